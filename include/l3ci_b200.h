@@ -91,6 +91,27 @@ L3CI_API int l3ci_add_rms_norm(const void* x, const void* residual, const void* 
 L3CI_API int l3ci_silu_mul(const void* gate, const void* up, void* out, int64_t rows, int64_t cols,
                            int64_t gate_row_stride, int64_t up_row_stride, l3ci_stream_t stream);
 
+/* Product of few rows (a decode step's tokens) with a weight matrix, and the activation that follows it:
+ *   out[r, n] = act( sum over k of x[r, k] * w[n, k] ),   x bf16 [rows, K], w bf16 [groups, N, K] dense, sums in fp32,
+ * rows <= L3CI_LINEAR_MAX_ROWS, K and x_st multiples of 8, x and w on 16 bytes; out bf16, or fp32 with out_f32.
+ * groups products at once: group g takes x + g * x_sg, w[g] and out + g * out_sg (strides: multiples of 8).
+ * L3CI_ACT_SILU_GATE: w is [groups, 2, N, K], gate rows then up rows, and out = silu(gate) * up (the two products of MLP.forward,
+ * model.py:134, with it).  early: w may be read before the stream's previous kernels have ended; for a w that was complete
+ * before the last kernel that waits for its predecessors ahead of letting this one start (weights of a model).  split: CTAs that share a tile's columns, 0 chooses (else 1, 2, 4 or 8).
+ * status (int32 on the device, may be null) receives L3CI_ERR_DEVICE_WAIT if a bounded wait ran out. */
+#define L3CI_LINEAR_MAX_ROWS 64
+typedef enum l3ci_act { L3CI_ACT_NONE = 0, L3CI_ACT_GELU = 1, L3CI_ACT_TANH = 2, L3CI_ACT_SILU_GATE = 3 } l3ci_act;
+typedef struct l3ci_linear_args {
+  const void* x;
+  const void* w;
+  void* out;
+  int32_t* status;
+  int64_t rows, x_st, out_st, x_sg, out_sg;
+  int32_t K, N, groups, act, out_f32, split, early;
+  l3ci_stream_t stream;
+} l3ci_linear_args;
+L3CI_API int l3ci_linear(const l3ci_linear_args* args);
+
 /* Greedy decode step: for every row b of bf16 logits [rows, vocab] (row_stride elements apart),
  *   tok = argmax (ties: smallest index, as torch.argmax; NaN counts as the maximum);
  *   out_tokens[b * out_stride + steps[b]] = tok (if steps[b] < out_cols);  steps[b] += 1;

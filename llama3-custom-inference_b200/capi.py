@@ -19,12 +19,22 @@ OK, ERR_INVALID, ERR_UNSUPPORTED, ERR_ALIGNMENT, ERR_SCRATCH, ERR_CUDA, ERR_DEVI
 # Every symbol include/l3ci_b200.h declares.
 EXPORTS = (
     "l3ci_status_string", "l3ci_last_error", "l3ci_version", "l3ci_set_device_wait_limit_ns", "l3ci_set_programmatic_launch",
-    "l3ci_rms_norm", "l3ci_add_rms_norm", "l3ci_silu_mul", "l3ci_greedy_step", "l3ci_top_p_step", "l3ci_rot_embed", "l3ci_rot_embed_kv_cache", "l3ci_rot_embed_kv_cache_at",
+    "l3ci_rms_norm", "l3ci_add_rms_norm", "l3ci_silu_mul", "l3ci_linear", "l3ci_greedy_step", "l3ci_top_p_step", "l3ci_rot_embed", "l3ci_rot_embed_kv_cache", "l3ci_rot_embed_kv_cache_at",
     "l3ci_flash_decode_scratch_bytes", "l3ci_flash_decode", "l3ci_flash_decode_static", "l3ci_flash_decode_poll",
     "l3ci_flash_decode_kernel_choice",
     "l3ci_lse_merge", "l3ci_lse_exchange_bytes", "l3ci_lse_exchange_merge", "l3ci_prefill_attention",
     "l3ci_flash_decode_exchange_bytes", "l3ci_flash_decode_exchange",
 )
+
+
+class LinearArgs(C.Structure):
+    """struct l3ci_linear_args"""
+    _fields_ = [(n, C.c_void_p) for n in ("x", "w", "out", "status")] + [(n, C.c_int64) for n in ("rows", "x_st", "out_st", "x_sg", "out_sg")] + [
+        (n, C.c_int32) for n in ("K", "N", "groups", "act", "out_f32", "split", "early")] + [("stream", C.c_void_p)]
+
+
+LINEAR_MAX_ROWS = 64
+ACT_NONE, ACT_GELU, ACT_TANH, ACT_SILU_GATE = range(4)
 
 
 class FlashDecodeArgs(C.Structure):
@@ -92,6 +102,8 @@ def load() -> C.CDLL:
     lib.l3ci_add_rms_norm.argtypes = [vp, vp, vp, vp, vp, i64, i64, f32, vp]
     lib.l3ci_silu_mul.restype = C.c_int
     lib.l3ci_silu_mul.argtypes = [vp, vp, vp, i64, i64, i64, i64, vp]
+    lib.l3ci_linear.restype = C.c_int
+    lib.l3ci_linear.argtypes = [C.POINTER(LinearArgs)]
     lib.l3ci_prefill_attention.restype = C.c_int
     lib.l3ci_prefill_attention.argtypes = [C.POINTER(PrefillArgs)]
     lib.l3ci_greedy_step.restype = C.c_int
@@ -173,6 +185,61 @@ def add_rms_norm(x, residual, weight, eps: float):
         _check(load().l3ci_add_rms_norm(x.data_ptr(), residual.data_ptr(), weight.data_ptr(), s.data_ptr(),
                                         out.data_ptr(), x.numel() // E, E, eps, _stream(x)), "l3ci_add_rms_norm")
     return s, out
+
+
+def _row_stride(x, width: int):
+    """Elements between the rows of x [..., width], its leading axes counted as one; None if no one stride fits."""
+    stride, reach = None, 0
+    for n, st in zip(reversed(x.shape[:-1]), reversed(x.stride()[:-1])):
+        if n == 1:
+            continue
+        if stride is None:
+            stride = st
+        elif st != reach:
+            return None
+        reach = st * n
+    return width if stride is None else stride
+
+
+def linear_args(x, w, act: int = ACT_NONE, out_dtype=None, split: int = 0, status=None, early: bool = False, out=None):
+    """Arguments of `l3ci_linear` and the tensor that it fills: x [..., K] and w [N, K] (gated: [2 N, K]), or groups of
+    products, x [groups, rows, K] and w [groups, N, K].  (None, None) where the call does not apply: more rows than it takes,
+    other types, layouts or alignments.  `out`: where the result goes, the last axis contiguous."""
+    import torch
+
+    if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and w.device == x.device and w.is_contiguous()):
+        return None, None
+    K, grouped = x.shape[-1], w.dim() == 3
+    if w.dim() not in (2, 3) or w.shape[-1] != K or K == 0 or K % 8 or x.stride(-1) != 1 or (grouped and (x.dim() != 3 or x.shape[0] != w.shape[0])):
+        return None, None
+    groups = w.shape[0] if grouped else 1
+    N, rows = w.shape[-2], x.numel() // (K * max(1, groups))
+    if act == ACT_SILU_GATE:
+        if N % 2:
+            return None, None
+        N //= 2
+    one = x[0] if grouped and groups else x
+    stride, group_stride = _row_stride(one, K), x.stride(0) if grouped else 0
+    if not 0 < rows <= LINEAR_MAX_ROWS or N == 0 or groups == 0 or stride is None:
+        return None, None
+    if stride % 8 or group_stride % 8 or (rows > 1 and stride < K and not grouped) or x.data_ptr() % 16 or w.data_ptr() % 16:
+        return None, None
+    if out is None:
+        out = torch.empty(*x.shape[:-1], N, dtype=out_dtype or x.dtype, device=x.device)
+    out_stride = _row_stride(out[0] if grouped else out, N)
+    a = LinearArgs(x=x.data_ptr(), w=w.data_ptr(), out=out.data_ptr(), status=None if status is None else status.data_ptr(), rows=rows, x_st=stride,
+                   out_st=out_stride, x_sg=group_stride, out_sg=out.stride(0) if grouped else 0, K=K, N=N, groups=groups, act=act,
+                   out_f32=int(out.dtype == torch.float32), split=split, early=int(early), stream=_stream(x))
+    return a, out
+
+
+def linear(x, w, act: int = ACT_NONE, out_dtype=None, split: int = 0, status=None, early: bool = False, out=None):
+    """act(x w^T) of few rows in one kernel (`l3ci_linear`); None where it does not apply."""
+    a, out = linear_args(x, w, act, out_dtype, split, status, early, out)
+    if a is not None:
+        with _on(x):
+            _check(load().l3ci_linear(C.byref(a)), "l3ci_linear")
+    return out
 
 
 def silu_mul(gate, up):

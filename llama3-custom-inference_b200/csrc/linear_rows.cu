@@ -1,0 +1,394 @@
+// out[rows, N] = act(x[rows, K] w[N, K]^T) of few rows (a decode step's tokens), bf16 operands, fp32 accumulation
+// (include/l3ci_b200.h, l3ci_linear).
+//
+// A product of up to 64 rows is bound by reading w once.  What kept the library's kernels from that rate inside a decode step was not
+// the stream itself but its edges: each product began to read its weights only when the kernel before it had ended, and drained
+// before the next one began.  Here
+//   * the weights take the 128-row side of the tcgen05 product and the tokens the narrow one (16, 32 or 64 columns): a CTA moves
+//     128 rows of w, 64 columns at a time, through a ring of bulk tensor copies, and the tensor cores keep up with a fraction of
+//     their rate, so nothing but the copies is timed;
+//   * w does not depend on the kernel before (`early`): the ring is filled before griddepcontrol.wait, and only the tokens are asked
+//     for after it.
+//     A CTA takes at most half of an SM's shared memory, so that it can start beside the CTAs of the kernel before;
+//   * few rows of w: a cluster of 2, 4 or 8 CTAs shares a tile's columns, and adds its parts through distributed shared memory in
+//     the order of the ranks (results do not depend on timing);
+//   * the activation that follows is done on the fp32 sums: gelu, tanh, or silu(gate) * up of a stacked matrix, a tile then being
+//     64 gate rows and the 64 up rows of the same outputs.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include "host_common.h"
+#include "ptx_sm100.cuh"
+#include "tcgen05.cuh"
+#include "tensor_map.h"
+
+namespace l3ci {
+namespace {
+
+constexpr int kTile = 128;                 // rows of w per tile
+constexpr int kDeep = 64;                  // columns per stage: 128 bytes
+constexpr int kThreads = 192;              // producer, MMA issue, four output warps
+constexpr int kWBytes = kTile * kDeep * 2;
+constexpr int kSwap = 8;                   // tokens whose up halves pass through shared memory at a time
+
+constexpr long long kAheadBytes = 80ll << 20;   // of 126 MB of L2
+
+template <int NP>
+struct LinShape {
+  static constexpr int kXBytes = NP * kDeep * 2;
+  static constexpr int kStageBytes = kWBytes + kXBytes;
+  static constexpr int kStages = NP == 16 ? 6 : NP == 32 ? 5 : 4;
+  static constexpr uint32_t kTmem = 2 * NP;          // two accumulators
+  static constexpr int kSwapBytes = kSwap * (kTile / 2) * 4;
+  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + kSwapBytes + (2 * kStages + 4) * 8 + 16;
+  static_assert(kStages * kStageBytes >= NP * kTile * 4, "the ring holds a tile's parts");
+  static_assert(2 * kSmem <= 232448, "two CTAs per SM");
+};
+
+struct LinParams {
+  l3ci_linear_args a;
+  int tiles, steps;                        // tiles of w, stages of K
+  int group_tiles;                         // tiles of one group
+  int ahead;                               // w fits L2 beside the rest: its tiles may be fetched there ahead of the ring
+};
+
+__device__ __forceinline__ float lin_act(float z, int act) {
+  if (act == L3CI_ACT_GELU) return 0.5f * z * (1.f + erff(z * 0.70710678118654752f));
+  if (act == L3CI_ACT_TANH) return tanhf(z);
+  return z;
+}
+__device__ __forceinline__ float lin_gate(float z, float u) { return z / (1.f + expf(-z)) * u; }
+
+__device__ __forceinline__ void store_out(const l3ci_linear_args& a, int grp, int t, int n, float v) {
+  const long long at = grp * a.out_sg + t * a.out_st + n;
+  if (a.out_f32) static_cast<float*>(a.out)[at] = v;
+  else static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(v);
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v) {
+  asm volatile("{\n\t.reg .u32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.f32 [r], %2;\n\t}\n" ::"r"(addr), "r"(rank), "f"(v)
+               : "memory");
+}
+__device__ __forceinline__ void output_warps_meet() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// Whether all four output warps are well: they meet at barriers together or not at all.
+__device__ __forceinline__ bool output_warps_agree(bool ok) {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n" : "=r"(r) : "r"((uint32_t)ok) : "memory");
+  return r != 0;
+}
+
+__device__ __forceinline__ void prefetch_l2(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
+
+// S: CTAs of a cluster, which share a tile's columns of w.  GATED: w holds N gate rows, then N up rows.
+template <int NP, int S, bool GATED>
+__global__ void __launch_bounds__(kThreads, 2)
+linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ LinParams p) {
+  using Sh = LinShape<NP>;
+  constexpr int kStages = Sh::kStages;
+  constexpr int kOuts = GATED ? kTile / 2 : kTile;     // outputs of a tile
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t ring = smem_u32(smem);
+  float* swap = reinterpret_cast<float*>(smem + kStages * Sh::kStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Sh::kStageBytes + Sh::kSwapBytes);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
+  const uint32_t full0 = smem_u32(bars), empty0 = full0 + kStages * 8, done0 = empty0 + kStages * 8, read0 = done0 + 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const l3ci_linear_args& a = p.a;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(full0 + i * 8, 1);
+      mbar_init(empty0 + i * 8, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(done0 + i * 8, 1);
+      mbar_init(read0 + i * 8, 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&xmap)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&wmap)) : "memory");
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), Sh::kTmem);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  // behind the allocation: a CTA of the next kernel must not hold the tensor memory that this one waits for
+  pdl_launch_dependents();
+  const uint32_t tmem = *tmem_slot;
+  const int rank = S > 1 ? (int)cluster_rank() : 0;
+  const int first = blockIdx.x / S, stride = gridDim.x / S;
+  const int k0 = (int)((long long)p.steps * rank / S), steps = (int)((long long)p.steps * (rank + 1) / S) - k0;   // this CTA's stages of a tile
+  bool ok = true;
+
+  if (warp == 0) {
+    // ---- producer ----
+    if (lane == 0) {
+      const uint64_t policy_w = l2_evict_first_policy();
+      uint64_t policy_x;
+      asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy_x));
+      const int tiles = first < p.tiles ? (p.tiles - first + stride - 1) / stride : 0;
+      const long long fills = (long long)tiles * steps;
+      auto load_w = [&](int s, int tile, int k) {
+        const uint32_t dst = ring + s * Sh::kStageBytes, bar = full0 + s * 8;
+        mbar_expect_tx(bar, Sh::kStageBytes);
+        const int grp = tile / p.group_tiles, row = tile % p.group_tiles * kOuts;
+        tma_load_4d(dst, &wmap, bar, (k0 + k) * kDeep, row, 0, grp, policy_w);
+        if (GATED) tma_load_4d(dst + kWBytes / 2, &wmap, bar, (k0 + k) * kDeep, row, 1, grp, policy_w);
+      };
+      auto load_x = [&](int s, int tile, int k) {
+        tma_load_4d(ring + s * Sh::kStageBytes + kWBytes, &xmap, full0 + s * 8, (k0 + k) * kDeep, 0, 0, tile / p.group_tiles, policy_x);
+      };
+      const int early = (int)(fills < kStages ? fills : kStages);
+      if (!a.early) pdl_wait();
+      for (int f = 0; f < early; ++f) load_w(f, first + f / steps * stride, f % steps);
+      if (a.early) {
+        // what of the first tile the ring does not hold goes as far as L2
+        for (int k = early; p.ahead && k < steps; ++k) {
+          const int grp = first / p.group_tiles, row = first % p.group_tiles * kOuts;
+          prefetch_l2(&wmap, (k0 + k) * kDeep, row, 0, grp);
+          if (GATED) prefetch_l2(&wmap, (k0 + k) * kDeep, row, 1, grp);
+        }
+        pdl_wait();
+      }
+      for (int f = 0; f < early; ++f) load_x(f, first + f / steps * stride, f % steps);
+      int tile = first + early / steps * stride, k = early % steps;
+      for (long long f = early; f < fills; ++f) {
+        const int s = (int)(f % kStages);
+        const uint32_t parity = (uint32_t)((f / kStages - 1) & 1);
+        if (!mbar_try_wait(empty0 + s * 8, parity)) {
+          const unsigned long long t0 = global_ns();
+          bool got = false;
+          for (uint32_t it = 0; !got; ++it) {
+            got = mbar_try_wait(empty0 + s * 8, parity);
+            if (!got && (it & 63u) == 63u && global_ns() - t0 > kWaitLimitNs) break;
+          }
+          if (!got) { ok = false; break; }
+        }
+        load_w(s, tile, k);
+        load_x(s, tile, k);
+        if (++k == steps) { k = 0; tile += stride; }
+      }
+    }
+    ok = __shfl_sync(kFullMask, ok, 0);
+  } else if (warp == 1) {
+    // ---- MMA issue: all lanes run the code, one elected lane predicates the instructions ----
+    pdl_wait();                          // (the bounds of the waits below count from here, not through the kernels before)
+    constexpr uint32_t idesc = instr_desc(kTile, NP, false);
+    const uint32_t elected = lane == 0 ? 1u : 0u;
+    int s = 0, round = 0;
+    uint32_t parity = 0;
+    for (int tile = first; tile < p.tiles && ok; tile += stride, ++round) {
+      const int acc = round & 1;
+      if (round >= 2 && !mbar_wait_bounded(read0 + acc * 8, ((round >> 1) - 1) & 1)) { ok = false; break; }
+      tc_fence_after();
+      for (int k = 0; k < steps; ++k) {
+        if (!mbar_wait_bounded(full0 + s * 8, parity)) { ok = false; break; }
+        tc_fence_after();
+        const uint64_t wd = smem_desc(ring + s * Sh::kStageBytes, 16, 1024);
+        const uint64_t xd = smem_desc(ring + s * Sh::kStageBytes + kWBytes, 16, 1024);
+#pragma unroll
+        for (int i = 0; i < kDeep / 16; ++i) mma_ss(tmem + acc * NP, wd + i * 2, xd + i * 2, idesc, (k > 0 || i > 0) ? 1u : 0u, elected);
+        tc_commit(empty0 + s * 8, elected);
+        if (++s == kStages) { s = 0; parity ^= 1; }
+      }
+      if (ok) tc_commit(done0 + acc * 8, elected);
+    }
+  } else {
+    // ---- output: a thread owns row r of the tile ----
+    pdl_wait();
+    const int q4 = warp & 3, r = q4 * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(q4 * 32) << 16;
+    const int rows = (int)a.rows;
+    int round = 0;
+    for (int tile = first; tile < p.tiles; tile += stride, ++round) {
+      const int acc = round & 1;
+      ok = mbar_wait_bounded(done0 + acc * 8, (round >> 1) & 1);
+      if (GATED && S == 1) ok = output_warps_agree(ok);
+      if (!ok) break;
+      tc_fence_after();
+      if constexpr (S == 1) {
+        const int grp = tile / p.group_tiles, n = tile % p.group_tiles * kOuts + (GATED ? r & 63 : r);
+#pragma unroll
+        for (int c = 0; c < NP; c += 16) {
+          if (c >= rows) break;
+          uint32_t v[16];
+          tmem_ld16(tmem + acc * NP + lane_addr + c, v);
+          tc_wait_ld();
+          if constexpr (GATED) {
+#pragma unroll
+            for (int h = 0; h < 16; h += kSwap) {
+              if (c + h >= rows) break;
+              if (r >= 64)
+#pragma unroll
+                for (int i = 0; i < kSwap; ++i) swap[i * 64 + r - 64] = __uint_as_float(v[h + i]);
+              output_warps_meet();
+              if (r < 64 && n < a.N)
+#pragma unroll
+                for (int i = 0; i < kSwap; ++i)
+                  if (c + h + i < rows) store_out(a, grp, c + h + i, n, lin_gate(__uint_as_float(v[h + i]), swap[i * 64 + r]));
+              output_warps_meet();
+            }
+          } else if (n < a.N) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (c + i < rows) store_out(a, grp, c + i, n, lin_act(__uint_as_float(v[i]), a.act));
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(read0 + acc * 8);
+      }
+    }
+  }
+  if constexpr (S > 1) {
+    // ---- one tile per cluster: every CTA has its part of the sums; CTA o adds up outputs o * kOuts / S onwards ----
+    constexpr int kSlice = kTile / S, kOwn = kOuts / S;   // rows of w and outputs of a CTA
+    __syncwarp();
+    cluster_meet();                                       // every ring of the cluster is done with: the parts go there
+    if (warp >= 2 && ok) {
+      const int q4 = warp & 3, r = q4 * 32 + lane, rows = (int)a.rows;
+      const int j = GATED ? r & 63 : r;
+      const uint32_t owner = (uint32_t)(j / kOwn);
+      // [token][rank][row of the slice]
+      const uint32_t at = ring + ((rank * kSlice + (GATED ? r / 64 * kOwn : 0) + j % kOwn) << 2);
+#pragma unroll
+      for (int c = 0; c < NP; c += 16) {
+        if (c >= rows) break;
+        uint32_t v[16];
+        tmem_ld16(tmem + ((uint32_t)(q4 * 32) << 16) + c, v);
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (c + i < rows) st_cluster(at + (uint32_t)(c + i) * kTile * 4, owner, __uint_as_float(v[i]));
+      }
+    }
+    __syncwarp();
+    cluster_meet();
+    const float* parts = reinterpret_cast<const float*>(smem);
+    for (int e = threadIdx.x; e < (int)a.rows * kOwn; e += kThreads) {
+      const int t = e / kOwn, j = e % kOwn, n = first % p.group_tiles * kOuts + rank * kOwn + j;
+      if (n >= a.N) continue;
+      float y = 0.f, u = 0.f;
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        y += parts[t * kTile + s * kSlice + j];
+        if (GATED) u += parts[t * kTile + s * kSlice + kOwn + j];
+      }
+      store_out(a, first / p.group_tiles, t, n, GATED ? lin_gate(y, u) : lin_act(y, a.act));
+    }
+  }
+  if (!ok && lane == 0 && a.status) atomicExch(a.status, (int)L3CI_ERR_DEVICE_WAIT);
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, Sh::kTmem);
+}
+
+template <int NP, int S, bool GATED>
+int launch(const l3ci_linear_args* a, cudaStream_t stream) {
+  using Sh = LinShape<NP>;
+  constexpr int kOuts = GATED ? kTile / 2 : kTile;
+  LinParams p = {};
+  p.a = *a;
+  p.group_tiles = (a->N + kOuts - 1) / kOuts;
+  p.tiles = p.group_tiles * a->groups;
+  p.steps = (a->K + kDeep - 1) / kDeep;
+  p.ahead = (long long)a->groups * a->N * a->K * (GATED ? 4 : 2) <= kAheadBytes;
+  const long long one = (long long)a->N * a->K;
+  CUtensorMap xmap, wmap;
+  if (int st = make_rows_map(&xmap, a->x, a->K, (int)a->rows, 1, a->groups, a->x_st, 0, a->x_sg, NP)) return st;
+  if (int st = make_rows_map(&wmap, a->w, a->K, a->N, GATED ? 2 : 1, a->groups, a->K, one, one * (GATED ? 2 : 1), kOuts)) return st;
+  auto kernel = linear_rows_kernel<NP, S, GATED>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  L3CI_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    L3CI_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::kSmem));
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
+  const int sms = sm_count() > 0 ? sm_count() : 148;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(S > 1 ? p.tiles * S : p.tiles < 2 * sms ? p.tiles : 2 * sms));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = Sh::kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (S > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = S;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (programmatic_launch_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xmap, wmap, p);
+  if (e != cudaSuccess) return fail(L3CI_ERR_CUDA, "launch of linear_rows_kernel failed: %s", cudaGetErrorString(e));
+  return L3CI_OK;
+}
+
+template <int NP, bool GATED>
+int launch_split(const l3ci_linear_args* a, cudaStream_t stream) {
+  const long long tiles = (a->N + (GATED ? kTile / 2 : kTile) - 1) / (GATED ? kTile / 2 : kTile) * (long long)a->groups;
+  int split = a->split;
+  if (split == 0) {
+    // the most CTAs that still run at once, each with two stages or more
+    const int sms = sm_count() > 0 ? sm_count() : 148, steps = (a->K + kDeep - 1) / kDeep;
+    split = 1;
+    while (split < 8 && tiles * split * 2 <= 2 * sms && steps >= 4 * split) split *= 2;
+  }
+  while (split > 1 && split > (a->K + kDeep - 1) / kDeep) split /= 2;   // every CTA has a stage
+  switch (split) {
+    case 1: return launch<NP, 1, GATED>(a, stream);
+    case 2: return launch<NP, 2, GATED>(a, stream);
+    case 4: return launch<NP, 4, GATED>(a, stream);
+    case 8: return launch<NP, 8, GATED>(a, stream);
+    default: return fail(L3CI_ERR_INVALID, "linear: split %d is not 1, 2, 4 or 8", split);
+  }
+}
+
+}  // namespace
+}  // namespace l3ci
+
+extern "C" int l3ci_linear(const l3ci_linear_args* a) {
+  using namespace l3ci;
+  clear_error();
+  if (!a) return fail(L3CI_ERR_INVALID, "linear: null arguments");
+  if (a->rows < 0 || a->K <= 0 || a->N < 0 || a->act < L3CI_ACT_NONE || a->act > L3CI_ACT_SILU_GATE || a->split < 0 || a->split > 8 || a->groups < 0)
+    return fail(L3CI_ERR_INVALID, "linear: rows=%lld K=%d N=%d groups=%d act=%d split=%d", (long long)a->rows, a->K, a->N, a->groups, a->act, a->split);
+  if (a->rows == 0 || a->N == 0 || a->groups == 0) return L3CI_OK;
+  if (a->rows > L3CI_LINEAR_MAX_ROWS) return fail(L3CI_ERR_UNSUPPORTED, "linear: %lld rows, at most %d", (long long)a->rows, L3CI_LINEAR_MAX_ROWS);
+  if (!a->x || !a->w || !a->out) return fail(L3CI_ERR_INVALID, "linear: null pointer");
+  if ((long long)a->groups * (a->N / (kTile / 2) + 1) > INT32_MAX / 16) return fail(L3CI_ERR_INVALID, "linear: %d groups of %d rows of w", a->groups, a->N);
+  if (a->K % 8 || a->x_st % 8 || a->x_sg % 8 || !aligned16(a->x) || !aligned16(a->w))
+    return fail(L3CI_ERR_ALIGNMENT, "linear: rows of x and w must be whole 16-byte vectors");
+  if (a->rows > 1 && a->out_st < a->N && (a->groups == 1 || a->out_sg < a->N)) return fail(L3CI_ERR_INVALID, "linear: rows of the result overlap");
+  if (a->x_st < 0 || a->x_sg < 0) return fail(L3CI_ERR_INVALID, "linear: negative stride");
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(a->stream);
+  const bool gated = a->act == L3CI_ACT_SILU_GATE;
+  if (a->rows <= 16) return gated ? launch_split<16, true>(a, s) : launch_split<16, false>(a, s);
+  if (a->rows <= 32) return gated ? launch_split<32, true>(a, s) : launch_split<32, false>(a, s);
+  return gated ? launch_split<64, true>(a, s) : launch_split<64, false>(a, s);
+}

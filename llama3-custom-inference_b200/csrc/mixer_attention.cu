@@ -34,8 +34,8 @@ __global__ void __launch_bounds__(kRowThreads) mixer_rows_kernel(const l3ci_mixe
   extern __shared__ float sh[];
   __shared__ float red[32];
   __shared__ float pk[MAPS][kRowThreads];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x, h = blockIdx.y, b = blockIdx.z, g = h / (a.H / a.G), tid = threadIdx.x;
   const int pos = a.positions[b] + t;
   // the keys in sight: the first `kept` ones, then those from `lo` on

@@ -130,8 +130,8 @@ mixer_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
     if (p.v_boxes) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&vmap)) : "memory");
   }
   __syncthreads();
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
 
   constexpr int kPairs = MAPS == 2 ? kMmRows / 2 : kMmRows;   // (token, head) pairs per unit
   const int unit = blockIdx.x / p.splits, split = blockIdx.x % p.splits;
@@ -479,8 +479,8 @@ __global__ void __launch_bounds__(kMergeMax) mixer_merge_kernel(const __grid_con
   __shared__ float red[32];
   __shared__ float wt[MAPS][kMaxSplits];
   __shared__ float4 sum[MAPS][kMergeMax];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const l3ci_mixer_attn_args& a = p.a;
   constexpr int kPairs = MAPS == 2 ? kMmRows / 2 : kMmRows;
   const int unit = blockIdx.x / kPairs, pair = blockIdx.x % kPairs;

@@ -35,8 +35,8 @@ moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ bia
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int e = tid; e < E; e += blockDim.x) count[e] = 0;
   __syncthreads();
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const long long row0 = (long long)blockIdx.x * tokens;
   const int n = (int)min((long long)tokens, rows - row0);
   float* z = row + warp * E;
@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(128)
 moe_gather_kernel(const S* __restrict__ h, const int* __restrict__ experts, const int* __restrict__ ranks, const int* __restrict__ counts,
                   S* __restrict__ out, int* __restrict__ part_rows, long long rows, int width, int E, int top) {
   extern __shared__ int at_s[];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const long long row = blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x / kWarp;
   for (int j = warp; j < top; j += warps) {
@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(256) moe_plain_kernel(const l3ci_moe_gemm_args
   constexpr int kMats = GATED ? 2 : 1;
   __shared__ float xs[kDeep][kTile + 4];
   __shared__ float ws[kMats][kDeep][kTile + 4];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   int expert, rows;
   long long row0;
   if (!expert_tile(a.counts, a.n_experts, kTile, blockIdx.x, expert, row0, rows)) return;

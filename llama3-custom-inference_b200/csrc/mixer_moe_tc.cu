@@ -75,8 +75,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const uint32_t tmem = *tmem_slot;
   const int steps = (a.K + kDeep - 1) / kDeep;
   // consecutive tiles share their rows' expert: the columns run fastest

@@ -199,8 +199,8 @@ recurrent_scan_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const bool fresh = a.positions[b] == 0;
   const int chunks = (T + kChunk - 1) / kChunk;
   const long long row0 = (long long)b * T;
@@ -535,8 +535,8 @@ __global__ void __launch_bounds__(kStepThreads, RP <= 4 ? 5 : RP <= 8 ? 3 : 2) r
   const int quads = V / 4, groups = kStepThreads / quads, quad = tid % quads, grp = tid / quads;
   const int h = blockIdx.x % a.H, b = blockIdx.x / a.H, R = a.H / a.G;
   const bool active = grp < groups;
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const bool fresh = a.positions[b] == 0;
   float4* state = reinterpret_cast<float4*>(a.state + b * a.state_sb + (long long)h * D * V) + quad;
   float4 s[RP];
@@ -635,8 +635,8 @@ template <typename S, int VEC, int LANES>
 __global__ void __launch_bounds__(256)
 head_norm_gate_vec_kernel(S* __restrict__ out, long long out_st, long long out_sh, const S* __restrict__ gate, long long gate_st,
                           long long gate_sh, const float* __restrict__ norm, long long norm_sh, int H, int V, long long units, int act, float eps) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const long long id = (long long)blockIdx.x * (256 / LANES) + threadIdx.x / LANES;
   const int c = (threadIdx.x % LANES) * VEC;
   const bool mine = id < units && c < V;
@@ -668,8 +668,8 @@ template <typename S, int VEC>
 __global__ void __launch_bounds__(256)
 head_norm_gate_kernel(S* __restrict__ out, long long out_st, long long out_sh, const S* __restrict__ gate, long long gate_st,
                       long long gate_sh, const float* __restrict__ norm, long long norm_sh, int H, int V, long long units, int act, float eps) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const long long id = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (id >= units) return;
@@ -737,8 +737,8 @@ __device__ __forceinline__ float decay_of(float y, float rate) {
 // TAPS > 0: the run's inputs are all asked for at once and every one is loaded once; 0: any number of taps.
 template <typename S, int VEC, int TAPS, int RUN>
 __global__ void __launch_bounds__(256, 3) delta_inputs_kernel(const l3ci_delta_inputs_args a, int runs, long long tasks) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long id = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (id >= tasks) return;

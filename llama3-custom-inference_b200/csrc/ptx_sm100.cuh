@@ -76,7 +76,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
 // Programmatic dependent launch.  pdl_wait: blocks until the kernel this one was launched behind has completed and
 // its memory operations are visible (at once when the kernel was launched the plain way); everything before it may
 // run while that kernel is still draining.  pdl_launch_dependents: lets the NEXT kernel of the stream be set up on the
-// SMs as they come free (it stops at its own pdl_wait until this grid has completed).
+// SMs as they come free (it stops at its own pdl_wait until this grid has completed).  Kernels call it first: the chain of
+// kernels behind then starts as far as the SMs have room, and what it may do ahead (l3ci_linear reads weights) overlaps them.
+// A kernel that allocates tensor memory calls it behind the allocation.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

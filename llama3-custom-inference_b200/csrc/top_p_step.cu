@@ -246,8 +246,8 @@ top_p_step_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lon
   __shared__ int s_owner;
   __shared__ long long s_token;
   __shared__ u64 s_slots[8];     // values for the peer CTA, one slot per exchange
-  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
   pdl_launch_dependents();  // the next one may be set up while this one runs
+  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
   const long long b = blockIdx.x / kCtas;
   const uint32_t rank = kCtas > 1 ? cluster_rank() : 0u;
   RowView rv;

@@ -337,6 +337,46 @@ Tensor silu_mul(Tensor gate, Tensor up) {
   return out;
 }
 
+// act(x w^T): few rows in one kernel (l3ci_linear; the weights are read ahead of the stream's previous kernels: w must not
+// be written by kernels of the same forward pass), more in torch's product and, gated, silu_mul.  `gated`: w holds gate
+// rows, then up rows, and the result is silu(gate) * up.
+Tensor linear(Tensor x, Tensor w, bool gated) {
+  check_bf16_cuda(x, "x");
+  check_bf16_cuda(w, "w");
+  TORCH_CHECK(x.dim() >= 1 && w.dim() == 2 && w.size(1) == x.size(-1), "w must be [N, K] with K the last axis of x");
+  TORCH_CHECK(w.get_device() == x.get_device(), "x and w on different devices");
+  TORCH_CHECK(!gated || w.size(0) % 2 == 0, "a gated product takes an even number of rows of w");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t K = x.size(-1), N = gated ? w.size(0) / 2 : w.size(0), rows = K ? x.numel() / K : 0;
+  // one row stride for all leading axes
+  int64_t stride = K, reach = 0;
+  bool regular = x.stride(-1) == 1;
+  for (int64_t d = x.dim() - 2; d >= 0; --d) {
+    if (x.size(d) == 1) continue;
+    if (reach == 0) stride = x.stride(d);
+    else regular = regular && x.stride(d) == reach;
+    reach = x.stride(d) * x.size(d);
+  }
+  auto at16 = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; };
+  if (regular && rows > 0 && rows <= L3CI_LINEAR_MAX_ROWS && N > 0 && K % 8 == 0 && stride % 8 == 0 && stride >= K && w.is_contiguous() &&
+      K <= INT32_MAX && w.size(0) <= INT32_MAX && at16(x) && at16(w)) {
+    auto sizes = x.sizes().vec();
+    sizes.back() = N;
+    Tensor out = torch::empty(sizes, x.options());
+    l3ci_linear_args a{};
+    a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
+    a.rows = rows; a.x_st = stride; a.out_st = N;
+    a.K = (int32_t)K; a.N = (int32_t)N; a.groups = 1;
+    a.act = gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE;
+    a.early = 1;
+    a.stream = current_stream();
+    check_status(l3ci_linear(&a), "linear");
+    return out;
+  }
+  Tensor y = at::linear(x, w);
+  return gated ? silu_mul(y.narrow(-1, 0, N), y.narrow(-1, N, N)) : y;
+}
+
 // Greedy decode step in place: argmax of logits [B, vocab] (bf16) per row, token written to out_tokens[b, steps[b]]
 // and next_input[b], steps / positions / seq_lens advanced by one.  model.py:370-381 as one kernel.
 void greedy_step(Tensor logits, Tensor out_tokens, Tensor steps, Tensor next_input, Tensor positions, Tensor seq_lens) {
@@ -489,6 +529,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_rms_norm", torch::wrap_pybind_function(add_rms_norm), "add_rms_norm", py::arg("x"), py::arg("residual"),
         py::arg("weight"), py::arg("eps"));
   m.def("silu_mul", torch::wrap_pybind_function(silu_mul), "silu_mul", py::arg("gate"), py::arg("up"));
+  m.def("linear", torch::wrap_pybind_function(linear), "linear", py::arg("x"), py::arg("w"), py::arg("gated") = false);
   m.def("greedy_step", torch::wrap_pybind_function(greedy_step), "greedy_step", py::arg("logits"), py::arg("out_tokens"),
         py::arg("steps"), py::arg("next_input"), py::arg("positions"), py::arg("seq_lens"));
   m.def("top_p_step", torch::wrap_pybind_function(top_p_step), "top_p_step", py::arg("logits"), py::arg("out_tokens"),

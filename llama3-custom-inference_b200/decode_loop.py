@@ -18,8 +18,10 @@ What differs from the reference's loop, all on the caller's side of the kernels:
   * which lets one decode step be captured in a CUDA graph and replayed: no per-step Python dispatch, no
     per-step mask construction (model.py:211) and no `all(eos_reached)` host sync (model.py:380).
   * the residual add runs inside the RMSNorm that follows it (`add_rms_norm`), `c_fc2` and `c_fc` are one GEMM
-    over the stacked weight, and `silu(gate) * up` is one kernel (`silu_mul`) instead of two elementwise passes.
-GEMMs and the embedding lookup are plain torch ops (cuBLAS); the token choice (greedy argmax, or nucleus sampling)
+    over the stacked weight, and `silu(gate) * up` is one kernel (`silu_mul`) instead of two elementwise passes, or
+    part of the product when the rows are few (`linear`).
+GEMMs of many rows and the embedding lookup are plain torch ops (cuBLAS), those of a decode step's rows a kernel of this
+package; the token choice (greedy argmax, or nucleus sampling)
 with its token bookkeeping is one kernel (`greedy_step` / `top_p_step`); prefill attention (torch SDPA in the reference, model.py:114-116) is `prefill_attention`.
 """
 from __future__ import annotations
@@ -115,13 +117,13 @@ class DecodeLoop:
         raise NotImplementedError
 
     @staticmethod
-    def logits(h: torch.Tensor, head: torch.Tensor, want=None):
-        """Output projection of the wanted places of h [B, T, width] (see `forward`)."""
+    def logits(h: torch.Tensor, head: torch.Tensor, want=None, linear=F.linear):
+        """Output projection (by `linear`) of the wanted places of h [B, T, width] (see `forward`)."""
         if want is None:
-            return F.linear(h[:, -1, :], head)
+            return linear(h[:, -1, :], head)
         if len(want) == 0:
             return None
-        return F.linear(h[:, torch.as_tensor(want, device=h.device)], head)
+        return linear(h[:, torch.as_tensor(want, device=h.device)], head)
 
     # ---- requests in portions -----------------------------------------------------------------------------
     @torch.inference_mode()
@@ -266,7 +268,6 @@ class Llama3Decoder(DecodeLoop):
         cfg, ext, w = self.cfg, self.ext, self.w
         B, T = tokens.shape
         E, D, Hq, Hkv = cfg.n_embd, cfg.head_dim, cfg.n_head, cfg.n_kv_head
-        F_ = cfg.hidden_dim
         slots = slice(0, B) if slots is None else slots
         x = F.embedding(tokens, w["wte"])                                            # model.py:208
         h = ext.rms_norm(x, w["h0.ln_1"], cfg.norm_eps)                                # model.py:147, 71
@@ -274,7 +275,7 @@ class Llama3Decoder(DecodeLoop):
             p = f"h{l}."
             cache_k, cache_v = self.cache_k[l][slots], self.cache_v[l][slots]
             _nvtx_push("layer")
-            qkv = F.linear(h, w[p + "attn"])                                           # model.py:95
+            qkv = ext.linear(h, w[p + "attn"])                                         # model.py:95
             _nvtx_push("rot_embd")
             _nvtx_push("use_kv")
             q = ext.rot_embed_kv_cache(qkv, self.freqs, cache_k, cache_v, 0, Hq, Hkv,
@@ -291,16 +292,15 @@ class Llama3Decoder(DecodeLoop):
                                                cache_v.transpose(1, 2), seq_lens=seq_lens,
                                                max_ctas=self._decode_kernel(B))     # model.py:118
             y = y.transpose(1, 2).reshape(B, T, E)                                     # model.py:120
-            x, h = ext.add_rms_norm(F.linear(y, w[p + "proj"]), x, w[p + "ln_2"], cfg.norm_eps)  # :121, 147-148
-            gu = F.linear(h, w[p + "gate_up"])                                         # c_fc2 | c_fc, model.py:134
-            m = F.linear(ext.silu_mul(gu[..., :F_], gu[..., F_:]), w[p + "mlp_proj"])
+            x, h = ext.add_rms_norm(ext.linear(y, w[p + "proj"]), x, w[p + "ln_2"], cfg.norm_eps)  # :121, 147-148
+            m = ext.linear(ext.linear(h, w[p + "gate_up"], gated=True), w[p + "mlp_proj"])   # c_fc2 | c_fc, model.py:134
             nxt = w[f"h{l + 1}.ln_1"] if l + 1 < cfg.n_layer else w["ln_f"]
             x, h = ext.add_rms_norm(m, x, nxt, cfg.norm_eps)                           # model.py:148, next 147 / 217
             _nvtx_pop()
         # the reference widens the logits to fp32 first (model.py:226); the widening is monotonic, so the argmax
         # of the bf16 values is the same index
         # model.py:225; the head is tied to the embedding (model.py:189) unless the checkpoint brought its own
-        return self.logits(h, w.get("lm_head", w["wte"]), want)
+        return self.logits(h, w.get("lm_head", w["wte"]), want, ext.linear)
 
 
 def config_from_hf(hf_config) -> DecoderConfig:

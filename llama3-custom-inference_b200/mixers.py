@@ -6,8 +6,9 @@ import ctypes as C
 from pathlib import Path
 
 import torch
+import torch.nn.functional as F
 
-from .capi import OK, L3ciError, _on, _stream
+from .capi import ACT_GELU, ACT_NONE, ACT_SILU_GATE, ACT_TANH, OK, L3ciError, LinearArgs, _on, _stream, linear_args
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libl3ci_mixers.so"
 
@@ -88,6 +89,7 @@ def load() -> C.CDLL:
     i64, i32, vp, f32 = C.c_int64, C.c_int32, C.c_void_p, C.c_float
     lib.l3ci_mixers_last_error.restype = C.c_char_p
     lib.l3ci_mixers_set_programmatic_launch.argtypes = [C.c_int]
+    lib.l3ci_linear.argtypes = [C.POINTER(LinearArgs)]
     lib.l3ci_add_dyn_tanh.argtypes = [vp, vp, vp, i64, vp, vp, vp, f32, vp, i64, i64, i32, vp]
     lib.l3ci_gelu.argtypes = [vp, vp, i64, i32, vp]
     lib.l3ci_latent_cache.argtypes = [vp, i64, vp, i64, vp, f32, vp, i64, i64, i64, vp] + [i32] * 7 + [vp]
@@ -120,6 +122,33 @@ def _cuda(*tensors):
     for t in tensors:
         if not t.is_cuda:
             raise ValueError("the mixer kernels take CUDA tensors: there is no CPU path")
+
+
+def few_rows(x, w, act: int = ACT_NONE, out_dtype=None, out=None):
+    """act(x w^T) of few rows in one kernel (`l3ci_linear`), groups of products where w is [groups, N, K]; None where it does
+    not apply.  w, the model's, is read ahead of the stream's previous kernels."""
+    a, out = linear_args(x, w, act, out_dtype, early=True, out=out)
+    if a is not None:
+        with _on(x):
+            _check(load().l3ci_linear(C.byref(a)), "l3ci_linear")
+    return out
+
+
+def linear(x, w, act: int = ACT_NONE):
+    """act(x w^T); ACT_SILU_GATE: w holds gate rows, then up rows."""
+    y = few_rows(x, w, act)
+    if y is not None:
+        return y
+    y = F.linear(x, w)
+    return y if act == ACT_NONE else gelu_(y) if act == ACT_GELU else tanh_(y) if act == ACT_TANH else gated_act(y)
+
+
+def product32(x, w):
+    """x [rows, K] w^T in fp32: products of two bf16 numbers are exact, the sum is not rounded to bf16."""
+    if x.dtype == torch.float32:
+        return torch.mm(x, w.t())
+    y = few_rows(x, w, out_dtype=torch.float32)
+    return torch.mm(x, w.t(), out_dtype=torch.float32) if y is None else y
 
 
 def embed_dyn_tanh(tokens, table, weight, bias, alpha: float):

@@ -189,6 +189,7 @@ class _LayerWeights:
             self.up = torch.cat([get("mix.uk"), get("mix.uv")])                       # latent -> keys | values of all heads
             split = m.heads * m.dim
             self.uk = self.up[:split].view(m.heads, m.dim, m.kv_rank)
+            self.uk_t = self.uk.transpose(1, 2).contiguous()                          # for the products of few rows
             self.uv = self.up[split:].view(m.heads, m.vdim, m.kv_rank)
         else:
             rows = [get("mix.q"), get("mix.k"), get("mix.v"), get("mix.g")]
@@ -234,7 +235,7 @@ class NibelornDecoder(DecodeLoop):
         B, T, _ = h.shape
         H, D, R, C, V = m.heads, m.dim, m.rot_dim, m.kv_rank, m.vdim
         cache = self.cache.layers[l]["latent"][slots]
-        qd = F.linear(h, w.proj)
+        qd = mixers.linear(h, w.proj)
         mixers.latent_cache(qd, self._tables[R, m.rot_base], w.latent_norm, self.cfg.eps, cache, positions, H, D, R, C)
         q = qd[..., :H * (D + R)].view(B, T, H, D + R)
         out = torch.empty(B, T, H, V, dtype=h.dtype, device=h.device)
@@ -245,12 +246,17 @@ class NibelornDecoder(DecodeLoop):
             mixers.attention(q[..., :D], kv[..., :H * D].view(B, S, H, D), kv[..., H * D:].view(B, S, H, V), out, positions,
                              qb=q[..., D:], kb=k_rot, scale=m.scale, start_pos=start_pos, variant=mixers.TC)
         else:
-            q_lat = torch.bmm(q[..., :D].reshape(B * T, H, D).transpose(0, 1), w.uk)               # [H, B * T, C]
+            q_rows = q[..., :D].reshape(B * T, H, D).transpose(0, 1)
+            q_lat = mixers.few_rows(q_rows, w.uk_t)                                                # [H, B * T, C]
+            if q_lat is None:
+                q_lat = torch.bmm(q_rows, w.uk)
             o_lat = torch.empty_like(q_lat)
             mixers.attention(q_lat.view(H, B, T, C).permute(1, 2, 0, 3), cache[:, :, None, :C], cache[:, :, None, :C],
                              o_lat.view(H, B, T, C).permute(1, 2, 0, 3), positions, qb=q[..., D:],
                              kb=cache[:, :, None, C:C + R], scale=m.scale, start_pos=start_pos)
-            torch.bmm(o_lat, w.uv.transpose(1, 2), out=out.view(B * T, H, V).transpose(0, 1))
+            heads_out = out.view(B * T, H, V).transpose(0, 1)
+            if mixers.few_rows(o_lat, w.uv, out=heads_out) is None:
+                torch.bmm(o_lat, w.uv.transpose(1, 2), out=heads_out)
         return out.view(B, T, H * V)
 
     def _expands(self, m: LatentAttention, T: int) -> bool:
@@ -263,7 +269,7 @@ class NibelornDecoder(DecodeLoop):
         H, G, D, V = m.heads, m.kv_heads, m.dim, m.vdim
         planes = self.cache.layers[l]
         k, v = planes["k"][slots], planes["v"][slots]
-        p = F.linear(h, w.proj)
+        p = mixers.linear(h, w.proj)
         at_k, at_v, at_g = 2 * H * D, 2 * (H + G) * D, 2 * (H + G) * D + G * V
         mixers.kv_cache_write(p, at_k, at_v, k, v, positions)
         out = torch.empty(B, T, H, V, dtype=h.dtype, device=h.device)
@@ -287,11 +293,11 @@ class NibelornDecoder(DecodeLoop):
                 following = self.w[l + 1].norm1 if l + 1 < len(layers) else self.final_norm
                 with nvtx_range("layer"):
                     mix = self._latent if isinstance(layer.mixer, LatentAttention) else self._differential
-                    y = F.linear(mix(l, h, positions, slots, start_pos), w.o)
+                    y = mixers.linear(mix(l, h, positions, slots, start_pos), w.o)
                     if layer.ff is not None:
                         h = mixers.add_dyn_tanh(y, x, *w.norm2.args)
-                        y = F.linear(mixers.gelu_(F.linear(h, w.ff_up)), w.ff_down)
+                        y = mixers.linear(mixers.linear(h, w.ff_up, mixers.ACT_GELU), w.ff_down)
                     h = mixers.add_dyn_tanh(y, x, *following.args)
                     if keep is not None:
                         keep.append(x.clone())
-            return self.logits(h, self.head, want)
+            return self.logits(h, self.head, want, mixers.linear)

@@ -19,7 +19,6 @@ from dataclasses import dataclass
 from typing import Optional
 
 import torch
-import torch.nn.functional as F
 
 from . import mixers
 from .decode_loop import DecodeLoop, full_precision_products, nvtx_range
@@ -277,7 +276,7 @@ class _LayerWeights:
             self.a_log, self.dt_bias, self.norm = f32("mix.A_log"), f32("mix.dt_bias"), f32("mix.norm")
         else:
             self.mu = torch.stack([f32("mix.mu." + s) for s in MIXES])
-            self.rkvg = torch.stack([get("mix." + s) for s in "rkvg"]).transpose(1, 2)   # [4, width, heads * dim]
+            self.rkvg = torch.stack([get("mix." + s) for s in "rkvg"])   # [4, heads * dim, width]
             self.w1, self.w2, self.w0 = get("mix.w1"), get("mix.w2"), f32("mix.w0")
             self.u, self.norm = f32("mix.u"), f32("mix.norm").view(m.heads, m.dim)
         self.o = get("mix.o")
@@ -320,7 +319,7 @@ class RupotarDecoder(DecodeLoop):
     def _attention(self, m: Attention, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, _ = h.shape
         qw, kw = m.heads * m.dim, m.kv_heads * m.dim
-        qkv = F.linear(h, w.proj)
+        qkv = mixers.linear(h, w.proj)
         k, v = planes["k"], planes["v"]
         mixers.qk_norm_cache(qkv, qw, kw, w.q_norm, w.k_norm, self.cfg.eps, k, v, positions)
         out = torch.empty(B, T, m.heads, m.vdim, dtype=h.dtype, device=h.device)
@@ -331,9 +330,9 @@ class RupotarDecoder(DecodeLoop):
     def _channel_delta(self, m: ChannelDelta, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, E = h.shape
         H, G, D, V = m.heads, m.kv_heads, m.dim, m.vdim
-        p = F.linear(h, w.proj)
+        p = mixers.linear(h, w.proj)
         low = p.view(B * T, -1)[:, w.at_low:]
-        up = torch.mm(low, w.up.t()).view(B, T, -1)
+        up = mixers.linear(low, w.up).view(B, T, -1)
         qk, v, beta, decay = mixers.delta_inputs(p, p[..., w.at_b:w.at_b + H], up[..., :H * D], w.conv, w.a_log, w.dt_bias, planes["tail"],
                                                  positions, H, G, D, V, UNIT_EPS)
         gate = up[..., w.at_gate:w.at_gate + H * V].view(B, T, H, V)
@@ -343,24 +342,23 @@ class RupotarDecoder(DecodeLoop):
     def _wkv(self, m: TimeMix, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, E = h.shape
         mixes = mixers.token_shift(h, w.mu, planes["last"], positions).view(len(MIXES), B * T, E)
-        r, k, v, g = torch.bmm(mixes[:4], w.rkvg).view(4, B, T, m.heads, m.dim)
-        decay = F.linear(mixers.tanh_(F.linear(mixes[4], w.w1)), w.w2).view(B, T, m.heads, m.dim)
+        rkvg = mixers.few_rows(mixes[:4], w.rkvg)
+        if rkvg is None:
+            rkvg = torch.bmm(mixes[:4], w.rkvg.transpose(1, 2))
+        r, k, v, g = rkvg.view(4, B, T, m.heads, m.dim)
+        decay = mixers.linear(mixers.linear(mixes[4], w.w1, mixers.ACT_TANH), w.w2).view(B, T, m.heads, m.dim)
         return mixers.recurrent_scan(r, k, v, decay, planes["state"], positions, w.norm, g, act=mixers.SILU, eps=self.cfg.eps, bonus=w.u,
                                      g_bias=w.w0)
 
     # ---- feed-forward: what `residual_norm` adds ---------------------------------------------------------------
     def _feed_forward(self, ff, w: _LayerWeights, h):
         if isinstance(ff, Dense):
-            return {"y": F.linear(mixers.gated_act(F.linear(h, w.gate_up)), w.down)}
+            return {"y": mixers.linear(mixers.linear(h, w.gate_up, mixers.ACT_SILU_GATE), w.down)}
         rows = h.view(-1, h.shape[-1])
-        experts, ranks, weights, counts = mixers.moe_route(self._product32(rows, w.router), w.router_b, ff.top)
+        experts, ranks, weights, counts = mixers.moe_route(mixers.product32(rows, w.router), w.router_b, ff.top)
         x, part_rows = mixers.moe_gather(rows, experts, ranks, counts)
         a = mixers.moe_gemm(x, w.gate_up, counts, limit=ff.limit, alpha=EXPERT_ALPHA)
         return {"y": mixers.moe_gemm(a, w.down, counts), "part_rows": part_rows, "part_weights": weights}
-
-    def _product32(self, x, w):
-        """x w^T in fp32: products of two bf16 numbers are exact, the sum is not rounded to bf16."""
-        return torch.mm(x, w.t()) if x.dtype == torch.float32 else torch.mm(x, w.t(), out_dtype=torch.float32)
 
     # ---- one forward pass over T new tokens per sequence ------------------------------------------------------
     def forward(self, tokens: torch.Tensor, positions: torch.Tensor, seq_lens: torch.Tensor, start_pos: int = 0,
@@ -391,13 +389,13 @@ class RupotarDecoder(DecodeLoop):
                 mix = self._attention if isinstance(m, Attention) else self._channel_delta if isinstance(m, ChannelDelta) else self._wkv
                 with nvtx_range("layer"):
                     if run.step is not None:
-                        h = mixers.residual_norm(self._product32(cat.view(B * T, 2 * E), self.loop_in), x, dtype=self.dtype, reset=True, step=self.loop_step[run.step],
+                        h = mixers.residual_norm(mixers.product32(cat.view(B * T, 2 * E), self.loop_in), x, dtype=self.dtype, reset=True, step=self.loop_step[run.step],
                                                  pre=w.norm1, eps=eps)
-                    added, post = {"y": F.linear(mix(m, w, planes, h, positions, start_pos), w.o)}, w.norm1b
+                    added, post = {"y": mixers.linear(mix(m, w, planes, h, positions, start_pos), w.o)}, w.norm1b
                     if ff is not None:
                         h = mixers.residual_norm(**added, x=x, dtype=self.dtype, post=post, pre=w.norm2, eps=eps)
                         added, post = self._feed_forward(ff, w, h), w.norm2b
                     h = mixers.residual_norm(**added, x=x, dtype=self.dtype, post=post, eps=eps, **before(r + 1))
                     if keep is not None:
                         keep.append(x.clone())
-            return self.logits(h, self.head, want)
+            return self.logits(h, self.head, want, mixers.linear)

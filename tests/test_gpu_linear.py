@@ -1,0 +1,89 @@
+"""`l3ci_linear`: products of few rows with a weight matrix, against fp64 sums of the same bf16 inputs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _want(x, w, act, capi):
+    y = x.double() @ w.double().T
+    if act == capi.ACT_GELU:
+        return 0.5 * y * (1.0 + torch.erf(y * 0.5 ** 0.5))
+    if act == capi.ACT_TANH:
+        return torch.tanh(y)
+    if act == capi.ACT_SILU_GATE:
+        n = w.shape[0] // 2
+        return y[..., :n] * torch.sigmoid(y[..., :n]) * y[..., n:]
+    return y
+
+
+def _check(got, want, K, f32):
+    """fp32 sums of K products of size about 1 / sqrt(K): the error of a sum is below sqrt(K) roundings of a partial sum of
+    size about 1, and the activations' slopes are below 2; a bf16 result adds half of a unit in the last place, 2^-9."""
+    err = (got.double() - want).abs()
+    bound = 2.0 * K ** 0.5 * 2.0 ** -23 * (1.0 + want.abs()) + (0.0 if f32 else 2.0 ** -8) * want.abs() + 1e-6
+    assert bool((err <= bound).all()), f"largest excess {(err - bound).max().item():.3g}"
+
+
+# rows: the edges of the 16-, 32- and 64-column forms; K: one 8-column vector, ends inside a stage, more stages than the ring
+# has; N: inside a tile, whole tiles and one row behind them, more tiles than CTAs
+@pytest.mark.parametrize("split", [0, 1, 2, 4, 8])
+@pytest.mark.parametrize("rows,K,N", [(1, 8, 1), (1, 2048, 4), (2, 72, 128), (16, 1000, 129), (17, 2048, 300), (32, 4096, 64), (33, 520, 1025),
+                                      (64, 2048, 2048), (7, 136, 40000)])
+@pytest.mark.parametrize("act", [0, 1, 2, 3])
+def test_products_of_few_rows(capi, device, rows, K, N, act, split):
+    g = torch.Generator(device=device).manual_seed(rows * 7919 + K + N)
+    x = torch.randn(rows, K, generator=g, device=device).bfloat16()
+    w = (torch.randn((2 if act == capi.ACT_SILU_GATE else 1) * N, K, generator=g, device=device) * K ** -0.5).bfloat16()
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    for out_dtype in (torch.bfloat16, torch.float32):
+        got = capi.linear(x, w, act, out_dtype=out_dtype, split=split, status=status)
+        assert got.dtype == out_dtype and got.shape == (rows, N)
+        _check(got, _want(x, w, act, capi), K, out_dtype == torch.float32)
+    assert status.item() == 0
+
+
+def test_rows_with_a_stride_and_what_does_not_apply(capi, device):
+    g = torch.Generator(device=device).manual_seed(5)
+    w = (torch.randn(96, 64, generator=g, device=device) / 8).bfloat16()
+    big = torch.randn(5, 3, 160, generator=g, device=device).bfloat16()
+    for x in (big[:, -1, 8:72], big[:, :, 16:80], big[:1, :, :64], big[:, :1, 96:]):
+        _check(capi.linear(x, w), _want(x, w, 0, capi), 64, False)
+    for x in (big[:, :2, :64], big[:, :, 4:68], big.float()[..., :64], big[..., :60], big.transpose(0, 1)[..., :64], big[:0, :, :64],
+              torch.zeros(65, 64, dtype=torch.bfloat16, device=device)):
+        weight = w if x.shape[-1] == 64 else w[:, :60]
+        assert capi.linear(x, weight) is None
+    assert capi.linear(big[..., :64], w[:, ::2]) is None and capi.linear(big[..., :64], w.float()) is None
+
+
+def test_chain_of_products_under_programmatic_launch(capi, device):
+    """Each product reads what the one before wrote, while its own weights were asked for early."""
+    g = torch.Generator(device=device).manual_seed(11)
+    sizes = [(2048, 2048), (3072, 2048), (2048, 3072), (512, 2048), (2048, 512)] * 4
+    ws = [(torch.randn(n, k, generator=g, device=device) * k ** -0.5).bfloat16() for n, k in sizes]
+    x0 = torch.randn(8, 2048, generator=g, device=device).bfloat16()
+
+    def chain():
+        x = x0
+        for w in ws:
+            x = capi.linear(x, w)
+        return x
+
+    with capi.programmatic_launch(False):
+        want = chain()
+    torch.cuda.synchronize()
+    with capi.programmatic_launch(True):
+        for _ in range(5):
+            assert torch.equal(chain(), want)
+
+
+@pytest.mark.parametrize("rows,groups,K,N", [(1, 4, 256, 256), (8, 16, 128, 512), (33, 3, 72, 130), (64, 16, 512, 128)])
+def test_groups_of_products(capi, device, rows, groups, K, N):
+    g = torch.Generator(device=device).manual_seed(rows + groups)
+    w = (torch.randn(groups, N, K, generator=g, device=device) * K ** -0.5).bfloat16()
+    x = torch.randn(rows, groups, K + 8, generator=g, device=device).bfloat16()[..., :K].transpose(0, 1)
+    want = torch.einsum("grk,gnk->grn", x.double(), w.double())
+    _check(capi.linear(x, w), want, K, False)
+    out = torch.empty(rows, groups, N, dtype=torch.bfloat16, device=device).transpose(0, 1)
+    assert capi.linear(x.contiguous(), w, out=out) is out
+    _check(out, want, K, False)
