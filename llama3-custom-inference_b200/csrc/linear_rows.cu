@@ -32,25 +32,28 @@ constexpr int kThreads = 192;              // producer, MMA issue, four output w
 constexpr int kWBytes = kTile * kDeep * 2;
 constexpr int kSwap = 8;                   // tokens whose up halves pass through shared memory at a time
 
-constexpr long long kAheadBytes = 80ll << 20;   // of 126 MB of L2
-
+// NP: tokens of the narrow side.  The product's least width is 16: of a tile of 8 tokens it reads 8 rows of what lies behind, into
+// columns of the accumulator that nobody reads.
 template <int NP>
 struct LinShape {
   static constexpr int kXBytes = NP * kDeep * 2;
   static constexpr int kStageBytes = kWBytes + kXBytes;
-  static constexpr int kStages = NP == 16 ? 6 : NP == 32 ? 5 : 4;
-  static constexpr uint32_t kTmem = 2 * NP;          // two accumulators
-  static constexpr int kSwapBytes = kSwap * (kTile / 2) * 4;
-  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + kSwapBytes + (2 * kStages + 4) * 8 + 16;
-  static_assert(kStages * kStageBytes >= NP * kTile * 4, "the ring holds a tile's parts");
-  static_assert(2 * kSmem <= 232448, "two CTAs per SM");
+  static constexpr int kStages = NP <= 16 ? 6 : NP == 32 ? 5 : 4;
+  static constexpr int kCols = NP < 16 ? 16 : NP;    // of the accumulator
+  static constexpr uint32_t kTmem = 2 * kCols;       // two accumulators
+  static constexpr int kPartBytes = NP * kTile * 4;  // a tile's parts from the cluster's CTAs
+  // the parts lie in the ring, behind one more meeting of the cluster, where a place of their own would cost a stage
+  static constexpr bool kInRing = NP > 8;
+  static constexpr int kExtraBytes = kInRing ? kSwap * (kTile / 2) * 4 : kPartBytes;
+  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + kExtraBytes + (2 * kStages + 4) * 8 + 16;
+  static_assert(kStages * kStageBytes >= kPartBytes && kExtraBytes >= kSwap * (kTile / 2) * 4, "room for parts and up halves");
+  static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs per SM");
 };
 
 struct LinParams {
   l3ci_linear_args a;
   int tiles, steps;                        // tiles of w, stages of K
   int group_tiles;                         // tiles of one group
-  int ahead;                               // w fits L2 beside the rest: its tiles may be fetched there ahead of the ring
 };
 
 __device__ __forceinline__ float lin_act(float z, int act) {
@@ -71,9 +74,8 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_meet() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v) {
   asm volatile("{\n\t.reg .u32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.f32 [r], %2;\n\t}\n" ::"r"(addr), "r"(rank), "f"(v)
                : "memory");
@@ -86,11 +88,6 @@ __device__ __forceinline__ bool output_warps_agree(bool ok) {
   return r != 0;
 }
 
-__device__ __forceinline__ void prefetch_l2(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-               : "memory");
-}
-
 // S: CTAs of a cluster, which share a tile's columns of w.  GATED: w holds N gate rows, then N up rows.
 template <int NP, int S, bool GATED>
 __global__ void __launch_bounds__(kThreads, 2)
@@ -101,8 +98,9 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t ring = smem_u32(smem);
-  float* swap = reinterpret_cast<float*>(smem + kStages * Sh::kStageBytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Sh::kStageBytes + Sh::kSwapBytes);
+  float* swap = reinterpret_cast<float*>(smem + kStages * Sh::kStageBytes);     // S == 1: the up halves
+  float* parts = Sh::kInRing ? reinterpret_cast<float*>(smem) : swap;           // S > 1: the cluster's parts
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Sh::kStageBytes + Sh::kExtraBytes);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + kStages * 8, done0 = empty0 + kStages * 8, read0 = done0 + 16;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -131,6 +129,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
   tc_fence_after();
   // behind the allocation: a CTA of the next kernel must not hold the tensor memory that this one waits for
   pdl_launch_dependents();
+  if constexpr (S > 1 && !Sh::kInRing) cluster_arrive();
   const uint32_t tmem = *tmem_slot;
   const int rank = S > 1 ? (int)cluster_rank() : 0;
   const int first = blockIdx.x / S, stride = gridDim.x / S;
@@ -143,54 +142,40 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
       const uint64_t policy_w = l2_evict_first_policy();
       uint64_t policy_x;
       asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy_x));
-      const int tiles = first < p.tiles ? (p.tiles - first + stride - 1) / stride : 0;
-      const long long fills = (long long)tiles * steps;
-      auto load_w = [&](int s, int tile, int k) {
+      // (one thread's instructions are all that a stage waits for: counters, no divisions, on the way to a copy)
+      struct At { int tile, grp, row, k; };
+      auto at_tile = [&](int tile) { return At{tile, tile / p.group_tiles, tile % p.group_tiles * kOuts, 0}; };
+      auto advance = [&](At& t) {
+        if (++t.k == steps) t = at_tile(t.tile + stride);
+      };
+      auto load_w = [&](int s, const At& t) {
         const uint32_t dst = ring + s * Sh::kStageBytes, bar = full0 + s * 8;
         mbar_expect_tx(bar, Sh::kStageBytes);
-        const int grp = tile / p.group_tiles, row = tile % p.group_tiles * kOuts;
-        tma_load_4d(dst, &wmap, bar, (k0 + k) * kDeep, row, 0, grp, policy_w);
-        if (GATED) tma_load_4d(dst + kWBytes / 2, &wmap, bar, (k0 + k) * kDeep, row, 1, grp, policy_w);
+        tma_load_4d(dst, &wmap, bar, (k0 + t.k) * kDeep, t.row, 0, t.grp, policy_w);
+        if (GATED) tma_load_4d(dst + kWBytes / 2, &wmap, bar, (k0 + t.k) * kDeep, t.row, 1, t.grp, policy_w);
       };
-      auto load_x = [&](int s, int tile, int k) {
-        tma_load_4d(ring + s * Sh::kStageBytes + kWBytes, &xmap, full0 + s * 8, (k0 + k) * kDeep, 0, 0, tile / p.group_tiles, policy_x);
+      auto load_x = [&](int s, const At& t) {
+        tma_load_4d(ring + s * Sh::kStageBytes + kWBytes, &xmap, full0 + s * 8, (k0 + t.k) * kDeep, 0, 0, t.grp, policy_x);
       };
-      const int early = (int)(fills < kStages ? fills : kStages);
       if (!a.early) pdl_wait();
-      for (int f = 0; f < early; ++f) load_w(f, first + f / steps * stride, f % steps);
-      if (a.early) {
-        // what of the first tile the ring does not hold goes as far as L2
-        for (int k = early; p.ahead && k < steps; ++k) {
-          const int grp = first / p.group_tiles, row = first % p.group_tiles * kOuts;
-          prefetch_l2(&wmap, (k0 + k) * kDeep, row, 0, grp);
-          if (GATED) prefetch_l2(&wmap, (k0 + k) * kDeep, row, 1, grp);
-        }
-        pdl_wait();
-      }
-      for (int f = 0; f < early; ++f) load_x(f, first + f / steps * stride, f % steps);
-      int tile = first + early / steps * stride, k = early % steps;
-      for (long long f = early; f < fills; ++f) {
-        const int s = (int)(f % kStages);
-        const uint32_t parity = (uint32_t)((f / kStages - 1) & 1);
-        if (!mbar_try_wait(empty0 + s * 8, parity)) {
-          const unsigned long long t0 = global_ns();
-          bool got = false;
-          for (uint32_t it = 0; !got; ++it) {
-            got = mbar_try_wait(empty0 + s * 8, parity);
-            if (!got && (it & 63u) == 63u && global_ns() - t0 > kWaitLimitNs) break;
-          }
-          if (!got) { ok = false; break; }
-        }
-        load_w(s, tile, k);
-        load_x(s, tile, k);
-        if (++k == steps) { k = 0; tile += stride; }
+      At w = at_tile(first), x = w;
+      int filled = 0;
+      for (; filled < kStages && w.tile < p.tiles; ++filled, advance(w)) load_w(filled, w);
+      if (a.early) pdl_wait();
+      for (int f = 0; f < filled; ++f, advance(x)) load_x(f, x);
+      uint32_t parity = 0;
+      for (int s = 0; w.tile < p.tiles; advance(w)) {
+        if (!mbar_wait_bounded_one(empty0 + s * 8, parity)) { ok = false; break; }
+        load_w(s, w);
+        load_x(s, w);
+        if (++s == kStages) { s = 0; parity ^= 1; }
       }
     }
     ok = __shfl_sync(kFullMask, ok, 0);
   } else if (warp == 1) {
     // ---- MMA issue: all lanes run the code, one elected lane predicates the instructions ----
     pdl_wait();                          // (the bounds of the waits below count from here, not through the kernels before)
-    constexpr uint32_t idesc = instr_desc(kTile, NP, false);
+    constexpr uint32_t idesc = instr_desc(kTile, Sh::kCols, false);
     const uint32_t elected = lane == 0 ? 1u : 0u;
     int s = 0, round = 0;
     uint32_t parity = 0;
@@ -204,7 +189,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
         const uint64_t wd = smem_desc(ring + s * Sh::kStageBytes, 16, 1024);
         const uint64_t xd = smem_desc(ring + s * Sh::kStageBytes + kWBytes, 16, 1024);
 #pragma unroll
-        for (int i = 0; i < kDeep / 16; ++i) mma_ss(tmem + acc * NP, wd + i * 2, xd + i * 2, idesc, (k > 0 || i > 0) ? 1u : 0u, elected);
+        for (int i = 0; i < kDeep / 16; ++i) mma_ss(tmem + acc * Sh::kCols, wd + i * 2, xd + i * 2, idesc, (k > 0 || i > 0) ? 1u : 0u, elected);
         tc_commit(empty0 + s * 8, elected);
         if (++s == kStages) { s = 0; parity ^= 1; }
       }
@@ -229,12 +214,12 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
         for (int c = 0; c < NP; c += 16) {
           if (c >= rows) break;
           uint32_t v[16];
-          tmem_ld16(tmem + acc * NP + lane_addr + c, v);
+          tmem_ld16(tmem + acc * Sh::kCols + lane_addr + c, v);
           tc_wait_ld();
           if constexpr (GATED) {
 #pragma unroll
             for (int h = 0; h < 16; h += kSwap) {
-              if (c + h >= rows) break;
+              if (c + h >= NP || c + h >= rows) break;
               if (r >= 64)
 #pragma unroll
                 for (int i = 0; i < kSwap; ++i) swap[i * 64 + r - 64] = __uint_as_float(v[h + i]);
@@ -261,13 +246,14 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
     // ---- one tile per cluster: every CTA has its part of the sums; CTA o adds up outputs o * kOuts / S onwards ----
     constexpr int kSlice = kTile / S, kOwn = kOuts / S;   // rows of w and outputs of a CTA
     __syncwarp();
-    cluster_meet();                                       // every ring of the cluster is done with: the parts go there
+    if constexpr (Sh::kInRing) cluster_arrive();
+    cluster_wait();                                       // the others' shared memory may be written: they have started, or are done with the ring
     if (warp >= 2 && ok) {
       const int q4 = warp & 3, r = q4 * 32 + lane, rows = (int)a.rows;
       const int j = GATED ? r & 63 : r;
       const uint32_t owner = (uint32_t)(j / kOwn);
       // [token][rank][row of the slice]
-      const uint32_t at = ring + ((rank * kSlice + (GATED ? r / 64 * kOwn : 0) + j % kOwn) << 2);
+      const uint32_t at = smem_u32(parts) + ((rank * kSlice + (GATED ? r / 64 * kOwn : 0) + j % kOwn) << 2);
 #pragma unroll
       for (int c = 0; c < NP; c += 16) {
         if (c >= rows) break;
@@ -276,12 +262,12 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
         tc_wait_ld();
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          if (c + i < rows) st_cluster(at + (uint32_t)(c + i) * kTile * 4, owner, __uint_as_float(v[i]));
+          if (c + i < NP && c + i < rows) st_cluster(at + (uint32_t)(c + i) * kTile * 4, owner, __uint_as_float(v[i]));
       }
     }
     __syncwarp();
-    cluster_meet();
-    const float* parts = reinterpret_cast<const float*>(smem);
+    cluster_arrive();
+    cluster_wait();
     for (int e = threadIdx.x; e < (int)a.rows * kOwn; e += kThreads) {
       const int t = e / kOwn, j = e % kOwn, n = first % p.group_tiles * kOuts + rank * kOwn + j;
       if (n >= a.N) continue;
@@ -310,7 +296,6 @@ int launch(const l3ci_linear_args* a, cudaStream_t stream) {
   p.group_tiles = (a->N + kOuts - 1) / kOuts;
   p.tiles = p.group_tiles * a->groups;
   p.steps = (a->K + kDeep - 1) / kDeep;
-  p.ahead = (long long)a->groups * a->N * a->K * (GATED ? 4 : 2) <= kAheadBytes;
   const long long one = (long long)a->N * a->K;
   CUtensorMap xmap, wmap;
   if (int st = make_rows_map(&xmap, a->x, a->K, (int)a->rows, 1, a->groups, a->x_st, 0, a->x_sg, NP)) return st;
@@ -388,6 +373,7 @@ extern "C" int l3ci_linear(const l3ci_linear_args* a) {
   if (a->x_st < 0 || a->x_sg < 0) return fail(L3CI_ERR_INVALID, "linear: negative stride");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(a->stream);
   const bool gated = a->act == L3CI_ACT_SILU_GATE;
+  if (a->rows <= 8) return gated ? launch_split<8, true>(a, s) : launch_split<8, false>(a, s);
   if (a->rows <= 16) return gated ? launch_split<16, true>(a, s) : launch_split<16, false>(a, s);
   if (a->rows <= 32) return gated ? launch_split<32, true>(a, s) : launch_split<32, false>(a, s);
   return gated ? launch_split<64, true>(a, s) : launch_split<64, false>(a, s);

@@ -73,6 +73,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
   }
   return true;
 }
+// The same by one thread.
+__device__ __forceinline__ bool mbar_wait_bounded_one(uint32_t bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = global_ns();
+  for (uint32_t it = 0;; ++it) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((it & 63u) == 63u && global_ns() - t0 > kWaitLimitNs) return false;
+  }
+}
 // Programmatic dependent launch.  pdl_wait: blocks until the kernel this one was launched behind has completed and
 // its memory operations are visible (at once when the kernel was launched the plain way); everything before it may
 // run while that kernel is still draining.  pdl_launch_dependents: lets the NEXT kernel of the stream be set up on the
