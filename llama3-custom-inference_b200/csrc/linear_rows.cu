@@ -76,10 +76,13 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v) {
-  asm volatile("{\n\t.reg .u32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.f32 [r], %2;\n\t}\n" ::"r"(addr), "r"(rank), "f"(v)
-               : "memory");
+// Address, among the cluster's, of what lies at `addr` in the shared memory of CTA `rank`.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
 }
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 __device__ __forceinline__ void output_warps_meet() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 // Whether all four output warps are well: they meet at barriers together or not at all.
 __device__ __forceinline__ bool output_warps_agree(bool ok) {
@@ -251,9 +254,9 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
     if (warp >= 2 && ok) {
       const int q4 = warp & 3, r = q4 * 32 + lane, rows = (int)a.rows;
       const int j = GATED ? r & 63 : r;
-      const uint32_t owner = (uint32_t)(j / kOwn);
-      // [token][rank][row of the slice]
-      const uint32_t at = smem_u32(parts) + ((rank * kSlice + (GATED ? r / 64 * kOwn : 0) + j % kOwn) << 2);
+      // [token][rank][row of the slice]: a warp's stores of one token are neighbours (16-byte stores of four tokens each, which are
+      // not, were slower)
+      const uint32_t at = cluster_addr(smem_u32(parts) + ((rank * kSlice + (GATED ? r / 64 * kOwn : 0) + j % kOwn) << 2), (uint32_t)(j / kOwn));
 #pragma unroll
       for (int c = 0; c < NP; c += 16) {
         if (c >= rows) break;
@@ -262,7 +265,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
         tc_wait_ld();
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          if (c + i < NP && c + i < rows) st_cluster(at + (uint32_t)(c + i) * kTile * 4, owner, __uint_as_float(v[i]));
+          if (c + i < NP && c + i < rows) st_cluster(at + (uint32_t)(c + i) * kTile * 4, v[i]);
       }
     }
     __syncwarp();

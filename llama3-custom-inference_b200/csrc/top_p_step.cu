@@ -102,6 +102,14 @@ __device__ __forceinline__ T ld_peer(const T* mine, uint32_t peer) {
     return *reinterpret_cast<T*>(&v);
   }
 }
+// Four words of a peer's shared memory.
+__device__ __forceinline__ uint4 ld_peer4(const uint32_t* mine, uint32_t peer) {
+  uint32_t remote;
+  uint4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(peer));
+  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(remote) : "memory");
+  return v;
+}
 // The CTAs' values of one quantity: each writes its own to a slot (no slot is used twice in a launch, so one cluster
 // barrier per exchange is enough) and reads the others' after the barrier.  `before`: the sum over the CTAs in front
 // of this one (the first CTA takes the front of the row); returns the sum over all.
@@ -404,6 +412,331 @@ top_p_step_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lon
   if constexpr (kCtas > 1) cluster_barrier();   // no CTA leaves while a peer may still read its shared memory
 }
 
+
+// ---- the same step by counts ---------------------------------------------------------------------------------------------------
+// The weight is a function of the logit's key, so the mass of a key is its count times its weight, exactly: the row needs one
+// histogram of counts over all 65 536 keys (16 bits each, 128 KB of shared memory) instead of a pass of three 64-bit-mass atomics
+// per search level, and the weights are evaluated once per key that occurs.  The CTA's share of the row stays in registers (64
+// entries a thread), is read from memory once, and the masses in index order are taken from there.  All sums are the integers of
+// the kernel above: same boundary, same ties, same draw, bit for bit.
+//   64 rows of 128 256 logits: 47 us; 82 with the masses' histograms, whose atomics met on a few dozen bins.
+constexpr int kKeyWords = 32768;                  // two keys' counts each
+constexpr int kHeld = 8;                          // 16-byte groups of a thread
+constexpr long long kMaxShare = 8191;             // groups of a CTA: a count of all its entries fits 16 bits
+
+__device__ __forceinline__ uint32_t bits_key(uint32_t u) {   // logit_key of a bf16 pattern
+  if (u == 0x8000u) return 0x8000u;
+  return (u & 0x8000u) ? (~u & 0xffffu) : (u | 0x8000u);
+}
+__device__ __forceinline__ float key_logit(uint32_t key) { return __uint_as_float(((key & 0x8000u) ? (key & 0x7fffu) : (~key & 0xffffu)) << 16); }
+
+// Sum over the warp's lanes in front of this one, and over all.
+template <typename T>
+__device__ __forceinline__ T warp_exclusive_scan(T v, T& total) {
+  const int lane = threadIdx.x & 31;
+  T inc = v;
+#pragma unroll
+  for (int d = 1; d < kWarp; d <<= 1) {
+    const T o = __shfl_up_sync(kFullMask, inc, d);
+    if (lane >= d) inc += o;
+  }
+  total = __shfl_sync(kFullMask, inc, kWarp - 1);
+  return inc - v;
+}
+
+template <int kCtas>
+__global__ void __launch_bounds__(kTopPBlock, 1)
+top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, long long row_stride, float inv_temperature,
+                   float top_p, unsigned long long seed, long long* __restrict__ out_tokens, long long out_stride,
+                   long long out_cols, long long* __restrict__ steps, long long* __restrict__ next_input,
+                   int* __restrict__ positions, int* __restrict__ seq_lens, int* __restrict__ nucleus_count,
+                   float* __restrict__ nucleus_mass) {
+  extern __shared__ __align__(16) uint32_t counts[];   // word k / 2 holds the counts of keys k (even: low half)
+  __shared__ float redf[kTopPWarps];
+  __shared__ u64 byte_mass[256], red[kTopPWarps];
+  __shared__ long long warp_eq[kTopPWarps], warp_above[kTopPWarps];
+  __shared__ u64 warp_mass[kTopPWarps];
+  __shared__ int s_pick;
+  __shared__ u64 s_above;
+  __shared__ u64 s_slots[4];     // values for the peers, one slot per exchange
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t rank = kCtas > 1 ? cluster_rank() : 0u;
+  for (int i = tid; i < kKeyWords / 4; i += kTopPBlock) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0u, 0u, 0u, 0u);
+  pdl_launch_dependents();  // the next one may be set up while this one runs
+  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
+  const long long b = blockIdx.x / kCtas;
+  const __nv_bfloat16* row = logits + b * row_stride;
+  const long long step = steps ? steps[b] : 0;            // (barriers of all CTAs follow before one of them writes it)
+  const bool vectors = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
+  // groups of 8 entries: the CTA's run, in it the warp's, there 32 neighbours at a time
+  const long long groups = (vocab + kVecElems - 1) / kVecElems;
+  const long long g_end = groups * (rank + 1) / kCtas, g_cta = groups * rank / kCtas;
+  const int per_warp = (int)((g_end - g_cta + kTopPWarps - 1) / kTopPWarps);
+  const long long g_warp = g_cta + (long long)warp * per_warp;
+  const int n_warp = (int)min((long long)per_warp, max(0ll, g_end - g_warp));   // groups of this warp
+  auto entries = [&](int it) {                            // of this lane's group of round `it`
+    if (it * 32 + lane >= n_warp) return 0;
+    const long long left = vocab - (g_warp + it * 32 + lane) * kVecElems;
+    return (int)(left < kVecElems ? left : kVecElems);
+  };
+  uint4 held[kHeld];
+#pragma unroll
+  for (int it = 0; it < kHeld; ++it) {
+    held[it] = make_uint4(0u, 0u, 0u, 0u);
+    const int n = entries(it);
+    if (n == 0) continue;
+    const __nv_bfloat16* at = row + (g_warp + it * 32 + lane) * kVecElems;
+    if (vectors && n == kVecElems) {
+      held[it] = __ldg(reinterpret_cast<const uint4*>(at));
+    } else {
+      const unsigned short* bits = reinterpret_cast<const unsigned short*>(at);
+      uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+      for (int j = 0; j < kVecElems; ++j)
+        if (j < n) w[j / 2] |= (uint32_t)__ldg(bits + j) << (16 * (j & 1));
+      held[it] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+  auto bits_of = [&](const uint4& v, int j) {
+    const uint32_t w = j < 2 ? v.x : j < 4 ? v.y : j < 6 ? v.z : v.w;
+    return (j & 1) ? w >> 16 : w & 0xffffu;
+  };
+  __syncthreads();                                        // the counts are cleared
+
+  // ---- 1. counts of the keys and the maximum ----
+  float m = -INFINITY;
+#pragma unroll
+  for (int it = 0; it < kHeld; ++it) {
+    if (it * 32 >= n_warp) break;
+    const int n = entries(it);
+    // equal neighbours (a flat row) are added at once
+    uint32_t run_key = 0u, run = 0u;
+#pragma unroll
+    for (int j = 0; j < kVecElems; ++j) {
+      if (j >= n) break;
+      const uint32_t u = bits_of(held[it], j), key = bits_key(u);
+      m = fmaxf(m, __uint_as_float(u << 16));
+      if (run > 0u && key != run_key) {
+        atomicAdd(counts + (run_key >> 1), run << (16 * (run_key & 1)));
+        run = 0u;
+      }
+      run_key = key;
+      ++run;
+    }
+    if (run > 0u) atomicAdd(counts + (run_key >> 1), run << (16 * (run_key & 1)));
+  }
+  m = group_max<kWarp>(m);
+  if (lane == 0) redf[warp] = m;
+  __syncthreads();
+  RowView rv;
+  rv.scale = inv_temperature * 1.4426950408889634f;
+  rv.shift = peer_max<kCtas>(group_max<kWarp>(redf[lane]), reinterpret_cast<float*>(&s_slots[0]), rank) * rv.scale;   // (its barrier: all counts are there)
+
+  // ---- 2. masses of the keys' high bytes: this CTA those of its 256 / kCtas ----
+  {
+    constexpr int kBins = 65536 / kCtas / kTopPBlock, kLanes = 256 / kBins;   // keys of a thread, threads of a byte
+    const int word0 = ((int)rank * (65536 / kCtas) + tid * kBins) / 2;
+    u64 q = 0;
+#pragma unroll
+    for (int i = 0; i < kBins / 8; ++i) {
+      uint32_t n[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) n[k] = 0u;
+      auto add = [&](const uint4& c) {
+        const uint32_t w[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { n[2 * k] += w[k] & 0xffffu; n[2 * k + 1] += w[k] >> 16; }
+      };
+      add(*reinterpret_cast<const uint4*>(counts + word0 + 4 * i));
+#pragma unroll
+      for (uint32_t pc = 0; pc < (uint32_t)kCtas; ++pc)
+        if (pc != rank) add(ld_peer4(counts + word0 + 4 * i, pc));
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (n[k]) q += (u64)n[k] * rv.weight(key_logit((uint32_t)(2 * (word0 + 4 * i) + k)));
+    }
+#pragma unroll
+    for (int d = kLanes / 2; d >= 1; d /= 2) q += __shfl_xor_sync(kFullMask, q, d);
+    if (tid % kLanes == 0) byte_mass[(int)rank * (256 / kCtas) + tid / kLanes] = q;
+  }
+  __syncthreads();
+  if constexpr (kCtas > 1) cluster_barrier();
+  const int d = 255 - tid;                                // (threads 0 to 255: a scan over threads is a suffix scan over values)
+  // the value of the digit in which the mass strictly above crosses `budget`; -1: all fit
+  auto crossing = [&](u64 h, u64 before, u64 total, u64 budget) {
+    if (tid == 0) { s_pick = -1; s_above = total; }
+    __syncthreads();
+    if (tid < 256 && before <= budget && before + h > budget) { s_pick = d; s_above = before; }
+    __syncthreads();
+    return s_pick;
+  };
+  u64 Z, h = 0;
+  if (tid < 256) {
+    const uint32_t owner = (uint32_t)(d / (256 / kCtas));
+    h = kCtas == 1 || owner == rank ? byte_mass[d] : ld_peer(byte_mass + d, owner);
+  }
+  u64 before = block_exclusive_scan<u64>(h, red, Z);
+  const u64 budget = (u64)((double)top_p * (double)Z);
+  const int hi = crossing(h, before, Z, budget);
+  const bool all_kept = hi < 0;                           // top_p >= 1
+  uint32_t key_star = 0u;
+  u64 bud = budget;
+  if (!all_kept) {
+    bud -= s_above;
+    h = 0;
+    if (tid < 256) {
+      const uint32_t key = ((uint32_t)hi << 8) | (uint32_t)d;
+      uint32_t n = (counts[key >> 1] >> (16 * (key & 1))) & 0xffffu;
+#pragma unroll
+      for (uint32_t pc = 0; pc < (uint32_t)kCtas; ++pc)
+        if (pc != rank) n += (ld_peer(counts + (key >> 1), pc) >> (16 * (key & 1))) & 0xffffu;
+      if (n) h = (u64)n * rv.weight(key_logit(key));
+    }
+    u64 total;
+    before = block_exclusive_scan<u64>(h, red, total);
+    const int lo = crossing(h, before, total, bud);
+    if (lo >= 0) bud -= s_above;
+    key_star = ((uint32_t)hi << 8) | (lo < 0 ? 0u : (uint32_t)lo);   // (the sums are exact: the second digit is found)
+  }
+  const u64 above = budget - bud;                         // mass of the entries strictly above the boundary
+  const u64 w_star = rv.weight(key_logit(key_star));
+
+  // ---- 3. the nucleus in index order: per warp, ties at the boundary counted ----
+  auto lane_sums = [&](int it, u64& w, int& eq, int& over) {   // this lane's group of round `it`
+    w = 0;
+    eq = over = 0;
+    const int n = entries(it);
+#pragma unroll
+    for (int j = 0; j < kVecElems; ++j) {
+      if (j >= n) break;
+      const uint32_t u = bits_of(held[it], j), key = bits_key(u);
+      if (all_kept || key > key_star) { w += rv.weight(__uint_as_float(u << 16)); ++over; }
+      else if (key == key_star) ++eq;
+    }
+  };
+  u64 w_warp = 0;
+  long long eq_warp = 0, over_warp = 0;
+  {
+    int eq_lane = 0, over_lane = 0;
+#pragma unroll
+    for (int it = 0; it < kHeld; ++it) {
+      if (it * 32 >= n_warp) break;
+      u64 w;
+      int eq, over;
+      lane_sums(it, w, eq, over);
+      w_warp += w;
+      eq_lane += eq;
+      over_lane += over;
+    }
+#pragma unroll
+    for (int k = 16; k >= 1; k /= 2) w_warp += __shfl_xor_sync(kFullMask, w_warp, k);
+    eq_warp = __reduce_add_sync(kFullMask, eq_lane);
+    over_warp = __reduce_add_sync(kFullMask, over_lane);
+  }
+  if (lane == 0) warp_eq[warp] = eq_warp;
+  __syncthreads();
+  // (every warp scans the 32 warps' values)
+  long long eq_total, front;
+  long long eq_before = __shfl_sync(kFullMask, warp_exclusive_scan<long long>(warp_eq[lane], eq_total), warp);
+  eq_total = peer_sum<kCtas>(eq_total, reinterpret_cast<long long*>(&s_slots[1]), rank, front);
+  eq_before += front;
+  // entries equal to the boundary, in index order: the j-th is kept while above + j * w* <= budget
+  long long eq_kept = 0;
+  if (!all_kept && eq_total > 0) {
+    eq_kept = w_star > 0 ? (long long)((budget > above ? budget - above : 0) / w_star) + 1 : eq_total;
+    if (eq_kept > eq_total) eq_kept = eq_total;
+  }
+  auto kept_of = [&](long long n_eq, long long seen) {
+    const long long k = eq_kept - seen;
+    return k < 0 ? 0 : k > n_eq ? n_eq : k;
+  };
+  const u64 mass_warp = w_warp + (u64)kept_of(eq_warp, eq_before) * w_star;
+  if (lane == 0) {
+    warp_mass[warp] = mass_warp;
+    warp_above[warp] = over_warp + kept_of(eq_warp, eq_before);
+  }
+  __syncthreads();
+  u64 mass_total, mass_front;
+  u64 mass_before = __shfl_sync(kFullMask, warp_exclusive_scan<u64>(warp_mass[lane], mass_total), warp);
+  mass_total = peer_sum<kCtas>(mass_total, &s_slots[2], rank, mass_front);
+  mass_before += mass_front;
+
+  // ---- 4. the draw: u in [0, 1) with 32 bits, target = floor(u * nucleus mass) < nucleus mass ----
+  const uint32_t r = philox_first((uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)b, (uint32_t)(b >> 32), (uint32_t)step,
+                                  (uint32_t)(step >> 32));
+  const u64 target = __umul64hi(mass_total, (u64)r << 32);
+  // one warp of one CTA has the target in its run; an empty nucleus (a row of NaNs) has no such warp: the first one stands in
+  const bool found = mass_warp > 0 && mass_before <= target && target < mass_before + mass_warp;
+  const bool stand_in = mass_total == 0 && rank == 0 && warp == 0;
+  if (found || stand_in) {
+    long long tok = -1;
+    if (found) {
+      u64 run = mass_before;
+      long long seen = eq_before;
+#pragma unroll
+      for (int it = 0; it < kHeld; ++it) {
+        if (it * 32 >= n_warp || __any_sync(kFullMask, tok >= 0)) break;
+        u64 w, w_all;
+        int eq, over;
+        lane_sums(it, w, eq, over);
+        int eq_all;
+        const int eq_front = warp_exclusive_scan<int>(eq, eq_all);
+        w += (u64)kept_of(eq, seen + eq_front) * w_star;
+        const u64 w_front = warp_exclusive_scan<u64>(w, w_all);
+        u64 mine = run + w_front;
+        if (w > 0 && mine <= target && target < mine + w) {
+          long long eq_seen = seen + eq_front;
+          const int n = entries(it);
+#pragma unroll
+          for (int j = 0; j < kVecElems; ++j) {
+            if (j >= n || tok >= 0) break;
+            const uint32_t u = bits_of(held[it], j), key = bits_key(u);
+            bool in = all_kept || key > key_star;
+            if (!in && key == key_star) { in = eq_seen < eq_kept; ++eq_seen; }
+            if (in) {
+              mine += rv.weight(__uint_as_float(u << 16));
+              if (mine > target) tok = (g_warp + it * 32 + lane) * kVecElems + j;
+            }
+          }
+        }
+        run += w_all;
+        seen += eq_all;
+      }
+    } else if (lane == 0) {
+      // the last entry of the nucleus among the first of the row
+      constexpr long long kRowThreads = (long long)kTopPBlock * kCtas;
+      const long long per = ((vocab + kRowThreads - 1) / kRowThreads + kVecElems - 1) / kVecElems * kVecElems;
+      tok = 0;
+      long long eq_seen = 0;
+      for (long long i = 0; i < per && i < vocab; ++i) {
+        const uint32_t key = bits_key(reinterpret_cast<const unsigned short*>(row)[i]);
+        bool in = all_kept || key > key_star;
+        if (!in && key == key_star) { in = eq_seen < eq_kept; ++eq_seen; }
+        if (in) tok = i;
+      }
+    }
+    if (tok >= 0) {                                       // one lane
+      if (out_tokens && steps) {
+        if (step >= 0 && step < out_cols) out_tokens[b * out_stride + step] = tok;
+        steps[b] = step + 1;
+      } else if (out_tokens) {
+        out_tokens[b * out_stride] = tok;
+      }
+      if (next_input) next_input[b] = tok;
+      if (positions) positions[b] += 1;
+      if (seq_lens) seq_lens[b] += 1;
+      if (nucleus_mass) nucleus_mass[b] = Z > 0 ? (float)((double)mass_total / (double)Z) : 0.f;
+    }
+  }
+  if (nucleus_count) {
+    long long total;
+    warp_exclusive_scan<long long>(warp_above[lane], total);
+    total = peer_sum<kCtas>(total, reinterpret_cast<long long*>(&s_slots[3]), rank, front);
+    if (tid == 0 && rank == 0) nucleus_count[b] = (int)total;
+  }
+  if constexpr (kCtas > 1) cluster_barrier();   // no CTA leaves while a peer may still read its shared memory
+}
+
 }  // namespace
 }  // namespace l3ci
 
@@ -424,15 +757,18 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
   const auto lp = static_cast<const __nv_bfloat16*>(logits);
   const float inv_t = 1.0f / temperature;
   const int sms = sm_count();
-  // Small batches: a cluster of CTAs per row, as many (8, 4, 2) as still run all at once, so that the batch covers
-  // the device (64 rows: 128 SMs; one row: 8).  A 148-SM part holds 15 clusters of 8, 33 of 4 or 74 of 2 of these
-  // CTAs at a time (cudaOccupancyMaxActiveClusters); the bounds scale with the SM count.
-  const int ctas_per_row = sms <= 0 ? 1 : rows * 148 <= 15LL * sms ? 8 : rows * 148 <= 33LL * sms ? 4 : 2 * rows <= sms ? 2 : 1;
-  // (a cluster size the device or its partition cannot place falls back to the next smaller one)
-  for (int c = ctas_per_row; c > 1; c /= 2) {
+  auto launch = [&](auto kernel, int c, int smem) {
+    static bool configured[64][9] = {};   // by device and CTAs per row
+    int dev = 0;
+    if (smem > 0 && (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !configured[dev][c])) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e != cudaSuccess) return e;
+      if (dev >= 0 && dev < 64) configured[dev][c] = true;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(c * rows));
     cfg.blockDim = dim3(kTopPBlock);
+    cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -440,14 +776,29 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    auto launch = [&](auto kernel) {
-      return cudaLaunchKernelEx(&cfg, kernel, lp, (long long)vocab, (long long)row_stride, inv_t, top_p, (unsigned long long)seed,
-                                reinterpret_cast<long long*>(out_tokens), (long long)out_stride, (long long)out_cols,
-                                reinterpret_cast<long long*>(steps), reinterpret_cast<long long*>(next_input), positions, seq_lens,
-                                nucleus_count, nucleus_mass);
-    };
-    const cudaError_t e = c == 8 ? launch(top_p_step_kernel<8>) : c == 4 ? launch(top_p_step_kernel<4>) : launch(top_p_step_kernel<2>);
+    cfg.numAttrs = c > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, lp, (long long)vocab, (long long)row_stride, inv_t, top_p, (unsigned long long)seed,
+                              reinterpret_cast<long long*>(out_tokens), (long long)out_stride, (long long)out_cols,
+                              reinterpret_cast<long long*>(steps), reinterpret_cast<long long*>(next_input), positions, seq_lens,
+                              nucleus_count, nucleus_mass);
+  };
+  // Small batches: a cluster of CTAs per row, as many (8, 4, 2) as still run all at once, so that the batch covers
+  // the device (64 rows: 128 SMs; one row: 8).  A 148-SM part holds 15 clusters of 8, 33 of 4 or 74 of 2 of these
+  // CTAs at a time (cudaOccupancyMaxActiveClusters); the bounds scale with the SM count.
+  const int ctas_per_row = sms <= 0 ? 1 : rows * 148 <= 15LL * sms ? 8 : rows * 148 <= 33LL * sms ? 4 : 2 * rows <= sms ? 2 : 1;
+  // By counts while a CTA's share of the row fits its registers and 16-bit counts: more CTAs per row where that takes more of
+  // them.  Longer rows yet, or a device that cannot place the cluster: by masses.
+  const long long groups = (vocab + kVecElems - 1) / kVecElems;
+  int by_counts = ctas_per_row;
+  while (by_counts < 8 && (groups + by_counts - 1) / by_counts > kMaxShare) by_counts *= 2;
+  if ((groups + by_counts - 1) / by_counts <= kMaxShare) {
+    cudaError_t e = by_counts == 8 ? launch(top_p_count_kernel<8>, 8, kKeyWords * 4) : by_counts == 4 ? launch(top_p_count_kernel<4>, 4, kKeyWords * 4)
+                    : by_counts == 2 ? launch(top_p_count_kernel<2>, 2, kKeyWords * 4) : launch(top_p_count_kernel<1>, 1, kKeyWords * 4);
+    if (e == cudaSuccess) return L3CI_OK;
+    (void)cudaGetLastError();   // not placed: nothing ran
+  }
+  for (int c = ctas_per_row; c > 1; c /= 2) {
+    const cudaError_t e = c == 8 ? launch(top_p_step_kernel<8>, 8, 0) : c == 4 ? launch(top_p_step_kernel<4>, 4, 0) : launch(top_p_step_kernel<2>, 2, 0);
     if (e == cudaSuccess) return L3CI_OK;
     (void)cudaGetLastError();   // not placed: nothing ran
   }

@@ -1,0 +1,39 @@
+"""The nucleus-sampling step by key counts against the same step by masses, which takes rows too long for the counts: an appended
+tail of -inf logits has no mass, so a row and the row with that tail must give the same token, nucleus size and mass."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+LONG = 8 * 8191 * 8 + 8      # one group more than eight CTAs count
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 8), (2, 1001), (40, 8191), (15, 65537), (16, 65536), (33, 128256), (74, 128256), (75, 65528), (75, 65529)])
+@pytest.mark.parametrize("kind", ["normal", "flat", "steps", "holes"])
+def test_counts_and_masses_agree(capi, device, rows, vocab, kind):
+    g = torch.Generator(device=device).manual_seed(rows + vocab)
+    x = torch.randn(rows, vocab, generator=g, device=device) * 2.5
+    if kind == "flat":
+        x.fill_(-1.25)
+    elif kind == "steps":
+        x = x.round()                                  # many ties at the boundary, zeros of both signs among them
+    elif kind == "holes":
+        x[torch.rand(rows, vocab, generator=g, device=device) < 0.9] = float("-inf")
+        x[:, vocab // 2] = 3.0
+    x = x.bfloat16()
+    long = torch.full((rows, LONG), float("-inf"), dtype=torch.bfloat16, device=device)
+    long[:, :vocab] = x
+
+    def run(logits):
+        out, i64, i32 = torch.zeros(rows, 2, dtype=torch.int64, device=device), dict(dtype=torch.int64, device=device), dict(dtype=torch.int32, device=device)
+        steps, cur, pos, lens, count = (torch.zeros(rows, **d) for d in (i64, i64, i32, i32, i32))
+        mass = torch.zeros(rows, device=device)
+        for _ in range(2):
+            capi.top_p_step(logits, 0.8, 0.9, 77, out, steps, cur, pos, lens, count, mass)
+        return out, steps, pos, lens, count, mass
+
+    odd = torch.empty(rows, vocab + 3, dtype=torch.bfloat16, device=device)      # rows that do not start on 16 bytes
+    odd[:, 3:] = x
+    want = run(long)
+    for logits in (x, odd[:, 3:]):
+        for a, b in zip(run(logits), want):
+            assert torch.equal(a, b)
