@@ -102,14 +102,6 @@ __device__ __forceinline__ T ld_peer(const T* mine, uint32_t peer) {
     return *reinterpret_cast<T*>(&v);
   }
 }
-// Four words of a peer's shared memory.
-__device__ __forceinline__ uint4 ld_peer4(const uint32_t* mine, uint32_t peer) {
-  uint32_t remote;
-  uint4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(peer));
-  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(remote) : "memory");
-  return v;
-}
 // The CTAs' values of one quantity: each writes its own to a slot (no slot is used twice in a launch, so one cluster
 // barrier per exchange is enough) and reads the others' after the barrier.  `before`: the sum over the CTAs in front
 // of this one (the first CTA takes the front of the row); returns the sum over all.
@@ -443,6 +435,47 @@ __device__ __forceinline__ T warp_exclusive_scan(T v, T& total) {
   total = __shfl_sync(kFullMask, inc, kWarp - 1);
   return inc - v;
 }
+// Sum of the CTAs' slots, and of those in front of this CTA, by every warp; behind a barrier of the cluster.  (One lane per CTA: a
+// read of a peer's shared memory by every thread took longer than the sums.)
+template <int kCtas, typename T>
+__device__ __forceinline__ T slots_sum(const T* slot, uint32_t rank, T& front) {
+  const uint32_t lane = threadIdx.x & 31;
+  T v = T(0);
+  if (lane < (uint32_t)kCtas) v = kCtas == 1 || lane == rank ? *slot : ld_peer(slot, lane);
+  T all;
+  front = __shfl_sync(kFullMask, warp_exclusive_scan<T>(v, all), (int)rank);
+  return all;
+}
+
+// Of 256 digits' masses (shared memory), by every warp: the largest digit whose mass together with that of the larger ones exceeds
+// `budget`, -1 if there is none; `above`: the mass of the larger ones; `total`: of all.  `budget_of(total)` gives the budget.
+template <typename F>
+__device__ __forceinline__ int digit_crossing(const u64* mass, F&& budget_of, u64& above, u64& total) {
+  const int lane = threadIdx.x & 31;
+  u64 h[8], sum = 0;                     // lane l: digits 255 - 8 l downwards
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    h[i] = mass[255 - 8 * lane - i];
+    sum += h[i];
+  }
+  u64 before = warp_exclusive_scan<u64>(sum, total);
+  const u64 budget = budget_of(total);
+  int pick = -1;
+  u64 at = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (pick < 0 && before <= budget && before + h[i] > budget) {
+      pick = 255 - 8 * lane - i;
+      at = before;
+    }
+    before += h[i];
+  }
+  const unsigned who = __ballot_sync(kFullMask, pick >= 0);
+  if (who == 0) return -1;
+  const int src = __ffs(who) - 1;
+  above = __shfl_sync(kFullMask, at, src);
+  return __shfl_sync(kFullMask, pick, src);
+}
 
 template <int kCtas>
 __global__ void __launch_bounds__(kTopPBlock, 1)
@@ -453,12 +486,12 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
                    float* __restrict__ nucleus_mass) {
   extern __shared__ __align__(16) uint32_t counts[];   // word k / 2 holds the counts of keys k (even: low half)
   __shared__ float redf[kTopPWarps];
-  __shared__ u64 byte_mass[256], red[kTopPWarps];
-  __shared__ long long warp_eq[kTopPWarps], warp_above[kTopPWarps];
+  __shared__ u64 own_mass[256], digit_mass[256];
+  __shared__ long long warp_eq[kTopPWarps], warp_over[kTopPWarps];
   __shared__ u64 warp_mass[kTopPWarps];
-  __shared__ int s_pick;
-  __shared__ u64 s_above;
-  __shared__ u64 s_slots[4];     // values for the peers, one slot per exchange
+  __shared__ float s_max;
+  __shared__ u64 s_mass;         // this CTA's, for the peers
+  __shared__ long long s_eq, s_kept;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = kCtas > 1 ? cluster_rank() : 0u;
   for (int i = tid; i < kKeyWords / 4; i += kTopPBlock) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -466,6 +499,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
   const long long b = blockIdx.x / kCtas;
   const __nv_bfloat16* row = logits + b * row_stride;
+  const unsigned short* row_bits = reinterpret_cast<const unsigned short*>(row);
   const long long step = steps ? steps[b] : 0;            // (barriers of all CTAs follow before one of them writes it)
   const bool vectors = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
   // groups of 8 entries: the CTA's run, in it the warp's, there 32 neighbours at a time
@@ -485,15 +519,14 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     held[it] = make_uint4(0u, 0u, 0u, 0u);
     const int n = entries(it);
     if (n == 0) continue;
-    const __nv_bfloat16* at = row + (g_warp + it * 32 + lane) * kVecElems;
+    const long long at = (g_warp + it * 32 + lane) * kVecElems;
     if (vectors && n == kVecElems) {
-      held[it] = __ldg(reinterpret_cast<const uint4*>(at));
+      held[it] = __ldg(reinterpret_cast<const uint4*>(row + at));
     } else {
-      const unsigned short* bits = reinterpret_cast<const unsigned short*>(at);
       uint32_t w[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
       for (int j = 0; j < kVecElems; ++j)
-        if (j < n) w[j / 2] |= (uint32_t)__ldg(bits + j) << (16 * (j & 1));
+        if (j < n) w[j / 2] |= (uint32_t)__ldg(row_bits + at + j) << (16 * (j & 1));
       held[it] = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
@@ -509,92 +542,85 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   for (int it = 0; it < kHeld; ++it) {
     if (it * 32 >= n_warp) break;
     const int n = entries(it);
-    // equal neighbours (a flat row) are added at once
-    uint32_t run_key = 0u, run = 0u;
+    const uint4 v = held[it];
+    if (n == kVecElems && v.x == v.y && v.y == v.z && v.z == v.w && v.x >> 16 == (v.x & 0xffffu)) {   // a flat row's lanes would queue at one word
+      const uint32_t key = bits_key(v.x & 0xffffu);
+      m = fmaxf(m, __uint_as_float(v.x << 16));
+      atomicAdd(counts + (key >> 1), 8u << (16 * (key & 1)));
+      continue;
+    }
 #pragma unroll
     for (int j = 0; j < kVecElems; ++j) {
       if (j >= n) break;
-      const uint32_t u = bits_of(held[it], j), key = bits_key(u);
+      const uint32_t u = bits_of(v, j), key = bits_key(u);
       m = fmaxf(m, __uint_as_float(u << 16));
-      if (run > 0u && key != run_key) {
-        atomicAdd(counts + (run_key >> 1), run << (16 * (run_key & 1)));
-        run = 0u;
-      }
-      run_key = key;
-      ++run;
+      atomicAdd(counts + (key >> 1), 1u << (16 * (key & 1)));
     }
-    if (run > 0u) atomicAdd(counts + (run_key >> 1), run << (16 * (run_key & 1)));
   }
   m = group_max<kWarp>(m);
   if (lane == 0) redf[warp] = m;
   __syncthreads();
+  m = group_max<kWarp>(redf[lane]);
+  if constexpr (kCtas > 1) {
+    if (tid == 0) s_max = m;
+    cluster_barrier();
+    if (lane < kCtas) m = ld_peer(&s_max, (uint32_t)lane);
+    m = group_max<kWarp>(m);
+  }
   RowView rv;
   rv.scale = inv_temperature * 1.4426950408889634f;
-  rv.shift = peer_max<kCtas>(group_max<kWarp>(redf[lane]), reinterpret_cast<float*>(&s_slots[0]), rank) * rv.scale;   // (its barrier: all counts are there)
+  rv.shift = m * rv.scale;
 
-  // ---- 2. masses of the keys' high bytes: this CTA those of its 256 / kCtas ----
-  {
-    constexpr int kBins = 65536 / kCtas / kTopPBlock, kLanes = 256 / kBins;   // keys of a thread, threads of a byte
-    const int word0 = ((int)rank * (65536 / kCtas) + tid * kBins) / 2;
+  // ---- 2. boundary of the nucleus, digit by digit of the key: the masses of this CTA's entries, then of all ----
+  // (a digit by a warp, neighbours to different ones: those that occur are neighbours)
+#pragma unroll 1
+  for (int i = 0; i < 8; ++i) {
+    const int d = i * kTopPWarps + warp;
+    const uint4 c = reinterpret_cast<const uint4*>(counts + d * 128)[lane];
     u64 q = 0;
+    if (__any_sync(kFullMask, (c.x | c.y | c.z | c.w) != 0u)) {
+      const uint32_t w[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-    for (int i = 0; i < kBins / 8; ++i) {
-      uint32_t n[8];
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t n = (k & 1) ? w[k / 2] >> 16 : w[k / 2] & 0xffffu;
+        if (n) q += (u64)n * rv.weight(key_logit((uint32_t)(d * 256 + lane * 8 + k)));
+      }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) n[k] = 0u;
-      auto add = [&](const uint4& c) {
-        const uint32_t w[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) { n[2 * k] += w[k] & 0xffffu; n[2 * k + 1] += w[k] >> 16; }
-      };
-      add(*reinterpret_cast<const uint4*>(counts + word0 + 4 * i));
-#pragma unroll
-      for (uint32_t pc = 0; pc < (uint32_t)kCtas; ++pc)
-        if (pc != rank) add(ld_peer4(counts + word0 + 4 * i, pc));
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (n[k]) q += (u64)n[k] * rv.weight(key_logit((uint32_t)(2 * (word0 + 4 * i) + k)));
+      for (int k = 16; k >= 1; k /= 2) q += __shfl_xor_sync(kFullMask, q, k);
     }
-#pragma unroll
-    for (int d = kLanes / 2; d >= 1; d /= 2) q += __shfl_xor_sync(kFullMask, q, d);
-    if (tid % kLanes == 0) byte_mass[(int)rank * (256 / kCtas) + tid / kLanes] = q;
+    if (lane == 0) own_mass[d] = q;
   }
   __syncthreads();
   if constexpr (kCtas > 1) cluster_barrier();
-  const int d = 255 - tid;                                // (threads 0 to 255: a scan over threads is a suffix scan over values)
-  // the value of the digit in which the mass strictly above crosses `budget`; -1: all fit
-  auto crossing = [&](u64 h, u64 before, u64 total, u64 budget) {
-    if (tid == 0) { s_pick = -1; s_above = total; }
-    __syncthreads();
-    if (tid < 256 && before <= budget && before + h > budget) { s_pick = d; s_above = before; }
-    __syncthreads();
-    return s_pick;
-  };
-  u64 Z, h = 0;
   if (tid < 256) {
-    const uint32_t owner = (uint32_t)(d / (256 / kCtas));
-    h = kCtas == 1 || owner == rank ? byte_mass[d] : ld_peer(byte_mass + d, owner);
+    u64 h = own_mass[tid];
+#pragma unroll
+    for (uint32_t pc = 0; pc < (uint32_t)kCtas; ++pc)
+      if (pc != rank) h += ld_peer(own_mass + tid, pc);
+    digit_mass[tid] = h;
   }
-  u64 before = block_exclusive_scan<u64>(h, red, Z);
-  const u64 budget = (u64)((double)top_p * (double)Z);
-  const int hi = crossing(h, before, Z, budget);
+  __syncthreads();
+  u64 Z, s_above = 0, budget = 0;
+  const int hi = digit_crossing(digit_mass, [&](u64 total) { return budget = (u64)((double)top_p * (double)total); }, s_above, Z);
   const bool all_kept = hi < 0;                           // top_p >= 1
   uint32_t key_star = 0u;
   u64 bud = budget;
   if (!all_kept) {
     bud -= s_above;
-    h = 0;
+    u64 h = 0;
     if (tid < 256) {
-      const uint32_t key = ((uint32_t)hi << 8) | (uint32_t)d;
+      const uint32_t key = ((uint32_t)hi << 8) | (uint32_t)tid;
       uint32_t n = (counts[key >> 1] >> (16 * (key & 1))) & 0xffffu;
 #pragma unroll
       for (uint32_t pc = 0; pc < (uint32_t)kCtas; ++pc)
         if (pc != rank) n += (ld_peer(counts + (key >> 1), pc) >> (16 * (key & 1))) & 0xffffu;
       if (n) h = (u64)n * rv.weight(key_logit(key));
     }
+    __syncthreads();                                      // the first digit's masses have been read
+    if (tid < 256) digit_mass[tid] = h;
+    __syncthreads();
     u64 total;
-    before = block_exclusive_scan<u64>(h, red, total);
-    const int lo = crossing(h, before, total, bud);
+    const int lo = digit_crossing(digit_mass, [&](u64) { return bud; }, s_above, total);
     if (lo >= 0) bud -= s_above;
     key_star = ((uint32_t)hi << 8) | (lo < 0 ? 0u : (uint32_t)lo);   // (the sums are exact: the second digit is found)
   }
@@ -602,16 +628,29 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   const u64 w_star = rv.weight(key_logit(key_star));
 
   // ---- 3. the nucleus in index order: per warp, ties at the boundary counted ----
+  // Few entries are in it: compares build a mask, and only the entries of its bits are weighed (read again: the row is in a cache).
+  // order(u): signed, -0 just below +0; at a boundary of 0 both tie
+  auto order = [](uint32_t u) { const int t = (int)(short)u; return t ^ ((t >> 31) & 0x7fff); };
+  const int star = all_kept ? -40000 : (int)key_star - 0x8000;
+  const int star_low = star == 0 ? -1 : star;
   auto lane_sums = [&](int it, u64& w, int& eq, int& over) {   // this lane's group of round `it`
     w = 0;
-    eq = over = 0;
     const int n = entries(it);
+    uint32_t in = 0u, ties = 0u;
 #pragma unroll
     for (int j = 0; j < kVecElems; ++j) {
-      if (j >= n) break;
-      const uint32_t u = bits_of(held[it], j), key = bits_key(u);
-      if (all_kept || key > key_star) { w += rv.weight(__uint_as_float(u << 16)); ++over; }
-      else if (key == key_star) ++eq;
+      const int t = order(bits_of(held[it], j));
+      in |= t > star ? 1u << j : 0u;
+      ties |= t <= star && t >= star_low ? 1u << j : 0u;
+    }
+    const uint32_t real = (1u << n) - 1u;
+    in &= real;
+    eq = __popc(ties & real);
+    over = __popc(in);
+    const unsigned short* at = row_bits + (g_warp + it * 32 + lane) * kVecElems;
+    while (in) {
+      w += rv.weight(__uint_as_float((uint32_t)__ldg(at + (__ffs(in) - 1)) << 16));
+      in &= in - 1;
     }
   };
   u64 w_warp = 0;
@@ -633,33 +672,41 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     eq_warp = __reduce_add_sync(kFullMask, eq_lane);
     over_warp = __reduce_add_sync(kFullMask, over_lane);
   }
-  if (lane == 0) warp_eq[warp] = eq_warp;
+  if (lane == 0) {
+    warp_eq[warp] = eq_warp;
+    warp_mass[warp] = w_warp;
+    warp_over[warp] = over_warp;
+  }
   __syncthreads();
   // (every warp scans the 32 warps' values)
-  long long eq_total, front;
+  long long eq_total, over_total, eq_front = 0;
+  u64 mass_cta, mass_front = 0;
   long long eq_before = __shfl_sync(kFullMask, warp_exclusive_scan<long long>(warp_eq[lane], eq_total), warp);
-  eq_total = peer_sum<kCtas>(eq_total, reinterpret_cast<long long*>(&s_slots[1]), rank, front);
-  eq_before += front;
+  u64 mass_before = __shfl_sync(kFullMask, warp_exclusive_scan<u64>(warp_mass[lane], mass_cta), warp);
+  warp_exclusive_scan<long long>(warp_over[lane], over_total);
+  u64 mass_total = mass_cta;
+  if constexpr (kCtas > 1) {
+    if (tid == 0) { s_eq = eq_total; s_mass = mass_cta; s_kept = over_total; }
+    cluster_barrier();
+    long long none;
+    eq_total = slots_sum<kCtas>(&s_eq, rank, eq_front);
+    mass_total = slots_sum<kCtas>(&s_mass, rank, mass_front);
+    over_total = slots_sum<kCtas>(&s_kept, rank, none);
+  }
+  eq_before += eq_front;
   // entries equal to the boundary, in index order: the j-th is kept while above + j * w* <= budget
   long long eq_kept = 0;
   if (!all_kept && eq_total > 0) {
     eq_kept = w_star > 0 ? (long long)((budget > above ? budget - above : 0) / w_star) + 1 : eq_total;
     if (eq_kept > eq_total) eq_kept = eq_total;
   }
-  auto kept_of = [&](long long n_eq, long long seen) {
+  auto kept_of = [&](long long n_eq, long long seen) {    // of n_eq ties behind `seen` others
     const long long k = eq_kept - seen;
     return k < 0 ? 0 : k > n_eq ? n_eq : k;
   };
+  mass_total += (u64)eq_kept * w_star;
+  mass_before += mass_front + (u64)kept_of(eq_before, 0) * w_star;
   const u64 mass_warp = w_warp + (u64)kept_of(eq_warp, eq_before) * w_star;
-  if (lane == 0) {
-    warp_mass[warp] = mass_warp;
-    warp_above[warp] = over_warp + kept_of(eq_warp, eq_before);
-  }
-  __syncthreads();
-  u64 mass_total, mass_front;
-  u64 mass_before = __shfl_sync(kFullMask, warp_exclusive_scan<u64>(warp_mass[lane], mass_total), warp);
-  mass_total = peer_sum<kCtas>(mass_total, &s_slots[2], rank, mass_front);
-  mass_before += mass_front;
 
   // ---- 4. the draw: u in [0, 1) with 32 bits, target = floor(u * nucleus mass) < nucleus mass ----
   const uint32_t r = philox_first((uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)b, (uint32_t)(b >> 32), (uint32_t)step,
@@ -677,15 +724,13 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
       for (int it = 0; it < kHeld; ++it) {
         if (it * 32 >= n_warp || __any_sync(kFullMask, tok >= 0)) break;
         u64 w, w_all;
-        int eq, over;
+        int eq, over, eq_all;
         lane_sums(it, w, eq, over);
-        int eq_all;
-        const int eq_front = warp_exclusive_scan<int>(eq, eq_all);
-        w += (u64)kept_of(eq, seen + eq_front) * w_star;
-        const u64 w_front = warp_exclusive_scan<u64>(w, w_all);
-        u64 mine = run + w_front;
+        const int ties_front = warp_exclusive_scan<int>(eq, eq_all);
+        w += (u64)kept_of(eq, seen + ties_front) * w_star;
+        u64 mine = run + warp_exclusive_scan<u64>(w, w_all);
         if (w > 0 && mine <= target && target < mine + w) {
-          long long eq_seen = seen + eq_front;
+          long long eq_seen = seen + ties_front;
           const int n = entries(it);
 #pragma unroll
           for (int j = 0; j < kVecElems; ++j) {
@@ -709,7 +754,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
       tok = 0;
       long long eq_seen = 0;
       for (long long i = 0; i < per && i < vocab; ++i) {
-        const uint32_t key = bits_key(reinterpret_cast<const unsigned short*>(row)[i]);
+        const uint32_t key = bits_key(row_bits[i]);
         bool in = all_kept || key > key_star;
         if (!in && key == key_star) { in = eq_seen < eq_kept; ++eq_seen; }
         if (in) tok = i;
@@ -728,12 +773,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
       if (nucleus_mass) nucleus_mass[b] = Z > 0 ? (float)((double)mass_total / (double)Z) : 0.f;
     }
   }
-  if (nucleus_count) {
-    long long total;
-    warp_exclusive_scan<long long>(warp_above[lane], total);
-    total = peer_sum<kCtas>(total, reinterpret_cast<long long*>(&s_slots[3]), rank, front);
-    if (tid == 0 && rank == 0) nucleus_count[b] = (int)total;
-  }
+  if (nucleus_count && tid == 0 && rank == 0) nucleus_count[b] = (int)(over_total + eq_kept);
   if constexpr (kCtas > 1) cluster_barrier();   // no CTA leaves while a peer may still read its shared memory
 }
 
