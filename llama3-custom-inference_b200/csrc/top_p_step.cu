@@ -411,7 +411,7 @@ top_p_step_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lon
 // per search level, and the weights are evaluated once per key that occurs.  The CTA's share of the row stays in registers (64
 // entries a thread), is read from memory once, and the masses in index order are taken from there.  All sums are the integers of
 // the kernel above: same boundary, same ties, same draw, bit for bit.
-//   64 rows of 128 256 logits: 47 us; 82 with the masses' histograms, whose atomics met on a few dozen bins.
+//   64 rows of 128 256 logits: 39 us; 82 with the masses' histograms, whose atomics met on a few dozen bins.
 constexpr int kKeyWords = 32768;                  // two keys' counts each
 constexpr int kHeld = 8;                          // 16-byte groups of a thread
 constexpr long long kMaxShare = 8191;             // groups of a CTA: a count of all its entries fits 16 bits
@@ -447,15 +447,16 @@ __device__ __forceinline__ T slots_sum(const T* slot, uint32_t rank, T& front) {
   return all;
 }
 
-// Of 256 digits' masses (shared memory), by every warp: the largest digit whose mass together with that of the larger ones exceeds
-// `budget`, -1 if there is none; `above`: the mass of the larger ones; `total`: of all.  `budget_of(total)` gives the budget.
+// Of 256 digits' masses (shared memory, digit d at digit_place(d)), by one warp: the largest digit whose mass together with that of
+// the larger ones exceeds the budget, -1 if there is none; `above`: the mass of the larger ones; `total`: of all.
+__device__ __forceinline__ int digit_place(int d) { return (255 - d) % 8 * 32 + (255 - d) / 8; }   // neighbouring lanes' digits on neighbouring banks
 template <typename F>
 __device__ __forceinline__ int digit_crossing(const u64* mass, F&& budget_of, u64& above, u64& total) {
   const int lane = threadIdx.x & 31;
   u64 h[8], sum = 0;                     // lane l: digits 255 - 8 l downwards
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    h[i] = mass[255 - 8 * lane - i];
+    h[i] = mass[i * 32 + lane];
     sum += h[i];
   }
   u64 before = warp_exclusive_scan<u64>(sum, total);
@@ -491,7 +492,11 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   __shared__ u64 warp_mass[kTopPWarps];
   __shared__ float s_max;
   __shared__ u64 s_mass;         // this CTA's, for the peers
-  __shared__ long long s_eq, s_kept;
+  __shared__ long long s_eq, s_over;
+  // what the first warp finds for all
+  __shared__ int s_pick[2];
+  __shared__ u64 s_above[2], s_total, s_budget, s_mass_front, s_mass_total;
+  __shared__ long long s_eq_front, s_eq_total, s_over_total;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = kCtas > 1 ? cluster_rank() : 0u;
   for (int i = tid; i < kKeyWords / 4; i += kTopPBlock) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -530,6 +535,8 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
       held[it] = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
+  const uint32_t r = philox_first((uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)b, (uint32_t)(b >> 32), (uint32_t)step,
+                                  (uint32_t)(step >> 32));
   auto bits_of = [&](const uint4& v, int j) {
     const uint32_t w = j < 2 ? v.x : j < 4 ? v.y : j < 6 ? v.z : v.w;
     return (j & 1) ? w >> 16 : w & 0xffffu;
@@ -597,16 +604,23 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
 #pragma unroll
     for (uint32_t pc = 0; pc < (uint32_t)kCtas; ++pc)
       if (pc != rank) h += ld_peer(own_mass + tid, pc);
-    digit_mass[tid] = h;
+    digit_mass[digit_place(tid)] = h;
   }
   __syncthreads();
-  u64 Z, s_above = 0, budget = 0;
-  const int hi = digit_crossing(digit_mass, [&](u64 total) { return budget = (u64)((double)top_p * (double)total); }, s_above, Z);
+  // (the scans by the first warp alone: 32 warps' shuffles took longer than the barriers)
+  if (warp == 0) {
+    u64 total, over = 0, limit = 0;
+    const int pick = digit_crossing(digit_mass, [&](u64 all) { return limit = (u64)((double)top_p * (double)all); }, over, total);
+    if (lane == 0) { s_pick[0] = pick; s_above[0] = over; s_total = total; s_budget = limit; }
+  }
+  __syncthreads();
+  const int hi = s_pick[0];
+  const u64 Z = s_total, budget = s_budget;
   const bool all_kept = hi < 0;                           // top_p >= 1
   uint32_t key_star = 0u;
   u64 bud = budget;
   if (!all_kept) {
-    bud -= s_above;
+    bud -= s_above[0];
     u64 h = 0;
     if (tid < 256) {
       const uint32_t key = ((uint32_t)hi << 8) | (uint32_t)tid;
@@ -616,19 +630,23 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
         if (pc != rank) n += (ld_peer(counts + (key >> 1), pc) >> (16 * (key & 1))) & 0xffffu;
       if (n) h = (u64)n * rv.weight(key_logit(key));
     }
-    __syncthreads();                                      // the first digit's masses have been read
-    if (tid < 256) digit_mass[tid] = h;
+    if (tid < 256) digit_mass[digit_place(tid)] = h;      // (the first digit's have been read)
     __syncthreads();
-    u64 total;
-    const int lo = digit_crossing(digit_mass, [&](u64) { return bud; }, s_above, total);
-    if (lo >= 0) bud -= s_above;
+    if (warp == 0) {
+      u64 total, over = 0;
+      const int pick = digit_crossing(digit_mass, [&](u64) { return bud; }, over, total);
+      if (lane == 0) { s_pick[1] = pick; s_above[1] = over; }
+    }
+    __syncthreads();
+    const int lo = s_pick[1];
+    if (lo >= 0) bud -= s_above[1];
     key_star = ((uint32_t)hi << 8) | (lo < 0 ? 0u : (uint32_t)lo);   // (the sums are exact: the second digit is found)
   }
   const u64 above = budget - bud;                         // mass of the entries strictly above the boundary
   const u64 w_star = rv.weight(key_logit(key_star));
 
   // ---- 3. the nucleus in index order: per warp, ties at the boundary counted ----
-  // Few entries are in it: compares build a mask, and only the entries of its bits are weighed (read again: the row is in a cache).
+  // Few entries are in it: compares build a mask, and only the entries of its bits are weighed.
   // order(u): signed, -0 just below +0; at a boundary of 0 both tie
   auto order = [](uint32_t u) { const int t = (int)(short)u; return t ^ ((t >> 31) & 0x7fff); };
   const int star = all_kept ? -40000 : (int)key_star - 0x8000;
@@ -636,20 +654,19 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   auto lane_sums = [&](int it, u64& w, int& eq, int& over) {   // this lane's group of round `it`
     w = 0;
     const int n = entries(it);
-    uint32_t in = 0u, ties = 0u;
+    uint32_t in = 0u, at_least = 0u;
 #pragma unroll
     for (int j = 0; j < kVecElems; ++j) {
       const int t = order(bits_of(held[it], j));
       in |= t > star ? 1u << j : 0u;
-      ties |= t <= star && t >= star_low ? 1u << j : 0u;
+      at_least |= t >= star_low ? 1u << j : 0u;
     }
     const uint32_t real = (1u << n) - 1u;
+    eq = __popc(at_least & ~in & real);
     in &= real;
-    eq = __popc(ties & real);
     over = __popc(in);
-    const unsigned short* at = row_bits + (g_warp + it * 32 + lane) * kVecElems;
     while (in) {
-      w += rv.weight(__uint_as_float((uint32_t)__ldg(at + (__ffs(in) - 1)) << 16));
+      w += rv.weight(__uint_as_float(bits_of(held[it], __ffs(in) - 1) << 16));
       in &= in - 1;
     }
   };
@@ -678,22 +695,32 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     warp_over[warp] = over_warp;
   }
   __syncthreads();
-  // (every warp scans the 32 warps' values)
-  long long eq_total, over_total, eq_front = 0;
-  u64 mass_cta, mass_front = 0;
-  long long eq_before = __shfl_sync(kFullMask, warp_exclusive_scan<long long>(warp_eq[lane], eq_total), warp);
-  u64 mass_before = __shfl_sync(kFullMask, warp_exclusive_scan<u64>(warp_mass[lane], mass_cta), warp);
-  warp_exclusive_scan<long long>(warp_over[lane], over_total);
-  u64 mass_total = mass_cta;
-  if constexpr (kCtas > 1) {
-    if (tid == 0) { s_eq = eq_total; s_mass = mass_cta; s_kept = over_total; }
-    cluster_barrier();
-    long long none;
-    eq_total = slots_sum<kCtas>(&s_eq, rank, eq_front);
-    mass_total = slots_sum<kCtas>(&s_mass, rank, mass_front);
-    over_total = slots_sum<kCtas>(&s_kept, rank, none);
+  if (warp == 0) {
+    long long eq_all, over_all;
+    u64 mass_all;
+    const long long eq = warp_exclusive_scan<long long>(warp_eq[lane], eq_all);
+    const u64 mass = warp_exclusive_scan<u64>(warp_mass[lane], mass_all);
+    over_all = warp_over[lane];
+#pragma unroll
+    for (int k = 16; k >= 1; k /= 2) over_all += __shfl_xor_sync(kFullMask, over_all, k);
+    warp_eq[lane] = eq;                                   // from here on: of the warps in front
+    warp_mass[lane] = mass;
+    if (lane == 0) { s_eq = eq_all; s_mass = mass_all; s_over = over_all; }
   }
-  eq_before += eq_front;
+  __syncwarp();
+  if constexpr (kCtas > 1) cluster_barrier();
+  if (warp == 0) {
+    long long eq_in_front, none;
+    u64 mass_in_front;
+    const long long eq_all = slots_sum<kCtas>(&s_eq, rank, eq_in_front), over_all = slots_sum<kCtas>(&s_over, rank, none);
+    const u64 mass_all = slots_sum<kCtas>(&s_mass, rank, mass_in_front);
+    if (lane == 0) {
+      s_eq_total = eq_all; s_eq_front = eq_in_front; s_over_total = over_all;
+      s_mass_total = mass_all; s_mass_front = mass_in_front;
+    }
+  }
+  __syncthreads();
+  const long long eq_total = s_eq_total, eq_before = warp_eq[warp] + s_eq_front;
   // entries equal to the boundary, in index order: the j-th is kept while above + j * w* <= budget
   long long eq_kept = 0;
   if (!all_kept && eq_total > 0) {
@@ -704,13 +731,11 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     const long long k = eq_kept - seen;
     return k < 0 ? 0 : k > n_eq ? n_eq : k;
   };
-  mass_total += (u64)eq_kept * w_star;
-  mass_before += mass_front + (u64)kept_of(eq_before, 0) * w_star;
+  const u64 mass_total = s_mass_total + (u64)eq_kept * w_star;
+  const u64 mass_before = warp_mass[warp] + s_mass_front + (u64)kept_of(eq_before, 0) * w_star;
   const u64 mass_warp = w_warp + (u64)kept_of(eq_warp, eq_before) * w_star;
 
   // ---- 4. the draw: u in [0, 1) with 32 bits, target = floor(u * nucleus mass) < nucleus mass ----
-  const uint32_t r = philox_first((uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)b, (uint32_t)(b >> 32), (uint32_t)step,
-                                  (uint32_t)(step >> 32));
   const u64 target = __umul64hi(mass_total, (u64)r << 32);
   // one warp of one CTA has the target in its run; an empty nucleus (a row of NaNs) has no such warp: the first one stands in
   const bool found = mass_warp > 0 && mass_before <= target && target < mass_before + mass_warp;
@@ -773,7 +798,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
       if (nucleus_mass) nucleus_mass[b] = Z > 0 ? (float)((double)mass_total / (double)Z) : 0.f;
     }
   }
-  if (nucleus_count && tid == 0 && rank == 0) nucleus_count[b] = (int)(over_total + eq_kept);
+  if (nucleus_count && tid == 0 && rank == 0) nucleus_count[b] = (int)(s_over_total + eq_kept);
   if constexpr (kCtas > 1) cluster_barrier();   // no CTA leaves while a peer may still read its shared memory
 }
 
