@@ -54,6 +54,7 @@ struct ScanParams {
   int splits, cols;              // column runs per head, columns per run
   int consumers;                 // warps
   int ring;                      // stages
+  int per_sm;                    // CTAs per SM
   int bulk;                      // the tokens' rows can be fetched by bulk tensor copies
   int wide;                      // state rows allow accesses of four columns
 };
@@ -903,7 +904,8 @@ int launch_scan(ScanParams p, cudaStream_t stream) {
   using St = ScanStage<S, Q, KIND, DP>;
   const l3ci_recurrent_scan_args& a = p.a;
   const size_t fixed = 128 + 3 * kMaxRing * 8 + (size_t)p.consumers * kPatchBytes;
-  p.ring = (int)((max_smem_optin() - fixed) / St::bytes(p.cols));
+  const int room = p.per_sm == 2 ? (max_smem_optin() + 1024) / 2 - 1024 : max_smem_optin();   // (1 KB of every CTA is the system's)
+  p.ring = (int)((room - (long long)fixed) / St::bytes(p.cols));
   if (p.ring > kMaxRing) p.ring = kMaxRing;
   if (p.ring < 1) return fail(L3CI_ERR_UNSUPPORTED, "recurrent_scan: D=%d V=%d", a.D, a.V);
   const size_t smem = fixed + (size_t)p.ring * St::bytes(p.cols);
@@ -959,16 +961,29 @@ int scan_typed(const l3ci_recurrent_scan_args* a, cudaStream_t stream) {
   auto rows16 = [](const void* x, size_t size, int64_t st, int64_t sh) { return aligned16(x) && st > 0 && sh > 0 && (st * size) % 16 == 0 && (sh * size) % 16 == 0; };
   p.bulk = rows16(a->q, sizeof(Q), a->qk_st, a->qk_sh) && rows16(a->k, sizeof(Q), a->qk_st, a->qk_sh) && rows16(a->g, sizeof(Q), a->g_st, a->g_sh) &&
            rows16(a->v, sizeof(S), a->v_st, a->v_sh);
-  // columns per warp and warps per CTA: as many as leave enough CTAs for the device
-  // (the delta rule wants the registers, time mixing the warps)
-  const struct { int C, W; } by_kind[2][4] = {{{8, 8}, {8, 4}, {2, 8}, {2, 4}}, {{4, 16}, {4, 8}, {2, 8}, {2, 4}}};
+  // Columns per warp, warps per CTA and CTAs per SM: the least time by waves of CTAs times what a wave takes.  `cost`: 5 us for 512
+  // tokens of 128 (delta rule) and 64 (time mixing) rows, measured over 16 to 128 and 32 to 256 heads; wider CTAs take longer per
+  // token, but a second wave costs a whole pass (48 heads of the delta rule: 219 us as 96 wide CTAs, 316 as 192 narrow ones in two
+  // waves).  Two CTAs of the delta rule fit an SM with three stages each: 96 heads then take 364 us, in whole waves 431.
+  struct Form { int C, W, per_sm, cost; };
+  const Form by_kind[2][5] = {{{8, 8, 1, 44}, {8, 4, 1, 33}, {8, 4, 2, 45}, {2, 8, 1, 20}, {2, 4, 1, 15}},
+                              {{4, 16, 1, 22}, {4, 8, 1, 14}, {2, 8, 1, 9}, {2, 4, 1, 8}, {}}};
   int C = 4;
-  for (const auto& s : by_kind[KIND]) {
-    C = s.C;
-    p.consumers = s.W;
-    p.cols = C * s.W;
-    p.splits = (a->V + p.cols - 1) / p.cols;
-    if (p.cols < 2 * a->V && heads * p.splits * 5 >= 4LL * sms) break;
+  long long best = -1;
+  for (const auto& f : by_kind[KIND]) {
+    const int cols = f.C * f.W, splits = (a->V + cols - 1) / (cols ? cols : 1);
+    // (not half of a CTA idle, where a narrower one is left; registers and stages of two CTAs: up to 128 rows)
+    if (cols == 0 || (cols > 8 && cols >= 2 * a->V) || (f.per_sm == 2 && a->D > 128)) continue;
+    const long long ctas = heads * splits, wave = (long long)f.per_sm * sms, rest = ctas % wave;
+    // (of two CTAs per SM, a last wave that gives no SM two takes the time of one)
+    const long long time = ctas / wave * f.cost + (rest == 0 ? 0 : f.per_sm == 2 && rest <= sms && ctas > wave ? f.cost * 2 / 3 : f.cost);
+    if (best >= 0 && time >= best) continue;
+    best = time;
+    C = f.C;
+    p.consumers = f.W;
+    p.cols = cols;
+    p.splits = splits;
+    p.per_sm = f.per_sm;
   }
   if (heads * p.splits > 0x7fffffffLL) return fail(L3CI_ERR_INVALID, "recurrent_scan: too many sequences");
   auto on = [](const void* x, int bytes) { return (reinterpret_cast<uintptr_t>(x) & (bytes - 1)) == 0; };
