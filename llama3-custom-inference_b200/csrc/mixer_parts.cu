@@ -83,7 +83,8 @@ gated_act_kernel(const S* __restrict__ gu, S* __restrict__ out, long long units,
   load_vec<S, VEC>(gu + row * 2 * ff + c, g);
   load_vec<S, VEC>(gu + row * 2 * ff + ff + c, u);
 #pragma unroll
-  for (int i = 0; i < VEC; ++i) g[i] = gated_activation(g[i], u[i], limit, alpha);
+  for (int i = 0; i < VEC; ++i)   // (rounded to bf16 right after: the short forms of exp and the division, which leave memory the bound)
+    g[i] = sizeof(S) == 2 ? gated_activation_fast(g[i], u[i], limit, alpha) : gated_activation(g[i], u[i], limit, alpha);
   store_vec<S, VEC>(out + row * ff + c, g);
 }
 
