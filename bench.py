@@ -1025,16 +1025,16 @@ def bench_end_to_end(args, ext, pkg, dev, rank, world):
                            "repository's kernels; the decode step is replayed from a CUDA graph",
                    "reference_published_rtx4060_tokens_per_s": 2041.67},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
-                     "peak_kind": peak_kind, "kernel": "whole decode step (cuBLAS GEMMs + this library's kernels)",
+                     "peak_kind": peak_kind, "kernel": "whole decode step",
                      "algorithmic_bytes_per_launch": gen_bytes // max(1, G - 1),
                      "note": "weights once per decode step + cached K/V of the step, averaged over the generation; the time "
                              "includes the prefill pass"},
-        "launches_per_decode_step": {"this_library": 82, "detail": "33 RMSNorm (32 fused with the residual add), 16 SiLU*mul, 16 fused "
-                                     "RoPE + cache write, 16 flash-decode, 1 greedy step; plus 81 cuBLAS GEMMs and the embedding lookup"},
+        "launches_per_decode_step": {"this_library": 131, "detail": "33 RMSNorm (32 fused with the residual add), 16 fused RoPE + cache write, 16 flash-decode, "
+                                     "65 products (16 with SiLU*mul), 1 greedy step; plus the embedding lookup"},
         "e2e": e2e,
-        # per decode step: 33 RMSNorm (32 with the residual add) + 16 SiLU*mul + 16 fused RoPE/cache + 16
-        # flash-decode + 1 greedy-step launches of this library; the prefill pass has no flash-decode
-        "gpu_launches": decode_steps * 82 + steps * 65, "clocks": sampler.summary(),
+        # per decode step: 33 RMSNorm (32 with the residual add) + 16 fused RoPE/cache + 16 flash-decode + 65 products
+        # + 1 greedy-step launches of this library; the prefill pass: norms, RoPE, attention, SiLU*mul and the head's product
+        "gpu_launches": decode_steps * 131 + steps * (33 + 16 * 3 + 1), "clocks": sampler.summary(),
     }
     if cpu is not None:
         line["cpu_baseline"] = cpu
@@ -1138,8 +1138,9 @@ def bench_nibelorn(args, ext, pkg, dev, rank, world):
                    "global_batch": 64 * world, "seq_len": 1024, "parallelism": "replicas x%d" % world,
                    "l2": "weights and cache of a step exceed L2"},
         "kernels": mixer_kernel_table(ext, pkg, dev, latent, differential) if rank == 0 else None,
-        # embedding, 16 x (cache write, attention, two norms, gelu), token choice; the split merges come on top
-        "gpu_launches": line["steps"] * (1 + 16 * 5 + 1),
+        # embedding, 16 x (cache write, attention, two norms), products: 8 x (6 + 4) and the head, token choice; the split merges
+        # come on top
+        "gpu_launches": line["steps"] * (1 + 16 * 4 + 8 * 10 + 1 + 1),
     }
 
 
@@ -1173,9 +1174,10 @@ def bench_rupotar(args, ext, pkg, dev, rank, world):
                    "global_batch": 64 * world, "seq_len": 1024, "parallelism": "replicas x%d" % world,
                    "l2": "weights and cache of a step exceed L2"},
         "kernels": rupotar_kernel_table(ext, pkg, dev, cfg) if rank == 0 else None,
-        # per step: embedding, token choice; per run two norms; per attention two (split merges on top), delta two, time mixing three
-        # (token shift, tanh, step); per dense one, experts four; per pass of the loop one more norm
-        "gpu_launches": line["steps"] * (2 + 16 * 2 + 8 * 2 + 4 * 2 + 4 * 3 + 8 * 1 + 8 * 4 + 2),
+        # per step: embedding, token choice; per run two norms; per attention two (split merges on top), delta two, time mixing two
+        # (token shift, step); experts four; per pass of the loop one more norm; products: 8 x 2 of attention, 4 x 3 of the delta
+        # rule, 4 x 4 of time mixing, 8 x 2 dense, 8 routers, 2 of the loop, the head
+        "gpu_launches": line["steps"] * (2 + 16 * 2 + 8 * 2 + 4 * 2 + 4 * 2 + 8 * 4 + 2 + 8 * 2 + 4 * 3 + 4 * 4 + 8 * 2 + 8 + 2 + 1),
     }
 
 

@@ -6,7 +6,7 @@
 // every entry whose PRECEDING mass exceeds p, renormalises, draws with torch.multinomial and maps the draw back
 // through the sort permutation: half a dozen full-vocabulary kernels per generated token.  The nucleus does not need
 // the order, only its boundary: entry i is kept iff the mass of the entries that sort strictly before it is <= p.
-// Here row b's CTA
+// Here row b's CTA (top_p_step_kernel)
 //   1. reduces (max, sum of exp) online in one pass over the row,
 //   2. finds the boundary of the nucleus by a two-level search over the bit pattern of the bf16 LOGITS (the weight
 //      e_i = exp((x_i - max) / T) is monotone in the logit, and a bf16 logit has only 65 536 patterns): each level
@@ -18,6 +18,7 @@
 //      where the running mass passes u * nucleus mass.  Any fixed order gives the multinomial distribution; index
 //      order needs no permutation.
 // Batches of up to half the SMs run as a cluster of two CTAs per row (see peer_value below).
+// Rows of up to 8 x 65 528 logits take the same steps by counts of keys instead of masses (top_p_count_kernel below), the longer ones these.
 // It then writes the token exactly as l3ci_greedy_step does.  Weights are recomputed from the logits in every pass
 // (same expression, same bits; the row is 256 KB and stays in L2), nothing is sorted and nothing leaves the SM.
 #include <cuda_bf16.h>
