@@ -228,8 +228,9 @@ flash_decode_small_kernel(const SmallParams p) {
   uint32_t cta_rank = 0;
   if constexpr (kCluster) cta_rank = cluster_cta_rank();
   const int n_units = p.B * p.Hkv;
-  pdl_launch_dependents();  // the next one may be set up while this one runs
+  // (waits first: calls back to back lost 1 % to CTAs of the next one that came early, 20.95 -> 21.19 us at 16 ragged sequences of 2048)
   pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
+  pdl_launch_dependents();  // the next one may be set up while this one runs
   const int unit0 = (int)(blockIdx.x >> lgC) * U;   // first unit of this CTA (of this cluster)
   const int unit = unit0 + (kWholeCta ? 0 : warp >> lgW);
   const bool has_unit = unit < n_units;
