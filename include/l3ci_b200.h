@@ -111,6 +111,10 @@ typedef struct l3ci_linear_args {
   l3ci_stream_t stream;
 } l3ci_linear_args;
 L3CI_API int l3ci_linear(const l3ci_linear_args* args);
+/* Elements between the rows of a tensor of these sizes and strides (in elements), all axes but the last counted as one axis of
+ * rows; the width where there is at most one row.  -1 where no one stride gives the rows (a broadcast axis, axes that do not
+ * follow one another), where rows overlap, or where the last axis is not contiguous.  Host only. */
+L3CI_API int64_t l3ci_row_stride(const int64_t* sizes, const int64_t* strides, int32_t dims);
 
 /* Greedy decode step: for every row b of bf16 logits [rows, vocab] (row_stride elements apart),
  *   tok = argmax (ties: smallest index, as torch.argmax; NaN counts as the maximum);

@@ -19,7 +19,7 @@ OK, ERR_INVALID, ERR_UNSUPPORTED, ERR_ALIGNMENT, ERR_SCRATCH, ERR_CUDA, ERR_DEVI
 # Every symbol include/l3ci_b200.h declares.
 EXPORTS = (
     "l3ci_status_string", "l3ci_last_error", "l3ci_version", "l3ci_set_device_wait_limit_ns", "l3ci_set_programmatic_launch",
-    "l3ci_rms_norm", "l3ci_add_rms_norm", "l3ci_silu_mul", "l3ci_linear", "l3ci_greedy_step", "l3ci_top_p_step", "l3ci_rot_embed", "l3ci_rot_embed_kv_cache", "l3ci_rot_embed_kv_cache_at",
+    "l3ci_rms_norm", "l3ci_add_rms_norm", "l3ci_silu_mul", "l3ci_linear", "l3ci_row_stride", "l3ci_greedy_step", "l3ci_top_p_step", "l3ci_rot_embed", "l3ci_rot_embed_kv_cache", "l3ci_rot_embed_kv_cache_at",
     "l3ci_flash_decode_scratch_bytes", "l3ci_flash_decode", "l3ci_flash_decode_static", "l3ci_flash_decode_poll",
     "l3ci_flash_decode_kernel_choice",
     "l3ci_lse_merge", "l3ci_lse_exchange_bytes", "l3ci_lse_exchange_merge", "l3ci_prefill_attention",
@@ -104,6 +104,8 @@ def load() -> C.CDLL:
     lib.l3ci_silu_mul.argtypes = [vp, vp, vp, i64, i64, i64, i64, vp]
     lib.l3ci_linear.restype = C.c_int
     lib.l3ci_linear.argtypes = [C.POINTER(LinearArgs)]
+    lib.l3ci_row_stride.restype = i64
+    lib.l3ci_row_stride.argtypes = [C.POINTER(i64), C.POINTER(i64), i32]
     lib.l3ci_prefill_attention.restype = C.c_int
     lib.l3ci_prefill_attention.argtypes = [C.POINTER(PrefillArgs)]
     lib.l3ci_greedy_step.restype = C.c_int
@@ -187,18 +189,11 @@ def add_rms_norm(x, residual, weight, eps: float):
     return s, out
 
 
-def _row_stride(x, width: int):
-    """Elements between the rows of x [..., width], its leading axes counted as one; None if no one stride fits."""
-    stride, reach = None, 0
-    for n, st in zip(reversed(x.shape[:-1]), reversed(x.stride()[:-1])):
-        if n == 1:
-            continue
-        if stride is None:
-            stride = st
-        elif st != reach:
-            return None
-        reach = st * n
-    return width if stride is None else stride
+def _row_stride(x):
+    """Elements between the rows of x [..., width], its leading axes counted as one; None if no one stride fits (l3ci_row_stride)."""
+    n = x.dim()
+    stride = load().l3ci_row_stride((C.c_int64 * n)(*x.shape), (C.c_int64 * n)(*x.stride()), n)
+    return None if stride < 0 else stride
 
 
 def linear_args(x, w, act: int = ACT_NONE, out_dtype=None, split: int = 0, status=None, early: bool = False, out=None):
@@ -210,7 +205,7 @@ def linear_args(x, w, act: int = ACT_NONE, out_dtype=None, split: int = 0, statu
     if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and w.device == x.device and w.is_contiguous()):
         return None, None
     K, grouped = x.shape[-1], w.dim() == 3
-    if w.dim() not in (2, 3) or w.shape[-1] != K or K == 0 or K % 8 or x.stride(-1) != 1 or (grouped and (x.dim() != 3 or x.shape[0] != w.shape[0])):
+    if w.dim() not in (2, 3) or w.shape[-1] != K or K == 0 or K % 8 or (grouped and (x.dim() != 3 or x.shape[0] != w.shape[0])):
         return None, None
     groups = w.shape[0] if grouped else 1
     N, rows = w.shape[-2], x.numel() // (K * max(1, groups))
@@ -219,14 +214,14 @@ def linear_args(x, w, act: int = ACT_NONE, out_dtype=None, split: int = 0, statu
             return None, None
         N //= 2
     one = x[0] if grouped and groups else x
-    stride, group_stride = _row_stride(one, K), x.stride(0) if grouped else 0
+    stride, group_stride = _row_stride(one), x.stride(0) if grouped else 0
     if not 0 < rows <= LINEAR_MAX_ROWS or N == 0 or groups == 0 or stride is None:
         return None, None
-    if stride % 8 or group_stride % 8 or (rows > 1 and stride < K and not grouped) or x.data_ptr() % 16 or w.data_ptr() % 16:
+    if stride % 8 or group_stride % 8 or x.data_ptr() % 16 or w.data_ptr() % 16:
         return None, None
     if out is None:
         out = torch.empty(*x.shape[:-1], N, dtype=out_dtype or x.dtype, device=x.device)
-    out_stride = _row_stride(out[0] if grouped else out, N)
+    out_stride = _row_stride(out[0] if grouped else out)
     a = LinearArgs(x=x.data_ptr(), w=w.data_ptr(), out=out.data_ptr(), status=None if status is None else status.data_ptr(), rows=rows, x_st=stride,
                    out_st=out_stride, x_sg=group_stride, out_sg=out.stride(0) if grouped else 0, K=K, N=N, groups=groups, act=act,
                    out_f32=int(out.dtype == torch.float32), split=split, early=int(early), stream=_stream(x))

@@ -364,6 +364,24 @@ int launch_split(const l3ci_linear_args* a, cudaStream_t stream) {
 }  // namespace
 }  // namespace l3ci
 
+extern "C" int64_t l3ci_row_stride(const int64_t* sizes, const int64_t* strides, int32_t dims) {
+  if (dims < 1) return -1;
+  const int64_t width = sizes[dims - 1];
+  if (strides[dims - 1] != 1 && width > 1) return -1;
+  int64_t stride = -1, reach = 0;          // of the axes seen so far: none yet
+  for (int d = dims - 2; d >= 0; --d) {
+    if (sizes[d] == 1) continue;
+    if (stride < 0) {
+      stride = strides[d];
+      if (stride < width) return -1;       // a broadcast axis among them
+    } else if (strides[d] != reach) {
+      return -1;
+    }
+    reach = strides[d] * sizes[d];
+  }
+  return stride < 0 ? width : stride;
+}
+
 extern "C" int l3ci_linear(const l3ci_linear_args* a) {
   using namespace l3ci;
   clear_error();

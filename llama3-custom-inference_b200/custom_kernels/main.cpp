@@ -348,17 +348,9 @@ Tensor linear(Tensor x, Tensor w, bool gated) {
   TORCH_CHECK(!gated || w.size(0) % 2 == 0, "a gated product takes an even number of rows of w");
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t K = x.size(-1), N = gated ? w.size(0) / 2 : w.size(0), rows = K ? x.numel() / K : 0;
-  // one row stride for all leading axes
-  int64_t stride = K, reach = 0;
-  bool regular = x.stride(-1) == 1;
-  for (int64_t d = x.dim() - 2; d >= 0; --d) {
-    if (x.size(d) == 1) continue;
-    if (reach == 0) stride = x.stride(d);
-    else regular = regular && x.stride(d) == reach;
-    reach = x.stride(d) * x.size(d);
-  }
+  const int64_t stride = l3ci_row_stride(x.sizes().data(), x.strides().data(), (int32_t)x.dim());
   auto at16 = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; };
-  if (regular && rows > 0 && rows <= L3CI_LINEAR_MAX_ROWS && N > 0 && K % 8 == 0 && stride % 8 == 0 && stride >= K && w.is_contiguous() &&
+  if (stride > 0 && stride % 8 == 0 && rows > 0 && rows <= L3CI_LINEAR_MAX_ROWS && N > 0 && K % 8 == 0 && w.is_contiguous() &&
       K <= INT32_MAX && w.size(0) <= INT32_MAX && at16(x) && at16(w)) {
     auto sizes = x.sizes().vec();
     sizes.back() = N;

@@ -87,3 +87,28 @@ def test_groups_of_products(capi, device, rows, groups, K, N):
     out = torch.empty(rows, groups, N, dtype=torch.bfloat16, device=device).transpose(0, 1)
     assert capi.linear(x.contiguous(), w, out=out) is out
     _check(out, want, K, False)
+
+
+def _ext_want(x, w, gated):
+    y = x.double() @ w.double().T
+    n = w.shape[0] // 2
+    return y[..., :n] * torch.sigmoid(y[..., :n]) * y[..., n:] if gated else y
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_extension_takes_any_layout_of_its_input(ext, device, gated):
+    """Broadcast, strided and ragged inputs: what one row stride describes goes to the kernel, the rest to torch's product."""
+    g = torch.Generator(device=device).manual_seed(3)
+    K = 64
+    w = (torch.randn(96, K, generator=g, device=device) / 8).bfloat16()
+    base = torch.randn(2, K, generator=g, device=device).bfloat16()
+    big = torch.randn(5, 3, 160, generator=g, device=device).bfloat16()
+    many = torch.randn(70, K, generator=g, device=device).bfloat16()
+    for x in (base[:, None].expand(2, 3, K), base[None].expand(3, 2, K), base[:1].expand(5, K), base[:, None, None].expand(2, 2, 3, K), base[0],
+              big[:, -1, 8:72], big[:, :, 16:80], big[:, :2, :K], big[:, :, 4:68], big.transpose(0, 1)[..., :K], big[:1, :, :K], many, many[:65],
+              many[:64], base.t().contiguous().t(), many.as_strided((4, K), (8, 1))):
+        got = ext.linear(x, w, gated=gated)
+        want = _ext_want(x, w, gated)
+        assert got.shape == want.shape
+        # as in _check; above 64 rows the gate and the up row are rounded to bf16 before their product, and so is silu(gate): 3 x 2^-9
+        assert bool(((got.double() - want).abs() <= 2.0 ** -6 * want.abs() + 2.0 ** -9).all())
