@@ -337,10 +337,10 @@ Tensor silu_mul(Tensor gate, Tensor up) {
   return out;
 }
 
-// act(x w^T): few rows in one kernel (l3ci_linear; the weights are read ahead of the stream's previous kernels: w must not
-// be written by kernels of the same forward pass), more in torch's product and, gated, silu_mul.  `gated`: w holds gate
-// rows, then up rows, and the result is silu(gate) * up.
-Tensor linear(Tensor x, Tensor w, bool gated) {
+// act(x w^T): few rows in one kernel (l3ci_linear), more in torch's product and, gated, silu_mul.  `gated`: w holds gate
+// rows, then up rows, and the result is silu(gate) * up.  `early`: the kernel may read w ahead of the stream's previous
+// kernels; for a w that was complete before the last one of them that waits for its predecessors ahead of letting others start.
+Tensor linear(Tensor x, Tensor w, bool gated, bool early) {
   check_bf16_cuda(x, "x");
   check_bf16_cuda(w, "w");
   TORCH_CHECK(x.dim() >= 1 && w.dim() == 2 && w.size(1) == x.size(-1), "w must be [N, K] with K the last axis of x");
@@ -360,7 +360,7 @@ Tensor linear(Tensor x, Tensor w, bool gated) {
     a.rows = rows; a.x_st = stride; a.out_st = N;
     a.K = (int32_t)K; a.N = (int32_t)N; a.groups = 1;
     a.act = gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE;
-    a.early = 1;
+    a.early = early;
     a.stream = current_stream();
     check_status(l3ci_linear(&a), "linear");
     return out;
@@ -521,7 +521,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_rms_norm", torch::wrap_pybind_function(add_rms_norm), "add_rms_norm", py::arg("x"), py::arg("residual"),
         py::arg("weight"), py::arg("eps"));
   m.def("silu_mul", torch::wrap_pybind_function(silu_mul), "silu_mul", py::arg("gate"), py::arg("up"));
-  m.def("linear", torch::wrap_pybind_function(linear), "linear", py::arg("x"), py::arg("w"), py::arg("gated") = false);
+  m.def("linear", torch::wrap_pybind_function(linear), "linear", py::arg("x"), py::arg("w"), py::arg("gated") = false,
+        py::arg("early") = false);
   m.def("greedy_step", torch::wrap_pybind_function(greedy_step), "greedy_step", py::arg("logits"), py::arg("out_tokens"),
         py::arg("steps"), py::arg("next_input"), py::arg("positions"), py::arg("seq_lens"));
   m.def("top_p_step", torch::wrap_pybind_function(top_p_step), "top_p_step", py::arg("logits"), py::arg("out_tokens"),

@@ -28,6 +28,7 @@ from __future__ import annotations
 
 from contextlib import contextmanager
 from dataclasses import dataclass
+from functools import partial
 from typing import Optional
 
 import torch
@@ -275,7 +276,7 @@ class Llama3Decoder(DecodeLoop):
             p = f"h{l}."
             cache_k, cache_v = self.cache_k[l][slots], self.cache_v[l][slots]
             _nvtx_push("layer")
-            qkv = ext.linear(h, w[p + "attn"])                                         # model.py:95
+            qkv = ext.linear(h, w[p + "attn"], early=True)                             # model.py:95
             _nvtx_push("rot_embd")
             _nvtx_push("use_kv")
             q = ext.rot_embed_kv_cache(qkv, self.freqs, cache_k, cache_v, 0, Hq, Hkv,
@@ -292,15 +293,16 @@ class Llama3Decoder(DecodeLoop):
                                                cache_v.transpose(1, 2), seq_lens=seq_lens,
                                                max_ctas=self._decode_kernel(B))     # model.py:118
             y = y.transpose(1, 2).reshape(B, T, E)                                     # model.py:120
-            x, h = ext.add_rms_norm(ext.linear(y, w[p + "proj"]), x, w[p + "ln_2"], cfg.norm_eps)  # :121, 147-148
-            m = ext.linear(ext.linear(h, w[p + "gate_up"], gated=True), w[p + "mlp_proj"])   # c_fc2 | c_fc, model.py:134
+            x, h = ext.add_rms_norm(ext.linear(y, w[p + "proj"], early=True), x, w[p + "ln_2"], cfg.norm_eps)  # :121, 147-148
+            a = ext.linear(h, w[p + "gate_up"], gated=True, early=True)                # c_fc2 | c_fc, model.py:134
+            m = ext.linear(a, w[p + "mlp_proj"], early=True)
             nxt = w[f"h{l + 1}.ln_1"] if l + 1 < cfg.n_layer else w["ln_f"]
             x, h = ext.add_rms_norm(m, x, nxt, cfg.norm_eps)                           # model.py:148, next 147 / 217
             _nvtx_pop()
         # the reference widens the logits to fp32 first (model.py:226); the widening is monotonic, so the argmax
         # of the bf16 values is the same index
         # model.py:225; the head is tied to the embedding (model.py:189) unless the checkpoint brought its own
-        return self.logits(h, w.get("lm_head", w["wte"]), want, ext.linear)
+        return self.logits(h, w.get("lm_head", w["wte"]), want, partial(ext.linear, early=True))
 
 
 def config_from_hf(hf_config) -> DecoderConfig:

@@ -124,30 +124,31 @@ def _cuda(*tensors):
             raise ValueError("the mixer kernels take CUDA tensors: there is no CPU path")
 
 
-def few_rows(x, w, act: int = ACT_NONE, out_dtype=None, out=None):
+def few_rows(x, w, act: int = ACT_NONE, out_dtype=None, out=None, early: bool = False):
     """act(x w^T) of few rows in one kernel (`l3ci_linear`), groups of products where w is [groups, N, K]; None where it does
-    not apply.  w, the model's, is read ahead of the stream's previous kernels."""
-    a, out = linear_args(x, w, act, out_dtype, early=True, out=out)
+    not apply.  `early`: w may be read ahead of the stream's previous kernels; for weights that were complete before the last one
+    of them that waits for its predecessors ahead of letting others start (a model's, in its forward pass)."""
+    a, out = linear_args(x, w, act, out_dtype, early=early, out=out)
     if a is not None:
         with _on(x):
             _check(load().l3ci_linear(C.byref(a)), "l3ci_linear")
     return out
 
 
-def linear(x, w, act: int = ACT_NONE):
-    """act(x w^T); ACT_SILU_GATE: w holds gate rows, then up rows."""
-    y = few_rows(x, w, act)
+def linear(x, w, act: int = ACT_NONE, early: bool = False):
+    """act(x w^T); ACT_SILU_GATE: w holds gate rows, then up rows.  `early`: see `few_rows`."""
+    y = few_rows(x, w, act, early=early)
     if y is not None:
         return y
     y = F.linear(x, w)
     return y if act == ACT_NONE else gelu_(y) if act == ACT_GELU else tanh_(y) if act == ACT_TANH else gated_act(y)
 
 
-def product32(x, w):
-    """x [rows, K] w^T in fp32: products of two bf16 numbers are exact, the sum is not rounded to bf16."""
+def product32(x, w, early: bool = False):
+    """x [rows, K] w^T in fp32: products of two bf16 numbers are exact, the sum is not rounded to bf16.  `early`: see `few_rows`."""
     if x.dtype == torch.float32:
         return torch.mm(x, w.t())
-    y = few_rows(x, w, out_dtype=torch.float32)
+    y = few_rows(x, w, out_dtype=torch.float32, early=early)
     return torch.mm(x, w.t(), out_dtype=torch.float32) if y is None else y
 
 

@@ -16,6 +16,7 @@ those of the experts are kernels of their own, the others torch's (cuBLAS).
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import partial
 from typing import Optional
 
 import torch
@@ -23,6 +24,11 @@ import torch
 from . import mixers
 from .decode_loop import DecodeLoop, full_precision_products, nvtx_range
 from .kv_cache import State
+
+# Products with the model's own weights, complete before a forward pass, whose first kernel waits ahead of letting others start.
+_linear = partial(mixers.linear, early=True)
+_few_rows = partial(mixers.few_rows, early=True)
+_product32 = partial(mixers.product32, early=True)
 
 POSITION_BASE = 10000.0     # sinusoidal positions
 SLOPE_RANGE = 8.0           # head h of H takes 2^(-8 (h + 1) / H) off a score per position of distance
@@ -319,7 +325,7 @@ class RupotarDecoder(DecodeLoop):
     def _attention(self, m: Attention, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, _ = h.shape
         qw, kw = m.heads * m.dim, m.kv_heads * m.dim
-        qkv = mixers.linear(h, w.proj)
+        qkv = _linear(h, w.proj)
         k, v = planes["k"], planes["v"]
         mixers.qk_norm_cache(qkv, qw, kw, w.q_norm, w.k_norm, self.cfg.eps, k, v, positions)
         out = torch.empty(B, T, m.heads, m.vdim, dtype=h.dtype, device=h.device)
@@ -330,9 +336,9 @@ class RupotarDecoder(DecodeLoop):
     def _channel_delta(self, m: ChannelDelta, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, E = h.shape
         H, G, D, V = m.heads, m.kv_heads, m.dim, m.vdim
-        p = mixers.linear(h, w.proj)
+        p = _linear(h, w.proj)
         low = p.view(B * T, -1)[:, w.at_low:]
-        up = mixers.linear(low, w.up).view(B, T, -1)
+        up = _linear(low, w.up).view(B, T, -1)
         qk, v, beta, decay = mixers.delta_inputs(p, p[..., w.at_b:w.at_b + H], up[..., :H * D], w.conv, w.a_log, w.dt_bias, planes["tail"],
                                                  positions, H, G, D, V, UNIT_EPS)
         gate = up[..., w.at_gate:w.at_gate + H * V].view(B, T, H, V)
@@ -342,20 +348,20 @@ class RupotarDecoder(DecodeLoop):
     def _wkv(self, m: TimeMix, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, E = h.shape
         mixes = mixers.token_shift(h, w.mu, planes["last"], positions).view(len(MIXES), B * T, E)
-        rkvg = mixers.few_rows(mixes[:4], w.rkvg)
+        rkvg = _few_rows(mixes[:4], w.rkvg)
         if rkvg is None:
             rkvg = torch.bmm(mixes[:4], w.rkvg.transpose(1, 2))
         r, k, v, g = rkvg.view(4, B, T, m.heads, m.dim)
-        decay = mixers.linear(mixers.linear(mixes[4], w.w1, mixers.ACT_TANH), w.w2).view(B, T, m.heads, m.dim)
+        decay = _linear(_linear(mixes[4], w.w1, mixers.ACT_TANH), w.w2).view(B, T, m.heads, m.dim)
         return mixers.recurrent_scan(r, k, v, decay, planes["state"], positions, w.norm, g, act=mixers.SILU, eps=self.cfg.eps, bonus=w.u,
                                      g_bias=w.w0)
 
     # ---- feed-forward: what `residual_norm` adds ---------------------------------------------------------------
     def _feed_forward(self, ff, w: _LayerWeights, h):
         if isinstance(ff, Dense):
-            return {"y": mixers.linear(mixers.linear(h, w.gate_up, mixers.ACT_SILU_GATE), w.down)}
+            return {"y": _linear(_linear(h, w.gate_up, mixers.ACT_SILU_GATE), w.down)}
         rows = h.view(-1, h.shape[-1])
-        experts, ranks, weights, counts = mixers.moe_route(mixers.product32(rows, w.router), w.router_b, ff.top)
+        experts, ranks, weights, counts = mixers.moe_route(_product32(rows, w.router), w.router_b, ff.top)
         x, part_rows = mixers.moe_gather(rows, experts, ranks, counts)
         a = mixers.moe_gemm(x, w.gate_up, counts, limit=ff.limit, alpha=EXPERT_ALPHA)
         return {"y": mixers.moe_gemm(a, w.down, counts), "part_rows": part_rows, "part_weights": weights}
@@ -389,13 +395,13 @@ class RupotarDecoder(DecodeLoop):
                 mix = self._attention if isinstance(m, Attention) else self._channel_delta if isinstance(m, ChannelDelta) else self._wkv
                 with nvtx_range("layer"):
                     if run.step is not None:
-                        h = mixers.residual_norm(mixers.product32(cat.view(B * T, 2 * E), self.loop_in), x, dtype=self.dtype, reset=True, step=self.loop_step[run.step],
+                        h = mixers.residual_norm(_product32(cat.view(B * T, 2 * E), self.loop_in), x, dtype=self.dtype, reset=True, step=self.loop_step[run.step],
                                                  pre=w.norm1, eps=eps)
-                    added, post = {"y": mixers.linear(mix(m, w, planes, h, positions, start_pos), w.o)}, w.norm1b
+                    added, post = {"y": _linear(mix(m, w, planes, h, positions, start_pos), w.o)}, w.norm1b
                     if ff is not None:
                         h = mixers.residual_norm(**added, x=x, dtype=self.dtype, post=post, pre=w.norm2, eps=eps)
                         added, post = self._feed_forward(ff, w, h), w.norm2b
                     h = mixers.residual_norm(**added, x=x, dtype=self.dtype, post=post, eps=eps, **before(r + 1))
                     if keep is not None:
                         keep.append(x.clone())
-            return self.logits(h, self.head, want, mixers.linear)
+            return self.logits(h, self.head, want, _linear)

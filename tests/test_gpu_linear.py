@@ -112,3 +112,29 @@ def test_extension_takes_any_layout_of_its_input(ext, device, gated):
         assert got.shape == want.shape
         # as in _check; above 64 rows the gate and the up row are rounded to bf16 before their product, and so is silu(gate): 3 x 2^-9
         assert bool(((got.double() - want).abs() <= 2.0 ** -6 * want.abs() + 2.0 ** -9).all())
+
+
+def _burst(ext, device, make):
+    """Products with weights that the kernel right in front writes, against the same products with the device idle between the two."""
+    g = torch.Generator(device=device).manual_seed(8)
+    x = torch.randn(8, 2048, generator=g, device=device).bfloat16()
+    ins = [torch.randn(2, 4096, 2048, generator=g, device=device).bfloat16() for _ in range(4)]
+    want = []
+    for a in ins:
+        w = make(a)
+        torch.cuda.synchronize()
+        want.append(ext.linear(x, w))
+        torch.cuda.synchronize()
+    for _ in range(5):
+        got = [ext.linear(x, make(a)) for a in ins]
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+
+
+def test_weights_written_by_the_kernel_in_front(ext, device):
+    """`early` is off unless asked for: the weights may be the result of the launch before."""
+    ones = torch.ones(2048, dtype=torch.bfloat16, device=device)
+    _burst(ext, device, lambda a: ext.silu_mul(a[0], a[1]))
+    _burst(ext, device, lambda a: ext.rms_norm(a[0], ones, 1e-5))
+    _burst(ext, device, lambda a: ext.linear(a[0][:64], a[1][:2048]))
+    _burst(ext, device, lambda a: a[0].clone().mul_(0.5))
