@@ -25,10 +25,10 @@ def _check(got, want, K, f32):
     assert bool((err <= bound).all()), f"largest excess {(err - bound).max().item():.3g}"
 
 
-# rows: the edges of the 16-, 32- and 64-column forms; K: one 8-column vector, ends inside a stage, more stages than the ring
+# rows: the edges of the 8-, 16-, 32- and 64-column forms; K: one 8-column vector, ends inside a stage, more stages than the ring
 # has; N: inside a tile, whole tiles and one row behind them, more tiles than CTAs
 @pytest.mark.parametrize("split", [0, 1, 2, 4, 8])
-@pytest.mark.parametrize("rows,K,N", [(1, 8, 1), (1, 2048, 4), (2, 72, 128), (16, 1000, 129), (17, 2048, 300), (32, 4096, 64), (33, 520, 1025),
+@pytest.mark.parametrize("rows,K,N", [(1, 8, 1), (1, 2048, 4), (2, 72, 128), (8, 2048, 300), (9, 136, 129), (16, 1000, 129), (17, 2048, 300), (32, 4096, 64), (33, 520, 1025),
                                       (64, 2048, 2048), (7, 136, 40000)])
 @pytest.mark.parametrize("act", [0, 1, 2, 3])
 def test_products_of_few_rows(capi, device, rows, K, N, act, split):
@@ -56,25 +56,36 @@ def test_rows_with_a_stride_and_what_does_not_apply(capi, device):
     assert capi.linear(big[..., :64], w[:, ::2]) is None and capi.linear(big[..., :64], w.float()) is None
 
 
-def test_chain_of_products_under_programmatic_launch(capi, device):
-    """Each product reads what the one before wrote, while its own weights were asked for early."""
+@pytest.mark.parametrize("split", [0, 1, 2, 4, 8])
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 33, 64])
+def test_chain_of_products_under_programmatic_launch(capi, device, rows, gated, split):
+    """Each product reads what the one before wrote, while its own weights were asked for ahead of it: the bits of plain launches,
+    and within the bound of the sums of fp64."""
     g = torch.Generator(device=device).manual_seed(11)
-    sizes = [(2048, 2048), (3072, 2048), (2048, 3072), (512, 2048), (2048, 512)] * 4
-    ws = [(torch.randn(n, k, generator=g, device=device) * k ** -0.5).bfloat16() for n, k in sizes]
-    x0 = torch.randn(8, 2048, generator=g, device=device).bfloat16()
+    sizes = [(2048, 2048), (3072, 2048), (2048, 3072), (520, 2048), (2048, 520)] * 2
+    act, n = (capi.ACT_SILU_GATE, 2) if gated else (capi.ACT_NONE, 1)
+    ws = [(torch.randn(n * N, K, generator=g, device=device) * K ** -0.5).bfloat16() for N, K in sizes]
+    x0 = torch.randn(rows, 2048, generator=g, device=device).bfloat16()
 
     def chain():
-        x = x0
+        xs = [x0]
         for w in ws:
-            x = capi.linear(x, w)
-        return x
+            xs.append(capi.linear(xs[-1], w, act, split=split, early=True))
+        return xs
 
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    torch.cuda.synchronize()                         # the weights are complete: they may be read ahead of the stream
     with capi.programmatic_launch(False):
         want = chain()
     torch.cuda.synchronize()
+    for x, w in zip(want, ws):
+        _check(capi.linear(x, w, act, split=split, status=status), _want(x, w, act, capi), x.shape[1], False)
+    assert status.item() == 0
     with capi.programmatic_launch(True):
         for _ in range(5):
-            assert torch.equal(chain(), want)
+            for a, b in zip(chain(), want):
+                assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("rows,groups,K,N", [(1, 4, 256, 256), (8, 16, 128, 512), (33, 3, 72, 130), (64, 16, 512, 128)])
