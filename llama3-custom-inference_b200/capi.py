@@ -199,9 +199,11 @@ def _row_stride(x):
 def linear_args(x, w, act: int = ACT_NONE, out_dtype=None, split: int = 0, status=None, early: bool = False, out=None):
     """Arguments of `l3ci_linear` and the tensor that it fills: x [..., K] and w [N, K] (gated: [2 N, K]), or groups of
     products, x [groups, rows, K] and w [groups, N, K].  (None, None) where the call does not apply: more rows than it takes,
-    other types, layouts or alignments.  `out`: where the result goes, the last axis contiguous."""
+    other types, layouts or alignments.  `out`: where the result goes, bf16 or fp32 rows [..., N] at one stride."""
     import torch
 
+    if (out_dtype if out is None else out.dtype) not in (None, torch.bfloat16, torch.float32):
+        raise ValueError("linear: the result is bf16 or fp32")
     if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and w.device == x.device and w.is_contiguous()):
         return None, None
     K, grouped = x.shape[-1], w.dim() == 3
@@ -217,11 +219,13 @@ def linear_args(x, w, act: int = ACT_NONE, out_dtype=None, split: int = 0, statu
     stride, group_stride = _row_stride(one), x.stride(0) if grouped else 0
     if not 0 < rows <= LINEAR_MAX_ROWS or N == 0 or groups == 0 or stride is None:
         return None, None
-    if stride % 8 or group_stride % 8 or x.data_ptr() % 16 or w.data_ptr() % 16:
+    if stride % 8 or group_stride % 8 or (groups > 1 and group_stride <= 0) or x.data_ptr() % 16 or w.data_ptr() % 16:
         return None, None
     if out is None:
         out = torch.empty(*x.shape[:-1], N, dtype=out_dtype or x.dtype, device=x.device)
     out_stride = _row_stride(out[0] if grouped else out)
+    if out.shape != (*x.shape[:-1], N) or out.device != x.device or out_stride is None or (groups > 1 and out.stride(0) <= 0):
+        raise ValueError("linear: the result's shape, device or strides")
     a = LinearArgs(x=x.data_ptr(), w=w.data_ptr(), out=out.data_ptr(), status=None if status is None else status.data_ptr(), rows=rows, x_st=stride,
                    out_st=out_stride, x_sg=group_stride, out_sg=out.stride(0) if grouped else 0, K=K, N=N, groups=groups, act=act,
                    out_f32=int(out.dtype == torch.float32), split=split, early=int(early), stream=_stream(x))

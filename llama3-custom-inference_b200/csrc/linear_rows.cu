@@ -395,7 +395,8 @@ extern "C" int l3ci_linear(const l3ci_linear_args* a) {
   if (a->K % 8 || a->x_st % 8 || a->x_sg % 8 || !aligned16(a->x) || !aligned16(a->w))
     return fail(L3CI_ERR_ALIGNMENT, "linear: rows of x and w must be whole 16-byte vectors");
   if (a->rows > 1 && a->out_st < a->N && (a->groups == 1 || a->out_sg < a->N)) return fail(L3CI_ERR_INVALID, "linear: rows of the result overlap");
-  if (a->x_st < 0 || a->x_sg < 0) return fail(L3CI_ERR_INVALID, "linear: negative stride");
+  if ((a->rows > 1 && a->x_st <= 0) || (a->groups > 1 && (a->x_sg <= 0 || a->out_sg <= 0)))
+    return fail(L3CI_ERR_INVALID, "linear: rows or groups without a stride of their own");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(a->stream);
   const bool gated = a->act == L3CI_ACT_SILU_GATE;
   if (a->rows <= 8) return gated ? launch_split<8, true>(a, s) : launch_split<8, false>(a, s);

@@ -106,3 +106,17 @@ def test_programmatic_launch_switch_round_trips(capi):
     with capi.programmatic_launch(False):
         assert lib.l3ci_set_programmatic_launch(0) == 0
     assert lib.l3ci_set_programmatic_launch(prev) == prev
+
+
+def test_products_without_strides_of_their_own_are_refused(capi):
+    lib = capi.load()
+
+    def args(**kw):
+        a = capi.LinearArgs(x=0x1000, w=0x1000, out=0x1000, rows=2, x_st=64, out_st=8, x_sg=128, out_sg=16, K=64, N=8, groups=2)
+        for k, v in kw.items():
+            setattr(a, k, v)
+        return lib.l3ci_linear(C.byref(a))
+
+    for bad in ({"x_sg": 0}, {"x_st": 0}, {"x_sg": -128}, {"x_st": -64}, {"out_sg": 0}, {"out_sg": -16}, {"groups": 1, "x_st": 0}):
+        assert args(**bad) == capi.ERR_INVALID, bad
+    assert args(rows=0) == args(groups=0) == args(N=0) == capi.OK

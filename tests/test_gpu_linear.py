@@ -149,3 +149,23 @@ def test_weights_written_by_the_kernel_in_front(ext, device):
     _burst(ext, device, lambda a: ext.rms_norm(a[0], ones, 1e-5))
     _burst(ext, device, lambda a: ext.linear(a[0][:64], a[1][:2048]))
     _burst(ext, device, lambda a: a[0].clone().mul_(0.5))
+
+
+def test_results_of_other_types_and_layouts_are_refused(capi, device):
+    g = torch.Generator(device=device).manual_seed(4)
+    x, w = torch.randn(4, 64, generator=g, device=device).bfloat16(), (torch.randn(24, 64, generator=g, device=device) / 8).bfloat16()
+
+    def empty(*shape, dtype=torch.bfloat16, dev=device):
+        return torch.empty(*shape, dtype=dtype, device=dev)
+
+    with pytest.raises(ValueError):
+        capi.linear(x, w, out_dtype=torch.float16)
+    for out in (empty(4, 24, dtype=torch.float16), empty(4, 16), empty(5, 24), empty(4, 24, dev="cpu"), empty(4, 48)[:, ::2], empty(24, 4).t(),
+                empty(1, 24).expand(4, 24), empty(2, 2, 24)):
+        with pytest.raises(ValueError):
+            capi.linear(x, w, out=out)
+    for out in (empty(4, 24), empty(4, 24, dtype=torch.float32), empty(4, 40)[:, 3:27], empty(8, 24)[::2]):
+        assert capi.linear(x, w, out=out) is out
+        _check(out, _want(x, w, 0, capi), 64, out.dtype == torch.float32)
+    # one x for all groups: not the kernel's
+    assert capi.linear(x[None].expand(3, 4, 64), w[None].expand(3, 24, 64).contiguous()) is None
