@@ -313,9 +313,11 @@ int rms_norm_dispatch(const void* x, const void* weight, void* out, int64_t rows
 }
 
 // out = bf16( bf16(silu(gate)) * up ): the two roundings of F.silu(gate) * up on bf16 tensors (model.py:134).
-// Bound by memory once the silu costs few enough instructions: with expf and an IEEE division the arithmetic took longer than the
-// bytes (8192 x 8192: 100 us, 4.0 TB/s; now 62 us, 6.5 TB/s).  The short forms of both are good to about 1e-6, next to the 2^-9 of the rounding behind
-// them.  Two vectors of each operand are asked for before the first is used.
+// silu(g) = g / (1 + exp(-g)) with expf and the short division, both sides a sixteenth: the divisor then stays below 2^126, beyond
+// which __fdividef is documented to give 0 (g below about -87.4).  With the 65 536 gates there are, every bit of the rounded silu is
+// that of expf and an IEEE division.  Bound by memory (8192 x 8192: 62 us, 6.5 TB/s; 100 us with the IEEE division and one vector
+// per thread).  Two vectors of each operand are asked for before the first is used.
+__device__ __forceinline__ float silu_short(float g) { return __fdividef(g * 0.0625f, fmaf(expf(-g), 0.0625f, 0.0625f)); }
 constexpr int kSiluVecs = 2;
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
@@ -341,7 +343,7 @@ silu_mul_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __r
     unpack8(g[v], a);
     unpack8(u[v], b);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = __fdividef(a[j], 1.0f + __expf(-a[j]));
+    for (int j = 0; j < 8; ++j) a[j] = silu_short(a[j]);
     const uint4 s = pack8(a);  // first rounding: silu(gate) as a bf16 tensor
     unpack8(s, a);
 #pragma unroll

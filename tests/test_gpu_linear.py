@@ -121,7 +121,7 @@ def test_extension_takes_any_layout_of_its_input(ext, device, gated):
         got = ext.linear(x, w, gated=gated)
         want = _ext_want(x, w, gated)
         assert got.shape == want.shape
-        # as in _check; above 64 rows the gate and the up row are rounded to bf16 before their product, and so is silu(gate): 3 x 2^-9
+        # as in _check; above 64 rows the gate and the up row are rounded to bf16 before their product, and so is silu(gate): 3 x 2^-8
         assert bool(((got.double() - want).abs() <= 2.0 ** -6 * want.abs() + 2.0 ** -9).all())
 
 
