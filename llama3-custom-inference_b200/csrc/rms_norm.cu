@@ -313,22 +313,23 @@ int rms_norm_dispatch(const void* x, const void* weight, void* out, int64_t rows
 }
 
 // out = bf16( bf16(silu(gate)) * up ): the two roundings of F.silu(gate) * up on bf16 tensors (model.py:134).
-// silu(g) = g / (1 + exp(-g)) with expf and the short division, both sides a sixteenth: the divisor then stays below 2^126, beyond
-// which __fdividef is documented to give 0 (g below about -87.4).  With the 65 536 gates there are, every bit of the rounded silu is
-// that of expf and an IEEE division.  Bound by memory (8192 x 8192: 62 us, 6.5 TB/s; 100 us with the IEEE division and one vector
-// per thread).  Two vectors of each operand are asked for before the first is used.
-__device__ __forceinline__ float silu_short(float g) { return __fdividef(g * 0.0625f, fmaf(expf(-g), 0.0625f, 0.0625f)); }
-constexpr int kSiluVecs = 2;
+// silu(g) = g / (1 + exp(-g)) by __expf and __fdividef, both sides of the division a sixteenth: the divisor then stays below 2^126,
+// beyond which __fdividef is documented to give 0 (g below about -87.4).  __expf's error grows with |g| (2 + 1.17 |g| units of the
+// last place); with the 65 536 gates there are, every bit of the rounded silu is that of expf and an IEEE division all the same.
+// Bound by memory (8192 x 8192: 59 us, 6.8 TB/s; 64 with expf; 86 with expf, an IEEE division and one vector per thread).  Two vectors
+// of each operand (kVecs) are asked for before the first is used where there are CTAs enough to fill the device all the same.
+__device__ __forceinline__ float silu_short(float g) { return __fdividef(g * 0.0625f, fmaf(__expf(-g), 0.0625f, 0.0625f)); }
+template <int kVecs>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
                 __nv_bfloat16* __restrict__ out, long long nvec, int row_vecs, long long gate_stride,
                 long long up_stride) {
   pdl_launch_dependents();  // the next one may be set up while this one runs
   pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
-  const long long i0 = (long long)blockIdx.x * (256 * kSiluVecs) + threadIdx.x;
-  uint4 g[kSiluVecs], u[kSiluVecs];
+  const long long i0 = (long long)blockIdx.x * (256 * kVecs) + threadIdx.x;
+  uint4 g[kVecs], u[kVecs];
 #pragma unroll
-  for (int v = 0; v < kSiluVecs; ++v) {
+  for (int v = 0; v < kVecs; ++v) {
     const long long i = i0 + v * 256;
     if (i >= nvec) break;
     const long long r = nvec <= 0xffffffffLL ? (long long)((unsigned)i / (unsigned)row_vecs) : i / row_vecs, c = (i - r * row_vecs) * kVecElems;
@@ -336,7 +337,7 @@ silu_mul_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __r
     u[v] = ld_stream16(up + r * up_stride + c);
   }
 #pragma unroll
-  for (int v = 0; v < kSiluVecs; ++v) {
+  for (int v = 0; v < kVecs; ++v) {
     const long long i = i0 + v * 256;
     if (i >= nvec) return;
     float a[8], b[8];
@@ -382,10 +383,15 @@ extern "C" int l3ci_silu_mul(const void* gate, const void* up, void* out, int64_
       !aligned16(gate) || !aligned16(up) || !aligned16(out))
     return fail(L3CI_ERR_ALIGNMENT, "silu_mul: rows must start on 16 bytes and cols be a multiple of 8");
   const long long nvec = rows * (cols / kVecElems);
-  const long long ctas = (nvec + 256 * kSiluVecs - 1) / (256 * kSiluVecs);
+  // one vector per thread up to eight CTAs per SM: 64 x 8192 in 1.94 us instead of 2.11, 300 x 2048 in 2.06 instead of 2.36
+  const int sms = sm_count() > 0 ? sm_count() : 148, vecs = nvec <= 256LL * 8 * sms ? 1 : 2;
+  const long long ctas = (nvec + 256 * vecs - 1) / (256 * vecs);
   if (ctas > 0x7fffffffLL) return fail(L3CI_ERR_INVALID, "silu_mul: tensor too large");
-  L3CI_LAUNCH("silu_mul_kernel", silu_mul_kernel, dim3((unsigned)ctas), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_),
-              static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up), static_cast<__nv_bfloat16*>(out), nvec,
-              (int)(cols / kVecElems), gate_row_stride, up_row_stride);
-  return L3CI_OK;
+  auto go = [&](auto kernel) -> int {
+    L3CI_LAUNCH("silu_mul_kernel", kernel, dim3((unsigned)ctas), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_),
+                static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up), static_cast<__nv_bfloat16*>(out), nvec,
+                (int)(cols / kVecElems), gate_row_stride, up_row_stride);
+    return L3CI_OK;
+  };
+  return vecs == 1 ? go(silu_mul_kernel<1>) : go(silu_mul_kernel<2>);
 }
