@@ -416,6 +416,11 @@ top_p_step_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lon
 constexpr int kKeyWords = 32768;                  // two keys' counts each
 constexpr int kHeld = 8;                          // 16-byte groups of a thread
 constexpr long long kMaxShare = 8191;             // groups of a CTA: a count of all its entries fits 16 bits
+// A weight is about 2^40 at most, except that of a logit without a number for one (NaN; an infinity or a value whose scaled
+// difference to the maximum overflows): 2^63 or more, so that masses wrap.  Masses of weights below 2^44 do not, over the 524 224
+// logits of the longest row.  A row with a larger weight is marked by this bit of its count.
+constexpr uint32_t kOddWeight = 1u << 12;         // in a weight's high word
+constexpr long long kOddRow = 1ll << 40;
 
 __device__ __forceinline__ uint32_t bits_key(uint32_t u) {   // logit_key of a bf16 pattern
   if (u == 0x8000u) return 0x8000u;
@@ -485,7 +490,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
                    float top_p, unsigned long long seed, long long* __restrict__ out_tokens, long long out_stride,
                    long long out_cols, long long* __restrict__ steps, long long* __restrict__ next_input,
                    int* __restrict__ positions, int* __restrict__ seq_lens, int* __restrict__ nucleus_count,
-                   float* __restrict__ nucleus_mass) {
+                   float* __restrict__ nucleus_mass, long long stand_in_run) {
   extern __shared__ __align__(16) uint32_t counts[];   // word k / 2 holds the counts of keys k (even: low half)
   __shared__ float redf[kTopPWarps];
   __shared__ u64 own_mass[256], digit_mass[256];
@@ -495,12 +500,16 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   __shared__ u64 s_mass;         // this CTA's, for the peers
   __shared__ long long s_eq, s_over;
   // what the first warp finds for all
-  __shared__ int s_pick[2];
+  __shared__ int s_pick[2], s_odd, s_first;
   __shared__ u64 s_above[2], s_total, s_budget, s_mass_front, s_mass_total;
   __shared__ long long s_eq_front, s_eq_total, s_over_total;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = kCtas > 1 ? cluster_rank() : 0u;
   for (int i = tid; i < kKeyWords / 4; i += kTopPBlock) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid == 0) {
+    s_odd = 0;
+    s_first = kTopPWarps;
+  }
   pdl_launch_dependents();  // the next one may be set up while this one runs
   pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
   const long long b = blockIdx.x / kCtas;
@@ -581,6 +590,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
 
   // ---- 2. boundary of the nucleus, digit by digit of the key: the masses of this CTA's entries, then of all ----
   // (a digit by a warp, neighbours to different ones: those that occur are neighbours)
+  uint32_t any = 0;                                       // high words of the weights
 #pragma unroll 1
   for (int i = 0; i < 8; ++i) {
     const int d = i * kTopPWarps + warp;
@@ -591,13 +601,18 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const uint32_t n = (k & 1) ? w[k / 2] >> 16 : w[k / 2] & 0xffffu;
-        if (n) q += (u64)n * rv.weight(key_logit((uint32_t)(d * 256 + lane * 8 + k)));
+        if (n) {
+          const u64 each = rv.weight(key_logit((uint32_t)(d * 256 + lane * 8 + k)));
+          any |= (uint32_t)(each >> 32);
+          q += (u64)n * each;
+        }
       }
 #pragma unroll
       for (int k = 16; k >= 1; k /= 2) q += __shfl_xor_sync(kFullMask, q, k);
     }
     if (lane == 0) own_mass[d] = q;
   }
+  if (any >= kOddWeight) s_odd = 1;
   __syncthreads();
   if constexpr (kCtas > 1) cluster_barrier();
   if (tid < 256) {
@@ -706,7 +721,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     for (int k = 16; k >= 1; k /= 2) over_all += __shfl_xor_sync(kFullMask, over_all, k);
     warp_eq[lane] = eq;                                   // from here on: of the warps in front
     warp_mass[lane] = mass;
-    if (lane == 0) { s_eq = eq_all; s_mass = mass_all; s_over = over_all; }
+    if (lane == 0) { s_eq = eq_all; s_mass = mass_all; s_over = over_all + (s_odd ? kOddRow : 0); }
   }
   __syncwarp();
   if constexpr (kCtas > 1) cluster_barrier();
@@ -738,9 +753,19 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
 
   // ---- 4. the draw: u in [0, 1) with 32 bits, target = floor(u * nucleus mass) < nucleus mass ----
   const u64 target = __umul64hi(mass_total, (u64)r << 32);
-  // one warp of one CTA has the target in its run; an empty nucleus (a row of NaNs) has no such warp: the first one stands in
-  const bool found = mass_warp > 0 && mass_before <= target && target < mass_before + mass_warp;
-  const bool stand_in = mass_total == 0 && rank == 0 && warp == 0;
+  // one warp of one CTA has the target in its run; an empty nucleus has no such warp: the first one stands in
+  bool found = mass_warp > 0 && mass_before <= target && target < mass_before + mass_warp;
+  bool stand_in = mass_total == 0 && rank == 0 && warp == 0;
+  if (s_over_total >= kOddRow) {                          // masses may have wrapped: any number of warps may have it, the first takes it
+    if (found && lane == 0) atomicMin(&s_first, warp);
+    __syncthreads();
+    if constexpr (kCtas > 1) cluster_barrier();
+    const int first = lane >= kCtas ? kTopPWarps : kCtas == 1 || lane == (int)rank ? s_first : ld_peer(&s_first, (uint32_t)lane);
+    const unsigned ctas = __ballot_sync(kFullMask, first < kTopPWarps);
+    const int cta = ctas ? __ffs(ctas) - 1 : 0, its = __shfl_sync(kFullMask, first, cta);
+    found = ctas && cta == (int)rank && its == warp;
+    stand_in = !ctas && rank == 0 && warp == 0;
+  }
   if (found || stand_in) {
     long long tok = -1;
     if (found) {
@@ -773,17 +798,24 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
         run += w_all;
         seen += eq_all;
       }
+      // one lane has it (of an odd row any number: the first of them, or the first entry of the warp)
+      const unsigned who = __ballot_sync(kFullMask, tok >= 0);
+      if (who == 0 && lane == 0) tok = g_warp * kVecElems;
+      if (who != 0 && lane != __ffs(who) - 1) tok = -1;
     } else if (lane == 0) {
-      // the last entry of the nucleus among the first of the row
-      constexpr long long kRowThreads = (long long)kTopPBlock * kCtas;
-      const long long per = ((vocab + kRowThreads - 1) / kRowThreads + kVecElems - 1) / kVecElems * kVecElems;
+      // of the first entries of the row, as many as a thread of the kernel above walks: the one that passes the target, or the last
+      // of the nucleus
       tok = 0;
       long long eq_seen = 0;
-      for (long long i = 0; i < per && i < vocab; ++i) {
-        const uint32_t key = bits_key(row_bits[i]);
+      u64 run = 0;
+      for (long long i = 0; i < stand_in_run && i < vocab; ++i) {
+        const uint32_t u = row_bits[i], key = bits_key(u);
         bool in = all_kept || key > key_star;
         if (!in && key == key_star) { in = eq_seen < eq_kept; ++eq_seen; }
-        if (in) tok = i;
+        if (!in) continue;
+        tok = i;
+        run += rv.weight(__uint_as_float(u << 16));
+        if (run > target) break;
       }
     }
     if (tok >= 0) {                                       // one lane
@@ -799,7 +831,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
       if (nucleus_mass) nucleus_mass[b] = Z > 0 ? (float)((double)mass_total / (double)Z) : 0.f;
     }
   }
-  if (nucleus_count && tid == 0 && rank == 0) nucleus_count[b] = (int)(s_over_total + eq_kept);
+  if (nucleus_count && tid == 0 && rank == 0) nucleus_count[b] = (int)(s_over_total % kOddRow + eq_kept);
   if constexpr (kCtas > 1) cluster_barrier();   // no CTA leaves while a peer may still read its shared memory
 }
 
@@ -823,7 +855,7 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
   const auto lp = static_cast<const __nv_bfloat16*>(logits);
   const float inv_t = 1.0f / temperature;
   const int sms = sm_count();
-  auto launch = [&](auto kernel, int c, int smem) {
+  auto launch = [&](auto kernel, int c, int smem, auto... more) {
     static bool configured[64][9] = {};   // by device and CTAs per row
     int dev = 0;
     if (smem > 0 && (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !configured[dev][c])) {
@@ -846,7 +878,7 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
     return cudaLaunchKernelEx(&cfg, kernel, lp, (long long)vocab, (long long)row_stride, inv_t, top_p, (unsigned long long)seed,
                               reinterpret_cast<long long*>(out_tokens), (long long)out_stride, (long long)out_cols,
                               reinterpret_cast<long long*>(steps), reinterpret_cast<long long*>(next_input), positions, seq_lens,
-                              nucleus_count, nucleus_mass);
+                              nucleus_count, nucleus_mass, more...);
   };
   // Small batches: a cluster of CTAs per row, as many (8, 4, 2) as still run all at once, so that the batch covers
   // the device (64 rows: 128 SMs; one row: 8).  A 148-SM part holds 15 clusters of 8, 33 of 4 or 74 of 2 of these
@@ -858,8 +890,10 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
   int by_counts = ctas_per_row;
   while (by_counts < 8 && (groups + by_counts - 1) / by_counts > kMaxShare) by_counts *= 2;
   if ((groups + by_counts - 1) / by_counts <= kMaxShare) {
-    cudaError_t e = by_counts == 8 ? launch(top_p_count_kernel<8>, 8, kKeyWords * 4) : by_counts == 4 ? launch(top_p_count_kernel<4>, 4, kKeyWords * 4)
-                    : by_counts == 2 ? launch(top_p_count_kernel<2>, 2, kKeyWords * 4) : launch(top_p_count_kernel<1>, 1, kKeyWords * 4);
+    const long long walkers = (long long)kTopPBlock * ctas_per_row, run = ((vocab + walkers - 1) / walkers + kVecElems - 1) / kVecElems * kVecElems;
+    auto counts = [&](auto kernel) { return launch(kernel, by_counts, kKeyWords * 4, run); };
+    const cudaError_t e = by_counts == 8 ? counts(top_p_count_kernel<8>) : by_counts == 4 ? counts(top_p_count_kernel<4>)
+                          : by_counts == 2 ? counts(top_p_count_kernel<2>) : counts(top_p_count_kernel<1>);
     if (e == cudaSuccess) return L3CI_OK;
     (void)cudaGetLastError();   // not placed: nothing ran
   }
