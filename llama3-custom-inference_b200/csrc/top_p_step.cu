@@ -416,6 +416,7 @@ top_p_step_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lon
 constexpr int kKeyWords = 32768;                  // two keys' counts each
 constexpr int kHeld = 8;                          // 16-byte groups of a thread
 constexpr long long kMaxShare = 8191;             // groups of a CTA: a count of all its entries fits 16 bits
+constexpr long long kFewLogits = 4096;            // logits of a one-CTA row that are few
 // A weight is about 2^40 at most, except that of a logit without a number for one (NaN; an infinity or a value whose scaled
 // difference to the maximum overflows): 2^63 or more, so that masses wrap.  Masses of weights below 2^44 do not, over the 524 224
 // logits of the longest row.  A row with a larger weight is marked by this bit of its count.
@@ -869,12 +870,17 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)c;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    if (c > 1) {
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)c;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+    } else {
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = c > 1 ? 1 : 0;
+    cfg.numAttrs = c > 1 || programmatic_launch_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, lp, (long long)vocab, (long long)row_stride, inv_t, top_p, (unsigned long long)seed,
                               reinterpret_cast<long long*>(out_tokens), (long long)out_stride, (long long)out_cols,
                               reinterpret_cast<long long*>(steps), reinterpret_cast<long long*>(next_input), positions, seq_lens,
@@ -885,11 +891,13 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
   // CTAs at a time (cudaOccupancyMaxActiveClusters); the bounds scale with the SM count.
   const int ctas_per_row = sms <= 0 ? 1 : rows * 148 <= 15LL * sms ? 8 : rows * 148 <= 33LL * sms ? 4 : 2 * rows <= sms ? 2 : 1;
   // By counts while a CTA's share of the row fits its registers and 16-bit counts: more CTAs per row where that takes more of
-  // them.  Longer rows yet, or a device that cannot place the cluster: by masses.
+  // them.  Longer rows yet, or a device that cannot place the cluster: by masses.  So are short rows of one CTA each, where clearing
+  // and summing 65 536 counts takes longer than the passes over the row (75 rows: of 1000 logits 11.4 us by masses, 13.8 by counts; 4096:
+  // 13.5, 13.8; 8000: 16.8, 13.7).
   const long long groups = (vocab + kVecElems - 1) / kVecElems;
   int by_counts = ctas_per_row;
   while (by_counts < 8 && (groups + by_counts - 1) / by_counts > kMaxShare) by_counts *= 2;
-  if ((groups + by_counts - 1) / by_counts <= kMaxShare) {
+  if ((groups + by_counts - 1) / by_counts <= kMaxShare && (by_counts > 1 || vocab > kFewLogits)) {
     const long long walkers = (long long)kTopPBlock * ctas_per_row, run = ((vocab + walkers - 1) / walkers + kVecElems - 1) / kVecElems * kVecElems;
     auto counts = [&](auto kernel) { return launch(kernel, by_counts, kKeyWords * 4, run); };
     const cudaError_t e = by_counts == 8 ? counts(top_p_count_kernel<8>) : by_counts == 4 ? counts(top_p_count_kernel<4>)
