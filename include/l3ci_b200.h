@@ -144,6 +144,9 @@ L3CI_API int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, in
                              float top_p, uint64_t seed, int64_t* out_tokens, int64_t out_stride, int64_t out_cols,
                              int64_t* steps, int64_t* next_input, int32_t* positions, int32_t* seq_lens,
                              int32_t* nucleus_count, float* nucleus_mass, l3ci_stream_t stream);
+/* The form in which l3ci_top_p_step takes rows of this size on the current device: CTAs per row (1, 2, 4 or 8), plus 16 where it
+ * counts keys; -1 for sizes it refuses.  For tests and measurements; no counterpart in the reference. */
+L3CI_API int l3ci_top_p_kernel_choice(int64_t rows, int64_t vocab);
 
 /* ------------------------------------------------------------------------------------------
  * Rotary embedding, interleaved-pair (Meta) convention:

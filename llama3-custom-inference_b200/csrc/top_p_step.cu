@@ -414,6 +414,7 @@ top_p_step_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lon
 // the kernel above: same boundary, same ties, same draw, bit for bit.
 //   64 rows of 128 256 logits: 39 us; 82 with the masses' histograms, whose atomics met on a few dozen bins.
 constexpr int kKeyWords = 32768;                  // two keys' counts each
+constexpr int kCountSmem = kKeyWords * 4;
 constexpr int kHeld = 8;                          // 16-byte groups of a thread
 constexpr long long kMaxShare = 8191;             // groups of a CTA: a count of all its entries fits 16 bits
 constexpr long long kFewLogits = 4096;            // logits of a one-CTA row that are few
@@ -836,8 +837,37 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   if constexpr (kCtas > 1) cluster_barrier();   // no CTA leaves while a peer may still read its shared memory
 }
 
+// CTAs per row, and whether keys are counted.
+struct TopPForm { int ctas; bool counts; int mass_ctas; };
+TopPForm top_p_form(long long rows, long long vocab) {
+  const int sms = sm_count();
+  // Small batches: a cluster of CTAs per row, as many (8, 4, 2) as still run all at once, so that the batch covers
+  // the device (64 rows: 128 SMs; one row: 8).  A 148-SM part holds 15 clusters of 8, 33 of 4 or 74 of 2 of these
+  // CTAs at a time (cudaOccupancyMaxActiveClusters); the bounds scale with the SM count.
+  const int mass_ctas = sms <= 0 ? 1 : rows * 148 <= 15LL * sms ? 8 : rows * 148 <= 33LL * sms ? 4 : 2 * rows <= sms ? 2 : 1;
+  // By counts while a CTA's share of the row fits its registers and 16-bit counts: more CTAs per row where that takes more of
+  // them.  Longer rows yet, or a device without the shared memory: by masses.  So are short rows of one CTA each, where clearing
+  // and summing 65 536 counts takes longer than the passes over the row (75 rows: of 1000 logits 11.4 us by masses, 13.8 by counts; 4096:
+  // 13.5, 13.8; 8000: 16.8, 13.7).
+  const long long groups = (vocab + kVecElems - 1) / kVecElems;
+  int ctas = mass_ctas;
+  while (ctas < 8 && (groups + ctas - 1) / ctas > kMaxShare) ctas *= 2;
+  const bool counts = (groups + ctas - 1) / ctas <= kMaxShare && (ctas > 1 || vocab > kFewLogits) && (sms <= 0 || max_smem_optin() >= kCountSmem + 8192);
+  return {counts ? ctas : mass_ctas, counts, mass_ctas};
+}
+// Errors of a launch whose cluster (or CTA) the device, or the part of it that this process has, cannot hold.
+bool not_placed(cudaError_t e) {
+  return e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources || e == cudaErrorInvalidConfiguration;
+}
+
 }  // namespace
 }  // namespace l3ci
+
+extern "C" int l3ci_top_p_kernel_choice(int64_t rows, int64_t vocab) {
+  if (rows <= 0 || vocab <= 0) return -1;
+  const l3ci::TopPForm f = l3ci::top_p_form(rows, vocab);
+  return f.ctas + (f.counts ? 16 : 0);
+}
 
 extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, int64_t row_stride, float temperature,
                                float top_p, uint64_t seed, int64_t* out_tokens, int64_t out_stride, int64_t out_cols,
@@ -855,7 +885,6 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   const auto lp = static_cast<const __nv_bfloat16*>(logits);
   const float inv_t = 1.0f / temperature;
-  const int sms = sm_count();
   auto launch = [&](auto kernel, int c, int smem, auto... more) {
     static bool configured[64][9] = {};   // by device and CTAs per row
     int dev = 0;
@@ -886,29 +915,23 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
                               reinterpret_cast<long long*>(steps), reinterpret_cast<long long*>(next_input), positions, seq_lens,
                               nucleus_count, nucleus_mass, more...);
   };
-  // Small batches: a cluster of CTAs per row, as many (8, 4, 2) as still run all at once, so that the batch covers
-  // the device (64 rows: 128 SMs; one row: 8).  A 148-SM part holds 15 clusters of 8, 33 of 4 or 74 of 2 of these
-  // CTAs at a time (cudaOccupancyMaxActiveClusters); the bounds scale with the SM count.
-  const int ctas_per_row = sms <= 0 ? 1 : rows * 148 <= 15LL * sms ? 8 : rows * 148 <= 33LL * sms ? 4 : 2 * rows <= sms ? 2 : 1;
-  // By counts while a CTA's share of the row fits its registers and 16-bit counts: more CTAs per row where that takes more of
-  // them.  Longer rows yet, or a device that cannot place the cluster: by masses.  So are short rows of one CTA each, where clearing
-  // and summing 65 536 counts takes longer than the passes over the row (75 rows: of 1000 logits 11.4 us by masses, 13.8 by counts; 4096:
-  // 13.5, 13.8; 8000: 16.8, 13.7).
-  const long long groups = (vocab + kVecElems - 1) / kVecElems;
-  int by_counts = ctas_per_row;
-  while (by_counts < 8 && (groups + by_counts - 1) / by_counts > kMaxShare) by_counts *= 2;
-  if ((groups + by_counts - 1) / by_counts <= kMaxShare && (by_counts > 1 || vocab > kFewLogits)) {
-    const long long walkers = (long long)kTopPBlock * ctas_per_row, run = ((vocab + walkers - 1) / walkers + kVecElems - 1) / kVecElems * kVecElems;
-    auto counts = [&](auto kernel) { return launch(kernel, by_counts, kKeyWords * 4, run); };
-    const cudaError_t e = by_counts == 8 ? counts(top_p_count_kernel<8>) : by_counts == 4 ? counts(top_p_count_kernel<4>)
-                          : by_counts == 2 ? counts(top_p_count_kernel<2>) : counts(top_p_count_kernel<1>);
+  const TopPForm form = top_p_form(rows, vocab);
+  auto failed = [](cudaError_t e) { return fail(L3CI_ERR_CUDA, "launch of the top_p_step kernel failed: %s", cudaGetErrorString(e)); };
+  if (form.counts) {
+    const long long walkers = (long long)kTopPBlock * form.mass_ctas, run = ((vocab + walkers - 1) / walkers + kVecElems - 1) / kVecElems * kVecElems;
+    auto counts = [&](auto kernel) { return launch(kernel, form.ctas, kCountSmem, run); };
+    const cudaError_t e = form.ctas == 8 ? counts(top_p_count_kernel<8>) : form.ctas == 4 ? counts(top_p_count_kernel<4>)
+                          : form.ctas == 2 ? counts(top_p_count_kernel<2>) : counts(top_p_count_kernel<1>);
     if (e == cudaSuccess) return L3CI_OK;
-    (void)cudaGetLastError();   // not placed: nothing ran
+    (void)cudaGetLastError();
+    if (!not_placed(e)) return failed(e);
   }
-  for (int c = ctas_per_row; c > 1; c /= 2) {
+  // (a cluster size the device or its partition cannot place falls back to the next smaller one)
+  for (int c = form.mass_ctas; c > 1; c /= 2) {
     const cudaError_t e = c == 8 ? launch(top_p_step_kernel<8>, 8, 0) : c == 4 ? launch(top_p_step_kernel<4>, 4, 0) : launch(top_p_step_kernel<2>, 2, 0);
     if (e == cudaSuccess) return L3CI_OK;
-    (void)cudaGetLastError();   // not placed: nothing ran
+    (void)cudaGetLastError();
+    if (!not_placed(e)) return failed(e);
   }
   L3CI_LAUNCH("top_p_step_kernel", top_p_step_kernel<1>, dim3((unsigned)rows), dim3(kTopPBlock), 0, stream,
               lp, (long long)vocab, (long long)row_stride, inv_t, top_p, (unsigned long long)seed,

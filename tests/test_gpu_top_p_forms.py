@@ -37,3 +37,20 @@ def test_counts_and_masses_agree(capi, device, rows, vocab, kind):
     for logits in (x, odd[:, 3:]):
         for a, b in zip(run(logits), want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["normal", "flat", "steps", "holes"])
+@pytest.mark.parametrize("rows,vocab", [(75, 1), (75, 4096), (75, 4097), (149, 4100)])
+def test_short_rows_of_one_cta(capi, device, rows, vocab, kind):
+    test_counts_and_masses_agree(capi, device, rows, vocab, kind)
+
+
+def test_the_form_taken(capi, device):
+    """CTAs per row, + 16 by counts.  A launch that fails for another reason than its place on the device is an error, not the other form."""
+    if torch.cuda.get_device_properties(device).multi_processor_count != 148:
+        pytest.skip("the bounds are those of 148 SMs")
+    choice = capi.load().l3ci_top_p_kernel_choice
+    for rows, vocab, want in ((1, 8, 24), (15, 128256, 24), (16, 128256, 20), (33, 8, 20), (34, 128256, 18), (74, 65528, 18), (75, 65528, 17),
+                              (75, 65529, 18), (75, 4097, 17), (75, 4096, 1), (256, 300000, 24), (1, LONG, 8), (33, LONG, 4), (80, LONG, 1)):
+        assert choice(rows, vocab) == want, (rows, vocab)
+    assert choice(0, 8) == choice(1, 0) == -1
