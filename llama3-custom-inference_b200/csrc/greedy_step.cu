@@ -49,8 +49,7 @@ greedy_step_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
                    int* __restrict__ seq_lens) {
   __shared__ float s_val[kGreedyBlock / kWarp];
   __shared__ long long s_idx[kGreedyBlock / kWarp];
-  pdl_launch_dependents();  // the next one may be set up while this one runs
-  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
+  pdl_begin();
   const long long b = blockIdx.x;
   const __nv_bfloat16* row = logits + b * row_stride;
   float best = -INFINITY;

@@ -35,8 +35,7 @@ moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ bia
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int e = tid; e < E; e += blockDim.x) count[e] = 0;
   __syncthreads();
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long row0 = (long long)blockIdx.x * tokens;
   const int n = (int)min((long long)tokens, rows - row0);
   float* z = row + warp * E;
@@ -93,8 +92,7 @@ __global__ void __launch_bounds__(128)
 moe_gather_kernel(const S* __restrict__ h, const int* __restrict__ experts, const int* __restrict__ ranks, const int* __restrict__ counts,
                   S* __restrict__ out, int* __restrict__ part_rows, long long rows, int width, int E, int top) {
   extern __shared__ int at_s[];
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long row = blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x / kWarp;
   for (int j = warp; j < top; j += warps) {

@@ -21,9 +21,7 @@ add_dyn_tanh_kernel(const S* __restrict__ y, const long long* __restrict__ token
                     float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float alpha,
                     S* __restrict__ out, int width) {
   // the first kernel of a forward pass lets none of it start early: later ones read the model's weights ahead of their own wait
-  if (!tokens) pdl_launch_dependents();
-  pdl_wait();
-  if (tokens) pdl_launch_dependents();
+  pdl_begin(!tokens);
   const long long row = blockIdx.x;
   float* xr = x + row * width;
   const S* add = y ? y + row * width : nullptr;
@@ -58,8 +56,7 @@ enum { kGelu = 0, kTanh = 1 };
 
 template <typename S, int VEC, int KIND>
 __global__ void __launch_bounds__(256) activation_kernel(const S* __restrict__ z, S* __restrict__ out, long long n) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long i0 = ((long long)blockIdx.x * 256 + threadIdx.x) * VEC;
   if (i0 >= n) return;
   float v[VEC];
@@ -75,8 +72,7 @@ __global__ void __launch_bounds__(256) activation_kernel(const S* __restrict__ z
 template <typename S, int VEC>
 __global__ void __launch_bounds__(256)
 gated_act_kernel(const S* __restrict__ gu, S* __restrict__ out, long long units, int per_row, float limit, float alpha) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
   if (id >= units) return;
   const long long row = units <= 0xffffffffLL ? (unsigned)id / (unsigned)per_row : id / per_row;
@@ -101,8 +97,7 @@ __global__ void __launch_bounds__(256)
 qk_norm_cache_kernel(S* __restrict__ qkv, const float* __restrict__ qw, const float* __restrict__ kw, S* __restrict__ ck,
                      S* __restrict__ cv, const int* __restrict__ positions, const QkNormRow p) {
   __shared__ float red[2][8];
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long row = blockIdx.x;
   const int b = (int)(row / p.T), t = (int)(row % p.T), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x / kWarp;
   const long long pos = (long long)positions[b] + t;
@@ -153,8 +148,7 @@ template <typename S, int VEC>
 __global__ void __launch_bounds__(256)
 token_shift_kernel(const S* __restrict__ h, const float* __restrict__ mu, S* __restrict__ last, long long last_sb,
                    const int* __restrict__ positions, S* __restrict__ out, int n_mix, int T, long long rows, int width) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long row = blockIdx.x;
   const int b = (int)(row / T), t = (int)(row % T);
   const bool fresh = positions[b] == 0;
@@ -194,8 +188,7 @@ __global__ void __launch_bounds__(256)
 latent_cache_kernel(S* __restrict__ qd, const float* __restrict__ table, const float* __restrict__ nw, S* __restrict__ cache,
                     const int* __restrict__ positions, const LatentRow p) {
   __shared__ float red[32];
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long row = blockIdx.x;
   const int b = (int)(row / p.T), t = (int)(row % p.T);
   const long long pos = (long long)positions[b] + t;
@@ -235,8 +228,7 @@ __global__ void __launch_bounds__(kLatentThreads)
 latent_cache_vec_kernel(__nv_bfloat16* __restrict__ qd, const float* __restrict__ table, const float* __restrict__ nw,
                         __nv_bfloat16* __restrict__ cache, const int* __restrict__ positions, const LatentRow p) {
   __shared__ float red[32];
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long row = blockIdx.x;
   const int b = (int)(row / p.T), t = (int)(row % p.T), tid = threadIdx.x;
   // the row's own loads do not wait for the position
@@ -311,8 +303,7 @@ template <int VPL>
 __global__ void __launch_bounds__(256)
 latent_cache_rows_kernel(__nv_bfloat16* __restrict__ qd, const float* __restrict__ table, const float* __restrict__ nw,
                          __nv_bfloat16* __restrict__ cache, const int* __restrict__ positions, const LatentRow p, long long rows) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -403,8 +394,7 @@ __global__ void __launch_bounds__(128)
 kv_cache_write_kernel(const S* __restrict__ src, long long stride, long long k_col, int k_width, long long v_col, int v_width,
                       S* __restrict__ ck, long long k_sb, long long k_st, S* __restrict__ cv, long long v_sb, long long v_st,
                       long long cache_len, const int* __restrict__ positions, int T, int rows) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   using R = typename Raw<VEC * sizeof(S)>::type;
   const unsigned per_row = (k_width + v_width) / VEC;
   R data[COPIES];

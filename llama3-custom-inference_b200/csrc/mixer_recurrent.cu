@@ -200,8 +200,7 @@ recurrent_scan_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const bool fresh = a.positions[b] == 0;
   const int chunks = (T + kChunk - 1) / kChunk;
   const long long row0 = (long long)b * T;
@@ -536,8 +535,7 @@ __global__ void __launch_bounds__(kStepThreads, RP <= 4 ? 5 : RP <= 8 ? 3 : 2) r
   const int quads = V / 4, groups = kStepThreads / quads, quad = tid % quads, grp = tid / quads;
   const int h = blockIdx.x % a.H, b = blockIdx.x / a.H, R = a.H / a.G;
   const bool active = grp < groups;
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const bool fresh = a.positions[b] == 0;
   float4* state = reinterpret_cast<float4*>(a.state + b * a.state_sb + (long long)h * D * V) + quad;
   float4 s[RP];
@@ -636,8 +634,7 @@ template <typename S, int VEC, int LANES>
 __global__ void __launch_bounds__(256)
 head_norm_gate_vec_kernel(S* __restrict__ out, long long out_st, long long out_sh, const S* __restrict__ gate, long long gate_st,
                           long long gate_sh, const float* __restrict__ norm, long long norm_sh, int H, int V, long long units, int act, float eps) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long id = (long long)blockIdx.x * (256 / LANES) + threadIdx.x / LANES;
   const int c = (threadIdx.x % LANES) * VEC;
   const bool mine = id < units && c < V;
@@ -669,8 +666,7 @@ template <typename S, int VEC>
 __global__ void __launch_bounds__(256)
 head_norm_gate_kernel(S* __restrict__ out, long long out_st, long long out_sh, const S* __restrict__ gate, long long gate_st,
                       long long gate_sh, const float* __restrict__ norm, long long norm_sh, int H, int V, long long units, int act, float eps) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const long long id = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (id >= units) return;
@@ -738,8 +734,7 @@ __device__ __forceinline__ float decay_of(float y, float rate) {
 // TAPS > 0: the run's inputs are all asked for at once and every one is loaded once; 0: any number of taps.
 template <typename S, int VEC, int TAPS, int RUN>
 __global__ void __launch_bounds__(256, 3) delta_inputs_kernel(const l3ci_delta_inputs_args a, int runs, long long tasks) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const long long id = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (id >= tasks) return;

@@ -73,9 +73,7 @@ __global__ void __launch_bounds__(512) residual_norm_kernel(const l3ci_residual_
   }
   const int valid = chunks * VEC;
   // the first kernel of a forward pass lets none of it start early: later ones read the model's weights ahead of their own wait
-  if (!a.tokens) pdl_launch_dependents();
-  pdl_wait();
-  if (a.tokens) pdl_launch_dependents();
+  pdl_begin(!a.tokens);
   const long long row = blockIdx.x;
   float* xr = a.x + row * width;
   float x[VPT * VEC], y[VPT * VEC];

@@ -37,8 +37,7 @@ rms_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 __nv_bfloat16* __restrict__ sum_out) {
   constexpr int kRows = RmsCfg<TPR>::kRowsPerCta;
   __shared__ float red[32];
-  pdl_launch_dependents();  // the next one may be set up while this one runs
-  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
+  pdl_begin();
   const int t = threadIdx.x % TPR;
   const long long row = (long long)blockIdx.x * kRows + threadIdx.x / TPR;
   const bool row_ok = row < rows;
@@ -151,8 +150,7 @@ __global__ void __launch_bounds__(kRowsBlock, (VPL >= 8 && kRes) ? 1 : 2)
 rms_norm_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                      __nv_bfloat16* __restrict__ out, long long rows, int nvec, long long x_stride, long long out_stride,
                      float embed_f, float eps, const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ sum_out) {
-  pdl_launch_dependents();  // the next one may be set up while this one runs
-  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (kRowsBlock / 32);
   long long row = (long long)blockIdx.x * (kRowsBlock / 32) + (threadIdx.x >> 5);
@@ -324,8 +322,7 @@ __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
                 __nv_bfloat16* __restrict__ out, long long nvec, int row_vecs, long long gate_stride,
                 long long up_stride) {
-  pdl_launch_dependents();  // the next one may be set up while this one runs
-  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
+  pdl_begin();
   const long long i0 = (long long)blockIdx.x * (256 * kVecs) + threadIdx.x;
   uint4 g[kVecs], u[kVecs];
 #pragma unroll

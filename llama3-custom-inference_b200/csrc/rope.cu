@@ -59,8 +59,7 @@ __global__ void __launch_bounds__(kTokenBlock)
 rot_embed_vec8_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ freq,
                       __nv_bfloat16* __restrict__ out, int S, int H, int vec_per_head_rt, long long sb, long long ss,
                       long long sh) {
-  pdl_launch_dependents();  // the next one may be set up while this one runs
-  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
+  pdl_begin();
   const int vec_per_head = VPH ? VPH : vec_per_head_rt;
   const long long token = blockIdx.x;
   const int s = (int)(token % S);
@@ -126,8 +125,7 @@ rot_embed_kv_cache_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __
                           long long qkv_sb, long long qkv_st, long long cache_sb, long long cache_st,
                           long long start_pos, const int* __restrict__ positions, long long freq_rows,
                           long long cache_len) {
-  pdl_launch_dependents();  // the next one may be set up while this one runs
-  pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
+  pdl_begin();
   const int vec_per_head = VPH ? VPH : vec_per_head_rt;
   const long long token = blockIdx.x;
   const int t = (int)(token % T);
