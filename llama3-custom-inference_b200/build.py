@@ -42,7 +42,7 @@ NVCC_FLAGS = [
 ]
 CUDA_SOURCES = ["host_common.cu", "linear_rows.cu", "rms_norm.cu", "rope.cu", "flash_decode.cu", "flash_decode_small.cu", "lse_merge.cu", "greedy_step.cu", "top_p_step.cu", "prefill_attention.cu", "prefill_attention_tc.cu"]
 
-MIXER_SOURCES = ["host_common.cu", "linear_rows.cu", "mixer_parts.cu", "mixer_attention.cu", "mixer_attention_mma.cu", "mixer_attention_tc.cu", "mixer_residual.cu", "mixer_recurrent.cu", "mixer_moe.cu", "mixer_moe_tc.cu"]
+MIXER_SOURCES = ["host_common.cu", "mixer_parts.cu", "mixer_attention.cu", "mixer_attention_mma.cu", "mixer_attention_tc.cu", "mixer_residual.cu", "mixer_recurrent.cu", "mixer_moe.cu", "mixer_moe_tc.cu"]
 
 
 def _nvcc() -> str:
@@ -91,7 +91,7 @@ def _build_shared(lib: Path, names: list[str], force: bool, verbose: bool) -> Pa
             if verbose:
                 print(out, file=sys.stderr)
     if force or jobs or not _newer(lib, objects):
-        # -Bsymbolic: both libraries hold host_common.o and linear_rows.o; each keeps to its own copy
+        # -Bsymbolic: both libraries hold host_common.o; each keeps to its own copy
         _run([nvcc, "-shared", "-o", str(lib), *map(str, objects), "-cudart", "static",
               "-Xlinker", "-soname," + lib.name, "-Xlinker", "-Bsymbolic"])
     return lib

@@ -337,35 +337,63 @@ Tensor silu_mul(Tensor gate, Tensor up) {
   return out;
 }
 
-// act(x w^T): few rows in one kernel (l3ci_linear), more in torch's product and, gated, silu_mul.  `gated`: w holds gate
-// rows, then up rows, and the result is silu(gate) * up.  `early`: the kernel may read w ahead of the stream's previous
-// kernels; for a w that was complete before the last one of them that waits for its predecessors ahead of letting others start.
+// act(x w^T) of few rows in one kernel (l3ci_linear): x [..., K] with w [N, K] (gated: [2 N, K], gate rows, then up rows), or groups
+// of products, x [groups, rows, K] with w [groups, N, K].  Nothing where that kernel does not apply: more rows, other types, layouts
+// or alignments.  `early`: the kernel may read w ahead of the stream's previous kernels; for a w that was complete before the last
+// one of them that waits for its predecessors ahead of letting others start.  f32: an fp32 result.  `into`: where the result goes.
+std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bool early, bool f32, const std::optional<Tensor>& into) {
+  if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != torch::kBFloat16 || w.scalar_type() != torch::kBFloat16 ||
+      w.get_device() != x.get_device() || x.dim() < 1)
+    return std::nullopt;
+  const bool grouped = w.dim() == 3, gated = act == L3CI_ACT_SILU_GATE;
+  const int64_t K = x.size(-1);
+  if ((w.dim() != 2 && !grouped) || w.size(-1) != K || (grouped && (x.dim() != 3 || x.size(0) != w.size(0)))) return std::nullopt;
+  const int64_t groups = grouped ? w.size(0) : 1, rows = K * groups ? x.numel() / (K * groups) : 0;
+  if (rows == 0 || rows > L3CI_LINEAR_MAX_ROWS || K % 8 || (gated && w.size(-2) % 2)) return std::nullopt;
+  const int64_t N = gated ? w.size(-2) / 2 : w.size(-2);
+  auto at16 = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; };
+  if (N == 0 || K > INT32_MAX || w.size(-2) > INT32_MAX || groups > INT32_MAX || !w.is_contiguous() || !at16(x) || !at16(w)) return std::nullopt;
+  auto row_stride = [&](const Tensor& t) {
+    const int64_t* sizes = t.sizes().data() + (grouped ? 1 : 0);
+    return l3ci_row_stride(sizes, t.strides().data() + (grouped ? 1 : 0), (int32_t)t.dim() - (grouped ? 1 : 0));
+  };
+  const int64_t stride = row_stride(x), group_stride = grouped ? x.stride(0) : 0;
+  if (stride < 0 || stride % 8 || group_stride % 8 || (groups > 1 && group_stride <= 0)) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(x.device());
+  auto sizes = x.sizes().vec();
+  sizes.back() = N;
+  Tensor out;
+  if (into) {
+    out = *into;
+    TORCH_CHECK(out.is_cuda() && out.get_device() == x.get_device() && out.sizes() == torch::IntArrayRef(sizes) &&
+                    (out.scalar_type() == torch::kBFloat16 || out.scalar_type() == torch::kFloat) && row_stride(out) > 0 &&
+                    (groups == 1 || out.stride(0) > 0),
+                "the result's type, shape, device or strides");
+  } else {
+    out = torch::empty(sizes, x.options().dtype(f32 ? torch::kFloat : torch::kBFloat16));
+  }
+  l3ci_linear_args a{};
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
+  a.rows = rows; a.x_st = stride; a.out_st = row_stride(out); a.x_sg = group_stride; a.out_sg = grouped ? out.stride(0) : 0;
+  a.K = (int32_t)K; a.N = (int32_t)N; a.groups = (int32_t)groups; a.act = (int32_t)act;
+  a.out_f32 = out.scalar_type() == torch::kFloat;
+  a.early = early;
+  a.stream = current_stream();
+  check_status(l3ci_linear(&a), "linear");
+  return out;
+}
+
+// act(x w^T) of any number of rows: few in one kernel (few_rows), more in torch's product and, gated, silu_mul.
 Tensor linear(Tensor x, Tensor w, bool gated, bool early) {
   check_bf16_cuda(x, "x");
   check_bf16_cuda(w, "w");
   TORCH_CHECK(x.dim() >= 1 && w.dim() == 2 && w.size(1) == x.size(-1), "w must be [N, K] with K the last axis of x");
   TORCH_CHECK(w.get_device() == x.get_device(), "x and w on different devices");
   TORCH_CHECK(!gated || w.size(0) % 2 == 0, "a gated product takes an even number of rows of w");
+  if (auto y = few_rows(x, w, gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE, early, false, std::nullopt)) return *y;
   const c10::cuda::CUDAGuard guard(x.device());
-  const int64_t K = x.size(-1), N = gated ? w.size(0) / 2 : w.size(0), rows = K ? x.numel() / K : 0;
-  const int64_t stride = l3ci_row_stride(x.sizes().data(), x.strides().data(), (int32_t)x.dim());
-  auto at16 = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; };
-  if (stride > 0 && stride % 8 == 0 && rows > 0 && rows <= L3CI_LINEAR_MAX_ROWS && N > 0 && K % 8 == 0 && w.is_contiguous() &&
-      K <= INT32_MAX && w.size(0) <= INT32_MAX && at16(x) && at16(w)) {
-    auto sizes = x.sizes().vec();
-    sizes.back() = N;
-    Tensor out = torch::empty(sizes, x.options());
-    l3ci_linear_args a{};
-    a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
-    a.rows = rows; a.x_st = stride; a.out_st = N;
-    a.K = (int32_t)K; a.N = (int32_t)N; a.groups = 1;
-    a.act = gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE;
-    a.early = early;
-    a.stream = current_stream();
-    check_status(l3ci_linear(&a), "linear");
-    return out;
-  }
   Tensor y = at::linear(x, w);
+  const int64_t N = w.size(0) / 2;
   return gated ? silu_mul(y.narrow(-1, 0, N), y.narrow(-1, N, N)) : y;
 }
 
@@ -523,6 +551,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("silu_mul", torch::wrap_pybind_function(silu_mul), "silu_mul", py::arg("gate"), py::arg("up"));
   m.def("linear", torch::wrap_pybind_function(linear), "linear", py::arg("x"), py::arg("w"), py::arg("gated") = false,
         py::arg("early") = false);
+  m.def("few_rows", torch::wrap_pybind_function(few_rows), "few_rows", py::arg("x"), py::arg("w"), py::arg("act") = (int64_t)L3CI_ACT_NONE,
+        py::arg("early") = false, py::arg("f32") = false, py::arg("into") = py::none());
   m.def("greedy_step", torch::wrap_pybind_function(greedy_step), "greedy_step", py::arg("logits"), py::arg("out_tokens"),
         py::arg("steps"), py::arg("next_input"), py::arg("positions"), py::arg("seq_lens"));
   m.def("top_p_step", torch::wrap_pybind_function(top_p_step), "top_p_step", py::arg("logits"), py::arg("out_tokens"),

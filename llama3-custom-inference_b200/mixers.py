@@ -8,7 +8,7 @@ from pathlib import Path
 import torch
 import torch.nn.functional as F
 
-from .capi import ACT_GELU, ACT_NONE, ACT_SILU_GATE, ACT_TANH, OK, L3ciError, LinearArgs, _on, _stream, linear_args
+from .capi import ACT_GELU, ACT_NONE, ACT_SILU_GATE, ACT_TANH, LINEAR_MAX_ROWS, OK, L3ciError, _on, _stream
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libl3ci_mixers.so"
 
@@ -89,7 +89,6 @@ def load() -> C.CDLL:
     i64, i32, vp, f32 = C.c_int64, C.c_int32, C.c_void_p, C.c_float
     lib.l3ci_mixers_last_error.restype = C.c_char_p
     lib.l3ci_mixers_set_programmatic_launch.argtypes = [C.c_int]
-    lib.l3ci_linear.argtypes = [C.POINTER(LinearArgs)]
     lib.l3ci_add_dyn_tanh.argtypes = [vp, vp, vp, i64, vp, vp, vp, f32, vp, i64, i64, i32, vp]
     lib.l3ci_gelu.argtypes = [vp, vp, i64, i32, vp]
     lib.l3ci_latent_cache.argtypes = [vp, i64, vp, i64, vp, f32, vp, i64, i64, i64, vp] + [i32] * 7 + [vp]
@@ -124,22 +123,36 @@ def _cuda(*tensors):
             raise ValueError("the mixer kernels take CUDA tensors: there is no CPU path")
 
 
+_ext = None
+
+
+def _extension():
+    """The torch extension module, whose `linear` and `few_rows` take the products: their checks cost the host less there than here."""
+    global _ext
+    if _ext is None:
+        from . import extension
+
+        _ext = extension()
+    return _ext
+
+
 def few_rows(x, w, act: int = ACT_NONE, out_dtype=None, out=None, early: bool = False):
     """act(x w^T) of few rows in one kernel (`l3ci_linear`), groups of products where w is [groups, N, K]; None where it does
     not apply.  `early`: w may be read ahead of the stream's previous kernels; for weights that were complete before the last one
     of them that waits for its predecessors ahead of letting others start (a model's, in its forward pass)."""
-    a, out = linear_args(x, w, act, out_dtype, early=early, out=out)
-    if a is not None:
-        with _on(x):
-            _check(load().l3ci_linear(C.byref(a)), "l3ci_linear")
-    return out
+    if out_dtype not in (None, torch.bfloat16, torch.float32):
+        raise ValueError("the result is bf16 or fp32")
+    if x.numel() > LINEAR_MAX_ROWS * x.shape[-1] * (x.shape[0] if w.dim() == 3 else 1):   # (a prompt's: the host is what it waits for)
+        return None
+    return _extension().few_rows(x, w, act, early, out_dtype == torch.float32, out)
 
 
 def linear(x, w, act: int = ACT_NONE, early: bool = False):
     """act(x w^T); ACT_SILU_GATE: w holds gate rows, then up rows.  `early`: see `few_rows`."""
-    y = few_rows(x, w, act, early=early)
-    if y is not None:
-        return y
+    if x.numel() <= LINEAR_MAX_ROWS * x.shape[-1]:
+        y = _extension().few_rows(x, w, act, early)
+        if y is not None:
+            return y
     y = F.linear(x, w)
     return y if act == ACT_NONE else gelu_(y) if act == ACT_GELU else tanh_(y) if act == ACT_TANH else gated_act(y)
 
