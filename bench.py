@@ -977,7 +977,7 @@ def bench_end_to_end(args, ext, pkg, dev, rank, world):
     sync_all(world)
     sampler.stop()
     ms = max_over_ranks(max(start.elapsed_time(end), wall * 1e3), world, dev)
-    if ext.flash_decode_status(toks) != 0:
+    if ext.flash_decode_status(toks) != 0 or ext.linear_status(toks) != 0:
         raise RuntimeError("device-side wait ran out")
     value = G * B * world * steps / (ms * 1e-3)
     # end to end through the public call with host inputs: prompts from pinned host memory, tokens read back

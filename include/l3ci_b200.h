@@ -98,7 +98,8 @@ L3CI_API int l3ci_silu_mul(const void* gate, const void* up, void* out, int64_t 
  * L3CI_ACT_SILU_GATE: w is [groups, 2, N, K], gate rows then up rows, and out = silu(gate) * up (the two products of MLP.forward,
  * model.py:134, with it).  early: w may be read before the stream's previous kernels have ended; for a w that was complete
  * before the last kernel that waits for its predecessors ahead of letting this one start (weights of a model).  split: CTAs that share a tile's columns, 0 chooses (else 1, 2, 4 or 8).
- * status (int32 on the device, may be null) receives L3CI_ERR_DEVICE_WAIT if a bounded wait ran out. */
+ * status (int32 on the device) receives L3CI_ERR_DEVICE_WAIT if a bounded wait ran out, and out is then not complete; null: a word of
+ * the library's own on the device, for l3ci_linear_poll. */
 #define L3CI_LINEAR_MAX_ROWS 64
 typedef enum l3ci_act { L3CI_ACT_NONE = 0, L3CI_ACT_GELU = 1, L3CI_ACT_TANH = 2, L3CI_ACT_SILU_GATE = 3 } l3ci_act;
 typedef struct l3ci_linear_args {
@@ -111,6 +112,9 @@ typedef struct l3ci_linear_args {
   l3ci_stream_t stream;
 } l3ci_linear_args;
 L3CI_API int l3ci_linear(const l3ci_linear_args* args);
+/* Waits for `stream`; L3CI_ERR_DEVICE_WAIT, once, if a launch of l3ci_linear without a status word of its own gave up on this device
+ * (should never happen). */
+L3CI_API int l3ci_linear_poll(l3ci_stream_t stream);
 /* Elements between the rows of a tensor of these sizes and strides (in elements), all axes but the last counted as one axis of
  * rows; the width where there is at most one row.  -1 where no one stride gives the rows (a broadcast axis, axes that do not
  * follow one another), where rows overlap, or where the last axis is not contiguous.  Host only. */

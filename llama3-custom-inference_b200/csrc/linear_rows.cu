@@ -53,6 +53,9 @@ struct LinShape {
   static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs per SM");
 };
 
+// Where a wait that ran out is recorded by calls without a status word of their own, until l3ci_linear_poll reads it.
+__device__ int g_wait_status = 0;
+
 struct LinParams {
   l3ci_linear_args a;
   int tiles, steps;                        // tiles of w, stages of K
@@ -141,6 +144,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
   const int first = blockIdx.x / S, stride = gridDim.x / S;
   const int k0 = (int)((long long)p.steps * rank / S), steps = (int)((long long)p.steps * (rank + 1) / S) - k0;   // this CTA's stages of a tile
   bool ok = true;
+  int asked = 0;                        // stages that this thread has asked for
 
   if (warp == 0) {
     // ---- producer ----
@@ -156,6 +160,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
       };
       auto load_w = [&](int s, const At& t) {
         const uint32_t dst = ring + s * Sh::kStageBytes, bar = full0 + s * 8;
+        ++asked;
         mbar_expect_tx(bar, Sh::kStageBytes);
         tma_load_4d(dst, &wmap, bar, (k0 + t.k) * kDeep, t.row, 0, t.grp, policy_w);
         if (GATED) tma_load_4d(dst + kWBytes / 2, &wmap, bar, (k0 + t.k) * kDeep, t.row, 1, t.grp, policy_w);
@@ -286,10 +291,12 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
       store_out(a, first / p.group_tiles, t, n, GATED ? lin_gate(y, u) : lin_act(y, a.act));
     }
   }
-  if (!ok && lane == 0 && a.status) atomicExch(a.status, (int)L3CI_ERR_DEVICE_WAIT);
+  if (!ok && lane == 0) atomicExch(a.status ? a.status : &g_wait_status, (int)L3CI_ERR_DEVICE_WAIT);
   __syncwarp();
   tc_fence_before();
-  __syncthreads();
+  // a wait ran out: the copies still under way land before the shared memory is given back (or their own waits run out too)
+  if (__syncthreads_or(!ok))
+    for (int f = asked > kStages ? asked - kStages : 0; f < asked; ++f) (void)mbar_wait_bounded_one(full0 + f % kStages * 8, (uint32_t)(f / kStages) & 1u);
   if (warp == 1) tmem_dealloc(tmem, Sh::kTmem);
 }
 
@@ -380,6 +387,20 @@ extern "C" int64_t l3ci_row_stride(const int64_t* sizes, const int64_t* strides,
     reach = strides[d] * sizes[d];
   }
   return stride < 0 ? width : stride;
+}
+
+extern "C" int l3ci_linear_poll(l3ci_stream_t stream_) {
+  using namespace l3ci;
+  clear_error();
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  int status = 0;
+  L3CI_CUDA_TRY(cudaMemcpyFromSymbolAsync(&status, g_wait_status, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+  L3CI_CUDA_TRY(cudaStreamSynchronize(stream));
+  if (status == 0) return L3CI_OK;
+  const int none = 0;
+  L3CI_CUDA_TRY(cudaMemcpyToSymbolAsync(g_wait_status, &none, sizeof(int), 0, cudaMemcpyHostToDevice, stream));
+  L3CI_CUDA_TRY(cudaStreamSynchronize(stream));
+  return fail(status, "linear: a bounded wait ran out in an earlier launch");
 }
 
 extern "C" int l3ci_linear(const l3ci_linear_args* a) {

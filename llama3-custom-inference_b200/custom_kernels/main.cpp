@@ -520,6 +520,15 @@ Tensor rot_embed_kv_cache(Tensor qkv, Tensor freq, Tensor cache_k, Tensor cache_
   return q_out;
 }
 
+// Status of the few-row products on the current stream of `like`'s device: 0, or 6 once after a device-side wait ran out.
+int64_t linear_status(Tensor like) {
+  TORCH_CHECK(like.is_cuda(), "like must be a CUDA tensor");
+  const c10::cuda::CUDAGuard guard(like.device());
+  const int status = l3ci_linear_poll(current_stream());
+  TORCH_CHECK(status != L3CI_ERR_CUDA, "linear_status: ", l3ci_last_error());
+  return status;
+}
+
 // Synchronises the current stream of `like`'s device and reports whether a device-side bounded
 // wait ran out in an earlier flash_attention_decode call on it (0 = fine).
 int64_t flash_decode_status(Tensor like) {
@@ -589,6 +598,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("prefill_attention", torch::wrap_pybind_function(prefill_attention), "prefill_attention", py::arg("query"),
         py::arg("keys"), py::arg("values"), py::kw_only(), py::arg("start_pos") = 0, py::arg("scale") = 0.0,
         py::arg("variant") = 0);
+  m.def("linear_status", torch::wrap_pybind_function(linear_status), "linear_status", py::arg("like"));
   m.def("flash_decode_status", torch::wrap_pybind_function(flash_decode_status), "flash_decode_status",
         py::arg("like"));
   m.def("c_abi_version", [] { return std::string(l3ci_version()); });

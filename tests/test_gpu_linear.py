@@ -169,3 +169,14 @@ def test_results_of_other_types_and_layouts_are_refused(capi, device):
         _check(out, _want(x, w, 0, capi), 64, out.dtype == torch.float32)
     # one x for all groups: not the kernel's
     assert capi.linear(x[None].expand(3, 4, 64), w[None].expand(3, 24, 64).contiguous()) is None
+
+
+def test_a_wait_that_runs_out_has_a_place_to_be_reported(capi, ext, device):
+    """Calls with and without a status word of their own leave both at zero (no wait of theirs can be made to run out: that would
+    need a copy that never lands)."""
+    g = torch.Generator(device=device).manual_seed(6)
+    x, w = torch.randn(9, 2048, generator=g, device=device).bfloat16(), torch.randn(256, 2048, generator=g, device=device).bfloat16()
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    capi.linear(x, w, status=status)
+    ext.linear(x, w)
+    assert ext.linear_status(x) == 0 and capi.load().l3ci_linear_poll(None) == capi.OK and status.item() == 0
