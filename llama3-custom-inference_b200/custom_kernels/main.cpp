@@ -393,8 +393,10 @@ Tensor linear(Tensor x, Tensor w, bool gated, bool early) {
   if (auto y = few_rows(x, w, gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE, early, false, std::nullopt)) return *y;
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y = at::linear(x, w);
+  if (!gated) return y;
   const int64_t N = w.size(0) / 2;
-  return gated ? silu_mul(y.narrow(-1, 0, N), y.narrow(-1, N, N)) : y;
+  const Tensor gate = y.narrow(-1, 0, N), up = y.narrow(-1, N, N);
+  return N > 0 && N % 8 == 0 ? silu_mul(gate, up) : at::mul(at::silu(gate), up);   // (silu_mul takes rows of whole 16-byte vectors)
 }
 
 // Greedy decode step in place: argmax of logits [B, vocab] (bf16) per row, token written to out_tokens[b, steps[b]]

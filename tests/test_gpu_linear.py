@@ -180,3 +180,12 @@ def test_a_wait_that_runs_out_has_a_place_to_be_reported(capi, ext, device):
     capi.linear(x, w, status=status)
     ext.linear(x, w)
     assert ext.linear_status(x) == 0 and capi.load().l3ci_linear_poll(None) == capi.OK and status.item() == 0
+
+
+@pytest.mark.parametrize("rows", [0, 1, 64, 65, 130])
+@pytest.mark.parametrize("N", [0, 1, 12, 16])
+def test_gated_products_of_any_width_and_number_of_rows(ext, device, rows, N):
+    g = torch.Generator(device=device).manual_seed(rows + N)
+    x, w = torch.randn(rows, 64, generator=g, device=device).bfloat16(), (torch.randn(2 * N, 64, generator=g, device=device) / 8).bfloat16()
+    got, want = ext.linear(x, w, gated=True), _ext_want(x, w, True)
+    assert got.shape == (rows, N) and bool(((got.double() - want).abs() <= 2.0 ** -6 * want.abs() + 2.0 ** -9).all())   # as above
