@@ -960,12 +960,15 @@ int scan_typed(const l3ci_recurrent_scan_args* a, cudaStream_t stream) {
   // tokens of 128 (delta rule) and 64 (time mixing) rows, measured over 16 to 128 and 32 to 256 heads; wider CTAs take longer per
   // token, but a second wave costs a whole pass (48 heads of the delta rule: 219 us as 96 wide CTAs, 316 as 192 narrow ones in two
   // waves).  Two CTAs of the delta rule fit an SM with three stages each: 96 heads then take 364 us, in whole waves 431.
+  // Of up to 64 rows the delta rule's CTAs leave room for a second one in other forms too, and two narrow ones are the faster (64 rows,
+  // 256 tokens, us by the costs above and by these: 48 heads 79, 75.5; 80 heads 88, 84; 96 heads 88, 85).
   struct Form { int C, W, per_sm, cost; };
-  const Form by_kind[2][5] = {{{8, 8, 1, 44}, {8, 4, 1, 33}, {8, 4, 2, 45}, {2, 8, 1, 20}, {2, 4, 1, 15}},
-                              {{4, 16, 1, 22}, {4, 8, 1, 14}, {2, 8, 1, 9}, {2, 4, 1, 8}, {}}};
+  const Form forms[3][6] = {{{8, 8, 1, 44}, {8, 4, 1, 33}, {8, 4, 2, 45}, {2, 8, 1, 20}, {2, 4, 1, 15}, {}},
+                            {{4, 16, 1, 22}, {4, 8, 1, 14}, {2, 8, 1, 9}, {2, 4, 1, 8}, {}, {}},
+                            {{8, 8, 1, 44}, {8, 4, 1, 33}, {8, 4, 2, 43}, {2, 8, 1, 20}, {2, 8, 2, 31}, {2, 4, 1, 15}}};
   int C = 4;
   long long best = -1;
-  for (const auto& f : by_kind[KIND]) {
+  for (const auto& f : forms[KIND == kDelta && a->D <= 64 ? 2 : KIND]) {
     const int cols = f.C * f.W, splits = (a->V + cols - 1) / (cols ? cols : 1);
     // (not half of a CTA idle, where a narrower one is left; registers and stages of two CTAs: up to 128 rows)
     if (cols == 0 || (cols > 8 && cols >= 2 * a->V) || (f.per_sm == 2 && a->D > 128)) continue;

@@ -38,3 +38,9 @@ def test_forms_agree(pkg, device, kind, H, D, batch):
         assert float((got[1][b] - want[b][1][0]).norm() / want[b][1][0].norm()) < 1e-4
         # bf16 outputs, normed: half a unit in the last place on either side
         assert float((got[0][b] - want[b][0][0]).norm() / want[b][0][0].norm()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("batch", [3, 5, 6, 12])
+@pytest.mark.parametrize("D", [32, 64])
+def test_forms_of_the_delta_rule_with_few_rows(pkg, device, D, batch):
+    test_forms_agree(pkg, device, "delta", 16, D, batch)
