@@ -337,11 +337,24 @@ Tensor silu_mul(Tensor gate, Tensor up) {
   return out;
 }
 
+// Whether the kernel for few rows is faster than torch's product (and the activation behind it).  A CTA reads its rows of x anew for
+// every tile of w and writes the results token by token, so it falls behind as rows / K grows.  Measured in chains, us (torch's) at 16,
+// 32, 48, 64 rows: w 2048 x 2048 4.6 (5.6), 5.3 (5.6), 6.0 (5.7), 6.8 (5.7); 2048 x 8192 9.9 (13.4), 10.6 (13.3), 11.6 (13.5), 12.3
+// (13.7); 2048 x 128 3.2 (2.4), 5.3 (2.4), 6.7 (2.4), 7.9 (2.6); gated 2 x 8192 x 2048 14.1 (15.8), 15.0 (15.6), 15.6 (16.3), 16.3 (15.9);
+// gelu 8192 x 2048 8.8 (10.7), 9.9 (10.9), 11.0 (11.4), 12.1 (11.5).  Without `early` it is about 1 us slower.  Few outputs (4 x 2048:
+// 5.2 (12.2) at 64 rows) and very many (128256 x 2048: 88 (95)) are its own at any number of rows.
+bool few_rows_pay(int64_t rows, int64_t K, int64_t N, int64_t groups, int64_t act, bool early) {
+  const int64_t least = early ? 16 : 8, limit = K / (early ? 64 : 128) + (act == L3CI_ACT_GELU || act == L3CI_ACT_SILU_GATE ? 16 : 0);
+  return rows <= least || rows <= limit || N * groups <= 256 || N >= 32768;
+}
+
 // act(x w^T) of few rows in one kernel (l3ci_linear): x [..., K] with w [N, K] (gated: [2 N, K], gate rows, then up rows), or groups
-// of products, x [groups, rows, K] with w [groups, N, K].  Nothing where that kernel does not apply: more rows, other types, layouts
-// or alignments.  `early`: the kernel may read w ahead of the stream's previous kernels; for a w that was complete before the last
+// of products, x [groups, rows, K] with w [groups, N, K].  Nothing where that kernel does not apply (more rows, other types, layouts
+// or alignments) or torch's product is the faster on the device (few_rows_pay).  `early`: the kernel may read w ahead of the stream's previous kernels; for a w that was complete before the last
 // one of them that waits for its predecessors ahead of letting others start.  f32: an fp32 result.  `into`: where the result goes.
-std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bool early, bool f32, const std::optional<Tensor>& into) {
+// `always`: wherever the kernel applies; for passes that wait for the host, which a launch of it costs about 4 us less than torch's
+// product (a prompt of 64 tokens, 16 layers: 1.0 ms instead of 1.4).
+std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bool early, bool f32, const std::optional<Tensor>& into, bool always) {
   if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != torch::kBFloat16 || w.scalar_type() != torch::kBFloat16 ||
       w.get_device() != x.get_device() || x.dim() < 1)
     return std::nullopt;
@@ -351,6 +364,7 @@ std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bo
   const int64_t groups = grouped ? w.size(0) : 1, rows = K * groups ? x.numel() / (K * groups) : 0;
   if (rows == 0 || rows > L3CI_LINEAR_MAX_ROWS || K % 8 || (gated && w.size(-2) % 2)) return std::nullopt;
   const int64_t N = gated ? w.size(-2) / 2 : w.size(-2);
+  if (!always && !few_rows_pay(rows, K, N, groups, act, early)) return std::nullopt;
   auto at16 = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; };
   if (N == 0 || K > INT32_MAX || w.size(-2) > INT32_MAX || groups > INT32_MAX || !w.is_contiguous() || !at16(x) || !at16(w)) return std::nullopt;
   auto row_stride = [&](const Tensor& t) {
@@ -384,13 +398,13 @@ std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bo
 }
 
 // act(x w^T) of any number of rows: few in one kernel (few_rows), more in torch's product and, gated, silu_mul.
-Tensor linear(Tensor x, Tensor w, bool gated, bool early) {
+Tensor linear(Tensor x, Tensor w, bool gated, bool early, bool always) {
   check_bf16_cuda(x, "x");
   check_bf16_cuda(w, "w");
   TORCH_CHECK(x.dim() >= 1 && w.dim() == 2 && w.size(1) == x.size(-1), "w must be [N, K] with K the last axis of x");
   TORCH_CHECK(w.get_device() == x.get_device(), "x and w on different devices");
   TORCH_CHECK(!gated || w.size(0) % 2 == 0, "a gated product takes an even number of rows of w");
-  if (auto y = few_rows(x, w, gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE, early, false, std::nullopt)) return *y;
+  if (auto y = few_rows(x, w, gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE, early, false, std::nullopt, always)) return *y;
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y = at::linear(x, w);
   if (!gated) return y;
@@ -561,9 +575,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("weight"), py::arg("eps"));
   m.def("silu_mul", torch::wrap_pybind_function(silu_mul), "silu_mul", py::arg("gate"), py::arg("up"));
   m.def("linear", torch::wrap_pybind_function(linear), "linear", py::arg("x"), py::arg("w"), py::arg("gated") = false,
-        py::arg("early") = false);
+        py::arg("early") = false, py::arg("always") = false);
   m.def("few_rows", torch::wrap_pybind_function(few_rows), "few_rows", py::arg("x"), py::arg("w"), py::arg("act") = (int64_t)L3CI_ACT_NONE,
-        py::arg("early") = false, py::arg("f32") = false, py::arg("into") = py::none());
+        py::arg("early") = false, py::arg("f32") = false, py::arg("into") = py::none(),
+        py::arg("always") = false);
   m.def("greedy_step", torch::wrap_pybind_function(greedy_step), "greedy_step", py::arg("logits"), py::arg("out_tokens"),
         py::arg("steps"), py::arg("next_input"), py::arg("positions"), py::arg("seq_lens"));
   m.def("top_p_step", torch::wrap_pybind_function(top_p_step), "top_p_step", py::arg("logits"), py::arg("out_tokens"),

@@ -35,6 +35,7 @@ import torch
 import torch.nn.functional as F
 
 from . import rope_table
+from .capi import LINEAR_MAX_ROWS
 from .kv_cache import StaticCache
 
 # Profiler range names of the reference's loop (model.py:99-109 "rot_embd" / "use_kv", :214-216 "layer", :364-366
@@ -270,13 +271,17 @@ class Llama3Decoder(DecodeLoop):
         B, T = tokens.shape
         E, D, Hq, Hkv = cfg.n_embd, cfg.head_dim, cfg.n_head, cfg.n_kv_head
         slots = slice(0, B) if slots is None else slots
+        # few rows: the weights are complete before the pass, whose first kernel is torch's; a portion of a prompt waits for the host
+        few = B * T <= LINEAR_MAX_ROWS
+        linear = partial(ext.linear, early=True, always=T > 1)
+        product = linear if few else F.linear
         x = F.embedding(tokens, w["wte"])                                            # model.py:208
         h = ext.rms_norm(x, w["h0.ln_1"], cfg.norm_eps)                                # model.py:147, 71
         for l in range(cfg.n_layer):
             p = f"h{l}."
             cache_k, cache_v = self.cache_k[l][slots], self.cache_v[l][slots]
             _nvtx_push("layer")
-            qkv = ext.linear(h, w[p + "attn"], early=True)                             # model.py:95
+            qkv = product(h, w[p + "attn"])                                            # model.py:95
             _nvtx_push("rot_embd")
             _nvtx_push("use_kv")
             q = ext.rot_embed_kv_cache(qkv, self.freqs, cache_k, cache_v, 0, Hq, Hkv,
@@ -293,16 +298,20 @@ class Llama3Decoder(DecodeLoop):
                                                cache_v.transpose(1, 2), seq_lens=seq_lens,
                                                max_ctas=self._decode_kernel(B))     # model.py:118
             y = y.transpose(1, 2).reshape(B, T, E)                                     # model.py:120
-            x, h = ext.add_rms_norm(ext.linear(y, w[p + "proj"], early=True), x, w[p + "ln_2"], cfg.norm_eps)  # :121, 147-148
-            a = ext.linear(h, w[p + "gate_up"], gated=True, early=True)                # c_fc2 | c_fc, model.py:134
-            m = ext.linear(a, w[p + "mlp_proj"], early=True)
+            x, h = ext.add_rms_norm(product(y, w[p + "proj"]), x, w[p + "ln_2"], cfg.norm_eps)  # :121, 147-148
+            if few:                                                                    # c_fc2 | c_fc, model.py:134
+                a = linear(h, w[p + "gate_up"], gated=True)
+            else:
+                gu = F.linear(h, w[p + "gate_up"])
+                a = ext.silu_mul(gu[..., :cfg.hidden_dim], gu[..., cfg.hidden_dim:])
+            m = product(a, w[p + "mlp_proj"])
             nxt = w[f"h{l + 1}.ln_1"] if l + 1 < cfg.n_layer else w["ln_f"]
             x, h = ext.add_rms_norm(m, x, nxt, cfg.norm_eps)                           # model.py:148, next 147 / 217
             _nvtx_pop()
         # the reference widens the logits to fp32 first (model.py:226); the widening is monotonic, so the argmax
         # of the bf16 values is the same index
         # model.py:225; the head is tied to the embedding (model.py:189) unless the checkpoint brought its own
-        return self.logits(h, w.get("lm_head", w["wte"]), want, partial(ext.linear, early=True))
+        return self.logits(h, w.get("lm_head", w["wte"]), want, linear)
 
 
 def config_from_hf(hf_config) -> DecoderConfig:

@@ -3,6 +3,7 @@ decoders other than Llama-3.  As in capi.py, torch owns the memory and names the
 from __future__ import annotations
 
 import ctypes as C
+from functools import partial
 from pathlib import Path
 
 import torch
@@ -136,33 +137,64 @@ def _extension():
     return _ext
 
 
-def few_rows(x, w, act: int = ACT_NONE, out_dtype=None, out=None, early: bool = False):
+def few_rows(x, w, act: int = ACT_NONE, out_dtype=None, out=None, early: bool = False, always: bool = False):
     """act(x w^T) of few rows in one kernel (`l3ci_linear`), groups of products where w is [groups, N, K]; None where it does
-    not apply.  `early`: w may be read ahead of the stream's previous kernels; for weights that were complete before the last one
-    of them that waits for its predecessors ahead of letting others start (a model's, in its forward pass)."""
+    not apply or torch's product is the faster on the device.  `early`: w may be read ahead of the stream's previous kernels; for
+    weights that were complete before the last one of them that waits for its predecessors ahead of letting others start (a model's,
+    in its forward pass).  `always`: wherever it applies, for passes that wait for the host."""
     if out_dtype not in (None, torch.bfloat16, torch.float32):
         raise ValueError("the result is bf16 or fp32")
-    if x.numel() > LINEAR_MAX_ROWS * x.shape[-1] * (x.shape[0] if w.dim() == 3 else 1):   # (a prompt's: the host is what it waits for)
-        return None
-    return _extension().few_rows(x, w, act, early, out_dtype == torch.float32, out)
+    return _extension().few_rows(x, w, act, early, out_dtype == torch.float32, out, always)
 
 
-def linear(x, w, act: int = ACT_NONE, early: bool = False):
-    """act(x w^T); ACT_SILU_GATE: w holds gate rows, then up rows.  `early`: see `few_rows`."""
-    if x.numel() <= LINEAR_MAX_ROWS * x.shape[-1]:
-        y = _extension().few_rows(x, w, act, early)
-        if y is not None:
-            return y
+def _many_rows(x, w, act: int = ACT_NONE):
     y = F.linear(x, w)
     return y if act == ACT_NONE else gelu_(y) if act == ACT_GELU else tanh_(y) if act == ACT_TANH else gated_act(y)
 
 
-def product32(x, w, early: bool = False):
-    """x [rows, K] w^T in fp32: products of two bf16 numbers are exact, the sum is not rounded to bf16.  `early`: see `few_rows`."""
+def linear(x, w, act: int = ACT_NONE, early: bool = False, always: bool = False):
+    """act(x w^T); ACT_SILU_GATE: w holds gate rows, then up rows.  `early`, `always`: see `few_rows`."""
+    y = few_rows(x, w, act, early=early, always=always)
+    return _many_rows(x, w, act) if y is None else y
+
+
+def product32(x, w, early: bool = False, always: bool = False):
+    """x [rows, K] w^T in fp32: products of two bf16 numbers are exact, the sum is not rounded to bf16.  `early`, `always`: see
+    `few_rows`."""
     if x.dtype == torch.float32:
         return torch.mm(x, w.t())
-    y = few_rows(x, w, out_dtype=torch.float32, early=early)
-    return torch.mm(x, w.t(), out_dtype=torch.float32) if y is None else y
+    y = few_rows(x, w, out_dtype=torch.float32, early=early, always=always)
+    return _many_rows32(x, w) if y is None else y
+
+
+def _many_rows32(x, w):
+    return torch.mm(x, w.t()) if x.dtype == torch.float32 else torch.mm(x, w.t(), out_dtype=torch.float32)
+
+
+class Products:
+    """`linear`, `few_rows` and `product32` with a model's own weights in a forward pass: they are complete before it, and its first
+    kernel waits ahead of letting others start, so that they may be read early."""
+
+    def __init__(self, **how):
+        self.linear, self.few_rows, self.product32 = (partial(f, early=True, **how) for f in (linear, few_rows, product32))
+
+
+class _ManyRows:
+    """The same in a pass over more rows than the kernel takes, which pays for no check."""
+    linear, product32 = staticmethod(_many_rows), staticmethod(_many_rows32)
+
+    @staticmethod
+    def few_rows(*_, **__):
+        return None
+
+
+_STEP, _PORTION, _MANY = Products(), Products(always=True), _ManyRows
+
+
+def products(B: int, T: int):
+    """What a pass over T tokens of B sequences multiplies with: a step (replayed from a graph) the fastest on the device, a portion of
+    a prompt, which waits for the host, the cheapest for the host."""
+    return _MANY if B * T > LINEAR_MAX_ROWS else _STEP if T == 1 else _PORTION
 
 
 def embed_dyn_tanh(tokens, table, weight, bias, alpha: float):

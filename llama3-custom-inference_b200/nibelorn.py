@@ -16,7 +16,6 @@ attention on the tensor cores.
 from __future__ import annotations
 
 from dataclasses import dataclass
-from functools import partial
 from typing import Optional
 
 import torch
@@ -25,9 +24,6 @@ import torch.nn.functional as F
 from . import mixers, rope_table
 from .decode_loop import DecodeLoop, full_precision_products, nvtx_range
 
-# Products with the model's own weights, complete before a forward pass, whose first kernel waits ahead of letting others start.
-_linear = partial(mixers.linear, early=True)
-_few_rows = partial(mixers.few_rows, early=True)
 
 EXPAND_FROM = 128   # portions of at least this many tokens expand the latents (a query block of the tcgen05 kernel)
 
@@ -240,7 +236,8 @@ class NibelornDecoder(DecodeLoop):
         B, T, _ = h.shape
         H, D, R, C, V = m.heads, m.dim, m.rot_dim, m.kv_rank, m.vdim
         cache = self.cache.layers[l]["latent"][slots]
-        qd = _linear(h, w.proj)
+        ops = mixers.products(B, T)
+        qd = ops.linear(h, w.proj)
         mixers.latent_cache(qd, self._tables[R, m.rot_base], w.latent_norm, self.cfg.eps, cache, positions, H, D, R, C)
         q = qd[..., :H * (D + R)].view(B, T, H, D + R)
         out = torch.empty(B, T, H, V, dtype=h.dtype, device=h.device)
@@ -252,7 +249,7 @@ class NibelornDecoder(DecodeLoop):
                              qb=q[..., D:], kb=k_rot, scale=m.scale, start_pos=start_pos, variant=mixers.TC)
         else:
             q_rows = q[..., :D].reshape(B * T, H, D).transpose(0, 1)
-            q_lat = _few_rows(q_rows, w.uk_t)                                                      # [H, B * T, C]
+            q_lat = ops.few_rows(q_rows, w.uk_t)                                                   # [H, B * T, C]
             if q_lat is None:
                 q_lat = torch.bmm(q_rows, w.uk)
             o_lat = torch.empty_like(q_lat)
@@ -260,7 +257,7 @@ class NibelornDecoder(DecodeLoop):
                              o_lat.view(H, B, T, C).permute(1, 2, 0, 3), positions, qb=q[..., D:],
                              kb=cache[:, :, None, C:C + R], scale=m.scale, start_pos=start_pos)
             heads_out = out.view(B * T, H, V).transpose(0, 1)
-            if _few_rows(o_lat, w.uv, out=heads_out) is None:
+            if ops.few_rows(o_lat, w.uv, out=heads_out) is None:
                 torch.bmm(o_lat, w.uv.transpose(1, 2), out=heads_out)
         return out.view(B, T, H * V)
 
@@ -274,7 +271,8 @@ class NibelornDecoder(DecodeLoop):
         H, G, D, V = m.heads, m.kv_heads, m.dim, m.vdim
         planes = self.cache.layers[l]
         k, v = planes["k"][slots], planes["v"][slots]
-        p = _linear(h, w.proj)
+        ops = mixers.products(B, T)
+        p = ops.linear(h, w.proj)
         at_k, at_v, at_g = 2 * H * D, 2 * (H + G) * D, 2 * (H + G) * D + G * V
         mixers.kv_cache_write(p, at_k, at_v, k, v, positions)
         out = torch.empty(B, T, H, V, dtype=h.dtype, device=h.device)
@@ -291,6 +289,7 @@ class NibelornDecoder(DecodeLoop):
         B, T = tokens.shape
         slots = slice(0, B) if slots is None else slots
         start_pos = start_pos if T > 1 else -1       # one token: positions live on the device alone (CUDA graph)
+        ops = mixers.products(B, T)
         with full_precision_products():
             x, h = mixers.embed_dyn_tanh(tokens, self.embed, *self.w[0].norm1.args)
             for l, layer in enumerate(layers):
@@ -298,11 +297,11 @@ class NibelornDecoder(DecodeLoop):
                 following = self.w[l + 1].norm1 if l + 1 < len(layers) else self.final_norm
                 with nvtx_range("layer"):
                     mix = self._latent if isinstance(layer.mixer, LatentAttention) else self._differential
-                    y = _linear(mix(l, h, positions, slots, start_pos), w.o)
+                    y = ops.linear(mix(l, h, positions, slots, start_pos), w.o)
                     if layer.ff is not None:
                         h = mixers.add_dyn_tanh(y, x, *w.norm2.args)
-                        y = _linear(_linear(h, w.ff_up, mixers.ACT_GELU), w.ff_down)
+                        y = ops.linear(ops.linear(h, w.ff_up, mixers.ACT_GELU), w.ff_down)
                     h = mixers.add_dyn_tanh(y, x, *following.args)
                     if keep is not None:
                         keep.append(x.clone())
-            return self.logits(h, self.head, want, _linear)
+            return self.logits(h, self.head, want, mixers.products(B, 1).linear)

@@ -16,7 +16,6 @@ those of the experts are kernels of their own, the others torch's (cuBLAS).
 from __future__ import annotations
 
 from dataclasses import dataclass
-from functools import partial
 from typing import Optional
 
 import torch
@@ -25,10 +24,6 @@ from . import mixers
 from .decode_loop import DecodeLoop, full_precision_products, nvtx_range
 from .kv_cache import State
 
-# Products with the model's own weights, complete before a forward pass, whose first kernel waits ahead of letting others start.
-_linear = partial(mixers.linear, early=True)
-_few_rows = partial(mixers.few_rows, early=True)
-_product32 = partial(mixers.product32, early=True)
 
 POSITION_BASE = 10000.0     # sinusoidal positions
 SLOPE_RANGE = 8.0           # head h of H takes 2^(-8 (h + 1) / H) off a score per position of distance
@@ -325,7 +320,7 @@ class RupotarDecoder(DecodeLoop):
     def _attention(self, m: Attention, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, _ = h.shape
         qw, kw = m.heads * m.dim, m.kv_heads * m.dim
-        qkv = _linear(h, w.proj)
+        qkv = mixers.products(B, T).linear(h, w.proj)
         k, v = planes["k"], planes["v"]
         mixers.qk_norm_cache(qkv, qw, kw, w.q_norm, w.k_norm, self.cfg.eps, k, v, positions)
         out = torch.empty(B, T, m.heads, m.vdim, dtype=h.dtype, device=h.device)
@@ -336,9 +331,10 @@ class RupotarDecoder(DecodeLoop):
     def _channel_delta(self, m: ChannelDelta, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, E = h.shape
         H, G, D, V = m.heads, m.kv_heads, m.dim, m.vdim
-        p = _linear(h, w.proj)
+        ops = mixers.products(B, T)
+        p = ops.linear(h, w.proj)
         low = p.view(B * T, -1)[:, w.at_low:]
-        up = _linear(low, w.up).view(B, T, -1)
+        up = ops.linear(low, w.up).view(B, T, -1)
         qk, v, beta, decay = mixers.delta_inputs(p, p[..., w.at_b:w.at_b + H], up[..., :H * D], w.conv, w.a_log, w.dt_bias, planes["tail"],
                                                  positions, H, G, D, V, UNIT_EPS)
         gate = up[..., w.at_gate:w.at_gate + H * V].view(B, T, H, V)
@@ -348,20 +344,21 @@ class RupotarDecoder(DecodeLoop):
     def _wkv(self, m: TimeMix, w: _LayerWeights, planes: dict, h, positions, start_pos: int):
         B, T, E = h.shape
         mixes = mixers.token_shift(h, w.mu, planes["last"], positions).view(len(MIXES), B * T, E)
-        rkvg = _few_rows(mixes[:4], w.rkvg)
+        ops = mixers.products(B, T)
+        rkvg = ops.few_rows(mixes[:4], w.rkvg)
         if rkvg is None:
             rkvg = torch.bmm(mixes[:4], w.rkvg.transpose(1, 2))
         r, k, v, g = rkvg.view(4, B, T, m.heads, m.dim)
-        decay = _linear(_linear(mixes[4], w.w1, mixers.ACT_TANH), w.w2).view(B, T, m.heads, m.dim)
+        decay = ops.linear(ops.linear(mixes[4], w.w1, mixers.ACT_TANH), w.w2).view(B, T, m.heads, m.dim)
         return mixers.recurrent_scan(r, k, v, decay, planes["state"], positions, w.norm, g, act=mixers.SILU, eps=self.cfg.eps, bonus=w.u,
                                      g_bias=w.w0)
 
     # ---- feed-forward: what `residual_norm` adds ---------------------------------------------------------------
-    def _feed_forward(self, ff, w: _LayerWeights, h):
+    def _feed_forward(self, ff, w: _LayerWeights, h, ops):
         if isinstance(ff, Dense):
-            return {"y": _linear(_linear(h, w.gate_up, mixers.ACT_SILU_GATE), w.down)}
+            return {"y": ops.linear(ops.linear(h, w.gate_up, mixers.ACT_SILU_GATE), w.down)}
         rows = h.view(-1, h.shape[-1])
-        experts, ranks, weights, counts = mixers.moe_route(_product32(rows, w.router), w.router_b, ff.top)
+        experts, ranks, weights, counts = mixers.moe_route(ops.product32(rows, w.router), w.router_b, ff.top)
         x, part_rows = mixers.moe_gather(rows, experts, ranks, counts)
         a = mixers.moe_gemm(x, w.gate_up, counts, limit=ff.limit, alpha=EXPERT_ALPHA)
         return {"y": mixers.moe_gemm(a, w.down, counts), "part_rows": part_rows, "part_weights": weights}
@@ -375,6 +372,7 @@ class RupotarDecoder(DecodeLoop):
         E = cfg.width
         slots = slice(0, B) if slots is None else slots
         start_pos = start_pos if T > 1 else -1       # one token: positions live on the device alone (CUDA graph)
+        ops = mixers.products(B, T)
         # [x; embedding output], the input of a pass
         cat = torch.empty(B, T, 2 * E, dtype=self.dtype, device=self.device) if cfg.loop is not None else None
 
@@ -395,13 +393,13 @@ class RupotarDecoder(DecodeLoop):
                 mix = self._attention if isinstance(m, Attention) else self._channel_delta if isinstance(m, ChannelDelta) else self._wkv
                 with nvtx_range("layer"):
                     if run.step is not None:
-                        h = mixers.residual_norm(_product32(cat.view(B * T, 2 * E), self.loop_in), x, dtype=self.dtype, reset=True, step=self.loop_step[run.step],
+                        h = mixers.residual_norm(ops.product32(cat.view(B * T, 2 * E), self.loop_in), x, dtype=self.dtype, reset=True, step=self.loop_step[run.step],
                                                  pre=w.norm1, eps=eps)
-                    added, post = {"y": _linear(mix(m, w, planes, h, positions, start_pos), w.o)}, w.norm1b
+                    added, post = {"y": ops.linear(mix(m, w, planes, h, positions, start_pos), w.o)}, w.norm1b
                     if ff is not None:
                         h = mixers.residual_norm(**added, x=x, dtype=self.dtype, post=post, pre=w.norm2, eps=eps)
-                        added, post = self._feed_forward(ff, w, h), w.norm2b
+                        added, post = self._feed_forward(ff, w, h, ops), w.norm2b
                     h = mixers.residual_norm(**added, x=x, dtype=self.dtype, post=post, eps=eps, **before(r + 1))
                     if keep is not None:
                         keep.append(x.clone())
-            return self.logits(h, self.head, want, _linear)
+            return self.logits(h, self.head, want, mixers.products(B, 1).linear)
