@@ -60,8 +60,8 @@ L3CI_API uint64_t l3ci_set_device_wait_limit_ns(uint64_t ns);
  * runs without clusters, RMSNorm,
  * SiLU*mul, the rotary kernels, the token-choice steps) are launched so that their grid may be set up on the SMs
  * while the previous kernel of the stream is still draining; each of them waits (griddepcontrol.wait) for that
- * kernel's completion and the visibility of its writes before its first global access, so results and stream order
- * are what they are without it: what overlaps is the launch itself and the start of the CTAs (about a microsecond
+ * kernel's completion and the visibility of its writes before its first global access (l3ci_linear with `early` reads
+ * its weights before), so results and stream order are what they are without it: what overlaps is the launch itself and the start of the CTAs (about a microsecond
  * per launch between kernels of this library, e.g. RoPE + cache write -> attention in a decode step, also inside a
  * captured CUDA graph).  No counterpart in the reference (legacy-stream <<<>>> launches). */
 L3CI_API int l3ci_set_programmatic_launch(int on);

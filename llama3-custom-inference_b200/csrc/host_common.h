@@ -66,7 +66,8 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // with the attribute that lets the grid be scheduled before the previous kernel of the stream has finished.  Kernels
 // launched this way call pdl_wait() (ptx_sm100.cuh) before they touch global memory: it returns once the previous
 // kernel has completed and its writes are visible, so the overlap is the launch itself, the CTAs' start and whatever
-// a kernel does before its first global access; a kernel launched the plain way passes through it at once.
+// a kernel does before its first global access; a kernel launched the plain way passes through it at once.  One
+// kernel reads ahead of it: linear_rows_kernel its weights, if the caller vouches for them (l3ci_linear_args.early).
 template <typename... Params, typename... Args>
 cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};

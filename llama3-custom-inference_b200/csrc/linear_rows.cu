@@ -4,7 +4,7 @@
 // A product of up to 64 rows is bound by reading w once.  What kept the library's kernels from that rate inside a decode step was not
 // the stream itself but its edges: each product began to read its weights only when the kernel before it had ended, and drained
 // before the next one began.  Here
-//   * the weights take the 128-row side of the tcgen05 product and the tokens the narrow one (16, 32 or 64 columns): a CTA moves
+//   * the weights take the 128-row side of the tcgen05 product and the tokens the narrow one (8, 16, 32 or 64): a CTA moves
 //     128 rows of w, 64 columns at a time, through a ring of bulk tensor copies, and the tensor cores keep up with a fraction of
 //     their rate, so nothing but the copies is timed;
 //   * w does not depend on the kernel before (`early`): the ring is filled before griddepcontrol.wait, and only the tokens are asked
@@ -14,9 +14,9 @@
 //     the order of the ranks (results do not depend on timing);
 //   * the activation that follows is done on the fp32 sums: gelu, tanh, or silu(gate) * up of a stacked matrix, a tile then being
 //     64 gate rows and the 64 up rows of the same outputs.
-// Measured one after another on weights beyond L2, us (the library's kernel): one row, w 2048 x 2048 3.6 (8.3), 2048 x 8192 8.5 (20.9),
-// gated 2 x 8192 x 2048 13.1 (13.8 without the gate), 128256 x 2048 82 (80); 64 rows 6.7 (5.7), 11.8 (13.4), 15.9 (13.8), 89 (93).  In a
-// step of the 1B model behind 4001 tokens, where the ring fills early: 686 us, 1121 with the library's.
+// Measured in chains on weights beyond L2, us (the library's product and its activation): one row, w 2048 x 2048 3.7 (8.1), 2048 x 8192
+// 9.2 (20.2), gated 2 x 8192 x 2048 13.7 (15.3), 128256 x 2048 82 (81); 64 rows 6.8 (5.7), 12.3 (13.7), 16.3 (15.9), 88 (95): the
+// extension leaves the shapes that lose to the library.  A step of the 1B model behind 4001 tokens: 690 us, 1103 to 1127 with the library's.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -28,7 +28,8 @@ __device__ __forceinline__ float gated_activation(float z, float u, float limit,
   return z / (1.f + expf(-z)) * u;
 }
 
-// The same to bf16 accuracy (relative error about 1e-6), without the divide's branches.
+// The same by the short forms of exp and the division: relative error about 2^-21 near 0, growing by 2^-23 for every unit that z (alpha z)
+// lies below it, and 0 where exp(-z) exceeds 2^126 (z below about -87.4).
 __device__ __forceinline__ float gated_activation_fast(float z, float u, float limit, float alpha) {
   if (limit > 0.f) {
     z = fminf(z, limit);

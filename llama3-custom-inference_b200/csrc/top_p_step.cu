@@ -6,21 +6,21 @@
 // every entry whose PRECEDING mass exceeds p, renormalises, draws with torch.multinomial and maps the draw back
 // through the sort permutation: half a dozen full-vocabulary kernels per generated token.  The nucleus does not need
 // the order, only its boundary: entry i is kept iff the mass of the entries that sort strictly before it is <= p.
-// Here row b's CTA (top_p_step_kernel)
-//   1. reduces (max, sum of exp) online in one pass over the row,
-//   2. finds the boundary of the nucleus by a two-level search over the bit pattern of the bf16 LOGITS (the weight
-//      e_i = exp((x_i - max) / T) is monotone in the logit, and a bf16 logit has only 65 536 patterns): each level
-//      histograms the MASS per byte value in shared memory (2^-40 fixed point, integer atomics: exact sums) and a
-//      block-wide suffix scan finds the byte in which the preceding mass crosses p * sum; entries whose logit equals the boundary pattern tie exactly and are kept in
-//      index order as long as the mass before them is <= p * sum (a stable descending sort puts them in that order),
-//   3. draws u in [0, 1) from a Philox4x32-10 stream keyed by (seed; row, step) and walks the nucleus in INDEX order
-//      (a block-wide scan of per-thread nucleus mass, then the owning thread walks its 128 entries) to the entry
-//      where the running mass passes u * nucleus mass.  Any fixed order gives the multinomial distribution; index
-//      order needs no permutation.
-// Batches of up to half the SMs run as a cluster of two CTAs per row (see peer_value below).
-// Rows of up to 8 x 65 528 logits take the same steps by counts of keys instead of masses (top_p_count_kernel below), the longer ones these.
-// It then writes the token exactly as l3ci_greedy_step does.  Weights are recomputed from the logits in every pass
-// (same expression, same bits; the row is 256 KB and stays in L2), nothing is sorted and nothing leaves the SM.
+// The weight e_i = exp((x_i - max) / T) is a function of the bf16 LOGIT, monotone, and a bf16 logit has only 65 536 patterns.
+//
+// top_p_count_kernel (rows of up to 8 x 65 528 logits, but for short ones of one CTA): a cluster of 8, 4 or 2 CTAs per row in small
+// batches, one CTA in larger ones,
+//   1. counts the keys (order-preserving patterns) of the row in shared memory in one pass, its share of the row then in registers,
+//   2. finds the boundary of the nucleus digit by digit of the key from count x weight (2^-40 fixed point, exact sums); entries whose
+//      logit equals the boundary pattern tie exactly and are kept in index order as long as the mass before them is <= p * sum (a
+//      stable descending sort puts them in that order),
+//   3. draws u in [0, 1) from a Philox4x32-10 stream keyed by (seed; row, step) and finds the entry where the mass of the nucleus in
+//      INDEX order passes u * nucleus mass: the warp, the 32 x 8 entries, the entry.  Any fixed order gives the multinomial
+//      distribution; index order needs no permutation.
+// top_p_step_kernel (longer rows, and short ones of one CTA): the same integers by masses.  Each level of the search is a pass over
+// the row that histograms the MASS per byte value in shared memory (integer atomics); weights are recomputed from the logits in every
+// pass (same expression, same bits; the row stays in L2).
+// Either writes the token exactly as l3ci_greedy_step does; nothing is sorted and nothing leaves the SMs.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>

@@ -5,8 +5,9 @@ are dynamic tanh (tanh(alpha x) w + b).  A layer may borrow another layer's weig
 own.  Sizes and constants come from config.json or a tensor's shape.
 
 Generation, requests, the cache and the CUDA graph of a decode step are `decode_loop.DecodeLoop`'s; this file holds the
-configuration, the weight layout and one forward pass over the mixer kernels (mixers.py).  Matrix products are torch's
-(cuBLAS), fused where inputs are shared: query and latent down-projection, or query, key, value and gate, are one.
+configuration, the weight layout and one forward pass over the mixer kernels (mixers.py).  Matrix products of
+few rows (a decode step's) are a kernel of this package, of many rows torch's (cuBLAS); they are fused where inputs are
+shared: query and latent down-projection, or query, key, value and gate, are one.
 
 Latent attention runs in two forms.  Decode and short portions keep the keys and values in the latent: the query is
 multiplied into it (q_n W_uk), scores and the weighted sum run over the cached rows alone, and W_uv is applied to the

@@ -11,7 +11,7 @@ Feed-forward: gated silu, or experts with a clamped activation.  Sizes and const
 
 Generation, requests, the cache and the CUDA graph of a decode step are `decode_loop.DecodeLoop`'s; this file holds the
 configuration, the weight layout and one forward pass over the kernels (mixers.py).  Matrix products of one input are fused;
-those of the experts are kernels of their own, the others torch's (cuBLAS).
+those of the experts and of few rows (a decode step's) are kernels of this package, the others torch's (cuBLAS).
 """
 from __future__ import annotations
 
