@@ -337,15 +337,15 @@ Tensor silu_mul(Tensor gate, Tensor up) {
   return out;
 }
 
-// Whether the kernel for few rows is faster than torch's product (and the activation behind it).  A CTA reads its rows of x anew for
-// every tile of w and writes the results token by token, so it falls behind as rows / K grows.  Measured in chains, us (torch's) at 16,
-// 32, 48, 64 rows: w 2048 x 2048 4.6 (5.6), 5.3 (5.6), 6.0 (5.7), 6.8 (5.7); 2048 x 8192 9.9 (13.4), 10.6 (13.3), 11.6 (13.5), 12.3
-// (13.7); 2048 x 128 3.2 (2.4), 5.3 (2.4), 6.7 (2.4), 7.9 (2.6); gated 2 x 8192 x 2048 14.1 (15.8), 15.0 (15.6), 15.6 (16.3), 16.3 (15.9);
-// gelu 8192 x 2048 8.8 (10.7), 9.9 (10.9), 11.0 (11.4), 12.1 (11.5).  Without `early` it is about 1 us slower.  Few outputs (4 x 2048:
-// 5.2 (12.2) at 64 rows) and very many (128256 x 2048: 88 (95)) are its own at any number of rows.
+// Whether the kernel for few rows is taken where torch's product could be.  A CTA reads its rows of x anew for every tile of w and
+// writes the results token by token, so it falls behind as rows / K grows.  Measured in chains, us (torch's) at 16, 32, 48, 64 rows: w
+// 2048 x 2048 4.6 (5.6), 5.3 (5.6), 6.0 (5.7), 6.8 (5.7); 2048 x 8192 9.9 (13.4), 10.6 (13.3), 11.6 (13.5), 12.3 (13.7); 2048 x 128
+// 3.2 (2.4), 5.3 (2.4), 6.7 (2.4), 7.9 (2.6).  Without `early` it is about 1 us slower.  Few outputs (4 x 2048: 5.2 (12.2) at 64 rows)
+// and very many (128256 x 2048: 88 (95)) are its own at any number of rows, and so are fused activations, which it applies to sums
+// that are not rounded to bf16: gated 2 x 8192 x 2048 14.1 (15.8), 15.0 (15.6), 15.6 (16.3), 16.3 (15.9); gelu 8192 x 2048 8.8 (10.7),
+// 9.9 (10.9), 11.0 (11.4), 12.1 (11.5).
 bool few_rows_pay(int64_t rows, int64_t K, int64_t N, int64_t groups, int64_t act, bool early) {
-  const int64_t least = early ? 16 : 8, limit = K / (early ? 64 : 128) + (act == L3CI_ACT_GELU || act == L3CI_ACT_SILU_GATE ? 16 : 0);
-  return rows <= least || rows <= limit || N * groups <= 256 || N >= 32768;
+  return act != L3CI_ACT_NONE || rows <= (early ? 16 : 8) || rows <= K / (early ? 64 : 128) || N * groups <= 256 || N >= 32768;
 }
 
 // act(x w^T) of few rows in one kernel (l3ci_linear): x [..., K] with w [N, K] (gated: [2 N, K], gate rows, then up rows), or groups
