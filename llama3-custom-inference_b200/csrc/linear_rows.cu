@@ -16,7 +16,7 @@
 //     64 gate rows and the 64 up rows of the same outputs.
 // Measured in chains on weights beyond L2, us (the library's product and its activation): one row, w 2048 x 2048 3.7 (8.1), 2048 x 8192
 // 9.2 (20.2), gated 2 x 8192 x 2048 13.7 (15.3), 128256 x 2048 82 (81); 64 rows 6.8 (5.7), 12.3 (13.7), 16.3 (15.9), 88 (95): the
-// extension leaves the shapes that lose to the library.  A step of the 1B model behind 4001 tokens: 690 us, 1103 to 1127 with the library's.
+// extension leaves the shapes that lose to the library.  A step of the 1B model behind 4001 tokens: 696 us, 1103 to 1127 with the library's.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
