@@ -1012,6 +1012,9 @@ def bench_end_to_end(args, ext, pkg, dev, rank, world):
     gen_bytes = (G - 1) * weight_bytes + kv_bytes_per_token * sum(P + t for t in range(1, G))
     peak, peak_kind = hbm_peak()
     achieved = gen_bytes * steps / (ms * 1e-3) / 1e9
+    # a step's products that are this library's: all of them up to 32 sequences, up to 64 gate and up, down and the head
+    products = 65 if B <= 32 else 33 if B <= 64 else 0
+    per_step = 33 + 16 + 16 + products + (0 if products else 16) + 1
     line = {
         "metric": "Llama-3.2-1B decode tokens/sec", "value": value, "unit": "tokens/s", "n_gpus": world, "steps": steps,
         "warmup": 1, "ms_per_step": ms / steps, "higher_is_better": True, "scaling": "weak",
@@ -1029,12 +1032,12 @@ def bench_end_to_end(args, ext, pkg, dev, rank, world):
                      "algorithmic_bytes_per_launch": gen_bytes // max(1, G - 1),
                      "note": "weights once per decode step + cached K/V of the step, averaged over the generation; the time "
                              "includes the prefill pass"},
-        "launches_per_decode_step": {"this_library": 131, "detail": "33 RMSNorm (32 fused with the residual add), 16 fused RoPE + cache write, 16 flash-decode, "
-                                     "65 products (16 with SiLU*mul), 1 greedy step; plus the embedding lookup"},
+        "launches_per_decode_step": {"this_library": per_step, "detail": "33 RMSNorm (32 fused with the residual add), 16 fused RoPE + cache write, 16 flash-decode, "
+                                     f"{products} products (16 with SiLU*mul), 1 greedy step; plus the embedding lookup and {65 - products} products of cuBLAS"},
         "e2e": e2e,
-        # per decode step: 33 RMSNorm (32 with the residual add) + 16 fused RoPE/cache + 16 flash-decode + 65 products
-        # + 1 greedy-step launches of this library; the prefill pass: norms, RoPE, attention, SiLU*mul and the head's product
-        "gpu_launches": decode_steps * 131 + steps * (33 + 16 * 3 + 1), "clocks": sampler.summary(),
+        # per decode step: 33 RMSNorm (32 with the residual add) + 16 fused RoPE/cache + 16 flash-decode + the products
+        # (else 16 SiLU*mul) + 1 greedy-step launches of this library; the prefill pass: norms, RoPE, attention, SiLU*mul and the head's product
+        "gpu_launches": decode_steps * per_step + steps * (33 + 16 * 3 + 1), "clocks": sampler.summary(),
     }
     if cpu is not None:
         line["cpu_baseline"] = cpu
@@ -1138,9 +1141,9 @@ def bench_nibelorn(args, ext, pkg, dev, rank, world):
                    "global_batch": 64 * world, "seq_len": 1024, "parallelism": "replicas x%d" % world,
                    "l2": "weights and cache of a step exceed L2"},
         "kernels": mixer_kernel_table(ext, pkg, dev, latent, differential) if rank == 0 else None,
-        # embedding, 16 x (cache write, attention, two norms), products: 8 x (6 + 4) and the head, token choice; the split merges
-        # come on top
-        "gpu_launches": line["steps"] * (1 + 16 * 4 + 8 * 10 + 1 + 1),
+        # embedding, 16 x (cache write, attention, two norms), products of 64 rows: 16 x 2 of the feed-forward and the head, token
+        # choice; the split merges come on top
+        "gpu_launches": line["steps"] * (1 + 16 * 4 + 16 * 2 + 1 + 1),
     }
 
 
@@ -1175,9 +1178,9 @@ def bench_rupotar(args, ext, pkg, dev, rank, world):
                    "l2": "weights and cache of a step exceed L2"},
         "kernels": rupotar_kernel_table(ext, pkg, dev, cfg) if rank == 0 else None,
         # per step: embedding, token choice; per run two norms; per attention two (split merges on top), delta two, time mixing two
-        # (token shift, step); experts four; per pass of the loop one more norm; products: 8 x 2 of attention, 4 x 3 of the delta
-        # rule, 4 x 4 of time mixing, 8 x 2 dense, 8 routers, 2 of the loop, the head
-        "gpu_launches": line["steps"] * (2 + 16 * 2 + 8 * 2 + 4 * 2 + 4 * 2 + 8 * 4 + 2 + 8 * 2 + 4 * 3 + 4 * 4 + 8 * 2 + 8 + 2 + 1),
+        # (token shift, step); experts four; per pass of the loop one more norm; products of 64 rows: 4 of time mixing, 8 x 2 dense, 8
+        # routers, 2 of the loop, the head
+        "gpu_launches": line["steps"] * (2 + 16 * 2 + 8 * 2 + 4 * 2 + 4 * 2 + 8 * 4 + 2 + 4 + 8 * 2 + 8 + 2 + 1),
     }
 
 
