@@ -1024,7 +1024,7 @@ def bench_end_to_end(args, ext, pkg, dev, rank, world):
         "config": {"workload": f"C5 random-init Llama-3.2-1B architecture, batch {B}/GPU, prompt {P}, {G} greedy tokens",
                    "global_batch": B * world, "parallelism": "replicas x%d" % world,
                    "l2": "working set per decode step (2.5 GB weights + KV cache) >> 126 MB L2",
-                   "note": "products of the prompt are cuBLAS via torch; those of a decode step, RMSNorm (+ residual add), SiLU*mul, RoPE + cache write, decode attention and the greedy step are this "
+                   "note": "products of the prompt, and beyond 32 sequences those of the attention layers, are cuBLAS via torch; the others, RMSNorm (+ residual add), SiLU*mul, RoPE + cache write, decode attention and the greedy step are this "
                            "repository's kernels; the decode step is replayed from a CUDA graph",
                    "reference_published_rtx4060_tokens_per_s": 2041.67},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
