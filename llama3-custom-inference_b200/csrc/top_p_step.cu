@@ -10,12 +10,12 @@
 //
 // top_p_count_kernel (rows of up to 8 x 65 528 logits, but for short ones of one CTA): a cluster of 8, 4 or 2 CTAs per row in small
 // batches, one CTA in larger ones,
-//   1. counts the keys (order-preserving patterns) of the row in shared memory in one pass, its share of the row then in registers,
+//   1. counts the keys (order-preserving patterns) of the row in shared memory in one pass,
 //   2. finds the boundary of the nucleus digit by digit of the key from count x weight (2^-40 fixed point, exact sums); entries whose
 //      logit equals the boundary pattern tie exactly and are kept in index order as long as the mass before them is <= p * sum (a
 //      stable descending sort puts them in that order),
 //   3. draws u in [0, 1) from a Philox4x32-10 stream keyed by (seed; row, step) and finds the entry where the mass of the nucleus in
-//      INDEX order passes u * nucleus mass: the warp, the 32 x 8 entries, the entry.  Any fixed order gives the multinomial
+//      INDEX order passes u * nucleus mass: the warp, the entry of its list.  Any fixed order gives the multinomial
 //      distribution; index order needs no permutation.
 // top_p_step_kernel (longer rows, and short ones of one CTA): the same integers by masses.  Each level of the search is a pass over
 // the row that histograms the MASS per byte value in shared memory (integer atomics); weights are recomputed from the logits in every
@@ -85,8 +85,11 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 template <typename T>
 __device__ __forceinline__ T ld_peer(const T* mine, uint32_t peer) {
@@ -409,20 +412,23 @@ top_p_step_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lon
 // ---- the same step by counts ---------------------------------------------------------------------------------------------------
 // The weight is a function of the logit's key, so the mass of a key is its count times its weight, exactly: the row needs one
 // histogram of counts over all 65 536 keys (16 bits each, 128 KB of shared memory) instead of a pass of three 64-bit-mass atomics
-// per search level, and the weights are evaluated once per key that occurs.  The CTA's share of the row stays in registers (64
-// entries a thread), is read from memory once, and the masses in index order are taken from there.  All sums are the integers of
-// the kernel above: same boundary, same ties, same draw, bit for bit.
-//   64 rows of 128 256 logits: 39 us; 82 with the masses' histograms, whose atomics met on a few dozen bins.
+// per search level, and the weights are evaluated once per key that occurs.  A second pass over the row (from L2) lists the few entries of
+// the nucleus.  All sums are the integers of the kernel above: same boundary, same ties, same draw, bit for bit.
+//   64 rows of 128 256 logits: 22.1 us; 82 with the masses' histograms, whose atomics met on a few dozen bins; 34.3 with the row in
+// registers, every lane weighing its own entries in unrolled loops: instruction fetch, and warps that waited for the lane with the most.
+// Left is the counting: 14 of 43 thousand cycles, shared-memory atomics of 32 lanes on 32 random banks.
 constexpr int kKeyWords = 32768;                  // two keys' counts each
-constexpr int kCountSmem = kKeyWords * 4;
-constexpr int kHeld = 8;                          // 16-byte groups of a thread
+constexpr int kGroup = 16;                        // neighbouring entries of a lane, at most
+constexpr int kListed = kWarp * kGroup;           // entries of a warp's list
+constexpr int kDense = 256;                       // of a round's 512, beyond which they are weighed without a list
+constexpr int kCountSmem = (kKeyWords + kTopPWarps * kListed) * 4;
 constexpr long long kMaxShare = 8191;             // groups of a CTA: a count of all its entries fits 16 bits
 constexpr long long kFewLogits = 4096;            // logits of a one-CTA row that are few
 // A weight is about 2^40 at most, except that of a logit without a number for one (NaN; an infinity or a value whose scaled
 // difference to the maximum overflows): 2^63 or more, so that masses wrap.  Masses of weights below 2^44 do not, over the 524 224
 // logits of the longest row.  A row with a larger weight is marked by this bit of its count.
 constexpr uint32_t kOddWeight = 1u << 12;         // in a weight's high word
-constexpr long long kOddRow = 1ll << 40;
+constexpr u64 kOddRow = 1u << 24;                 // above the entries of the longest row, with room for eight CTAs' marks
 
 __device__ __forceinline__ uint32_t bits_key(uint32_t u) {   // logit_key of a bf16 pattern
   if (u == 0x8000u) return 0x8000u;
@@ -443,13 +449,21 @@ __device__ __forceinline__ T warp_exclusive_scan(T v, T& total) {
   total = __shfl_sync(kFullMask, inc, kWarp - 1);
   return inc - v;
 }
-// Sum of the CTAs' slots, and of those in front of this CTA, by every warp; behind a barrier of the cluster.  (One lane per CTA: a
-// read of a peer's shared memory by every thread took longer than the sums.)
+// Writes a value into the place of `mine` in a peer's shared memory.  (Of the few values of a meeting, which the CTAs then read from their
+// own memory: a read of a peer's takes as long as the barrier once more.  The masses of the digits are read: 256 of them took longer to write.)
+template <typename T>
+__device__ __forceinline__ void st_peer(T* mine, uint32_t peer, T v) {
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "32- or 64-bit values");
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(peer));
+  if constexpr (sizeof(T) == 4) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(*reinterpret_cast<uint32_t*>(&v)) : "memory");
+  else asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(*reinterpret_cast<u64*>(&v)) : "memory");
+}
+// Sum of the CTAs' values, one per lane from slot 0 on, and of those in front of this CTA.
 template <int kCtas, typename T>
-__device__ __forceinline__ T slots_sum(const T* slot, uint32_t rank, T& front) {
+__device__ __forceinline__ T slots_sum(const T* slots, uint32_t rank, T& front) {
   const uint32_t lane = threadIdx.x & 31;
-  T v = T(0);
-  if (lane < (uint32_t)kCtas) v = kCtas == 1 || lane == rank ? *slot : ld_peer(slot, lane);
+  const T v = lane < (uint32_t)kCtas ? slots[lane] : T(0);
   T all;
   front = __shfl_sync(kFullMask, warp_exclusive_scan<T>(v, all), (int)rank);
   return all;
@@ -495,16 +509,17 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
                    float* __restrict__ nucleus_mass, long long stand_in_run) {
   extern __shared__ __align__(16) uint32_t counts[];   // word k / 2 holds the counts of keys k (even: low half)
   __shared__ float redf[kTopPWarps];
-  __shared__ u64 own_mass[256], digit_mass[256];
-  __shared__ long long warp_eq[kTopPWarps], warp_over[kTopPWarps];
+  __shared__ u64 own_mass[256], digit_mass[256];   // of this CTA, of all
+  __shared__ u64 warp_ties[kTopPWarps];          // ties << 32 | entries above them
   __shared__ u64 warp_mass[kTopPWarps];
-  __shared__ float s_max;
-  __shared__ u64 s_mass;         // this CTA's, for the peers
-  __shared__ long long s_eq, s_over;
+  uint32_t* s_list = counts + kKeyWords;         // entries of the nucleus, by warp
+  __shared__ float s_max[kCtas];
+  __shared__ u64 s_mass[kCtas], s_ties[kCtas];   // the CTAs'; of s_ties bit 24 onwards: CTAs with an odd row
   // what the first warp finds for all
   __shared__ int s_pick[2], s_odd, s_first;
   __shared__ u64 s_above[2], s_total, s_budget, s_mass_front, s_mass_total;
-  __shared__ long long s_eq_front, s_eq_total, s_over_total;
+  __shared__ long long s_eq_front, s_eq_kept, s_over_total;
+  __shared__ int s_any_odd;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = kCtas > 1 ? cluster_rank() : 0u;
   for (int i = tid; i < kKeyWords / 4; i += kTopPBlock) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -512,6 +527,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     s_odd = 0;
     s_first = kTopPWarps;
   }
+  if constexpr (kCtas > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (waited for ahead of the first write to a peer: all of them have started)
   pdl_launch_dependents();  // the next one may be set up while this one runs
   pdl_wait();               // the previous kernel of the stream has completed; its writes are visible
   const long long b = blockIdx.x / kCtas;
@@ -519,72 +535,85 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   const unsigned short* row_bits = reinterpret_cast<const unsigned short*>(row);
   const long long step = steps ? steps[b] : 0;            // (barriers of all CTAs follow before one of them writes it)
   const bool vectors = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
-  // groups of 8 entries: the CTA's run, in it the warp's, there 32 neighbours at a time
-  const long long groups = (vocab + kVecElems - 1) / kVecElems;
-  const long long g_end = groups * (rank + 1) / kCtas, g_cta = groups * rank / kCtas;
-  const int per_warp = (int)((g_end - g_cta + kTopPWarps - 1) / kTopPWarps);
-  const long long g_warp = g_cta + (long long)warp * per_warp;
-  const int n_warp = (int)min((long long)per_warp, max(0ll, g_end - g_warp));   // groups of this warp
-  auto entries = [&](int it) {                            // of this lane's group of round `it`
-    if (it * 32 + lane >= n_warp) return 0;
-    const long long left = vocab - (g_warp + it * 32 + lane) * kVecElems;
-    return (int)(left < kVecElems ? left : kVecElems);
-  };
-  uint4 held[kHeld];
-#pragma unroll
-  for (int it = 0; it < kHeld; ++it) {
-    held[it] = make_uint4(0u, 0u, 0u, 0u);
+  // vectors of 8 entries: the CTA's run, in it the warp's, an even number; there a round of 32 neighbouring groups at a time
+  const long long vecs = (vocab + kVecElems - 1) / kVecElems;
+  const long long v_end = vecs * (rank + 1) / kCtas, v_cta = vecs * rank / kCtas;
+  const int per_warp = (int)((v_end - v_cta + 2 * kTopPWarps - 1) / (2 * kTopPWarps)) * 2;
+  const long long v_warp = v_cta + (long long)warp * per_warp, first = v_warp * kVecElems;
+  const int n_warp = (int)max(0ll, min(min((long long)per_warp, v_end - v_warp) * kVecElems, vocab - first));   // entries of this warp
+  // (short runs: half a group each, so that all lanes have some)
+  const int group = per_warp <= kWarp ? kGroup / 2 : kGroup, round = kWarp * group;
+  auto entries = [&](int it) { return max(0, min(group, n_warp - it * round - lane * group)); };   // of this lane's group of round `it`
+  struct Group { uint4 v[2]; };
+  auto load = [&](int it) {                               // zeros where the lane has none
+    Group g;
     const int n = entries(it);
-    if (n == 0) continue;
-    const long long at = (g_warp + it * 32 + lane) * kVecElems;
-    if (vectors && n == kVecElems) {
-      held[it] = __ldg(reinterpret_cast<const uint4*>(row + at));
-    } else {
-      uint32_t w[4] = {0u, 0u, 0u, 0u};
+    const unsigned short* at = row_bits + first + it * round + lane * group;
 #pragma unroll
-      for (int j = 0; j < kVecElems; ++j)
-        if (j < n) w[j / 2] |= (uint32_t)__ldg(row_bits + at + j) << (16 * (j & 1));
-      held[it] = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int i = 0; i < 2; ++i) {
+      g.v[i] = make_uint4(0u, 0u, 0u, 0u);
+      const int left = n - i * kVecElems;
+      if (vectors && left >= kVecElems) {
+        g.v[i] = __ldg(reinterpret_cast<const uint4*>(at) + i);
+      } else if (left > 0) {
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int j = 0; j < kVecElems; ++j)
+          if (j < left) w[j / 2] |= (uint32_t)__ldg(at + i * kVecElems + j) << (16 * (j & 1));
+        g.v[i] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
     }
-  }
+    return g;
+  };
+  // Calls visit(round, group) for the warp's rounds, the next group under way.  (Loops that are not unrolled: a launch meets a cold
+  // instruction cache, and unrolled by rounds, with the row in registers, fetching the kernel took a third of its time.)
+  auto rounds = [&](auto&& visit) {
+    Group next = {};
+#pragma unroll 1
+    for (int it = -1; it * round < n_warp; ++it) {
+      const Group g = next;
+      next = load(it + 1);
+      if (it >= 0) visit(it, g);
+    }
+  };
   const uint32_t r = philox_first((uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)b, (uint32_t)(b >> 32), (uint32_t)step,
                                   (uint32_t)(step >> 32));
-  auto bits_of = [&](const uint4& v, int j) {
-    const uint32_t w = j < 2 ? v.x : j < 4 ? v.y : j < 6 ? v.z : v.w;
+  auto bits_of = [&](const Group& g, int j) {
+    const uint4 v = j < kVecElems ? g.v[0] : g.v[1];
+    const uint32_t w = (j & 4) ? (j & 2) ? v.w : v.z : (j & 2) ? v.y : v.x;
     return (j & 1) ? w >> 16 : w & 0xffffu;
   };
   __syncthreads();                                        // the counts are cleared
 
   // ---- 1. counts of the keys and the maximum ----
   float m = -INFINITY;
-#pragma unroll
-  for (int it = 0; it < kHeld; ++it) {
-    if (it * 32 >= n_warp) break;
+  rounds([&](int it, const Group& g) {
     const int n = entries(it);
-    const uint4 v = held[it];
-    if (n == kVecElems && v.x == v.y && v.y == v.z && v.z == v.w && v.x >> 16 == (v.x & 0xffffu)) {   // a flat row's lanes would queue at one word
-      const uint32_t key = bits_key(v.x & 0xffffu);
+    const uint4 v = g.v[0], u = g.v[1];
+    if (n == kGroup && v.x == v.y && v.y == v.z && v.z == v.w && v.x >> 16 == (v.x & 0xffffu) && u.x == v.x && u.y == v.x && u.z == v.x && u.w == v.x) {
+      const uint32_t key = bits_key(v.x & 0xffffu);       // a flat row's lanes would queue at one word
       m = fmaxf(m, __uint_as_float(v.x << 16));
-      atomicAdd(counts + (key >> 1), 8u << (16 * (key & 1)));
-      continue;
+      atomicAdd(counts + (key >> 1), (uint32_t)kGroup << (16 * (key & 1)));
+      return;
     }
 #pragma unroll
-    for (int j = 0; j < kVecElems; ++j) {
+    for (int j = 0; j < kGroup; ++j) {
       if (j >= n) break;
-      const uint32_t u = bits_of(v, j), key = bits_key(u);
+      const uint32_t u = bits_of(g, j), key = bits_key(u);
       m = fmaxf(m, __uint_as_float(u << 16));
       atomicAdd(counts + (key >> 1), 1u << (16 * (key & 1)));
     }
-  }
+  });
   m = group_max<kWarp>(m);
   if (lane == 0) redf[warp] = m;
   __syncthreads();
   m = group_max<kWarp>(redf[lane]);
   if constexpr (kCtas > 1) {
-    if (tid == 0) s_max = m;
+    cluster_wait();
+    if (tid < kCtas) st_peer(&s_max[rank], (uint32_t)tid, m);
     cluster_barrier();
-    if (lane < kCtas) m = ld_peer(&s_max, (uint32_t)lane);
-    m = group_max<kWarp>(m);
+#pragma unroll
+    for (int c = 0; c < kCtas; ++c) m = fmaxf(m, s_max[c]);
   }
   RowView rv;
   rv.scale = inv_temperature * 1.4426950408889634f;
@@ -601,13 +630,11 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     if (__any_sync(kFullMask, (c.x | c.y | c.z | c.w) != 0u)) {
       const uint32_t w[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
+      for (int k = 0; k < 8; ++k) {     // (no branches: the eight are under way together)
         const uint32_t n = (k & 1) ? w[k / 2] >> 16 : w[k / 2] & 0xffffu;
-        if (n) {
-          const u64 each = rv.weight(key_logit((uint32_t)(d * 256 + lane * 8 + k)));
-          any |= (uint32_t)(each >> 32);
-          q += (u64)n * each;
-        }
+        const u64 each = rv.weight(key_logit((uint32_t)(d * 256 + lane * 8 + k)));
+        any |= n ? (uint32_t)(each >> 32) : 0u;
+        q += (u64)n * each;
       }
 #pragma unroll
       for (int k = 16; k >= 1; k /= 2) q += __shfl_xor_sync(kFullMask, q, k);
@@ -615,8 +642,8 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     if (lane == 0) own_mass[d] = q;
   }
   if (any >= kOddWeight) s_odd = 1;
-  __syncthreads();
   if constexpr (kCtas > 1) cluster_barrier();
+  else __syncthreads();
   if (tid < 256) {
     u64 h = own_mass[tid];
 #pragma unroll
@@ -664,87 +691,140 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   const u64 w_star = rv.weight(key_logit(key_star));
 
   // ---- 3. the nucleus in index order: per warp, ties at the boundary counted ----
-  // Few entries are in it: compares build a mask, and only the entries of its bits are weighed.
+  // Few entries are in it: packed compares build masks, the entries of their bits go into the warp's list, and its lanes weigh one each.
+  // A round that has more than half of its entries in it is weighed as it is (rows of 128256 logits of one size: 32 us; by lists 59).
   // order(u): signed, -0 just below +0; at a boundary of 0 both tie
   auto order = [](uint32_t u) { const int t = (int)(short)u; return t ^ ((t >> 31) & 0x7fff); };
   const int star = all_kept ? -40000 : (int)key_star - 0x8000;
   const int star_low = star == 0 ? -1 : star;
-  auto lane_sums = [&](int it, u64& w, int& eq, int& over) {   // this lane's group of round `it`
-    w = 0;
+  const bool plain = !s_odd && !all_kept;                 // every entry has a number: bf16's own compare orders them (and ties -0 and +0)
+  auto at_least = [&](int it, const Group& g) {           // bit j: entry j of the group is in the nucleus or ties
     const int n = entries(it);
-    uint32_t in = 0u, at_least = 0u;
+    uint32_t in = 0u;
+    if (plain) {
+      const uint32_t star2 = ((key_star & 0x8000u) ? (key_star & 0x7fffu) : (~key_star & 0xffffu)) * 0x10001u;
+      const __nv_bfloat162 limit = *reinterpret_cast<const __nv_bfloat162*>(&star2);
+      uint32_t in_high = 0u;                              // of the words' high halves, 16 bits up
 #pragma unroll
-    for (int j = 0; j < kVecElems; ++j) {
-      const int t = order(bits_of(held[it], j));
-      in |= t > star ? 1u << j : 0u;
-      at_least |= t >= star_low ? 1u << j : 0u;
+      for (int k = 0; k < kGroup / 2; ++k) {
+        const uint4 v = g.v[k / 4];
+        const uint32_t w = k % 4 == 0 ? v.x : k % 4 == 1 ? v.y : k % 4 == 2 ? v.z : v.w;
+        const uint32_t mask = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w), limit);
+        in |= mask & (1u << (2 * k));
+        in_high |= mask & (0x20000u << (2 * k));
+      }
+      in = (in | in_high >> 16) & ((1u << n) - 1u);
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < n; ++j) in |= (order(bits_of(g, j)) >= star_low ? 1u : 0u) << j;
     }
-    const uint32_t real = (1u << n) - 1u;
-    eq = __popc(at_least & ~in & real);
-    in &= real;
-    over = __popc(in);
-    while (in) {
-      w += rv.weight(__uint_as_float(bits_of(held[it], __ffs(in) - 1) << 16));
-      in &= in - 1;
+    return in;
+  };
+  auto weigh = [&](const Group& g, uint32_t in, u64& w, int& ties) {   // entry by entry
+    w = 0;
+    ties = 0;
+#pragma unroll
+    for (int j = 0; j < kGroup; ++j) {
+      const uint32_t u = bits_of(g, j);
+      const bool tie = order(u) <= star, mine = in >> j & 1u;
+      const u64 each = rv.weight(__uint_as_float(u << 16));
+      w += mine && !tie ? each : 0;
+      ties += mine && tie;
     }
   };
+  uint32_t* list = s_list + warp * kListed;               // in index order: pattern, place in the warp's run << 16
+  auto entry = [&](int i, int n, bool& tie) {             // entry i of the list's n, and whether it ties at the boundary
+    const uint32_t e = i < n ? list[i] : 0u;
+    tie = i < n && order(e & 0xffffu) <= star;
+    return e;
+  };
   u64 w_warp = 0;
-  long long eq_warp = 0, over_warp = 0;
-  {
-    int eq_lane = 0, over_lane = 0;
-#pragma unroll
-    for (int it = 0; it < kHeld; ++it) {
-      if (it * 32 >= n_warp) break;
+  int eq_warp = 0, over_warp = 0, listed = 0;
+  bool whole = true;                                      // the list has them all
+  rounds([&](int it, const Group& g) {
+    uint32_t in = at_least(it, g);
+    int all;
+    int at = warp_exclusive_scan<int>(__popc(in), all);
+    if (all > kDense || listed + all > kListed) {
       u64 w;
-      int eq, over;
-      lane_sums(it, w, eq, over);
+      int ties;
+      weigh(g, in, w, ties);
       w_warp += w;
-      eq_lane += eq;
-      over_lane += over;
+      ties = __reduce_add_sync(kFullMask, ties);
+      eq_warp += ties;
+      over_warp += all - ties;
+      whole = false;
+      return;
     }
-#pragma unroll
-    for (int k = 16; k >= 1; k /= 2) w_warp += __shfl_xor_sync(kFullMask, w_warp, k);
-    eq_warp = __reduce_add_sync(kFullMask, eq_lane);
-    over_warp = __reduce_add_sync(kFullMask, over_lane);
+    at += listed;
+    listed += all;
+#pragma unroll 1
+    for (; in; in &= in - 1) {
+      const int j = __ffs(in) - 1;
+      list[at++] = bits_of(g, j) | (uint32_t)(it * round + lane * group + j) << 16;
+    }
+  });
+  __syncwarp();
+#pragma unroll 1
+  for (int i = 0; i < listed; i += kWarp) {
+    bool tie;
+    const uint32_t e = entry(i + lane, listed, tie);
+    const u64 w = rv.weight(__uint_as_float(e << 16));
+    w_warp += i + lane < listed && !tie ? w : 0;
+    const int ties = __popc(__ballot_sync(kFullMask, tie));
+    eq_warp += ties;
+    over_warp += min(listed - i, kWarp) - ties;
   }
+#pragma unroll
+  for (int k = 16; k >= 1; k /= 2) w_warp += __shfl_xor_sync(kFullMask, w_warp, k);
   if (lane == 0) {
-    warp_eq[warp] = eq_warp;
+    warp_ties[warp] = (u64)eq_warp << 32 | (u64)over_warp;
     warp_mass[warp] = w_warp;
-    warp_over[warp] = over_warp;
   }
   __syncthreads();
   if (warp == 0) {
-    long long eq_all, over_all;
-    u64 mass_all;
-    const long long eq = warp_exclusive_scan<long long>(warp_eq[lane], eq_all);
+    u64 ties_all, mass_all;
+    const u64 ties = warp_exclusive_scan<u64>(warp_ties[lane], ties_all);
     const u64 mass = warp_exclusive_scan<u64>(warp_mass[lane], mass_all);
-    over_all = warp_over[lane];
-#pragma unroll
-    for (int k = 16; k >= 1; k /= 2) over_all += __shfl_xor_sync(kFullMask, over_all, k);
-    warp_eq[lane] = eq;                                   // from here on: of the warps in front
+    warp_ties[lane] = ties;                               // from here on: of the warps in front
     warp_mass[lane] = mass;
-    if (lane == 0) { s_eq = eq_all; s_mass = mass_all; s_over = over_all + (s_odd ? kOddRow : 0); }
+    if (s_odd) ties_all |= kOddRow;
+    if (lane < kCtas) {
+      if constexpr (kCtas > 1) {
+        st_peer(&s_ties[rank], (uint32_t)lane, ties_all);
+        st_peer(&s_mass[rank], (uint32_t)lane, mass_all);
+      } else {
+        s_ties[0] = ties_all;
+        s_mass[0] = mass_all;
+      }
+    }
   }
   __syncwarp();
   if constexpr (kCtas > 1) cluster_barrier();
   if (warp == 0) {
-    long long eq_in_front, none;
-    u64 mass_in_front;
-    const long long eq_all = slots_sum<kCtas>(&s_eq, rank, eq_in_front), over_all = slots_sum<kCtas>(&s_over, rank, none);
-    const u64 mass_all = slots_sum<kCtas>(&s_mass, rank, mass_in_front);
+    u64 ties_in_front, mass_in_front;
+    const u64 ties_all = slots_sum<kCtas>(s_ties, rank, ties_in_front);
+    const u64 mass_all = slots_sum<kCtas>(s_mass, rank, mass_in_front);
+    const long long eq_all = (long long)(ties_all >> 32), eq_in_front = (long long)(ties_in_front >> 32);
+    const int over_all = (int)(ties_all & (kOddRow - 1));
+    // entries equal to the boundary, in index order: the j-th is kept while above + j * w* <= budget
+    long long kept = 0;
+    if (!all_kept && eq_all > 0) {
+      kept = eq_all;
+      if (w_star > 0) {
+        const u64 room = budget > above ? budget - above : 0;
+        // (a division of 64 bits only where not all are kept)
+        if (__umul64hi(w_star, (u64)(eq_all - 1)) != 0 || w_star * (u64)(eq_all - 1) > room) kept = (long long)(room / w_star) + 1;
+      }
+      if (kept > eq_all) kept = eq_all;
+    }
     if (lane == 0) {
-      s_eq_total = eq_all; s_eq_front = eq_in_front; s_over_total = over_all;
+      s_eq_kept = kept; s_eq_front = eq_in_front; s_over_total = over_all; s_any_odd = (ties_all & 0xffffffffu) >= kOddRow;
       s_mass_total = mass_all; s_mass_front = mass_in_front;
     }
   }
   __syncthreads();
-  const long long eq_total = s_eq_total, eq_before = warp_eq[warp] + s_eq_front;
-  // entries equal to the boundary, in index order: the j-th is kept while above + j * w* <= budget
-  long long eq_kept = 0;
-  if (!all_kept && eq_total > 0) {
-    eq_kept = w_star > 0 ? (long long)((budget > above ? budget - above : 0) / w_star) + 1 : eq_total;
-    if (eq_kept > eq_total) eq_kept = eq_total;
-  }
+  const long long eq_kept = s_eq_kept, eq_before = (long long)(warp_ties[warp] >> 32) + s_eq_front;
   auto kept_of = [&](long long n_eq, long long seen) {    // of n_eq ties behind `seen` others
     const long long k = eq_kept - seen;
     return k < 0 ? 0 : k > n_eq ? n_eq : k;
@@ -758,7 +838,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   // one warp of one CTA has the target in its run; an empty nucleus has no such warp: the first one stands in
   bool found = mass_warp > 0 && mass_before <= target && target < mass_before + mass_warp;
   bool stand_in = mass_total == 0 && rank == 0 && warp == 0;
-  if (s_over_total >= kOddRow) {                          // masses may have wrapped: any number of warps may have it, the first takes it
+  if (s_any_odd) {                          // masses may have wrapped: any number of warps may have it, the first takes it
     if (found && lane == 0) atomicMin(&s_first, warp);
     __syncthreads();
     if constexpr (kCtas > 1) cluster_barrier();
@@ -773,36 +853,50 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
     if (found) {
       u64 run = mass_before;
       long long seen = eq_before;
-#pragma unroll
-      for (int it = 0; it < kHeld; ++it) {
-        if (it * 32 >= n_warp || __any_sync(kFullMask, tok >= 0)) break;
-        u64 w, w_all;
-        int eq, over, eq_all;
-        lane_sums(it, w, eq, over);
-        const int ties_front = warp_exclusive_scan<int>(eq, eq_all);
-        w += (u64)kept_of(eq, seen + ties_front) * w_star;
-        u64 mine = run + warp_exclusive_scan<u64>(w, w_all);
-        if (w > 0 && mine <= target && target < mine + w) {
-          long long eq_seen = seen + ties_front;
-          const int n = entries(it);
-#pragma unroll
-          for (int j = 0; j < kVecElems; ++j) {
-            if (j >= n || tok >= 0) break;
-            const uint32_t u = bits_of(held[it], j), key = bits_key(u);
-            bool in = all_kept || key > key_star;
-            if (!in && key == key_star) { in = eq_seen < eq_kept; ++eq_seen; }
-            if (in) {
-              mine += rv.weight(__uint_as_float(u << 16));
-              if (mine > target) tok = (g_warp + it * 32 + lane) * kVecElems + j;
+      if (whole) {
+#pragma unroll 1
+        for (int i = 0; i < listed && !__any_sync(kFullMask, tok >= 0); i += kWarp) {
+          bool tie;
+          const uint32_t e = entry(i + lane, listed, tie);
+          const unsigned ties = __ballot_sync(kFullMask, tie);
+          u64 w = rv.weight(__uint_as_float(e << 16)), w_all;
+          if (tie) w = seen + __popc(ties & ((1u << lane) - 1u)) < eq_kept ? w_star : 0;
+          if (i + lane >= listed) w = 0;
+          const u64 mine = run + warp_exclusive_scan<u64>(w, w_all);
+          if (w > 0 && mine <= target && target < mine + w) tok = first + (e >> 16);
+          run += w_all;
+          seen += __popc(ties);
+        }
+      } else {
+        rounds([&](int it, const Group& g) {
+          if (__any_sync(kFullMask, tok >= 0)) return;
+          const uint32_t in = at_least(it, g);
+          u64 w, w_all;
+          int ties, ties_all;
+          weigh(g, in, w, ties);
+          const int ties_front = warp_exclusive_scan<int>(ties, ties_all);
+          w += (u64)kept_of(ties, seen + ties_front) * w_star;
+          u64 mine = run + warp_exclusive_scan<u64>(w, w_all);
+          if (w > 0 && mine <= target && target < mine + w) {
+            long long eq_seen = seen + ties_front;
+#pragma unroll 1
+            for (int j = 0; j < kGroup && tok < 0; ++j) {
+              const uint32_t u = bits_of(g, j);
+              bool mine_too = in >> j & 1u;
+              if (mine_too && order(u) <= star) { mine_too = eq_seen < eq_kept; ++eq_seen; }
+              if (mine_too) {
+                mine += rv.weight(__uint_as_float(u << 16));
+                if (mine > target) tok = first + it * round + lane * group + j;
+              }
             }
           }
-        }
-        run += w_all;
-        seen += eq_all;
+          run += w_all;
+          seen += ties_all;
+        });
       }
       // one lane has it (of an odd row any number: the first of them, or the first entry of the warp)
       const unsigned who = __ballot_sync(kFullMask, tok >= 0);
-      if (who == 0 && lane == 0) tok = g_warp * kVecElems;
+      if (who == 0 && lane == 0) tok = first;
       if (who != 0 && lane != __ffs(who) - 1) tok = -1;
     } else if (lane == 0) {
       // of the first entries of the row, as many as a thread of the kernel above walks: the one that passes the target, or the last
@@ -810,6 +904,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
       tok = 0;
       long long eq_seen = 0;
       u64 run = 0;
+#pragma unroll 1
       for (long long i = 0; i < stand_in_run && i < vocab; ++i) {
         const uint32_t u = row_bits[i], key = bits_key(u);
         bool in = all_kept || key > key_star;
@@ -833,7 +928,7 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
       if (nucleus_mass) nucleus_mass[b] = Z > 0 ? (float)((double)mass_total / (double)Z) : 0.f;
     }
   }
-  if (nucleus_count && tid == 0 && rank == 0) nucleus_count[b] = (int)(s_over_total % kOddRow + eq_kept);
+  if (nucleus_count && tid == 0 && rank == 0) nucleus_count[b] = (int)(s_over_total + eq_kept);
   if constexpr (kCtas > 1) cluster_barrier();   // no CTA leaves while a peer may still read its shared memory
 }
 
@@ -898,18 +993,21 @@ extern "C" int l3ci_top_p_step(const void* logits, int64_t rows, int64_t vocab, 
     cfg.blockDim = dim3(kTopPBlock);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    int n = 0;
     if (c > 1) {
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)c;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-    } else {
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      attr[n].id = cudaLaunchAttributeClusterDimension;
+      attr[n].val.clusterDim.x = (unsigned)c;
+      attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+      ++n;
+    }
+    if (programmatic_launch_enabled()) {
+      attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[n].val.programmaticStreamSerializationAllowed = 1;
+      ++n;
     }
     cfg.attrs = attr;
-    cfg.numAttrs = c > 1 || programmatic_launch_enabled() ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, lp, (long long)vocab, (long long)row_stride, inv_t, top_p, (unsigned long long)seed,
                               reinterpret_cast<long long*>(out_tokens), (long long)out_stride, (long long)out_cols,
                               reinterpret_cast<long long*>(steps), reinterpret_cast<long long*>(next_input), positions, seq_lens,
