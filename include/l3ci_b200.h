@@ -112,6 +112,9 @@ typedef struct l3ci_linear_args {
   l3ci_stream_t stream;
 } l3ci_linear_args;
 L3CI_API int l3ci_linear(const l3ci_linear_args* args);
+/* The same; with a limit above 0 the gated activation is z sigmoid(alpha z) (u + 1) of z = min(gate, limit), u = clamp(up, -limit, limit)
+ * (experts whose rows lie in places of their own, one group each). */
+L3CI_API int l3ci_linear_gated(const l3ci_linear_args* args, float limit, float alpha);
 /* Waits for `stream`; L3CI_ERR_DEVICE_WAIT, once, if a launch of l3ci_linear without a status word of its own gave up on this device
  * (should never happen). */
 L3CI_API int l3ci_linear_poll(l3ci_stream_t stream);

@@ -141,6 +141,10 @@ L3CI_API int l3ci_moe_route(const float* logits, const float* bias, int32_t* exp
 L3CI_API int l3ci_moe_gather(const void* h, const int32_t* experts, const int32_t* ranks, const int32_t* counts, void* out,
                              int32_t* part_rows, int64_t rows, int64_t width, int32_t n_experts, int32_t top, int32_t dtype,
                              l3ci_stream_t stream);
+/* The same into places by expert: at = expert * rows + rank (a token has an expert once, so none has more than `rows` pairs); places
+ * without a pair keep what they held.  For few tokens, whose experts' products are then groups of l3ci_linear_gated. */
+L3CI_API int l3ci_moe_gather_places(const void* h, const int32_t* experts, const int32_t* ranks, void* out, int32_t* part_rows, int64_t rows,
+                                    int64_t width, int32_t n_experts, int32_t top, int32_t dtype, l3ci_stream_t stream);
 /* Products of the sorted rows x [rows, K] with their experts' matrices w.
  *   gated == 0: w [E, N, K], out [rows, N] = x w^T.
  *   gated == 1: w [E, 2, N, K] (gate, up), out [rows, N] = the clamped activation of l3ci_gated_act of x gate^T, x up^T.

@@ -12,7 +12,7 @@
 //     A CTA takes at most half of an SM's shared memory, so that it can start beside the CTAs of the kernel before;
 //   * few rows of w: a cluster of 2, 4 or 8 CTAs shares a tile's columns, and adds its parts through distributed shared memory in
 //     the order of the ranks (results do not depend on timing);
-//   * the activation that follows is done on the fp32 sums: gelu, tanh, or silu(gate) * up of a stacked matrix, a tile then being
+//   * the activation that follows is done on the fp32 sums: gelu, tanh, or silu(gate) * up (or its clamped form) of a stacked matrix, a tile then being
 //     64 gate rows and the 64 up rows of the same outputs.
 // Measured in chains on weights beyond L2, us (the library's product and its activation): one row, w 2048 x 2048 3.7 (8.1), 2048 x 8192
 // 9.2 (20.2), gated 2 x 8192 x 2048 13.7 (15.3), 128256 x 2048 82 (81); 64 rows 6.8 (5.7), 12.3 (13.7), 16.3 (15.9), 88 (95): the
@@ -21,7 +21,10 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "host_common.h"
+#include "mixer_types.cuh"
 #include "ptx_sm100.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.h"
@@ -60,6 +63,7 @@ struct LinParams {
   l3ci_linear_args a;
   int tiles, steps;                        // tiles of w, stages of K
   int group_tiles;                         // tiles of one group
+  float limit, alpha;                      // of a gated activation
 };
 
 __device__ __forceinline__ float lin_act(float z, int act) {
@@ -67,7 +71,6 @@ __device__ __forceinline__ float lin_act(float z, int act) {
   if (act == L3CI_ACT_TANH) return tanhf(z);
   return z;
 }
-__device__ __forceinline__ float lin_gate(float z, float u) { return z / (1.f + expf(-z)) * u; }
 
 __device__ __forceinline__ void store_out(const l3ci_linear_args& a, int grp, int t, int n, float v) {
   const long long at = grp * a.out_sg + t * a.out_st + n;
@@ -238,7 +241,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
               if (r < 64 && n < a.N)
 #pragma unroll
                 for (int i = 0; i < kSwap; ++i)
-                  if (c + h + i < rows) store_out(a, grp, c + h + i, n, lin_gate(__uint_as_float(v[h + i]), swap[i * 64 + r]));
+                  if (c + h + i < rows) store_out(a, grp, c + h + i, n, gated_activation(__uint_as_float(v[h + i]), swap[i * 64 + r], p.limit, p.alpha));
               output_warps_meet();
             }
           } else if (n < a.N) {
@@ -288,7 +291,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
         y += parts[t * kTile + s * kSlice + j];
         if (GATED) u += parts[t * kTile + s * kSlice + kOwn + j];
       }
-      store_out(a, first / p.group_tiles, t, n, GATED ? lin_gate(y, u) : lin_act(y, a.act));
+      store_out(a, first / p.group_tiles, t, n, GATED ? gated_activation(y, u, p.limit, p.alpha) : lin_act(y, a.act));
     }
   }
   if (!ok && lane == 0) atomicExch(a.status ? a.status : &g_wait_status, (int)L3CI_ERR_DEVICE_WAIT);
@@ -301,11 +304,13 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
 }
 
 template <int NP, int S, bool GATED>
-int launch(const l3ci_linear_args* a, cudaStream_t stream) {
+int launch(const l3ci_linear_args* a, float limit, float alpha, cudaStream_t stream) {
   using Sh = LinShape<NP>;
   constexpr int kOuts = GATED ? kTile / 2 : kTile;
   LinParams p = {};
   p.a = *a;
+  p.limit = limit;
+  p.alpha = alpha;
   p.group_tiles = (a->N + kOuts - 1) / kOuts;
   p.tiles = p.group_tiles * a->groups;
   p.steps = (a->K + kDeep - 1) / kDeep;
@@ -348,7 +353,7 @@ int launch(const l3ci_linear_args* a, cudaStream_t stream) {
 }
 
 template <int NP, bool GATED>
-int launch_split(const l3ci_linear_args* a, cudaStream_t stream) {
+int launch_split(const l3ci_linear_args* a, float limit, float alpha, cudaStream_t stream) {
   const long long tiles = (a->N + (GATED ? kTile / 2 : kTile) - 1) / (GATED ? kTile / 2 : kTile) * (long long)a->groups;
   int split = a->split;
   if (split == 0) {
@@ -360,10 +365,10 @@ int launch_split(const l3ci_linear_args* a, cudaStream_t stream) {
   }
   while (split > 1 && split > (a->K + kDeep - 1) / kDeep) split /= 2;   // every CTA has a stage
   switch (split) {
-    case 1: return launch<NP, 1, GATED>(a, stream);
-    case 2: return launch<NP, 2, GATED>(a, stream);
-    case 4: return launch<NP, 4, GATED>(a, stream);
-    case 8: return launch<NP, 8, GATED>(a, stream);
+    case 1: return launch<NP, 1, GATED>(a, limit, alpha, stream);
+    case 2: return launch<NP, 2, GATED>(a, limit, alpha, stream);
+    case 4: return launch<NP, 4, GATED>(a, limit, alpha, stream);
+    case 8: return launch<NP, 8, GATED>(a, limit, alpha, stream);
     default: return fail(L3CI_ERR_INVALID, "linear: split %d is not 1, 2, 4 or 8", split);
   }
 }
@@ -403,9 +408,10 @@ extern "C" int l3ci_linear_poll(l3ci_stream_t stream_) {
   return fail(status, "linear: a bounded wait ran out in an earlier launch");
 }
 
-extern "C" int l3ci_linear(const l3ci_linear_args* a) {
+extern "C" int l3ci_linear_gated(const l3ci_linear_args* a, float limit, float alpha) {
   using namespace l3ci;
   clear_error();
+  if (a && limit != 0.f && (a->act != L3CI_ACT_SILU_GATE || !(limit > 0.f))) return fail(L3CI_ERR_INVALID, "linear: a limit of %g with activation %d", limit, a->act);
   if (!a) return fail(L3CI_ERR_INVALID, "linear: null arguments");
   if (a->rows < 0 || a->K <= 0 || a->N < 0 || a->act < L3CI_ACT_NONE || a->act > L3CI_ACT_SILU_GATE || a->split < 0 || a->split > 8 || a->groups < 0)
     return fail(L3CI_ERR_INVALID, "linear: rows=%lld K=%d N=%d groups=%d act=%d split=%d", (long long)a->rows, a->K, a->N, a->groups, a->act, a->split);
@@ -420,8 +426,14 @@ extern "C" int l3ci_linear(const l3ci_linear_args* a) {
     return fail(L3CI_ERR_INVALID, "linear: rows or groups without a stride of their own");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(a->stream);
   const bool gated = a->act == L3CI_ACT_SILU_GATE;
-  if (a->rows <= 8) return gated ? launch_split<8, true>(a, s) : launch_split<8, false>(a, s);
-  if (a->rows <= 16) return gated ? launch_split<16, true>(a, s) : launch_split<16, false>(a, s);
-  if (a->rows <= 32) return gated ? launch_split<32, true>(a, s) : launch_split<32, false>(a, s);
-  return gated ? launch_split<64, true>(a, s) : launch_split<64, false>(a, s);
+  auto go = [&](auto np) {
+    constexpr int NP = decltype(np)::value;
+    return gated ? launch_split<NP, true>(a, limit, alpha, s) : launch_split<NP, false>(a, limit, alpha, s);
+  };
+  if (a->rows <= 8) return go(std::integral_constant<int, 8>{});
+  if (a->rows <= 16) return go(std::integral_constant<int, 16>{});
+  if (a->rows <= 32) return go(std::integral_constant<int, 32>{});
+  return go(std::integral_constant<int, 64>{});
 }
+
+extern "C" int l3ci_linear(const l3ci_linear_args* a) { return l3ci_linear_gated(a, 0.f, 0.f); }

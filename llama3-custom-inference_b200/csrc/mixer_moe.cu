@@ -90,7 +90,7 @@ moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ bia
 template <typename S, int VEC>
 __global__ void __launch_bounds__(128)
 moe_gather_kernel(const S* __restrict__ h, const int* __restrict__ experts, const int* __restrict__ ranks, const int* __restrict__ counts,
-                  S* __restrict__ out, int* __restrict__ part_rows, long long rows, int width, int E, int top) {
+                  S* __restrict__ out, int* __restrict__ part_rows, long long rows, int width, int E, int top, long long places) {
   extern __shared__ int at_s[];
   pdl_begin();
   const long long row = blockIdx.x;
@@ -98,8 +98,12 @@ moe_gather_kernel(const S* __restrict__ h, const int* __restrict__ experts, cons
   for (int j = warp; j < top; j += warps) {
     const int e = experts[row * top + j];
     int before = 0;
-    for (int i = lane; i < e; i += 32) before += counts[i];
-    before = __reduce_add_sync(kFullMask, before);
+    if (counts) {
+      for (int i = lane; i < e; i += 32) before += counts[i];
+      before = __reduce_add_sync(kFullMask, before);
+    } else {
+      before = e * (int)rows;
+    }
     if (lane == 0) {
       const int at = before + ranks[row * top + j];
       part_rows[row * top + j] = at;
@@ -112,7 +116,7 @@ moe_gather_kernel(const S* __restrict__ h, const int* __restrict__ experts, cons
     const R x = *reinterpret_cast<const R*>(h + row * width + c);
     for (int j = 0; j < top; ++j) {
       const long long at = at_s[j];
-      if (at >= 0 && at < rows * top) *reinterpret_cast<R*>(out + at * width + c) = x;
+      if (at >= 0 && at < places) *reinterpret_cast<R*>(out + at * width + c) = x;
     }
   }
 }
@@ -220,15 +224,15 @@ int l3ci_moe_route(const float* logits, const float* bias, int32_t* experts, int
   return L3CI_OK;
 }
 
-int l3ci_moe_gather(const void* h, const int32_t* experts, const int32_t* ranks, const int32_t* counts, void* out, int32_t* part_rows,
-                    int64_t rows, int64_t width, int32_t E, int32_t top, int32_t dtype, l3ci_stream_t stream_) {
+static int gather(const void* h, const int32_t* experts, const int32_t* ranks, const int32_t* counts, bool by_counts, void* out, int32_t* part_rows,
+                  int64_t rows, int64_t width, int32_t E, int32_t top, int32_t dtype, l3ci_stream_t stream_) {
   using namespace l3ci;
   clear_error();
   if (rows < 0 || rows > 0x7fffffffLL || width <= 0 || width > 0x3fffffffLL || E <= 0 || E > kMaxExperts || top <= 0 || top > E ||
-      rows * top > 0x7fffffffLL || (dtype != L3CI_BF16 && dtype != L3CI_F32))
+      rows * top > 0x7fffffffLL || (!by_counts && rows * E > 0x7fffffffLL) || (dtype != L3CI_BF16 && dtype != L3CI_F32))
     return fail(L3CI_ERR_INVALID, "moe_gather: rows=%lld width=%lld experts=%d top=%d", (long long)rows, (long long)width, E, top);
   if (rows == 0) return L3CI_OK;
-  if (!h || !experts || !ranks || !counts || !out || !part_rows) return fail(L3CI_ERR_INVALID, "moe_gather: null pointer");
+  if (!h || !experts || !ranks || (by_counts && !counts) || !out || !part_rows) return fail(L3CI_ERR_INVALID, "moe_gather: null pointer");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
   auto typed = [&](auto zero) -> int {
     using S = decltype(zero);
@@ -236,12 +240,22 @@ int l3ci_moe_gather(const void* h, const int32_t* experts, const int32_t* ranks,
     const bool v = width % kVec == 0 && aligned16(h) && aligned16(out);
     auto go = [&](auto kernel) -> int {
       L3CI_LAUNCH("moe_gather_kernel", kernel, dim3((unsigned)rows), dim3(128), sizeof(int) * top, s, static_cast<const S*>(h), experts, ranks, counts,
-                  static_cast<S*>(out), part_rows, (long long)rows, (int)width, E, top);
+                  static_cast<S*>(out), part_rows, (long long)rows, (int)width, E, top, (long long)rows * (by_counts ? top : E));
       return L3CI_OK;
     };
     return v ? go(moe_gather_kernel<S, kVec>) : go(moe_gather_kernel<S, 1>);
   };
   return dtype == L3CI_BF16 ? typed(__nv_bfloat16{}) : typed(float{});
+}
+
+int l3ci_moe_gather(const void* h, const int32_t* experts, const int32_t* ranks, const int32_t* counts, void* out, int32_t* part_rows,
+                    int64_t rows, int64_t width, int32_t E, int32_t top, int32_t dtype, l3ci_stream_t stream) {
+  return gather(h, experts, ranks, counts, true, out, part_rows, rows, width, E, top, dtype, stream);
+}
+
+int l3ci_moe_gather_places(const void* h, const int32_t* experts, const int32_t* ranks, void* out, int32_t* part_rows, int64_t rows,
+                           int64_t width, int32_t E, int32_t top, int32_t dtype, l3ci_stream_t stream) {
+  return gather(h, experts, ranks, nullptr, false, out, part_rows, rows, width, E, top, dtype, stream);
 }
 
 int l3ci_moe_gemm_variant(const l3ci_moe_gemm_args* a) {

@@ -353,8 +353,9 @@ bool few_rows_pay(int64_t rows, int64_t K, int64_t N, int64_t groups, int64_t ac
 // or alignments) or torch's product is the faster on the device (few_rows_pay).  `early`: the kernel may read w ahead of the stream's previous kernels; for a w that was complete before the last
 // one of them that waits for its predecessors ahead of letting others start.  f32: an fp32 result.  `into`: where the result goes.
 // `always`: wherever the kernel applies; for passes that wait for the host, which a launch of it costs about 4 us less than torch's
-// product (a prompt of 64 tokens, 16 layers: 1.0 ms instead of 1.4).
-std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bool early, bool f32, const std::optional<Tensor>& into, bool always) {
+// product (a prompt of 64 tokens, 16 layers: 1.0 ms instead of 1.4).  `limit`, `alpha`: of a gated activation's clamped form.
+std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bool early, bool f32, const std::optional<Tensor>& into, bool always,
+                               double limit, double alpha) {
   if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != torch::kBFloat16 || w.scalar_type() != torch::kBFloat16 ||
       w.get_device() != x.get_device() || x.dim() < 1)
     return std::nullopt;
@@ -393,7 +394,7 @@ std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bo
   a.out_f32 = out.scalar_type() == torch::kFloat;
   a.early = early;
   a.stream = current_stream();
-  check_status(l3ci_linear(&a), "linear");
+  check_status(l3ci_linear_gated(&a, (float)limit, (float)alpha), "linear");
   return out;
 }
 
@@ -404,7 +405,7 @@ Tensor linear(Tensor x, Tensor w, bool gated, bool early, bool always) {
   TORCH_CHECK(x.dim() >= 1 && w.dim() == 2 && w.size(1) == x.size(-1), "w must be [N, K] with K the last axis of x");
   TORCH_CHECK(w.get_device() == x.get_device(), "x and w on different devices");
   TORCH_CHECK(!gated || w.size(0) % 2 == 0, "a gated product takes an even number of rows of w");
-  if (auto y = few_rows(x, w, gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE, early, false, std::nullopt, always)) return *y;
+  if (auto y = few_rows(x, w, gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE, early, false, std::nullopt, always, 0.0, 0.0)) return *y;
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y = at::linear(x, w);
   if (!gated) return y;
@@ -578,7 +579,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("early") = false, py::arg("always") = false);
   m.def("few_rows", torch::wrap_pybind_function(few_rows), "few_rows", py::arg("x"), py::arg("w"), py::arg("act") = (int64_t)L3CI_ACT_NONE,
         py::arg("early") = false, py::arg("f32") = false, py::arg("into") = py::none(),
-        py::arg("always") = false);
+        py::arg("always") = false, py::arg("limit") = 0.0, py::arg("alpha") = 0.0);
   m.def("greedy_step", torch::wrap_pybind_function(greedy_step), "greedy_step", py::arg("logits"), py::arg("out_tokens"),
         py::arg("steps"), py::arg("next_input"), py::arg("positions"), py::arg("seq_lens"));
   m.def("top_p_step", torch::wrap_pybind_function(top_p_step), "top_p_step", py::arg("logits"), py::arg("out_tokens"),

@@ -17,7 +17,7 @@ EXPORTS = ("l3ci_mixers_last_error", "l3ci_mixers_set_programmatic_launch", "l3c
            "l3ci_latent_cache", "l3ci_kv_cache_write", "l3ci_mixer_attention", "l3ci_mixer_attention_scratch_bytes",
            "l3ci_mixer_attention_variant", "l3ci_residual_norm", "l3ci_tanh", "l3ci_gated_act", "l3ci_qk_norm_cache",
            "l3ci_token_shift", "l3ci_delta_inputs", "l3ci_recurrent_scan", "l3ci_moe_route", "l3ci_moe_gather",
-           "l3ci_moe_gemm", "l3ci_moe_gemm_variant")
+           "l3ci_moe_gather_places", "l3ci_moe_gemm", "l3ci_moe_gemm_variant")
 
 DTYPE_CODES = {torch.bfloat16: 0, torch.float32: 1}
 ROWS, MMA, TC = 1, 2, 3   # variants of l3ci_mixer_attention (0: choose)
@@ -107,6 +107,7 @@ def load() -> C.CDLL:
     lib.l3ci_recurrent_scan.argtypes = [C.POINTER(RecurrentScanArgs)]
     lib.l3ci_moe_route.argtypes = [vp, vp, vp, vp, vp, vp, i64, i32, i32, vp]
     lib.l3ci_moe_gather.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i32, i32, i32, vp]
+    lib.l3ci_moe_gather_places.argtypes = [vp, vp, vp, vp, vp, i64, i64, i32, i32, i32, vp]
     lib.l3ci_moe_gemm.argtypes = [C.POINTER(MoeGemmArgs)]
     lib.l3ci_moe_gemm_variant.argtypes = [C.POINTER(MoeGemmArgs)]
     _lib = lib
@@ -137,14 +138,16 @@ def _extension():
     return _ext
 
 
-def few_rows(x, w, act: int = ACT_NONE, out_dtype=None, out=None, early: bool = False, always: bool = False):
+def few_rows(x, w, act: int = ACT_NONE, out_dtype=None, out=None, early: bool = False, always: bool = False, limit: float = 0.0,
+             alpha: float = 0.0):
     """act(x w^T) of few rows in one kernel (`l3ci_linear`), groups of products where w is [groups, N, K]; None where it does
     not apply or torch's product is the faster on the device.  `early`: w may be read ahead of the stream's previous kernels; for
     weights that were complete before the last one of them that waits for its predecessors ahead of letting others start (a model's,
-    in its forward pass).  `always`: wherever it applies, for passes that wait for the host."""
+    in its forward pass).  `always`: wherever it applies, for passes that wait for the host.  `limit`, `alpha`: the clamped form of a gated
+    activation (`gated_act`)."""
     if out_dtype not in (None, torch.bfloat16, torch.float32):
         raise ValueError("the result is bf16 or fp32")
-    return _extension().few_rows(x, w, act, early, out_dtype == torch.float32, out, always)
+    return _extension().few_rows(x, w, act, early, out_dtype == torch.float32, out, always, limit, alpha)
 
 
 def _many_rows(x, w, act: int = ACT_NONE):
@@ -421,6 +424,27 @@ def moe_gather(h, experts, ranks, counts):
         _check(load().l3ci_moe_gather(h.data_ptr(), experts.data_ptr(), ranks.data_ptr(), counts.data_ptr(), out.data_ptr(),
                                       part_rows.data_ptr(), rows, h.shape[1], counts.numel(), top, DTYPE_CODES[h.dtype], _stream(h)),
                "l3ci_moe_gather")
+    return out, part_rows
+
+
+def moe_places_pay(rows: int, experts: int, top: int) -> bool:
+    """Whether the experts of few tokens are groups of products over places of their own (every expert's weights are read then, chosen or
+    not) rather than products of the sorted rows (tiles of 128 of them): up to 32 tokens, where even routing leaves out few experts.  Routing,
+    gathering and both products, width 2048, experts of 2048, us by sorted rows and by places: 4 of 4 experts, 8 tokens 43.8, 29.7, 32 tokens
+    39.5, 33.5, 64 tokens 43.2, 41.1; 4 of 16, 8 tokens (a tenth left out) 81.3, 73.7, 32 tokens 85.1, 81.0, 48 tokens 88.3, 89.9; 4 of 32, 12 tokens (a
+    fifth left out) 114.8, 132.7, 24 tokens 141.9, 137.3."""
+    return rows <= 32 and (1.0 - top / experts) ** rows <= 0.11
+
+
+def moe_places(h, experts, ranks, n_experts: int):
+    """h's rows in places by expert [experts, rows, width] (those without a pair: anything), and the place of every (row, choice) pair."""
+    _cuda(h, experts, ranks)
+    rows, top = experts.shape
+    out = torch.empty(n_experts, rows, h.shape[1], dtype=h.dtype, device=h.device)
+    part_rows = torch.empty(rows, top, dtype=torch.int32, device=h.device)
+    with _on(h):
+        _check(load().l3ci_moe_gather_places(h.data_ptr(), experts.data_ptr(), ranks.data_ptr(), out.data_ptr(), part_rows.data_ptr(), rows,
+                                             h.shape[1], n_experts, top, DTYPE_CODES[h.dtype], _stream(h)), "l3ci_moe_gather_places")
     return out, part_rows
 
 
