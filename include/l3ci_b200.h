@@ -115,7 +115,10 @@ L3CI_API int l3ci_linear(const l3ci_linear_args* args);
 /* The same; with a limit above 0 the gated activation is z sigmoid(alpha z) (u + 1) of z = min(gate, limit), u = clamp(up, -limit, limit)
  * (experts whose rows lie in places of their own, one group each). */
 L3CI_API int l3ci_linear_gated(const l3ci_linear_args* args, float limit, float alpha);
-/* Waits for `stream`; L3CI_ERR_DEVICE_WAIT, once, if a launch of l3ci_linear without a status word of its own gave up on this device
+/* The same of any number of rows, tiles of 256 x 256 over pairs of SMs (a prompt's products with an activation): groups 1, out bf16, N and
+ * out_st multiples of 8, out on 16 bytes; split and early are not used, status is the library's word. */
+L3CI_API int l3ci_linear_many(const l3ci_linear_args* args);
+/* Waits for `stream`; L3CI_ERR_DEVICE_WAIT, once, if a launch of l3ci_linear without a status word of its own, or of l3ci_linear_many, gave up on this device
  * (should never happen). */
 L3CI_API int l3ci_linear_poll(l3ci_stream_t stream);
 /* Elements between the rows of a tensor of these sizes and strides (in elements), all axes but the last counted as one axis of

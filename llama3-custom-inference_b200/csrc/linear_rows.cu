@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "host_common.h"
+#include "linear_many.h"
 #include "mixer_types.cuh"
 #include "ptx_sm100.cuh"
 #include "tcgen05.cuh"
@@ -398,14 +399,18 @@ extern "C" int l3ci_linear_poll(l3ci_stream_t stream_) {
   using namespace l3ci;
   clear_error();
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  int status = 0;
-  L3CI_CUDA_TRY(cudaMemcpyFromSymbolAsync(&status, g_wait_status, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+  void* own = nullptr;
+  L3CI_CUDA_TRY(cudaGetSymbolAddress(&own, g_wait_status));
+  int* words[2] = {static_cast<int*>(own), linear_many_wait_status()};
+  int status[2] = {0, 0};
+  for (int i = 0; i < 2; ++i)
+    if (words[i]) L3CI_CUDA_TRY(cudaMemcpyAsync(&status[i], words[i], sizeof(int), cudaMemcpyDeviceToHost, stream));
   L3CI_CUDA_TRY(cudaStreamSynchronize(stream));
-  if (status == 0) return L3CI_OK;
-  const int none = 0;
-  L3CI_CUDA_TRY(cudaMemcpyToSymbolAsync(g_wait_status, &none, sizeof(int), 0, cudaMemcpyHostToDevice, stream));
+  if (status[0] == 0 && status[1] == 0) return L3CI_OK;
+  for (int i = 0; i < 2; ++i)
+    if (words[i]) L3CI_CUDA_TRY(cudaMemsetAsync(words[i], 0, sizeof(int), stream));
   L3CI_CUDA_TRY(cudaStreamSynchronize(stream));
-  return fail(status, "linear: a bounded wait ran out in an earlier launch");
+  return fail(status[0] ? status[0] : status[1], "linear: a bounded wait ran out in an earlier launch");
 }
 
 extern "C" int l3ci_linear_gated(const l3ci_linear_args* a, float limit, float alpha) {

@@ -12,6 +12,7 @@
 // forwards raw pointers to the C ABI of include/l3ci_b200.h.
 #include <torch/extension.h>
 
+#include <ATen/cuda/CUDAContextLight.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -398,7 +399,45 @@ std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bo
   return out;
 }
 
-// act(x w^T) of any number of rows: few in one kernel (few_rows), more in torch's product and, gated, silu_mul.
+// Whether a product of many rows with its activation is the faster by l3ci_linear_many, tiles of 256 x 256 on pairs of SMs, than by torch's
+// product and a pass for the activation: where there are tiles for more than one wave of pairs and the last wave is not nearly empty.  Both
+// in turn, us: gated 2 x 8192 x 2048, rows 256 19.9 and 19.5, 512 31.1 and 30.4, 2048 127.2 and 101.7, 6001 378 and 323, 8192 515 and 432; gelu
+// 8192 x 2048, rows 512 21.5 and 22.9, 1024 35.3 and 33.9, 2048 67.6 and 62.5, 8192 303 and 252.  (Without an activation it is the library's
+// equal at best: 8192 rows 202.3 and 196.7, 2048 rows 49.7 and 52.5.)
+bool many_rows_pay(int64_t rows, int64_t N, bool gated, int sms) {
+  const int64_t outs = gated ? 128 : 256, tiles = (rows + 255) / 256 * ((N + outs - 1) / outs), pairs = sms / 2;
+  const int64_t waves = (tiles + pairs - 1) / pairs;
+  return pairs > 0 && 2 * tiles >= 3 * pairs && 20 * tiles >= 17 * waves * pairs;
+}
+
+// act(x w^T) of many rows in one kernel (l3ci_linear_many); nothing where it does not apply or does not pay.
+std::optional<Tensor> many_rows(const Tensor& x, const Tensor& w, int64_t act) {
+  if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != torch::kBFloat16 || w.scalar_type() != torch::kBFloat16 ||
+      w.get_device() != x.get_device() || x.dim() < 1 || w.dim() != 2 || act == L3CI_ACT_NONE)
+    return std::nullopt;
+  const bool gated = act == L3CI_ACT_SILU_GATE;
+  const int64_t K = x.size(-1), N = gated ? w.size(0) / 2 : w.size(0), rows = K ? x.numel() / K : 0;
+  if (w.size(1) != K || K % 8 || N == 0 || N % 8 || (gated && w.size(0) % 2) || !w.is_contiguous() || rows > INT32_MAX || K > INT32_MAX || w.size(0) > INT32_MAX ||
+      !many_rows_pay(rows, N, gated, at::cuda::getDeviceProperties(x.get_device())->multiProcessorCount))
+    return std::nullopt;
+  auto at16 = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; };
+  const int64_t stride = l3ci_row_stride(x.sizes().data(), x.strides().data(), (int32_t)x.dim());
+  if (stride < 0 || stride % 8 || !at16(x) || !at16(w)) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(x.device());
+  auto sizes = x.sizes().vec();
+  sizes.back() = N;
+  Tensor out = torch::empty(sizes, x.options());
+  l3ci_linear_args a{};
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
+  a.rows = rows; a.x_st = stride; a.out_st = N;
+  a.K = (int32_t)K; a.N = (int32_t)N; a.groups = 1; a.act = (int32_t)act;
+  a.stream = current_stream();
+  check_status(l3ci_linear_many(&a), "linear_many");
+  return out;
+}
+
+// act(x w^T) of any number of rows: few in one kernel (few_rows), many gated ones in another (many_rows), else torch's product and, gated,
+// silu_mul.
 Tensor linear(Tensor x, Tensor w, bool gated, bool early, bool always) {
   check_bf16_cuda(x, "x");
   check_bf16_cuda(w, "w");
@@ -406,6 +445,8 @@ Tensor linear(Tensor x, Tensor w, bool gated, bool early, bool always) {
   TORCH_CHECK(w.get_device() == x.get_device(), "x and w on different devices");
   TORCH_CHECK(!gated || w.size(0) % 2 == 0, "a gated product takes an even number of rows of w");
   if (auto y = few_rows(x, w, gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE, early, false, std::nullopt, always, 0.0, 0.0)) return *y;
+  if (gated)
+    if (auto y = many_rows(x, w, L3CI_ACT_SILU_GATE)) return *y;
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y = at::linear(x, w);
   if (!gated) return y;
@@ -580,6 +621,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("few_rows", torch::wrap_pybind_function(few_rows), "few_rows", py::arg("x"), py::arg("w"), py::arg("act") = (int64_t)L3CI_ACT_NONE,
         py::arg("early") = false, py::arg("f32") = false, py::arg("into") = py::none(),
         py::arg("always") = false, py::arg("limit") = 0.0, py::arg("alpha") = 0.0);
+  m.def("many_rows", torch::wrap_pybind_function(many_rows), "many_rows", py::arg("x"), py::arg("w"), py::arg("act"));
   m.def("greedy_step", torch::wrap_pybind_function(greedy_step), "greedy_step", py::arg("logits"), py::arg("out_tokens"),
         py::arg("steps"), py::arg("next_input"), py::arg("positions"), py::arg("seq_lens"));
   m.def("top_p_step", torch::wrap_pybind_function(top_p_step), "top_p_step", py::arg("logits"), py::arg("out_tokens"),

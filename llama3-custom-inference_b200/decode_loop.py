@@ -299,11 +299,7 @@ class Llama3Decoder(DecodeLoop):
                                                max_ctas=self._decode_kernel(B))     # model.py:118
             y = y.transpose(1, 2).reshape(B, T, E)                                     # model.py:120
             x, h = ext.add_rms_norm(product(y, w[p + "proj"]), x, w[p + "ln_2"], cfg.norm_eps)  # :121, 147-148
-            if few:                                                                    # c_fc2 | c_fc, model.py:134
-                a = linear(h, w[p + "gate_up"], gated=True)
-            else:
-                gu = F.linear(h, w[p + "gate_up"])
-                a = ext.silu_mul(gu[..., :cfg.hidden_dim], gu[..., cfg.hidden_dim:])
+            a = linear(h, w[p + "gate_up"], gated=True)                                # c_fc2 | c_fc, model.py:134
             m = product(a, w[p + "mlp_proj"])
             nxt = w[f"h{l + 1}.ln_1"] if l + 1 < cfg.n_layer else w["ln_f"]
             x, h = ext.add_rms_norm(m, x, nxt, cfg.norm_eps)                           # model.py:148, next 147 / 217
