@@ -401,9 +401,9 @@ std::optional<Tensor> few_rows(const Tensor& x, const Tensor& w, int64_t act, bo
 
 // Whether a product of many rows with its activation is the faster by l3ci_linear_many, tiles of 256 x 256 on pairs of SMs, than by torch's
 // product and a pass for the activation: where there are tiles for more than one wave of pairs and the last wave is not nearly empty.  Both
-// in turn, us: gated 2 x 8192 x 2048, rows 256 19.9 and 19.5, 512 31.1 and 30.4, 2048 127.2 and 101.7, 6001 378 and 323, 8192 515 and 432; gelu
-// 8192 x 2048, rows 512 21.5 and 22.9, 1024 35.3 and 33.9, 2048 67.6 and 62.5, 8192 303 and 252.  (Without an activation it is the library's
-// equal at best: 8192 rows 202.3 and 196.7, 2048 rows 49.7 and 52.5.)
+// in turn, us: gated 2 x 8192 x 2048, rows 256 19.9 and 19.5, 512 30.8 and 29.0, 2048 128 and 98.6, 6001 362 and 304, 8192 495 and 413; gelu
+// 8192 x 2048, rows 512 21.5 and 22.9, 1024 48.2 and 44.2, 2048 69.3 and 59.5, 8192 301 and 226.  (Without an activation it is the library's
+// equal at best: 8192 rows 215 and 208, 2048 rows 48.7 and 51.3.)
 bool many_rows_pay(int64_t rows, int64_t N, bool gated, int sms) {
   const int64_t outs = gated ? 128 : 256, tiles = (rows + 255) / 256 * ((N + outs - 1) / outs), pairs = sms / 2;
   const int64_t waves = (tiles + pairs - 1) / pairs;
