@@ -86,14 +86,10 @@ __device__ __forceinline__ uint64_t l2_evict_normal_policy() {
 }
 
 // Finishes one (token, head) row of differential attention from the normalised outputs of its maps: the factor that
-// the difference o (sum of squares `ss` over Dv columns) is multiplied by.
-__device__ __forceinline__ float differential_factor(const l3ci_mixer_attn_args& a, float ss, int b, int t, int h) {
-  float f = a.post * __frsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)a.Dv), a.eps));
-  if (a.gate) {
-    const float z = __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[b * a.g_sb + t * a.g_st + h]);
-    f *= 1.f / (1.f + expf(-z));
-  }
-  return f;
+// the difference o (sum of squares `ss` over Dv columns) is multiplied by; `gate`: the row's, if there are gates.
+__device__ __forceinline__ float differential_factor(const l3ci_mixer_attn_args& a, float ss, float gate) {
+  const float f = a.post * __frsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)a.Dv), a.eps));
+  return a.gate ? f * (1.f / (1.f + expf(-gate))) : f;
 }
 
 template <int KS, int NB, int MAPS>
@@ -443,7 +439,8 @@ mixer_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
     for (int w = 0; w < kWarps; ++w) ss += s_ss[w * 8 + gid];
     if (gid < n_pairs) {
       const int idx = pair0 + gid;
-      const float f = differential_factor(a, ss, b, idx / p.R, g * p.R + idx % p.R);
+      const float gate = a.gate ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[b * a.g_sb + idx / p.R * a.g_st + g * p.R + idx % p.R]) : 0.f;
+      const float f = differential_factor(a, ss, gate);
       __nv_bfloat16* dst = out_row(gid);
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
@@ -488,6 +485,26 @@ __global__ void __launch_bounds__(kMergeMax) mixer_merge_kernel(const __grid_con
   const int idx = rb * kPairs + pair;
   if (idx >= a.T * p.R) return;
   const int t = idx / p.R, h = g * p.R + idx % p.R, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // what the rows below need from memory is asked for at once, beside the maxima: one trip instead of two (8 sequences, 4096 keys: 4.5 to 5.5 us in a
+  // step, 3.9 to 4.8 so)
+  const int col0 = blockIdx.y * p.merge_cols, quads = min(p.merge_cols, a.Dv - col0) / 4;
+  int lanes = 16;                                                // threads along the columns, a power of two
+  while (lanes < quads) lanes *= 2;
+  const int groups = blockDim.x / lanes, grp = tid / lanes, c = tid % lanes;
+  const long long step = (long long)kMmRows * p.dv_pad;
+  constexpr int kFetched = 4;                                    // splits of a group, at most
+  float4 fetched[MAPS][kFetched];
+#pragma unroll
+  for (int m = 0; m < MAPS; ++m)
+#pragma unroll
+    for (int i = 0; i < kFetched; ++i) {
+      fetched[m][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < quads && grp + i * groups < p.splits)
+        fetched[m][i] = *reinterpret_cast<const float4*>(p.o_part + ((long long)unit * p.splits * kMmRows + pair + 8 * m) * p.dv_pad + col0 + 4 * c +
+                                                         (grp + i * groups) * step);
+    }
+  float gate = 0.f;
+  if (MAPS == 2 && a.gate) gate = __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[b * a.g_sb + t * a.g_st + h]);
   // weight of split s: exp2(m_s - max) / sum of l_s exp2(m_s - max); 0 for a split without a visible key
   if (warp < MAPS) {
     const float2* ml = reinterpret_cast<const float2*>(p.ml_part) + (long long)unit * p.splits * kMmRows + pair + 8 * warp;
@@ -505,27 +522,25 @@ __global__ void __launch_bounds__(kMergeMax) mixer_merge_kernel(const __grid_con
     for (int s = lane; s < p.splits; s += 32) wt[warp][s] *= inv;
   }
   __syncthreads();
-  const int col0 = blockIdx.y * p.merge_cols, quads = min(p.merge_cols, a.Dv - col0) / 4;
-  int lanes = 16;                                                // threads along the columns, a power of two
-  while (lanes < quads) lanes *= 2;
-  const int groups = blockDim.x / lanes, grp = tid / lanes, c = tid % lanes;
-  const long long step = (long long)kMmRows * p.dv_pad;
 #pragma unroll
   for (int m = 0; m < MAPS; ++m) {
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](int s, const float4& y) {
+      const float w = wt[m][s];
+      if (w != 0.f) {   // a record of weight 0 may never have been written
+        x.x = fmaf(y.x, w, x.x);
+        x.y = fmaf(y.y, w, x.y);
+        x.z = fmaf(y.z, w, x.z);
+        x.w = fmaf(y.w, w, x.w);
+      }
+    };
     if (c < quads) {
+#pragma unroll
+      for (int i = 0; i < kFetched; ++i)
+        if (grp + i * groups < p.splits) add(grp + i * groups, fetched[m][i]);
       const float* src = p.o_part + ((long long)unit * p.splits * kMmRows + pair + 8 * m) * p.dv_pad + col0 + 4 * c;
 #pragma unroll 4
-      for (int s = grp; s < p.splits; s += groups) {
-        const float w = wt[m][s];
-        const float4 y = *reinterpret_cast<const float4*>(src + s * step);
-        if (w != 0.f) {   // a record of weight 0 may never have been written
-          x.x = fmaf(y.x, w, x.x);
-          x.y = fmaf(y.y, w, x.y);
-          x.z = fmaf(y.z, w, x.z);
-          x.w = fmaf(y.w, w, x.w);
-        }
-      }
+      for (int s = grp + kFetched * groups; s < p.splits; s += groups) add(s, *reinterpret_cast<const float4*>(src + s * step));
     }
     sum[m][tid] = x;
   }
@@ -546,7 +561,7 @@ __global__ void __launch_bounds__(kMergeMax) mixer_merge_kernel(const __grid_con
   }
   float f = 1.f;
   if (MAPS == 2)
-    f = differential_factor(a, cta_sum(o[0] * o[0] + o[1] * o[1] + o[2] * o[2] + o[3] * o[3], red, blockDim.x / kWarp), b, t, h);
+    f = differential_factor(a, cta_sum(o[0] * o[0] + o[1] * o[1] + o[2] * o[2] + o[3] * o[3], red, blockDim.x / kWarp), gate);
   if (grp == 0 && c < quads) {
     __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.out) + b * a.o_sb + t * a.o_st + h * a.o_sh + col0 + 4 * c;
     reinterpret_cast<uint32_t*>(dst)[0] = pack_bf16x2(o[0] * f, o[1] * f);   // rows start on 4 bytes
