@@ -131,6 +131,11 @@ typedef struct l3ci_recurrent_scan_args {
 } l3ci_recurrent_scan_args;
 
 L3CI_API int l3ci_recurrent_scan(const l3ci_recurrent_scan_args* args);
+/* The same by chunks of 16 tokens, for prompts in bf16 with 64 or 128 key channels.  scratch: on 16 bytes, at least what
+ * one chunk of all heads takes (L3CI_ERR_SCRATCH); l3ci_recurrent_scan_scratch_bytes tells what it takes at best, and 0 where it does not apply or
+ * l3ci_recurrent_scan is the faster. */
+L3CI_API int l3ci_recurrent_scan_chunks(const l3ci_recurrent_scan_args* args, void* scratch, size_t scratch_bytes);
+L3CI_API size_t l3ci_recurrent_scan_scratch_bytes(const l3ci_recurrent_scan_args* args);
 
 /* Mixture of experts.  Route: of the fp32 logits [rows, E] + bias [E] the `top` largest of a token (ties: the smaller index),
  * weights = softmax over these; experts, ranks int32 [rows, top] (rank: place of the pair among the pairs of its expert),

@@ -26,6 +26,7 @@
 
 #include "../../include/l3ci_mixers.h"
 #include "host_common.h"
+#include "mixer_recurrent.h"
 #include "mixer_types.cuh"
 #include "ptx_sm100.cuh"
 #include "tcgen05.cuh"
@@ -148,29 +149,6 @@ __device__ __forceinline__ float scatter_sum(float (&v)[N], int lane) {
   for (int k = 16; k >= 1; k /= 2)
     if (k < 32 / N) r += __shfl_xor_sync(kFullMask, r, k);
   return r;
-}
-
-// The convolution's carried inputs: row r of the tail becomes the input of token T - (taps - 1) + r.  Channel c of a sequence,
-// by one thread.
-template <typename S>
-__device__ __forceinline__ void move_tail(const l3ci_recurrent_scan_args& a, S* tail, const S* in, long long channels, long long c, bool fresh) {
-  const int rows = a.taps - 1;
-  for (int r = 0; r < rows; ++r) {
-    const int t = a.T - rows + r;
-    tail[r * channels + c] = t >= 0 ? in[t * a.conv_st + c] : fresh ? from_f32<S>(0.f) : tail[(r + a.T) * channels + c];
-  }
-}
-
-// Those of head h's values and, by the first head that reads them, of its queries and keys; `i` of `n` threads.
-template <typename S>
-__device__ __forceinline__ void move_tails(const l3ci_recurrent_scan_args& a, int b, int h, int i, int n, bool fresh) {
-  const int GD = a.G * a.D, R = a.H / a.G;
-  const long long channels = 2LL * GD + (long long)a.H * a.V;
-  S* tail = static_cast<S*>(a.tail) + b * a.tail_sb;
-  const S* in = static_cast<const S*>(a.conv_in) + (long long)b * a.T * a.conv_st;
-  for (int c = i; c < a.V; c += n) move_tail<S>(a, tail, in, channels, 2LL * GD + (long long)h * a.V + c, fresh);
-  if (h % R == 0)
-    for (int c = i; c < 2 * a.D; c += n) move_tail<S>(a, tail, in, channels, c < a.D ? (h / R) * a.D + c : GD + (h / R) * a.D + c - a.D, fresh);
 }
 
 // S: storage type of v, gate, out; Q: type of q, k, g.
@@ -944,6 +922,26 @@ int step_launch(const l3ci_recurrent_scan_args* a, cudaStream_t stream) {
                                                                          : go(recurrent_step_kernel<S, Q, KIND, 16>);
 }
 
+// Norm and gate of the rows that a scan has written.
+template <typename S>
+int norm_and_gate(const l3ci_recurrent_scan_args* a, cudaStream_t stream) {
+  const long long units = (long long)a->B * a->H * a->T;
+  if ((units + 7) / 8 > 0x7fffffffLL) return fail(L3CI_ERR_INVALID, "recurrent_scan: too many rows");
+  auto go = [&](auto kernel, int per_cta) -> int {
+    L3CI_LAUNCH("head_norm_gate_kernel", kernel, dim3((unsigned)((units + per_cta - 1) / per_cta)), dim3(256), 0, stream, static_cast<S*>(a->out),
+                (long long)a->out_st, (long long)a->out_sh, static_cast<const S*>(a->gate), (long long)a->gate_st, (long long)a->gate_sh,
+                a->norm, (long long)a->norm_sh, a->H, a->V, units, a->act, a->eps);
+    return L3CI_OK;
+  };
+  constexpr int kVec = 16 / sizeof(S);
+  const bool vec = (a->V | a->out_st | a->out_sh | a->gate_st | a->gate_sh | a->norm_sh) % kVec == 0 && aligned16(a->out) && aligned16(a->gate) &&
+                   aligned16(a->norm);
+  if (vec && a->V <= 8 * kVec) return go(head_norm_gate_vec_kernel<S, kVec, 8>, 32);
+  if (vec && a->V <= 16 * kVec) return go(head_norm_gate_vec_kernel<S, kVec, 16>, 16);
+  if (vec && a->V <= 32 * kVec) return go(head_norm_gate_vec_kernel<S, kVec, 32>, 8);
+  return go(head_norm_gate_kernel<S, 1>, 8);
+}
+
 template <typename S, typename Q, int KIND>
 int scan_typed(const l3ci_recurrent_scan_args* a, cudaStream_t stream) {
   if (step_applies<S, Q, KIND>(a)) return step_launch<S, Q, KIND>(a, stream);
@@ -993,22 +991,20 @@ int scan_typed(const l3ci_recurrent_scan_args* a, cudaStream_t stream) {
   };
   st = C == 2 ? by_rows(std::integral_constant<int, 2>{}) : by_rows(std::integral_constant<int, KIND == kDelta ? 8 : 4>{});
   if (st) return st;
-  // norm and gate of the rows the scan has written
-  const long long units = heads * a->T;
-  if ((units + 7) / 8 > 0x7fffffffLL) return fail(L3CI_ERR_INVALID, "recurrent_scan: too many rows");
-  auto go = [&](auto kernel, int per_cta) -> int {
-    L3CI_LAUNCH("head_norm_gate_kernel", kernel, dim3((unsigned)((units + per_cta - 1) / per_cta)), dim3(256), 0, stream, static_cast<S*>(a->out),
-                (long long)a->out_st, (long long)a->out_sh, static_cast<const S*>(a->gate), (long long)a->gate_st, (long long)a->gate_sh,
-                a->norm, (long long)a->norm_sh, a->H, a->V, units, a->act, a->eps);
-    return L3CI_OK;
-  };
-  constexpr int kVec = 16 / sizeof(S);
-  const bool vec = (a->V | a->out_st | a->out_sh | a->gate_st | a->gate_sh | a->norm_sh) % kVec == 0 && aligned16(a->out) && aligned16(a->gate) &&
-                   aligned16(a->norm);
-  if (vec && a->V <= 8 * kVec) return go(head_norm_gate_vec_kernel<S, kVec, 8>, 32);
-  if (vec && a->V <= 16 * kVec) return go(head_norm_gate_vec_kernel<S, kVec, 16>, 16);
-  if (vec && a->V <= 32 * kVec) return go(head_norm_gate_vec_kernel<S, kVec, 32>, 8);
-  return go(head_norm_gate_kernel<S, 1>, 8);
+  return norm_and_gate<S>(a, stream);
+}
+
+int check_scan(const l3ci_recurrent_scan_args* a) {
+  if (!a) return fail(L3CI_ERR_INVALID, "recurrent_scan: null args");
+  if (a->B < 0 || a->T < 0 || a->H <= 0 || a->G <= 0 || a->H % a->G || a->D <= 0 || a->V <= 0 || (a->kind != 0 && a->kind != 1) ||
+      (a->dtype != L3CI_BF16 && a->dtype != L3CI_F32) || (a->kind == 1 && a->G != a->H) || (a->tail && a->taps < 1))
+    return fail(L3CI_ERR_INVALID, "recurrent_scan: bad size B=%d T=%d H=%d G=%d D=%d V=%d kind=%d", a->B, a->T, a->H, a->G, a->D, a->V, a->kind);
+  if (a->D > kMaxD) return fail(L3CI_ERR_UNSUPPORTED, "recurrent_scan: %d key channels per head, at most %d", a->D, kMaxD);
+  if (a->B == 0 || a->T == 0) return L3CI_OK;
+  if (!a->q || !a->k || !a->v || !a->g || !a->state || !a->out || !a->positions || !a->norm || !a->gate || (a->kind == 0 && !a->beta) ||
+      (a->kind == 1 && (!a->bonus || !a->g_bias)) || (a->tail && !a->conv_in))
+    return fail(L3CI_ERR_INVALID, "recurrent_scan: null pointer");
+  return L3CI_OK;
 }
 
 }  // namespace
@@ -1057,19 +1053,27 @@ int l3ci_delta_inputs(const l3ci_delta_inputs_args* a) {
 int l3ci_recurrent_scan(const l3ci_recurrent_scan_args* a) {
   using namespace l3ci;
   clear_error();
-  if (!a) return fail(L3CI_ERR_INVALID, "recurrent_scan: null args");
-  if (a->B < 0 || a->T < 0 || a->H <= 0 || a->G <= 0 || a->H % a->G || a->D <= 0 || a->V <= 0 || (a->kind != 0 && a->kind != 1) ||
-      (a->dtype != L3CI_BF16 && a->dtype != L3CI_F32) || (a->kind == 1 && a->G != a->H) || (a->tail && a->taps < 1))
-    return fail(L3CI_ERR_INVALID, "recurrent_scan: bad size B=%d T=%d H=%d G=%d D=%d V=%d kind=%d", a->B, a->T, a->H, a->G, a->D, a->V, a->kind);
-  if (a->D > kMaxD) return fail(L3CI_ERR_UNSUPPORTED, "recurrent_scan: %d key channels per head, at most %d", a->D, kMaxD);
+  if (int st = check_scan(a)) return st;
   if (a->B == 0 || a->T == 0) return L3CI_OK;
-  if (!a->q || !a->k || !a->v || !a->g || !a->state || !a->out || !a->positions || !a->norm || !a->gate || (a->kind == 0 && !a->beta) ||
-      (a->kind == 1 && (!a->bonus || !a->g_bias)) || (a->tail && !a->conv_in))
-    return fail(L3CI_ERR_INVALID, "recurrent_scan: null pointer");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(a->stream);
   if (a->kind == 0)
     return a->dtype == L3CI_BF16 ? scan_typed<__nv_bfloat16, float, kDelta>(a, s) : scan_typed<float, float, kDelta>(a, s);
   return a->dtype == L3CI_BF16 ? scan_typed<__nv_bfloat16, __nv_bfloat16, kTimeMix>(a, s) : scan_typed<float, float, kTimeMix>(a, s);
+}
+
+size_t l3ci_recurrent_scan_scratch_bytes(const l3ci_recurrent_scan_args* a) {
+  using namespace l3ci;
+  clear_error();
+  return check_scan(a) == L3CI_OK && a->B > 0 && a->T > 0 ? scan_chunks_scratch(a) : 0;
+}
+
+int l3ci_recurrent_scan_chunks(const l3ci_recurrent_scan_args* a, void* scratch, size_t scratch_bytes) {
+  using namespace l3ci;
+  clear_error();
+  if (int st = check_scan(a)) return st;
+  if (a->B == 0 || a->T == 0) return L3CI_OK;
+  if (int st = scan_chunks_launch(a, scratch, scratch_bytes)) return st;
+  return norm_and_gate<__nv_bfloat16>(a, reinterpret_cast<cudaStream_t>(a->stream));
 }
 
 }  // extern "C"

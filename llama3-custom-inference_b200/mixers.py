@@ -16,7 +16,8 @@ LIB_PATH = Path(__file__).resolve().parent / "lib" / "libl3ci_mixers.so"
 EXPORTS = ("l3ci_mixers_last_error", "l3ci_mixers_set_programmatic_launch", "l3ci_add_dyn_tanh", "l3ci_gelu",
            "l3ci_latent_cache", "l3ci_kv_cache_write", "l3ci_mixer_attention", "l3ci_mixer_attention_scratch_bytes",
            "l3ci_mixer_attention_variant", "l3ci_residual_norm", "l3ci_tanh", "l3ci_gated_act", "l3ci_qk_norm_cache",
-           "l3ci_token_shift", "l3ci_delta_inputs", "l3ci_recurrent_scan", "l3ci_moe_route", "l3ci_moe_gather",
+           "l3ci_token_shift", "l3ci_delta_inputs", "l3ci_recurrent_scan", "l3ci_recurrent_scan_chunks",
+           "l3ci_recurrent_scan_scratch_bytes", "l3ci_moe_route", "l3ci_moe_gather",
            "l3ci_moe_gather_places", "l3ci_moe_gemm", "l3ci_moe_gemm_variant")
 
 DTYPE_CODES = {torch.bfloat16: 0, torch.float32: 1}
@@ -105,6 +106,9 @@ def load() -> C.CDLL:
     lib.l3ci_token_shift.argtypes = [vp, vp, vp, i64, vp, vp, i32, i32, i32, i64, i32, vp]
     lib.l3ci_delta_inputs.argtypes = [C.POINTER(DeltaInputsArgs)]
     lib.l3ci_recurrent_scan.argtypes = [C.POINTER(RecurrentScanArgs)]
+    lib.l3ci_recurrent_scan_chunks.argtypes = [C.POINTER(RecurrentScanArgs), vp, C.c_size_t]
+    lib.l3ci_recurrent_scan_scratch_bytes.argtypes = [C.POINTER(RecurrentScanArgs)]
+    lib.l3ci_recurrent_scan_scratch_bytes.restype = C.c_size_t
     lib.l3ci_moe_route.argtypes = [vp, vp, vp, vp, vp, vp, i64, i32, i32, vp]
     lib.l3ci_moe_gather.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i32, i32, i32, vp]
     lib.l3ci_moe_gather_places.argtypes = [vp, vp, vp, vp, vp, i64, i64, i32, i32, i32, vp]
@@ -373,10 +377,11 @@ def delta_inputs(p, b, a_proj, conv, a_log, dt_bias, tail, positions, H: int, G:
 
 
 def recurrent_scan(q, k, v, g, state, positions, norm, gate, *, act: int, eps: float, beta=None, bonus=None, g_bias=None,
-                   conv_in=None, tail=None, taps: int = 1, status=None):
+                   conv_in=None, tail=None, taps: int = 1, status=None, scratch=None):
     """q, k [B, T, G, D], v, gate [B, T, H, V], g [B, T, H, D], state [B, H, D, V] (fp32, carried), norm [V] or [H, V].  beta (delta rule) or bonus
     and g_bias (time mixing) choose the recurrence.  Returns the normed and gated output [B, T, H * V].  conv_in [B, T, W],
-    tail: the convolution's inputs and its carried ones, moved on."""
+    tail: the convolution's inputs and its carried ones, moved on.  scratch (uint8): by chunks of tokens in this memory, whatever the sizes; else
+    where chunks are the faster."""
     _cuda(q, k, v, g, state, positions, gate)
     B, T, H, V = v.shape
     G, D = q.shape[2:]
@@ -399,7 +404,13 @@ def recurrent_scan(q, k, v, g, state, positions, norm, gate, *, act: int, eps: f
         assert tail[0].is_contiguous() and conv_in.dtype == tail.dtype == v.dtype
         a.conv_in, a.conv_st, a.tail, a.tail_sb = conv_in.data_ptr(), _row_stride(conv_in), tail.data_ptr(), tail.stride(0)
     with _on(v):
-        _check(load().l3ci_recurrent_scan(C.byref(a)), "l3ci_recurrent_scan")
+        if scratch is None and T > 1:
+            need = load().l3ci_recurrent_scan_scratch_bytes(C.byref(a))
+            scratch = torch.empty(need, dtype=torch.uint8, device=v.device) if need else None
+        if scratch is not None:
+            _check(load().l3ci_recurrent_scan_chunks(C.byref(a), scratch.data_ptr(), scratch.numel()), "l3ci_recurrent_scan_chunks")
+        else:
+            _check(load().l3ci_recurrent_scan(C.byref(a)), "l3ci_recurrent_scan")
     return out.view(B, T, H * V)
 
 
