@@ -60,8 +60,8 @@ __device__ __forceinline__ float sinusoid(int p, double freq, bool cosine) {
   return cosine ? cosf(angle) : sinf(angle);
 }
 
-// Y: type of y.
-template <typename S, typename Y, int VEC, int VPT>
+// Y: type of y.  AHEAD: the norms' vectors are asked for with the row.
+template <typename S, typename Y, int VEC, int VPT, bool AHEAD = false>
 __global__ void __launch_bounds__(512) residual_norm_kernel(const l3ci_residual_norm_args a) {
   __shared__ float sm[2][kMaxWarps][3];
   const int tid = threadIdx.x, width = (int)a.width;
@@ -79,9 +79,9 @@ __global__ void __launch_bounds__(512) residual_norm_kernel(const l3ci_residual_
   float x[VPT * VEC], y[VPT * VEC];
 #pragma unroll
   for (int i = 0; i < VPT * VEC; ++i) x[i] = y[i] = 0.f;
-  // a thread of few columns asks for the norms' vectors along with the row: behind the statistics they were a trip to memory each (8 rows of 2048,
-  // 4.5 us in a step, 4.1 so)
-  constexpr bool kAhead = VPT == 1;
+  // few rows: a thread asks for the norms' vectors along with the row; behind the statistics they were a trip to memory each (8 rows of 2048,
+  // 4.5 us in a step, 4.1 so, 3.7 with half a vector a thread).  Not with more rows than SMs: the registers leave room for fewer of them.
+  constexpr bool kAhead = AHEAD && VPT == 1;
   float post_w[kAhead ? VEC : 1], post_b[kAhead ? VEC : 1], pre_w[kAhead ? VEC : 1], pre_b[kAhead ? VEC : 1];
   if constexpr (kAhead) {
     if (chunks > 0) {
@@ -245,10 +245,16 @@ int residual_norm_typed(const l3ci_residual_norm_args* a) {
   int threads = 32, vpt = 1;
   while ((many && vec ? kManyVpt : 1) * threads < units && threads < 512) threads *= 2;
   while ((long long)vpt * threads < units) vpt *= 2;
+  // a row that has an SM to itself: half a vector a thread, where 512 threads are enough (a launch's code comes cold: fewer instructions; 8 rows of
+  // 2048, back to back, 3.45 and 3.00 us)
+  const bool few = vec && a->rows <= (sm_count() > 0 ? sm_count() : 148), half = few && units <= 256;
+  if (half) threads = 2 * threads > 512 ? 512 : 2 * threads;
   auto go = [&](auto kernel) -> int {
     L3CI_LAUNCH("residual_norm_kernel", kernel, dim3((unsigned)a->rows), dim3(threads), 0, reinterpret_cast<cudaStream_t>(a->stream), *a);
     return L3CI_OK;
   };
+  if (half) return go(residual_norm_kernel<S, Y, kVec / 2, 1, true>);
+  if (few && vpt == 1) return go(residual_norm_kernel<S, Y, kVec, 1, true>);
   if (vec) {
     switch (vpt) {
       case 1: return go(residual_norm_kernel<S, Y, kVec, 1>);
