@@ -115,6 +115,19 @@ L3CI_API int l3ci_linear(const l3ci_linear_args* args);
 /* The same; with a limit above 0 the gated activation is z sigmoid(alpha z) (u + 1) of z = min(gate, limit), u = clamp(up, -limit, limit)
  * (experts whose rows lie in places of their own, one group each). */
 L3CI_API int l3ci_linear_gated(const l3ci_linear_args* args, float limit, float alpha);
+/* The query, key and value projections of a decode step and what l3ci_rot_embed_kv_cache_at does to them (model.py:95-108), the same bits as by two calls:
+ * w [(Hq + 2 Hkv) D, K]; rows b * T + t of x; rotated queries to out [rows, Hq * D] (out_st), rotated keys and values to the rows of the caches at
+ * positions[b] + t (a position outside the table or the cache is skipped).  Up to 32 rows and projections that clusters of 4 or 8 CTAs share, else
+ * L3CI_ERR_UNSUPPORTED: two calls. */
+typedef struct l3ci_linear_rope {
+  const float* freq_table;
+  const int32_t* positions;
+  void* cache_k;
+  void* cache_v;
+  int64_t freq_rows, cache_sb, cache_st, cache_len;
+  int32_t T, Hq, Hkv, D;
+} l3ci_linear_rope;
+L3CI_API int l3ci_linear_rot_embed_kv_cache(const l3ci_linear_args* args, const l3ci_linear_rope* rope);
 /* The same of any number of rows, tiles of 256 x 256 over pairs of SMs (a prompt's products with an activation): groups 1, out bf16, N and
  * out_st multiples of 8, out on 16 bytes; split and early are not used, status is the library's word. */
 L3CI_API int l3ci_linear_many(const l3ci_linear_args* args);

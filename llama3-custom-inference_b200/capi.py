@@ -19,7 +19,7 @@ OK, ERR_INVALID, ERR_UNSUPPORTED, ERR_ALIGNMENT, ERR_SCRATCH, ERR_CUDA, ERR_DEVI
 # Every symbol include/l3ci_b200.h declares.
 EXPORTS = (
     "l3ci_status_string", "l3ci_last_error", "l3ci_version", "l3ci_set_device_wait_limit_ns", "l3ci_set_programmatic_launch",
-    "l3ci_rms_norm", "l3ci_add_rms_norm", "l3ci_silu_mul", "l3ci_linear", "l3ci_linear_gated", "l3ci_linear_many", "l3ci_linear_poll", "l3ci_row_stride", "l3ci_greedy_step", "l3ci_top_p_step", "l3ci_top_p_kernel_choice", "l3ci_rot_embed", "l3ci_rot_embed_kv_cache", "l3ci_rot_embed_kv_cache_at",
+    "l3ci_rms_norm", "l3ci_add_rms_norm", "l3ci_silu_mul", "l3ci_linear", "l3ci_linear_gated", "l3ci_linear_many", "l3ci_linear_rot_embed_kv_cache", "l3ci_linear_poll", "l3ci_row_stride", "l3ci_greedy_step", "l3ci_top_p_step", "l3ci_top_p_kernel_choice", "l3ci_rot_embed", "l3ci_rot_embed_kv_cache", "l3ci_rot_embed_kv_cache_at",
     "l3ci_flash_decode_scratch_bytes", "l3ci_flash_decode", "l3ci_flash_decode_static", "l3ci_flash_decode_poll",
     "l3ci_flash_decode_kernel_choice",
     "l3ci_lse_merge", "l3ci_lse_exchange_bytes", "l3ci_lse_exchange_merge", "l3ci_prefill_attention",
@@ -106,6 +106,8 @@ def load() -> C.CDLL:
     lib.l3ci_linear.argtypes = [C.POINTER(LinearArgs)]
     lib.l3ci_linear_gated.restype = C.c_int
     lib.l3ci_linear_gated.argtypes = [C.POINTER(LinearArgs), C.c_float, C.c_float]
+    lib.l3ci_linear_rot_embed_kv_cache.restype = C.c_int
+    lib.l3ci_linear_rot_embed_kv_cache.argtypes = [C.POINTER(LinearArgs), vp]
     lib.l3ci_linear_many.restype = C.c_int
     lib.l3ci_linear_many.argtypes = [C.POINTER(LinearArgs)]
     lib.l3ci_linear_poll.restype = C.c_int

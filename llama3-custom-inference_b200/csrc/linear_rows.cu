@@ -16,7 +16,8 @@
 //     64 gate rows and the 64 up rows of the same outputs.
 // Measured in chains on weights beyond L2, us (the library's product and its activation): one row, w 2048 x 2048 3.7 (8.1), 2048 x 8192
 // 9.2 (20.2), gated 2 x 8192 x 2048 13.7 (15.3), 128256 x 2048 82 (81); 64 rows 6.8 (5.7), 12.3 (13.7), 16.3 (15.9), 88 (95): the
-// extension leaves the shapes that lose to the library.  A step of the 1B model behind 4001 tokens: 696 us, 1103 to 1127 with the library's.
+// extension leaves the shapes that lose to the library.  A step of the 1B model behind 4001 tokens: 696 us, 1103 to 1127 with the library's, and
+// 668 with the rotation and the cache write in the projections' last step (a launch a layer less; figures at the kernel).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -65,6 +66,7 @@ struct LinParams {
   int tiles, steps;                        // tiles of w, stages of K
   int group_tiles;                         // tiles of one group
   float limit, alpha;                      // of a gated activation
+  l3ci_linear_rope rope;                   // (kernels with ROPE)
 };
 
 __device__ __forceinline__ float lin_act(float z, int act) {
@@ -101,11 +103,16 @@ __device__ __forceinline__ bool output_warps_agree(bool ok) {
   return r != 0;
 }
 
-// S: CTAs of a cluster, which share a tile's columns of w.  GATED: w holds N gate rows, then N up rows.
-template <int NP, int S, bool GATED>
+// S: CTAs of a cluster, which share a tile's columns of w.  GATE: 1 silu(gate) * up of w's N gate rows and N up rows, 2 its clamped form
+// (a kernel of its own: both in one took a layer's step of 64 rows 1 us), 0 none.
+// ROPE: the outputs are queries, keys and values, which the last step rotates and puts where l3ci_rot_embed_kv_cache_at does, with its
+// bits.  That call took 2.4 us of a layer's 43 at one token and 4001 positions, nearly all of it a launch and a trip to memory each way;
+// here the table and the positions come while the sums still run.  A step of one token 696 -> 668 us.
+template <int NP, int S, int GATE, bool ROPE>
 __global__ void __launch_bounds__(kThreads, 2)
 linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ LinParams p) {
   using Sh = LinShape<NP>;
+  constexpr bool GATED = GATE > 0;
   constexpr int kStages = Sh::kStages;
   constexpr int kOuts = GATED ? kTile / 2 : kTile;     // outputs of a tile
   extern __shared__ uint8_t smem_raw[];
@@ -149,6 +156,27 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
   const int k0 = (int)((long long)p.steps * rank / S), steps = (int)((long long)p.steps * (rank + 1) / S) - k0;   // this CTA's stages of a tile
   bool ok = true;
   int asked = 0;                        // stages that this thread has asked for
+
+  constexpr int kOwn = kOuts / S;       // outputs of a cluster's CTA
+  // a pair of outputs that are rotated together, of the output warps' threads: the first one's place is looked up ahead of the sums
+  struct Pair { int t, j, n; long long pos; float2 turn; };
+  auto pair_at = [&](int e) {
+    Pair x;
+    x.t = e / (kOwn / 2);
+    x.j = e % (kOwn / 2) * 2;
+    x.n = first * kOuts + rank * kOwn + x.j;
+    x.pos = -1;
+    x.turn = make_float2(1.f, 0.f);
+    if (ROPE && warp >= 2 && x.t < (int)a.rows && x.n < a.N) {
+      const long long pos = (long long)p.rope.positions[x.t / p.rope.T] + x.t % p.rope.T;
+      if (pos >= 0 && pos < p.rope.freq_rows && pos < p.rope.cache_len) {
+        x.pos = pos;
+        if (x.n < (p.rope.Hq + p.rope.Hkv) * p.rope.D) x.turn = *reinterpret_cast<const float2*>(p.rope.freq_table + pos * p.rope.D + x.n % p.rope.D);
+      }
+    }
+    return x;
+  };
+  Pair pair{};
 
   if (warp == 0) {
     // ---- producer ----
@@ -213,6 +241,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
   } else {
     // ---- output: a thread owns row r of the tile ----
     pdl_wait();
+    if constexpr (ROPE) pair = pair_at((int)threadIdx.x - 64);
     const int q4 = warp & 3, r = q4 * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(q4 * 32) << 16;
     const int rows = (int)a.rows;
@@ -242,7 +271,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
               if (r < 64 && n < a.N)
 #pragma unroll
                 for (int i = 0; i < kSwap; ++i)
-                  if (c + h + i < rows) store_out(a, grp, c + h + i, n, gated_activation(__uint_as_float(v[h + i]), swap[i * 64 + r], p.limit, p.alpha));
+                  if (c + h + i < rows) store_out(a, grp, c + h + i, n, gated_activation(__uint_as_float(v[h + i]), swap[i * 64 + r], GATE == 2 ? p.limit : 0.f, p.alpha));
               output_warps_meet();
             }
           } else if (n < a.N) {
@@ -259,7 +288,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
   }
   if constexpr (S > 1) {
     // ---- one tile per cluster: every CTA has its part of the sums; CTA o adds up outputs o * kOuts / S onwards ----
-    constexpr int kSlice = kTile / S, kOwn = kOuts / S;   // rows of w and outputs of a CTA
+    constexpr int kSlice = kTile / S;                     // rows of w of a CTA
     __syncwarp();
     if constexpr (Sh::kInRing) cluster_arrive();
     cluster_wait();                                       // the others' shared memory may be written: they have started, or are done with the ring
@@ -283,7 +312,30 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
     __syncwarp();
     cluster_arrive();
     cluster_wait();
-    for (int e = threadIdx.x; e < (int)a.rows * kOwn; e += kThreads) {
+    if constexpr (ROPE) {
+      const l3ci_linear_rope& rp = p.rope;
+      const int q_cols = rp.Hq * rp.D, k_cols = rp.Hkv * rp.D;
+      for (int e = (int)threadIdx.x - 64; e >= 0 && e < (int)a.rows * (kOwn / 2); e += 128, pair = pair_at(e)) {
+        if (pair.pos < 0) continue;                       // (a position outside the table or the cache is skipped, not written)
+        float x = 0.f, y = 0.f;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          x += parts[pair.t * kTile + s * kSlice + pair.j];
+          y += parts[pair.t * kTile + s * kSlice + pair.j + 1];
+        }
+        x = __bfloat162float(__float2bfloat16_rn(x));     // (the projections are bf16 where they are two calls)
+        y = __bfloat162float(__float2bfloat16_rn(y));
+        const long long row = (long long)(pair.t / rp.T) * rp.cache_sb + pair.pos * rp.cache_st;
+        __nv_bfloat16* to = pair.n < q_cols ? static_cast<__nv_bfloat16*>(a.out) + pair.t * a.out_st + pair.n
+                            : pair.n < q_cols + k_cols ? static_cast<__nv_bfloat16*>(rp.cache_k) + row + pair.n - q_cols
+                                                       : static_cast<__nv_bfloat16*>(rp.cache_v) + row + pair.n - q_cols - k_cols;
+        const float c = pair.turn.x, sn = pair.turn.y;
+        const bool turns = pair.n < q_cols + k_cols;      // (a value is copied: an infinite neighbour must not reach it)
+        *reinterpret_cast<__nv_bfloat162*>(to) = __floats2bfloat162_rn(turns ? __fmaf_rn(x, c, -__fmul_rn(y, sn)) : x,
+                                                                       turns ? __fmaf_rn(x, sn, __fmul_rn(y, c)) : y);
+      }
+    }
+    for (int e = threadIdx.x; !ROPE && e < (int)a.rows * kOwn; e += kThreads) {
       const int t = e / kOwn, j = e % kOwn, n = first % p.group_tiles * kOuts + rank * kOwn + j;
       if (n >= a.N) continue;
       float y = 0.f, u = 0.f;
@@ -292,7 +344,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
         y += parts[t * kTile + s * kSlice + j];
         if (GATED) u += parts[t * kTile + s * kSlice + kOwn + j];
       }
-      store_out(a, first / p.group_tiles, t, n, GATED ? gated_activation(y, u, p.limit, p.alpha) : lin_act(y, a.act));
+      store_out(a, first / p.group_tiles, t, n, GATED ? gated_activation(y, u, GATE == 2 ? p.limit : 0.f, p.alpha) : lin_act(y, a.act));
     }
   }
   if (!ok && lane == 0) atomicExch(a.status ? a.status : &g_wait_status, (int)L3CI_ERR_DEVICE_WAIT);
@@ -304,14 +356,16 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
   if (warp == 1) tmem_dealloc(tmem, Sh::kTmem);
 }
 
-template <int NP, int S, bool GATED>
-int launch(const l3ci_linear_args* a, float limit, float alpha, cudaStream_t stream) {
+template <int NP, int S, int GATE, bool ROPE = false>
+int launch(const l3ci_linear_args* a, float limit, float alpha, cudaStream_t stream, const l3ci_linear_rope* rope = nullptr) {
   using Sh = LinShape<NP>;
+  constexpr bool GATED = GATE > 0;
   constexpr int kOuts = GATED ? kTile / 2 : kTile;
   LinParams p = {};
   p.a = *a;
   p.limit = limit;
   p.alpha = alpha;
+  if (rope) p.rope = *rope;
   p.group_tiles = (a->N + kOuts - 1) / kOuts;
   p.tiles = p.group_tiles * a->groups;
   p.steps = (a->K + kDeep - 1) / kDeep;
@@ -319,7 +373,7 @@ int launch(const l3ci_linear_args* a, float limit, float alpha, cudaStream_t str
   CUtensorMap xmap, wmap;
   if (int st = make_rows_map(&xmap, a->x, a->K, (int)a->rows, 1, a->groups, a->x_st, 0, a->x_sg, NP)) return st;
   if (int st = make_rows_map(&wmap, a->w, a->K, a->N, GATED ? 2 : 1, a->groups, a->K, one, one * (GATED ? 2 : 1), kOuts)) return st;
-  auto kernel = linear_rows_kernel<NP, S, GATED>;
+  auto kernel = linear_rows_kernel<NP, S, GATE, ROPE>;
   static bool configured[64] = {false};
   int dev = 0;
   L3CI_CUDA_TRY(cudaGetDevice(&dev));
@@ -353,8 +407,9 @@ int launch(const l3ci_linear_args* a, float limit, float alpha, cudaStream_t str
   return L3CI_OK;
 }
 
-template <int NP, bool GATED>
+template <int NP, int GATE>
 int launch_split(const l3ci_linear_args* a, float limit, float alpha, cudaStream_t stream) {
+  constexpr bool GATED = GATE > 0;
   const long long tiles = (a->N + (GATED ? kTile / 2 : kTile) - 1) / (GATED ? kTile / 2 : kTile) * (long long)a->groups;
   int split = a->split;
   if (split == 0) {
@@ -366,10 +421,10 @@ int launch_split(const l3ci_linear_args* a, float limit, float alpha, cudaStream
   }
   while (split > 1 && split > (a->K + kDeep - 1) / kDeep) split /= 2;   // every CTA has a stage
   switch (split) {
-    case 1: return launch<NP, 1, GATED>(a, limit, alpha, stream);
-    case 2: return launch<NP, 2, GATED>(a, limit, alpha, stream);
-    case 4: return launch<NP, 4, GATED>(a, limit, alpha, stream);
-    case 8: return launch<NP, 8, GATED>(a, limit, alpha, stream);
+    case 1: return launch<NP, 1, GATE>(a, limit, alpha, stream);
+    case 2: return launch<NP, 2, GATE>(a, limit, alpha, stream);
+    case 4: return launch<NP, 4, GATE>(a, limit, alpha, stream);
+    case 8: return launch<NP, 8, GATE>(a, limit, alpha, stream);
     default: return fail(L3CI_ERR_INVALID, "linear: split %d is not 1, 2, 4 or 8", split);
   }
 }
@@ -433,7 +488,7 @@ extern "C" int l3ci_linear_gated(const l3ci_linear_args* a, float limit, float a
   const bool gated = a->act == L3CI_ACT_SILU_GATE;
   auto go = [&](auto np) {
     constexpr int NP = decltype(np)::value;
-    return gated ? launch_split<NP, true>(a, limit, alpha, s) : launch_split<NP, false>(a, limit, alpha, s);
+    return !gated ? launch_split<NP, 0>(a, limit, alpha, s) : limit > 0.f ? launch_split<NP, 2>(a, limit, alpha, s) : launch_split<NP, 1>(a, limit, alpha, s);
   };
   if (a->rows <= 8) return go(std::integral_constant<int, 8>{});
   if (a->rows <= 16) return go(std::integral_constant<int, 16>{});
@@ -442,3 +497,32 @@ extern "C" int l3ci_linear_gated(const l3ci_linear_args* a, float limit, float a
 }
 
 extern "C" int l3ci_linear(const l3ci_linear_args* a) { return l3ci_linear_gated(a, 0.f, 0.f); }
+
+extern "C" int l3ci_linear_rot_embed_kv_cache(const l3ci_linear_args* a, const l3ci_linear_rope* rope) {
+  using namespace l3ci;
+  clear_error();
+  if (!a || !rope) return fail(L3CI_ERR_INVALID, "linear_rot_embed_kv_cache: null arguments");
+  if (a->rows < 0 || a->K <= 0 || a->N <= 0 || a->act != L3CI_ACT_NONE || a->groups != 1 || a->out_f32 || rope->T <= 0 || rope->Hq <= 0 || rope->Hkv <= 0 || rope->D <= 0 ||
+      a->rows % rope->T || a->N != (rope->Hq + 2 * rope->Hkv) * rope->D || rope->freq_rows < 0 || rope->cache_len < 0)
+    return fail(L3CI_ERR_INVALID, "linear_rot_embed_kv_cache: rows=%lld K=%d N=%d T=%d heads %d, %d of %d", (long long)a->rows, a->K, a->N, rope->T, rope->Hq, rope->Hkv, rope->D);
+  if (a->rows == 0) return L3CI_OK;
+  if (!a->x || !a->w || !a->out || !rope->freq_table || !rope->positions || !rope->cache_k || !rope->cache_v)
+    return fail(L3CI_ERR_INVALID, "linear_rot_embed_kv_cache: null pointer");
+  if (a->K % 8 || a->x_st % 8 || !aligned16(a->x) || !aligned16(a->w)) return fail(L3CI_ERR_ALIGNMENT, "linear: rows of x and w must be whole 16-byte vectors");
+  auto on4 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 3) == 0; };
+  if (rope->D % 2 || !on4(a->out) || a->out_st % 2 || !on4(rope->cache_k) || !on4(rope->cache_v) || rope->cache_sb % 2 || rope->cache_st % 2 || !on4(rope->positions) ||
+      (reinterpret_cast<uintptr_t>(rope->freq_table) & 7))
+    return fail(L3CI_ERR_ALIGNMENT, "linear_rot_embed_kv_cache: pairs must start on 4 bytes, the table on 8");
+  if (a->rows > 1 && (a->x_st <= 0 || a->out_st < rope->Hq * rope->D)) return fail(L3CI_ERR_INVALID, "linear_rot_embed_kv_cache: rows without a stride of their own");
+  // clusters of 8 or 4 CTAs a tile, up to 32 rows (16 threads a row in the last step): a decode step's projections; others are two calls
+  const int sms = sm_count() > 0 ? sm_count() : 148, steps = (a->K + kDeep - 1) / kDeep;
+  const long long tiles = (a->N + kTile - 1) / kTile;
+  const int split = tiles * 8 <= 2 * sms && steps >= 16 ? 8 : tiles * 4 <= 2 * sms && steps >= 8 ? 4 : 0;
+  if (split == 0 || a->rows > 32) return fail(L3CI_ERR_UNSUPPORTED, "linear_rot_embed_kv_cache: %lld rows, K=%d, N=%d", (long long)a->rows, a->K, a->N);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(a->stream);
+  auto go = [&](auto np) {
+    constexpr int NP = decltype(np)::value;
+    return split == 8 ? launch<NP, 8, 0, true>(a, 0.f, 0.f, s, rope) : launch<NP, 4, 0, true>(a, 0.f, 0.f, s, rope);
+  };
+  return a->rows <= 8 ? go(std::integral_constant<int, 8>{}) : a->rows <= 16 ? go(std::integral_constant<int, 16>{}) : go(std::integral_constant<int, 32>{});
+}

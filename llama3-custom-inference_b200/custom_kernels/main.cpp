@@ -578,6 +578,50 @@ Tensor rot_embed_kv_cache(Tensor qkv, Tensor freq, Tensor cache_k, Tensor cache_
   return q_out;
 }
 
+// linear(x, w) of few rows, then rot_embed_kv_cache of its rows, in one kernel: the rotated queries; nothing where that kernel does not apply or
+// does not pay (the rule of `linear`; more than 32 rows).  `early`, `always`: as in `linear`.
+std::optional<Tensor> linear_rot_embed_kv_cache(Tensor x, Tensor w, Tensor freq, Tensor cache_k, Tensor cache_v, int64_t n_head, int64_t n_kv_head,
+                                                Tensor positions, bool early, bool always) {
+  check_bf16_cuda(x, "x");
+  check_bf16_cuda(w, "w");
+  check_bf16_cuda(cache_k, "cache_k");
+  check_bf16_cuda(cache_v, "cache_v");
+  TORCH_CHECK(x.dim() == 3 && w.dim() == 2 && w.size(1) == x.size(2), "x must be [B, T, K], w [N, K]");
+  TORCH_CHECK(n_head > 0 && n_kv_head > 0 && w.size(0) % (n_head + 2 * n_kv_head) == 0, "w's rows do not match the head counts");
+  const int64_t B = x.size(0), T = x.size(1), K = x.size(2), N = w.size(0), D = N / (n_head + 2 * n_kv_head);
+  TORCH_CHECK(cache_k.dim() == 4 && cache_k.sizes() == cache_v.sizes() && cache_k.strides() == cache_v.strides(),
+              "cache_k and cache_v must be [maxB, maxLen, n_kv_head, D] with equal layout");
+  TORCH_CHECK(cache_k.size(2) == n_kv_head && cache_k.size(3) == D && cache_k.stride(3) == 1 && cache_k.stride(2) == D,
+              "cache rows must be [n_kv_head, D] contiguous");
+  TORCH_CHECK(B <= cache_k.size(0), "batch does not fit the cache");
+  TORCH_CHECK(freq.is_cuda() && freq.scalar_type() == torch::kFloat32 && freq.dim() == 2 && freq.size(1) == D, "freq must be the whole float32 [rows, D] table");
+  TORCH_CHECK(positions.is_cuda() && positions.scalar_type() == torch::kInt32 && positions.dim() == 1 && positions.size(0) == B && positions.is_contiguous(),
+              "positions must be a contiguous int32 CUDA tensor of shape [B]");
+  for (const Tensor& t : {w, cache_k, cache_v, freq, positions}) TORCH_CHECK(t.get_device() == x.get_device(), "tensors on different devices");
+  const int64_t rows = B * T;
+  if (rows == 0 || rows > 32 || K % 8 || !w.is_contiguous() || !freq.is_contiguous() ||
+      (!always && !few_rows_pay(rows, K, N, 1, L3CI_ACT_NONE, early)))
+    return std::nullopt;
+  const int64_t stride = l3ci_row_stride(x.sizes().data(), x.strides().data(), 3);
+  if (stride < 0 || stride % 8) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor q = torch::empty({B, T, n_head, D}, x.options());
+  l3ci_linear_args a{};
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = q.data_ptr();
+  a.rows = rows; a.x_st = stride; a.out_st = n_head * D;
+  a.K = (int32_t)K; a.N = (int32_t)N; a.groups = 1; a.act = L3CI_ACT_NONE; a.early = early;
+  a.stream = current_stream();
+  l3ci_linear_rope r{};
+  r.freq_table = freq.data_ptr<float>(); r.positions = positions.data_ptr<int32_t>();
+  r.cache_k = cache_k.data_ptr(); r.cache_v = cache_v.data_ptr();
+  r.freq_rows = freq.size(0); r.cache_sb = cache_k.stride(0); r.cache_st = cache_k.stride(1); r.cache_len = cache_k.size(1);
+  r.T = (int32_t)T; r.Hq = (int32_t)n_head; r.Hkv = (int32_t)n_kv_head; r.D = (int32_t)D;
+  const int status = l3ci_linear_rot_embed_kv_cache(&a, &r);
+  if (status == L3CI_ERR_UNSUPPORTED || status == L3CI_ERR_ALIGNMENT) return std::nullopt;
+  check_status(status, "linear_rot_embed_kv_cache");
+  return q;
+}
+
 // Status of the few-row products on the current stream of `like`'s device: 0, or 6 once after a device-side wait ran out.
 int64_t linear_status(Tensor like) {
   TORCH_CHECK(like.is_cuda(), "like must be a CUDA tensor");
@@ -621,6 +665,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("few_rows", torch::wrap_pybind_function(few_rows), "few_rows", py::arg("x"), py::arg("w"), py::arg("act") = (int64_t)L3CI_ACT_NONE,
         py::arg("early") = false, py::arg("f32") = false, py::arg("into") = py::none(),
         py::arg("always") = false, py::arg("limit") = 0.0, py::arg("alpha") = 0.0);
+  m.def("linear_rot_embed_kv_cache", torch::wrap_pybind_function(linear_rot_embed_kv_cache), "linear_rot_embed_kv_cache", py::arg("x"), py::arg("w"), py::arg("freq"),
+        py::arg("cache_k"), py::arg("cache_v"), py::arg("n_head"), py::arg("n_kv_head"), py::arg("positions"), py::arg("early") = false, py::arg("always") = false);
   m.def("many_rows", torch::wrap_pybind_function(many_rows), "many_rows", py::arg("x"), py::arg("w"), py::arg("act"));
   m.def("greedy_step", torch::wrap_pybind_function(greedy_step), "greedy_step", py::arg("logits"), py::arg("out_tokens"),
         py::arg("steps"), py::arg("next_input"), py::arg("positions"), py::arg("seq_lens"));

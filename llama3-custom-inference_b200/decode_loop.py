@@ -281,11 +281,15 @@ class Llama3Decoder(DecodeLoop):
             p = f"h{l}."
             cache_k, cache_v = self.cache_k[l][slots], self.cache_v[l][slots]
             _nvtx_push("layer")
-            qkv = product(h, w[p + "attn"])                                            # model.py:95
             _nvtx_push("rot_embd")
             _nvtx_push("use_kv")
-            q = ext.rot_embed_kv_cache(qkv, self.freqs, cache_k, cache_v, 0, Hq, Hkv,
-                                       positions=positions)                            # model.py:96-108
+            q = None
+            if few:                                                                    # model.py:95-108
+                q = ext.linear_rot_embed_kv_cache(h, w[p + "attn"], self.freqs, cache_k, cache_v, Hq, Hkv, positions, early=True, always=T > 1)
+            if q is None:
+                qkv = product(h, w[p + "attn"])                                        # model.py:95
+                q = ext.rot_embed_kv_cache(qkv, self.freqs, cache_k, cache_v, 0, Hq, Hkv,
+                                           positions=positions)                        # model.py:96-108
             _nvtx_pop()
             _nvtx_pop()
             if T > 1:
