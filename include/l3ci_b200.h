@@ -129,7 +129,9 @@ typedef struct l3ci_linear_rope {
 } l3ci_linear_rope;
 L3CI_API int l3ci_linear_rot_embed_kv_cache(const l3ci_linear_args* args, const l3ci_linear_rope* rope);
 /* The same of any number of rows, tiles of 256 x 256 over pairs of SMs (a prompt's products with an activation): groups 1, out bf16, N and
- * out_st multiples of 8, out on 16 bytes; split and early are not used, status is the library's word. */
+ * out_st multiples of 8, out on 16 bytes; split and early are not used, status is the library's word.  act may also be
+ * L3CI_ACT_SILU_MUL: silu(gate) * up with the roundings of l3ci_silu_mul on a bf16 product, the same bits. */
+#define L3CI_ACT_SILU_MUL 4
 L3CI_API int l3ci_linear_many(const l3ci_linear_args* args);
 /* Waits for `stream`; L3CI_ERR_DEVICE_WAIT, once, if a launch of l3ci_linear without a status word of its own, or of l3ci_linear_many, gave up on this device
  * (should never happen). */

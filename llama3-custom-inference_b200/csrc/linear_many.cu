@@ -1,5 +1,5 @@
 // out[rows, N] = act(x[rows, K] w[N, K]^T) of many rows (prompts) with the activation on the fp32 sums (include/l3ci_b200.h,
-// l3ci_linear_many): bf16 operands, gelu, tanh, or silu(gate) * up of a stacked matrix.
+// l3ci_linear_many): bf16 operands, gelu, tanh, or silu(gate) * up of a stacked matrix (or the same with silu_mul's roundings).
 //
 // The library's product writes twice the outputs of a gated product (268 MB a layer for 8192 tokens of the 1B model), and a pass of
 // its own reads them again.  Here the activation is done on the way out, under the next tile's product.
@@ -111,10 +111,14 @@ __device__ __forceinline__ void pair_commit(uint32_t bar, uint32_t elected) {
                ::"r"(bar), "r"(elected), "h"((uint16_t)3) : "memory");
 }
 
+// A pair of gate and up sums as a bf16 product has them, and silu's own rounding: l3ci_silu_mul's bits.
+__device__ __forceinline__ float bf16_of(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+__device__ __forceinline__ float silu_mul(float z, float u) { return bf16_of(gated(bf16_of(z), 1.f)) * bf16_of(u); }
+
 template <int ACT>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_many_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ ManyParams p) {
-  constexpr bool GATED = ACT == L3CI_ACT_SILU_GATE;
+  constexpr bool GATED = ACT == L3CI_ACT_SILU_GATE || ACT == L3CI_ACT_SILU_MUL;
   constexpr int kOuts = GATED ? kHalf : 2 * kHalf;       // output columns of a tile
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -234,7 +238,8 @@ linear_many_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               f[i] = __uint_as_float(y[v * 8 + i]);
-              if (GATED) f[i] = gated(f[i], __uint_as_float(z[v * 8 + i]));
+              if (ACT == L3CI_ACT_SILU_MUL) f[i] = silu_mul(f[i], __uint_as_float(z[v * 8 + i]));
+              else if (GATED) f[i] = gated(f[i], __uint_as_float(z[v * 8 + i]));
               else if (ACT == L3CI_ACT_TANH) f[i] = tanhf(f[i]);
             }
             if (ACT == L3CI_ACT_GELU)
@@ -272,7 +277,7 @@ linear_many_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
 
 template <int ACT>
 int launch(const l3ci_linear_args* a) {
-  constexpr bool GATED = ACT == L3CI_ACT_SILU_GATE;
+  constexpr bool GATED = ACT == L3CI_ACT_SILU_GATE || ACT == L3CI_ACT_SILU_MUL;
   ManyParams p = {};
   const int outs = GATED ? kHalf : 2 * kHalf;
   p.m_tiles = (a->rows + 2 * kHalf - 1) / (2 * kHalf);
@@ -326,7 +331,7 @@ extern "C" int l3ci_linear_many(const l3ci_linear_args* a) {
   using namespace l3ci;
   clear_error();
   if (!a) return fail(L3CI_ERR_INVALID, "linear_many: null arguments");
-  if (a->rows < 0 || a->rows > INT32_MAX || a->K <= 0 || a->N < 0 || a->act < L3CI_ACT_NONE || a->act > L3CI_ACT_SILU_GATE || a->groups != 1 || a->out_f32)
+  if (a->rows < 0 || a->rows > INT32_MAX || a->K <= 0 || a->N < 0 || a->act < L3CI_ACT_NONE || a->act > L3CI_ACT_SILU_MUL || a->groups != 1 || a->out_f32)
     return fail(L3CI_ERR_INVALID, "linear_many: rows=%lld K=%d N=%d groups=%d act=%d", (long long)a->rows, a->K, a->N, a->groups, a->act);
   if (a->rows == 0 || a->N == 0) return L3CI_OK;
   if (!a->x || !a->w || !a->out) return fail(L3CI_ERR_INVALID, "linear_many: null pointer");
@@ -337,6 +342,7 @@ extern "C" int l3ci_linear_many(const l3ci_linear_args* a) {
     case L3CI_ACT_GELU: return launch<L3CI_ACT_GELU>(a);
     case L3CI_ACT_TANH: return launch<L3CI_ACT_TANH>(a);
     case L3CI_ACT_SILU_GATE: return launch<L3CI_ACT_SILU_GATE>(a);
+    case L3CI_ACT_SILU_MUL: return launch<L3CI_ACT_SILU_MUL>(a);
     default: return launch<L3CI_ACT_NONE>(a);
   }
 }

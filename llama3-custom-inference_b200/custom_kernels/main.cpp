@@ -415,7 +415,7 @@ std::optional<Tensor> many_rows(const Tensor& x, const Tensor& w, int64_t act) {
   if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != torch::kBFloat16 || w.scalar_type() != torch::kBFloat16 ||
       w.get_device() != x.get_device() || x.dim() < 1 || w.dim() != 2 || act == L3CI_ACT_NONE)
     return std::nullopt;
-  const bool gated = act == L3CI_ACT_SILU_GATE;
+  const bool gated = act == L3CI_ACT_SILU_GATE || act == L3CI_ACT_SILU_MUL;
   const int64_t K = x.size(-1), N = gated ? w.size(0) / 2 : w.size(0), rows = K ? x.numel() / K : 0;
   if (w.size(1) != K || K % 8 || N == 0 || N % 8 || (gated && w.size(0) % 2) || !w.is_contiguous() || rows > INT32_MAX || K > INT32_MAX || w.size(0) > INT32_MAX ||
       !many_rows_pay(rows, N, gated, at::cuda::getDeviceProperties(x.get_device())->multiProcessorCount))
@@ -446,7 +446,7 @@ Tensor linear(Tensor x, Tensor w, bool gated, bool early, bool always) {
   TORCH_CHECK(!gated || w.size(0) % 2 == 0, "a gated product takes an even number of rows of w");
   if (auto y = few_rows(x, w, gated ? L3CI_ACT_SILU_GATE : L3CI_ACT_NONE, early, false, std::nullopt, always, 0.0, 0.0)) return *y;
   if (gated)
-    if (auto y = many_rows(x, w, L3CI_ACT_SILU_GATE)) return *y;
+    if (auto y = many_rows(x, w, L3CI_ACT_SILU_MUL)) return *y;     // (silu_mul's bits)
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y = at::linear(x, w);
   if (!gated) return y;

@@ -47,9 +47,20 @@ def test_products_with_activations(capi, device, rows, K, N, act):
     assert capi.load().l3ci_linear_poll(torch.cuda.current_stream().cuda_stream) == capi.OK
 
 
+@pytest.mark.parametrize("rows,K,N", [(300, 640, 1032), (2049, 2048, 8192)])
+def test_silu_mul_of_a_product_bit_for_bit(ext, capi, device, rows, K, N):
+    """The form that stands for a bf16 product and silu_mul: their bits, where this kernel's sums are the plain product's."""
+    x, w = rand(rows, K, seed=3), rand(2 * N, K, seed=4, scale=8 * K ** -0.5)
+    plain, out = torch.empty(rows, 2 * N, dtype=BF16, device=device), torch.empty(rows, N, dtype=BF16, device=device)
+    a = capi.LinearArgs(x=x.data_ptr(), w=w.data_ptr(), out=out.data_ptr(), rows=rows, x_st=K, out_st=N, K=K, N=N, groups=1, act=4,
+                        stream=torch.cuda.current_stream().cuda_stream)
+    assert many(capi, x, w, 0, plain) == capi.OK and capi.load().l3ci_linear_many(C.byref(a)) == capi.OK
+    assert torch.equal(out, ext.silu_mul(plain[:, :N], plain[:, N:]))
+
+
 def test_refused(capi, device):
     x, w, out = rand(300, 64), rand(64, 64), torch.empty(300, 64, dtype=BF16, device=device)
     assert many(capi, x[:, :60], w[:, :60], 0, out) == capi.ERR_ALIGNMENT
-    assert many(capi, x, w, 4, out) == capi.ERR_INVALID
+    assert many(capi, x, w, 5, out) == capi.ERR_INVALID
     assert many(capi, x[:1].expand(300, 64), w, 0, out) == capi.ERR_INVALID
     assert many(capi, x, w[:60], 0, out[:, :60]) == capi.ERR_ALIGNMENT
