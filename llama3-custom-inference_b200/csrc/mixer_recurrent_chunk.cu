@@ -11,13 +11,15 @@
 //     multiplied on from token to token, so that every decay is a product of factors at most 1 and none is divided by; L's and M's rows are the
 //     lanes' sums, T's columns a lane's each.
 //   chunk_scan_kernel    a warp per 16 columns of the state, whose transpose it keeps in accumulators of m16n8k8 products: per chunk U, the
-//     outputs and the new state are 312 of them (128 rows).  Operands are 32-bit, each split into two tf32 parts and multiplied in three
-//     products.  An accumulator's columns are the next product's depth, taken in the order in which they lie.  Chunks come through a ring of bulk
+//     outputs and the new state are 312 of them (128 rows).  Operands are 32-bit, split into tf32 parts: two and three
+//     products for the sums over the state, three and six (all but what lies below 2^-33) for U and the new state.  An accumulator's columns are the next product's depth, taken in the order in which they lie.  Chunks come through a ring of bulk
 //     copies.
-// 1777 tokens of 3 x 16 heads of 128 x 128 (delta rule): 349 us, token by token 741; 3 x 32 heads of 64 x 64 (time mixing): 222, 374.  Two thirds are the
-// scan, a warp per scheduler and 4000 cycles a chunk, of which the products alone are 2500.  With U and W instead of T in the chunks the rows of
+// 1777 tokens of 3 x 16 heads of 128 x 128 (delta rule): 429 us, token by token 741; 3 x 32 heads of 64 x 64 (time mixing): 231, 374.  Most of it is the
+// scan, a warp per scheduler, of which the products alone are 3300 cycles a chunk.  With U and W instead of T in the chunks the rows of
 // the forward substitution took longer than the scan; with the values read by the scan's lanes themselves a chunk took 1.4 times as long.
-// Errors against 64 bits: outputs the same (their rounding to bf16), states 1.3e-7 to 1.7e-7 of their norm, token by token 1.3e-7 to 1.4e-7.
+// Errors against 64 bits: outputs the same (their rounding to bf16); states after such prompts, of their norm, delta rule of four layers 1.43,
+// 1.29, 1.27, 1.76 e-7, token by token 1.52, 1.24, 1.24, 2.34, time mixing 1.76 to 1.97 e-7 and 1.86 to 2.02.  By three products throughout (346
+// us) it was 1.6 to 2.1 e-7: the bit that two parts leave out, and the product of the small parts.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -58,6 +60,15 @@ __device__ __forceinline__ Split split(float x) {
   s.lo = __float_as_uint(x - __uint_as_float(s.hi)) + 0x1000u;
   return s;
 }
+
+// The same without loss: lo as it is, of which a product takes the first 11 bits; the rest of it is a third part.
+__device__ __forceinline__ Split split_whole(float x) {
+  Split s;
+  s.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  s.lo = __float_as_uint(x - __uint_as_float(s.hi));
+  return s;
+}
+__device__ __forceinline__ uint32_t rest(uint32_t lo) { return __float_as_uint(__uint_as_float(lo) - __uint_as_float(lo & 0xffffe000u)); }
 
 struct ChunkParams {
   l3ci_recurrent_scan_args a;
@@ -222,7 +233,7 @@ chunk_inputs_kernel(const __grid_constant__ ChunkParams p, long long units) {
       f2_unpack(t[i + 1][j], y[0], y[1]);
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const Split sx = split(x[e]), sy = split(y[e]);
+        const Split sx = split_whole(x[e]), sy = split_whole(y[e]);
         *reinterpret_cast<uint4*>(block + Sh::kAtK + i / 2 * Sh::kKPitch + 4 * (d0 + 2 * j + e)) = make_uint4(sx.hi, sy.hi, sx.lo, sy.lo);
       }
     }
@@ -237,18 +248,36 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 }
 // An accumulator as the left operand of the next product, in two parts: its columns 2 t and 2 t + 1 are the depths t and t + 4.
 struct Left { uint32_t hi[4], lo[4]; };
+template <bool WHOLE = false>
 __device__ __forceinline__ Left left(const float (&c)[4]) {
   Left l;
   const int from[4] = {0, 2, 1, 3};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const Split s = split(c[from[i]]);
+    const Split s = WHOLE ? split_whole(c[from[i]]) : split(c[from[i]]);
     l.hi[i] = s.hi;
     l.lo[i] = s.lo;
   }
   return l;
 }
 struct Right { Split x, y; };
+// c (large products: their accumulator is cut off, not rounded) and d (small ones) += l r of split_whole's parts, all but what lies below 2^-33; EXACT: l has no small parts
+template <bool EXACT>
+__device__ __forceinline__ void mma_whole(float (&c)[4], float (&d)[4], const Left& l, const Right& r) {
+  const uint32_t rx = rest(r.x.lo), ry = rest(r.y.lo);
+  mma_tf32(d, l.hi, rx, ry);
+  mma_tf32(d, l.hi, r.x.lo, r.y.lo);
+  if (!EXACT) {
+    uint32_t lr[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) lr[i] = rest(l.lo[i]);
+    mma_tf32(d, lr, r.x.hi, r.y.hi);
+    mma_tf32(d, l.lo, r.x.lo, r.y.lo);
+    mma_tf32(d, l.lo, r.x.hi, r.y.hi);
+  }
+  mma_tf32(c, l.hi, r.x.hi, r.y.hi);
+}
+
 __device__ __forceinline__ Right right(const float* p) {
   const uint4 v = *reinterpret_cast<const uint4*>(p);
   return {{v.x, v.z}, {v.y, v.w}};
@@ -324,7 +353,7 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
       float ws[3][2][4] = {}, os[3][2][4] = {};
 #pragma unroll
       for (int x = 0; x < NT; ++x) {
-        const Left l = left(S[x]);
+        const Left l = left<>(S[x]);
         Right w[2], q[2];
 #pragma unroll
         for (int tt = 0; tt < 2; ++tt) {
@@ -343,14 +372,19 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
       }
       // U^T, and the outputs with it: sums over the chunk's tokens j, rows i of T and of M
       Left u[2];
-      auto by_rows = [&](const float* rows, const Left (&l)[2], float (&c)[3][2][4], bool exact) {   // exact: l has no small part
+      auto by_rows = [&](const float* rows, const Left (&l)[2], float (&c)[3][2][4], bool exact, bool whole) {   // exact: l has no small part
 #pragma unroll
         for (int tt = 0; tt < 2; ++tt) {
           Right m[2];
 #pragma unroll
           for (int ti = 0; ti < 2; ++ti) {
             const float2 f = *reinterpret_cast<const float2*>(rows + (8 * ti + g) * kMPitch + 8 * tt + 2 * t4);
-            m[ti] = {split(f.x), split(f.y)};
+            m[ti] = whole ? Right{split_whole(f.x), split_whole(f.y)} : Right{split(f.x), split(f.y)};
+          }
+          if (whole) {
+#pragma unroll
+            for (int ti = 0; ti < 2; ++ti) mma_whole<false>(c[tt][ti], c[2][ti], l[tt], m[ti]);
+            continue;
           }
 #pragma unroll
           for (int part = 0; part < (exact ? 2 : 3); ++part)
@@ -367,19 +401,19 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
           v[e] = to_f32(*reinterpret_cast<const __nv_bfloat16*>(vs + (8 * tt + 2 * t4 + (e & 1)) * kVPitch + (e >> 1) * 16));
           if (KIND == kDelta) v[e] -= ws[0][tt][e] + ws[1][tt][e] + ws[2][tt][e];
         }
-        u[tt] = left(v);
+        u[tt] = left<true>(v);
       }
       if (KIND == kDelta) {
         float us[3][2][4] = {};
-        by_rows(st + Sh::kAtT, u, us, false);
+        by_rows(st + Sh::kAtT, u, us, false, true);
 #pragma unroll
         for (int tt = 0; tt < 2; ++tt) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) us[0][tt][e] += us[1][tt][e] + us[2][tt][e];
-          u[tt] = left(us[0][tt]);
+          u[tt] = left<true>(us[0][tt]);
         }
       }
-      by_rows(st + Sh::kAtM, u, os, KIND == kTimeMix);      // (time mixing's U are bf16)
+      by_rows(st + Sh::kAtM, u, os, KIND == kTimeMix, false);      // (time mixing's U are bf16)
       const int n = min(kChunk, p.tokens - i * kChunk);
 #pragma unroll
       for (int ti = 0; ti < 2; ++ti)
@@ -393,23 +427,20 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
 #pragma unroll
       for (int x0 = 0; x0 < NT; x0 += kTogether) {
         Right k[kTogether][2];
-        float add[kTogether][4] = {};
+        float add[kTogether][4] = {}, small[kTogether][4] = {}, odd[kTogether][4] = {};
 #pragma unroll
         for (int x = 0; x < kTogether; ++x)
 #pragma unroll
           for (int tt = 0; tt < 2; ++tt) k[x][tt] = right(st + Sh::kAtK + (4 * tt + t4) * Sh::kKPitch + 4 * (8 * (x0 + x) + g));
 #pragma unroll
-        for (int part = KIND == kTimeMix ? 1 : 2; part >= 0; --part)
+        for (int tt = 0; tt < 2; ++tt)
 #pragma unroll
-          for (int tt = 0; tt < 2; ++tt)
-#pragma unroll
-            for (int x = 0; x < kTogether; ++x)
-              mma_tf32(add[x], part == 2 ? u[tt].lo : u[tt].hi, part == 1 ? k[x][tt].x.lo : k[x][tt].x.hi, part == 1 ? k[x][tt].y.lo : k[x][tt].y.hi);
+          for (int x = 0; x < kTogether; ++x) mma_whole<KIND == kTimeMix>(tt > 0 ? odd[x] : add[x], small[x], u[tt], k[x][tt]);
 #pragma unroll
         for (int x = 0; x < kTogether; ++x) {
           const float2 f = *reinterpret_cast<const float2*>(st + Sh::kAtG + 8 * (x0 + x) + 2 * t4);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) S[x0 + x][e] = fmaf(S[x0 + x][e], e & 1 ? f.y : f.x, add[x][e]);
+          for (int e = 0; e < 4; ++e) S[x0 + x][e] = fmaf(S[x0 + x][e], e & 1 ? f.y : f.x, add[x][e] + (odd[x][e] + small[x][e]));
         }
       }
       __syncwarp();
@@ -485,11 +516,11 @@ bool applies(const l3ci_recurrent_scan_args* a) {
 }  // namespace
 
 size_t scan_chunks_scratch(const l3ci_recurrent_scan_args* a) {
-  // From where the chunks are the faster, in CTAs of the scan and tokens (us by tokens and by chunks): 32 CTAs of the delta rule 192 tokens 44.1 and 44.3,
-  // 384 79.9 and 69.5, of time mixing 384 40.4 and 42.1, 512 50.2 and 50.2; 64 CTAs 64 tokens 29.5 and 29.4, time mixing 128 25.5 and 24.7; 96 CTAs
-  // 48 tokens 30.7 and 27.6, 19.6 and 19.4; 256 CTAs 32 tokens 43.0 and 33.8.
+  // From where the chunks are the faster, in CTAs of the scan and tokens (us by tokens and by chunks): 32 CTAs of the delta rule 384 tokens 79.5 and
+  // 87.0, of time mixing 40.2 and 44.3, and a token more costs both the same; 64 CTAs 96 tokens 38.9 and 37.9, time mixing 128 25.5 and 25.6; 96
+  // CTAs 48 tokens 30.7 and 30.0, 64 24.1 and 22.2; 256 CTAs 48 tokens 54.8 and 43.6, 33.9 and 28.1.
   const long long ctas = (long long)a->B * a->H * ((a->V + kBlockCols - 1) / kBlockCols);
-  if (!applies(a) || a->T < 40 || a->T * ctas * ctas < 470000) return 0;
+  if (!applies(a) || ctas < 64 || a->T < 40 || a->T * ctas * ctas < 540000) return 0;
   const size_t one = chunk_bytes(a), all = (size_t)((a->T + kChunk - 1) / kChunk);
   return one * all <= kMaxScratch ? one * all : one > kMaxScratch ? one : kMaxScratch / one * one;
 }

@@ -97,9 +97,9 @@ def test_where_chunks_are_taken(pkg, device):
         a.state_sb = H * D * V
         return lib.l3ci_recurrent_scan_scratch_bytes(C.byref(a))
 
-    assert need(1, 459, 16, 128, 128) == 29 * one(16, 128, True) and need(1, 458, 16, 128, 128) == 0
-    assert need(3, 52, 16, 128, 128) == 4 * one(48, 128, True) and need(16, 39, 16, 128, 128) == 0
-    assert need(3, 52, 32, 64, 64, kind=1) == 4 * one(96, 64, False)
+    assert need(2, 132, 16, 128, 128) == 9 * one(32, 128, True) and need(2, 131, 16, 128, 128) == 0 and need(1, 6000, 16, 128, 128) == 0
+    assert need(3, 59, 16, 128, 128) == 4 * one(48, 128, True) and need(16, 39, 16, 128, 128) == 0
+    assert need(3, 59, 32, 64, 64, kind=1) == 4 * one(96, 64, False)
     assert 0 < need(8, 6000, 16, 128, 128) <= 256 << 20                             # longer prompts: segments
     assert need(3, 1000, 16, 128, 128, dtype=1) == need(3, 1000, 16, 32, 128) == need(3, 1000, 16, 128, 124) == need(3, 1000, 16, 128, 128, shift=2) == 0
     a = A()
