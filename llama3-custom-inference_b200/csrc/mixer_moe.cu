@@ -53,7 +53,14 @@ moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ bia
       }
       const unsigned most = __reduce_max_sync(kFullMask, best);
       at = __reduce_min_sync(kFullMask, best == most ? at : E);
-      if (at >= E) at = j;                                        // nothing but NaN left: any place within bounds
+      if (at >= E) {                                              // nothing but NaN left: the smallest index that is not taken (a token has an expert once)
+        for (int e = lane; e < E && at >= E; e += 32) {
+          bool taken = false;
+          for (int i = 0; i < j; ++i) taken = taken || chosen[t * top + i] == e;
+          if (!taken) at = e;
+        }
+        at = __reduce_min_sync(kFullMask, at);
+      }
       const float v = z[at];
       if (j == 0) first = v;
       const float p = expf(v - first);

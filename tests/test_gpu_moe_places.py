@@ -39,6 +39,35 @@ def test_experts_of_few_tokens(pkg, device, rows, E, top, width, ff):
         assert rel.max().item() < 1e-2      # bf16 activations (2^-9 each) and rows of y (2^-9): 4e-3 at most of their norms' quotient
 
 
+@pytest.mark.parametrize("rows,E,top,bad", [(8, 4, 4, [2]), (32, 4, 4, [0, 1, 3]), (9, 40, 38, [0, 7, 33, 39]), (200, 4, 3, [1, 2])])
+def test_router_logits_without_numbers(pkg, device, rows, E, top, bad):
+    """A token whose logits run out of numbers has every expert once all the same: no expert more pairs than it has places, all places
+    within the products' rows, and the other tokens' results untouched."""
+    mx, width, ff = pkg.mixers, 64, 40
+    h, z = rand(rows, width, seed=1).to(device), rand(rows, E, seed=2, scale=5).float().to(device)
+    odd = torch.arange(rows, device=device) % 3 == 1
+    w, down = rand(E, 2 * ff, width, seed=3, scale=0.1).to(device), rand(E, width, ff, seed=4, scale=0.1).to(device)
+
+    def run(z):
+        experts, ranks, weights, counts = mx.moe_route(z, torch.zeros(E, device=device), top)
+        assert bool((experts.sort(dim=1).values.diff(dim=1) > 0).all()) and int(experts.min()) >= 0 and int(experts.max()) < E
+        assert int(counts.sum()) == rows * top and int(counts.max()) <= rows and int(ranks.max()) < rows and int(ranks.min()) >= 0
+        if rows > 32:
+            return experts, None
+        x, part_rows = mx.moe_places(h, experts, ranks, E)
+        assert part_rows.unique().numel() == rows * top and int(part_rows.max()) < rows * E
+        y = mx.few_rows(mx.few_rows(x, w, mx.ACT_SILU_GATE, always=True, limit=0.7, alpha=1.702), down, always=True)
+        stream = torch.zeros(rows, width, device=device)
+        mx.residual_norm(y, stream, dtype=torch.bfloat16, part_rows=part_rows, part_weights=weights)
+        return experts, stream
+
+    without = torch.where(odd[:, None], torch.full_like(z, float("nan")).index_fill(1, torch.tensor([e for e in range(E) if e not in bad], device=device), 1.0), z)
+    (experts, stream), (_, want) = run(without), run(z)
+    assert bool((experts[odd][:, :E - len(bad)] == torch.tensor([e for e in range(E) if e not in bad], device=device)[:top]).all())
+    if stream is not None:
+        assert torch.equal(stream[~odd], want[~odd]) and bool(stream[odd].isnan().all()) and bool(want.isfinite().all())
+
+
 def test_a_limit_belongs_to_a_gate(pkg, device):
     mx, x, w = pkg.mixers, rand(4, 64).to(device), rand(32, 64).to(device)
     for act, limit in ((mx.ACT_NONE, 1.0), (mx.ACT_GELU, 1.0), (mx.ACT_SILU_GATE, -1.0), (mx.ACT_SILU_GATE, float("nan"))):
