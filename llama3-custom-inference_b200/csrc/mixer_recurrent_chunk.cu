@@ -299,7 +299,6 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + kMaxStages * 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int vb = blockIdx.x % p.col_blocks, bh = blockIdx.x / p.col_blocks, h = bh % a.H, b = bh / a.H;
-  const bool fresh = a.positions[b] == 0 && p.t0 == 0;
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.ring; ++i) {
       mbar_init(full0 + i * 8, 1);
@@ -310,6 +309,7 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
   }
   __syncthreads();
   pdl_begin();
+  const bool fresh = a.positions[b] == 0 && p.t0 == 0;
   bool ok = true;
   int asked = 0;
   if (warp == kScanWarps) {
