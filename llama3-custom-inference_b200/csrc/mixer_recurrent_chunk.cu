@@ -6,20 +6,25 @@
 //                      S <- diag(G) S + sum_j (k_j G_{>j}) u_j^T,
 // with G_i the product of the decays up to token i, L_ij and M_ij the products of k_i, q_i with k_j decayed from j to i.  With T the inverse of
 // (1 + beta L) times beta, U = T (V - (k G) S), and all but the terms with S is known ahead, for all chunks at once.  Time mixing is the same with
-// U = V, decays up to i - 1 and the bonus on the diagonal of M.
+// U = V, decays up to i - 1 and the bonus on the diagonal of M.  (The chunked delta rule: Yang et al., "Parallelizing Linear Transformers with the
+// Delta Rule over Sequence Length".)
 //   chunk_inputs_kernel  a warp per head and chunk, lanes over channels: the decayed keys of the chunk's tokens stay in registers and are
 //     multiplied on from token to token, so that every decay is a product of factors at most 1 and none is divided by; L's and M's rows are the
 //     lanes' sums, T's columns a lane's each.
-//   chunk_scan_kernel    a warp per 16 columns of the state, whose transpose it keeps in accumulators of m16n8k8 products: per chunk U, the
-//     outputs and the new state are 312 of them (128 rows).  Operands are 32-bit, split into tf32 parts: two and three
-//     products for the sums over the state, three and six (all but what lies below 2^-33) for U and the new state.  An accumulator's columns are the next product's depth, taken in the order in which they lie.  Chunks come through a ring of bulk
-//     copies.
-// 1777 tokens of 3 x 16 heads of 128 x 128 (delta rule): 429 us, token by token 741; 3 x 32 heads of 64 x 64 (time mixing): 231, 374.  Most of it is the
-// scan, a warp per scheduler, of which the products alone are 3300 cycles a chunk.  With U and W instead of T in the chunks the rows of
-// the forward substitution took longer than the scan; with the values read by the scan's lanes themselves a chunk took 1.4 times as long.
-// Errors against 64 bits: outputs the same (their rounding to bf16); states after such prompts, of their norm, delta rule of four layers 1.43,
-// 1.29, 1.27, 1.76 e-7, token by token 1.52, 1.24, 1.24, 2.34, time mixing 1.76 to 1.97 e-7 and 1.86 to 2.02.  By three products throughout (346
-// us) it was 1.6 to 2.1 e-7: the bit that two parts leave out, and the product of the small parts.
+//   chunk_scan_kernel    a warp per 8 columns of the state, in its registers: sixteen lanes share four columns, four neighbouring rows of every
+//     64 a lane.  Per chunk the sums W S and Q S, four tokens at a time over the sixteen lanes; U and the outputs, a token's column by one lane;
+//     the new state.  Chunks come through a ring of bulk copies.
+// All in 32-bit multiply-adds, a sum over the tokens up to its own only.  Products on the tensor cores, of operands in two or three tf32
+// parts, were as fast for the delta rule and a quarter faster for time mixing, but their accumulators are cut off, not rounded: states that
+// decay within a few tokens were twice as far from 64 bits as token by token.  And 0 times a later token's NaN is NaN.
+// States against 64 bits, of their norm, in 1e-8 (40 to 4000 tokens, 64 and 128 channels; in brackets token by token): delta rule without
+// decay 14 to 36 (14 to 35), decays of about e^-0.0008 a token 17 to 39 (19 to 43), e^-0.08 9.6 to 10.2 (9.5 to 10.0), e^-0.8 4.8 to
+// 5.4 (4.9 to 5.6), e^-8 3.4 to 4.5 (4.2 to 4.5); time mixing, decays of about e^-e^-5 a token 18 to 41 (18 to 41), e^-e^-3 12.4 to 13.3
+// (12.1 to 12.9), e^-e^-1 5.6 to 6.2 (5.5 to 6.1), e^-e 3.0 to 3.2 (3.0 to 3.2).  Outputs: the same, but for their rounding to bf16.
+// us, by chunks and token by token: delta rule, 1777 tokens of 3 x 16 heads of 128 x 128 445 and 740; time mixing, 3 x 32 heads of 64 x 64
+// 298 and 370.  Bound by shared memory: of the scan's 6.8 thousand cycles a chunk (128 x 128) the rows of W, Q and K, which every warp reads,
+// and the shuffles take 4 to 5.  Eight columns a lane instead of four and four warps instead of eight (half of those rows): 577 and 484 us, one
+// warp a scheduler waits out its own instructions.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -33,48 +38,32 @@ namespace {
 
 constexpr int kChunk = 16;
 constexpr int kDelta = 0, kTimeMix = 1;
-constexpr int kScanWarps = 4;
-constexpr int kBlockCols = 16 * kScanWarps;       // state columns of a CTA
-constexpr int kVPitch = kBlockCols * 2 + 16;      // bytes of a token's values in a stage
-constexpr int kMPitch = 20;                       // floats; pitches: neighbouring rows on other banks
+constexpr int kOwn = 4;                           // a lane's columns
+constexpr int kCols = 2 * kOwn;                   // a warp's: sixteen lanes share kOwn of them
+constexpr int kTogether = 16 / kOwn;              // tokens whose sums over the state are taken together: one for each of the lanes
+constexpr int kPatch = kChunk + 4;                // floats of a column's tokens in a patch: neighbours on other banks
+constexpr int kMaxWarps = 8;
+constexpr int kMaxCols = kMaxWarps * kCols;       // of a CTA
+constexpr int kVPitch = kMaxCols * 2 + 16;        // bytes of a token's values in a stage
+constexpr int kStages = 4;
 
-// A chunk's block of D channels, in floats: W = k G (delta rule) and Q = q G, K decayed to the chunk's end, M, T (delta rule), the chunk's decays.  W,
-// Q and K lie as the scan's lanes take them, 16 bytes each, split into their tf32 parts: of a token, hi and lo of two channels; of K, of a channel,
-// hi and lo of two tokens.
+// A chunk's block of D channels, in floats: W = k G (delta rule) and Q = q G, K decayed to the chunk's end, 16 tokens each, M, T (delta
+// rule), the chunk's decays.
 template <int KIND, int D>
 struct ChunkShape {
-  static constexpr int kWPitch = 2 * D + 16, kKPitch = 4 * D + 8;    // of a token, of two tokens
-  static constexpr int kW = KIND == kDelta ? kChunk * kWPitch : 0;
-  static constexpr int kQ = kChunk * kWPitch, kK = kChunk / 2 * kKPitch, kM = kChunk * kMPitch;
-  static constexpr int kAtQ = kW, kAtK = kAtQ + kQ, kAtM = kAtK + kK, kAtT = kAtM + kM, kAtG = kAtT + (KIND == kDelta ? kM : 0);
+  static constexpr int kRows = kChunk * D, kSquare = kChunk * kChunk;
+  static constexpr int kAtQ = KIND == kDelta ? kRows : 0, kAtK = kAtQ + kRows, kAtM = kAtK + kRows, kAtT = kAtM + kSquare,
+                       kAtG = kAtT + (KIND == kDelta ? kSquare : 0);
   static constexpr int kFloats = kAtG + D;
   static constexpr int kStage = kFloats * 4 + kChunk * kVPitch;      // bytes in the scan: the block and the values
   static_assert(kFloats % 4 == 0, "bulk copies of whole 16-byte vectors");
 };
 
-// A 32-bit number as two of the 11 bits that a tf32 product takes.  (Integer instructions: the conversion's own runs at an eighth of their rate.)
-struct Split { uint32_t hi, lo; };
-__device__ __forceinline__ Split split(float x) {
-  Split s;
-  s.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  s.lo = __float_as_uint(x - __uint_as_float(s.hi)) + 0x1000u;
-  return s;
-}
-
-// The same without loss: lo as it is, of which a product takes the first 11 bits; the rest of it is a third part.
-__device__ __forceinline__ Split split_whole(float x) {
-  Split s;
-  s.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  s.lo = __float_as_uint(x - __uint_as_float(s.hi));
-  return s;
-}
-__device__ __forceinline__ uint32_t rest(uint32_t lo) { return __float_as_uint(__uint_as_float(lo) - __uint_as_float(lo & 0xffffe000u)); }
-
 struct ChunkParams {
   l3ci_recurrent_scan_args a;
   float* blocks;                 // [B * H][chunks]
   int t0, tokens, chunks;        // of this segment
-  int col_blocks, last, ring;
+  int col_blocks, warps, last;
 };
 
 // ---- the chunks' inputs -----------------------------------------------------------------------------------------------------------
@@ -104,21 +93,15 @@ chunk_inputs_kernel(const __grid_constant__ ChunkParams p, long long units) {
     f2_unpack(s, u, v);
     return u + v;
   };
-  f2 t[kChunk][P2], run[P2], gb[P2], bonus[P2];   // decayed keys; product of the decays so far
-  // a pair of channels of a token, of W or Q
-  auto put = [&](float* row, int j, f2 v) {
-    float x, y;
-    f2_unpack(v, x, y);
-    const Split sx = split(x), sy = split(y);
-    *reinterpret_cast<uint4*>(row + 2 * (d0 + 2 * j)) = make_uint4(sx.hi, sy.hi, sx.lo, sy.lo);
-  };
+  f2 t[kChunk][P2], run[P2], rest[P2], gb[P2], bonus[P2];   // decayed keys; product of the decays so far, what its roundings left
+  auto put = [&](float* row, int j, f2 v) { *reinterpret_cast<f2*>(row + d0 + 2 * j) = v; };
   float t_col[kChunk];                            // column lane % 16 of T
 #pragma unroll
   for (int j = 0; j < kChunk; ++j) t_col[j] = 0.f;
 #pragma unroll
   for (int j = 0; j < P2; ++j) {
     run[j] = pair_of(1.f, 1.f);
-    gb[j] = bonus[j] = 0ull;
+    rest[j] = gb[j] = bonus[j] = 0ull;
     if (KIND == kTimeMix) {
       gb[j] = pair_of(a.g_bias[h * D + d0 + 2 * j], a.g_bias[h * D + d0 + 2 * j + 1]);
       bonus[j] = pair_of(a.bonus[h * D + d0 + 2 * j], a.bonus[h * D + d0 + 2 * j + 1]);
@@ -166,12 +149,15 @@ chunk_inputs_kernel(const __grid_constant__ ChunkParams p, long long units) {
         qg[j] = f2_mul(q[j], run[j]);
         kg[j] = f2_mul(k[j], run[j]);
       } else {
-        qg[j] = f2_mul(q[j], run[j]);
+        // (without the rest states of slow decays were 1.06 times as far from 64 bits as token by token; of the delta rule they are nearer anyway)
+        qg[j] = f2_mul(q[j], f2_add(run[j], rest[j]));
         kg[j] = f2_mul(bonus[j], k[j]);
-        run[j] = f2_mul(run[j], g[j]);
+        const f2 product = f2_mul(run[j], g[j]);
+        rest[j] = f2_fma(rest[j], g[j], f2_fma(run[j], g[j], product ^ 0x8000000080000000ull));
+        run[j] = product;
       }
-      put(block + Sh::kAtQ + i * Sh::kWPitch, j, qg[j]);
-      if (KIND == kDelta) put(block + i * Sh::kWPitch, j, kg[j]);
+      put(block + Sh::kAtQ + i * D, j, qg[j]);
+      if (KIND == kDelta) put(block + i * D, j, kg[j]);
     }
     float sums[32];
 #pragma unroll
@@ -208,7 +194,7 @@ chunk_inputs_kernel(const __grid_constant__ ChunkParams p, long long units) {
         sums[x] = mine + __shfl_xor_sync(kFullMask, send, m);
       }
     }
-    if (lane >= kChunk) block[Sh::kAtM + i * kMPitch + lane - kChunk] = lane - kChunk <= i ? sums[0] : 0.f;
+    if (lane >= kChunk) block[Sh::kAtM + i * kChunk + lane - kChunk] = sums[0];   // (those of later tokens are not read)
     if (KIND == kDelta) {
       const float row_l = lane < i ? -sums[0] : 0.f;
       float col = lane % kChunk == i ? 1.f : 0.f;
@@ -221,88 +207,39 @@ chunk_inputs_kernel(const __grid_constant__ ChunkParams p, long long units) {
       col *= beta;
 #pragma unroll
       for (int j = 0; j < kChunk; ++j) t_col[j] = j == i ? col : t_col[j];
-      if (lane < kChunk) block[Sh::kAtT + i * kMPitch + lane] = col;
+      if (lane < kChunk) block[Sh::kAtT + i * kChunk + lane] = col;
     }
   }
 #pragma unroll
-  for (int i = 0; i < kChunk; i += 2)
+  for (int i = 0; i < kChunk; ++i)
 #pragma unroll
-    for (int j = 0; j < P2; ++j) {
-      float x[2], y[2];
-      f2_unpack(t[i][j], x[0], x[1]);
-      f2_unpack(t[i + 1][j], y[0], y[1]);
+    for (int j = 0; j < P2; ++j) put(block + Sh::kAtK + i * D, j, t[i][j]);
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const Split sx = split_whole(x[e]), sy = split_whole(y[e]);
-        *reinterpret_cast<uint4*>(block + Sh::kAtK + i / 2 * Sh::kKPitch + 4 * (d0 + 2 * j + e)) = make_uint4(sx.hi, sy.hi, sx.lo, sy.lo);
-      }
-    }
-#pragma unroll
-  for (int j = 0; j < P2; ++j) *reinterpret_cast<f2*>(block + Sh::kAtG + d0 + 2 * j) = run[j];
+  for (int j = 0; j < P2; ++j) put(block + Sh::kAtG, j, f2_add(run[j], rest[j]));
 }
 
 // ---- the scan ----------------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// An accumulator as the left operand of the next product, in two parts: its columns 2 t and 2 t + 1 are the depths t and t + 4.
-struct Left { uint32_t hi[4], lo[4]; };
-template <bool WHOLE = false>
-__device__ __forceinline__ Left left(const float (&c)[4]) {
-  Left l;
-  const int from[4] = {0, 2, 1, 3};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const Split s = WHOLE ? split_whole(c[from[i]]) : split(c[from[i]]);
-    l.hi[i] = s.hi;
-    l.lo[i] = s.lo;
-  }
-  return l;
-}
-struct Right { Split x, y; };
-// c (large products: their accumulator is cut off, not rounded) and d (small ones) += l r of split_whole's parts, all but what lies below 2^-33; EXACT: l has no small parts
-template <bool EXACT>
-__device__ __forceinline__ void mma_whole(float (&c)[4], float (&d)[4], const Left& l, const Right& r) {
-  const uint32_t rx = rest(r.x.lo), ry = rest(r.y.lo);
-  mma_tf32(d, l.hi, rx, ry);
-  mma_tf32(d, l.hi, r.x.lo, r.y.lo);
-  if (!EXACT) {
-    uint32_t lr[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) lr[i] = rest(l.lo[i]);
-    mma_tf32(d, lr, r.x.hi, r.y.hi);
-    mma_tf32(d, l.lo, r.x.lo, r.y.lo);
-    mma_tf32(d, l.lo, r.x.hi, r.y.hi);
-  }
-  mma_tf32(c, l.hi, r.x.hi, r.y.hi);
-}
-
-__device__ __forceinline__ Right right(const float* p) {
-  const uint4 v = *reinterpret_cast<const uint4*>(p);
-  return {{v.x, v.z}, {v.y, v.w}};
-}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
-constexpr int kMaxStages = 4;
-
 template <int KIND, int D>
-__global__ void __launch_bounds__(32 * (kScanWarps + 1), 1)
+__global__ void __launch_bounds__(32 * (kMaxWarps + 1), 1)
 chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
   using Sh = ChunkShape<KIND, D>;
-  constexpr int NT = D / 8;                       // accumulators of 8 state rows
+  typedef unsigned long long f2;
+  constexpr int kRuns = D / 64;                   // a lane's rows: 4 neighbours of every 64
   extern __shared__ __align__(128) uint8_t ring_smem[];
-  __shared__ __align__(8) uint64_t bars[2 * kMaxStages];
+  __shared__ __align__(16) float patches[kMaxWarps][2][kCols * kPatch];      // of a warp, by column: V - W S, U
+  __shared__ __align__(8) uint64_t bars[2 * kStages];
   const l3ci_recurrent_scan_args& a = p.a;
-  const uint32_t full0 = smem_u32(bars), empty0 = full0 + kMaxStages * 8;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const uint32_t full0 = smem_u32(bars), empty0 = full0 + kStages * 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int vb = blockIdx.x % p.col_blocks, bh = blockIdx.x / p.col_blocks, h = bh % a.H, b = bh / a.H;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < p.ring; ++i) {
+    for (int i = 0; i < kStages; ++i) {
       mbar_init(full0 + i * 8, 1);
-      mbar_init(empty0 + i * 8, kScanWarps);
+      mbar_init(empty0 + i * 8, p.warps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -312,11 +249,12 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
   const bool fresh = a.positions[b] == 0 && p.t0 == 0;
   bool ok = true;
   int asked = 0;
-  if (warp == kScanWarps) {
+  const int col0 = vb * p.warps * kCols;
+  if (warp == p.warps) {
     // ---- producer: a chunk's block, and a token's values by each of 16 lanes ----
     const float* block = p.blocks + (long long)bh * p.chunks * Sh::kFloats;
-    const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(a.v) + ((long long)b * a.T + p.t0) * a.v_st + h * a.v_sh + vb * kBlockCols;
-    const uint32_t v_bytes = min(kBlockCols, a.V - vb * kBlockCols) * 2;
+    const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(a.v) + ((long long)b * a.T + p.t0) * a.v_st + h * a.v_sh + col0;
+    const uint32_t v_bytes = min(p.warps * kCols, a.V - col0) * 2;
     for (int i = 0, s = 0, parity = 1; i < p.chunks; ++i) {
       if (!mbar_wait_bounded(empty0 + s * 8, parity)) { ok = false; break; }
       const uint32_t dst = smem_u32(ring_smem + s * Sh::kStage), bar = full0 + s * 8;
@@ -328,147 +266,209 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
       __syncwarp();
       if (lane < kChunk)    // (a token behind the last one has no share in anything: the last one's values again)
         bulk_load(dst + Sh::kFloats * 4 + lane * kVPitch, v + (long long)min(i * kChunk + lane, p.tokens - 1) * a.v_st, v_bytes, bar);
-      if (++s == p.ring) { s = 0; parity ^= 1; }
+      if (++s == kStages) { s = 0; parity ^= 1; }
     }
     __syncwarp();
     if (a.tail && p.last && vb == 0) move_tails<__nv_bfloat16>(a, b, h, lane, 32, a.positions[b] == 0);
   } else {
-    const int c0 = vb * kBlockCols + warp * 16;
+    // Sixteen lanes share kOwn columns of all rows.  A lane's column c is column c ^ me of them, and token x of those taken together token
+    // x ^ mine, so that the lanes' sums are added up without choosing what to send: a lane ends with column `me` of token `mine`.
+    const int r = lane & 15, group = lane >> 4, me = r % kOwn, mine = r / kOwn, col = group * kOwn + me;
+    const int c0 = col0 + warp * kCols + group * kOwn;
+    const bool real = c0 < a.V;                   // (of a group all columns are, or none)
     float* state = a.state + b * a.state_sb + (long long)h * D * a.V + c0;
-    float S[NT][4];
+    auto row_of = [&](int j) { return j / 2 * 64 + 4 * r + j % 2 * 2; };                        // first row of pair j
+    f2 S[kOwn][2 * kRuns];
 #pragma unroll
-    for (int x = 0; x < NT; ++x)
+    for (int c = 0; c < kOwn; ++c)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int d = 8 * x + 2 * t4 + (e & 1), col = g + (e >> 1) * 8;
-        S[x][e] = !fresh && c0 + col < a.V ? state[(long long)d * a.V + col] : 0.f;
+      for (int j = 0; j < 2 * kRuns; ++j) {
+        const float* at = state + (long long)row_of(j) * a.V + (c ^ me);
+        S[c][j] = !fresh && real ? f2_packf(at[0], at[a.V]) : 0ull;
       }
-    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + ((long long)b * a.T + p.t0) * a.out_st + h * a.out_sh + c0;
+    float *seen = patches[warp][0], *u = patches[warp][1];
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + ((long long)b * a.T + p.t0) * a.out_st + h * a.out_sh + c0 + me;
+    auto load4 = [](const float* x, f2 (&y)[2]) {
+      const ulonglong2 z = *reinterpret_cast<const ulonglong2*>(x);
+      y[0] = z.x;
+      y[1] = z.y;
+    };
     for (int i = 0, s = 0, parity = 0; i < p.chunks; ++i) {
       if (!mbar_wait_bounded(full0 + s * 8, parity)) { ok = false; break; }
       const float* st = reinterpret_cast<const float*>(ring_smem + s * Sh::kStage);
-      const uint8_t* vs = ring_smem + s * Sh::kStage + Sh::kFloats * 4 + (warp * 16 + g) * 2;
-      // (W S)^T and (Q S)^T, by token tiles of 8; the large products in two runs, the small ones in a third: an accumulator is cut off, not
-      // rounded, at every step
-      float ws[3][2][4] = {}, os[3][2][4] = {};
+      const uint8_t* values = ring_smem + s * Sh::kStage + Sh::kFloats * 4 + (warp * kCols + col) * 2;
+      const int n = min(kChunk, p.tokens - i * kChunk);
+      float v[kChunk / kTogether];
 #pragma unroll
-      for (int x = 0; x < NT; ++x) {
-        const Left l = left<>(S[x]);
-        Right w[2], q[2];
+      for (int i2 = 0; i2 < kChunk / kTogether; ++i2)
+        v[i2] = real ? to_f32(*reinterpret_cast<const __nv_bfloat16*>(values + (i2 * kTogether + mine) * kVPitch)) : 0.f;
+      auto put = [&](float* of, int i2, float y) { of[col * kPatch + i2 * kTogether + mine] = y; };
+      if (KIND == kTimeMix) {                     // (U = V)
 #pragma unroll
-        for (int tt = 0; tt < 2; ++tt) {
-          const int at = (8 * tt + g) * Sh::kWPitch + 16 * x + 4 * t4;
-          q[tt] = right(st + Sh::kAtQ + at);
-          if (KIND == kDelta) w[tt] = right(st + at);
-        }
-#pragma unroll
-        for (int part = 0; part < 3; ++part)
-#pragma unroll
-          for (int tt = 0; tt < 2; ++tt) {
-            const int run = part == 0 ? x % 2 : 2;
-            if (KIND == kDelta) mma_tf32(ws[run][tt], part == 2 ? l.lo : l.hi, part == 1 ? w[tt].x.lo : w[tt].x.hi, part == 1 ? w[tt].y.lo : w[tt].y.hi);
-            mma_tf32(os[run][tt], part == 2 ? l.lo : l.hi, part == 1 ? q[tt].x.lo : q[tt].x.hi, part == 1 ? q[tt].y.lo : q[tt].y.hi);
-          }
+        for (int i2 = 0; i2 < kChunk / kTogether; ++i2) put(u, i2, v[i2]);
+        __syncwarp();
       }
-      // U^T, and the outputs with it: sums over the chunk's tokens j, rows i of T and of M
-      Left u[2];
-      auto by_rows = [&](const float* rows, const Left (&l)[2], float (&c)[3][2][4], bool exact, bool whole) {   // exact: l has no small part
+      // ---- sums over the state: W S of the delta rule, Q S ----
+      constexpr int kSums = KIND == kDelta ? 2 : 1;
+      float sums[kChunk / kTogether][kSums];
 #pragma unroll
-        for (int tt = 0; tt < 2; ++tt) {
-          Right m[2];
+      for (int i2 = 0; i2 < kChunk / kTogether; ++i2)
 #pragma unroll
-          for (int ti = 0; ti < 2; ++ti) {
-            const float2 f = *reinterpret_cast<const float2*>(rows + (8 * ti + g) * kMPitch + 8 * tt + 2 * t4);
-            m[ti] = whole ? Right{split_whole(f.x), split_whole(f.y)} : Right{split(f.x), split(f.y)};
-          }
-          if (whole) {
+        for (int k = 0; k < kSums; ++k) {
+          f2 part[kTogether][kOwn];
 #pragma unroll
-            for (int ti = 0; ti < 2; ++ti) mma_whole<false>(c[tt][ti], c[2][ti], l[tt], m[ti]);
-            continue;
-          }
+          for (int x = 0; x < kTogether; ++x)
 #pragma unroll
-          for (int part = 0; part < (exact ? 2 : 3); ++part)
+            for (int j = 0; j < kRuns; ++j) {
+              f2 y[2];
+              load4(st + (k == kSums - 1 ? Sh::kAtQ : 0) + (i2 * kTogether + (x ^ mine)) * D + j * 64 + 4 * r, y);
 #pragma unroll
-            for (int ti = 0; ti < 2; ++ti)
-              mma_tf32(c[part == 0 ? tt : 2][ti], part == 2 ? l[tt].lo : l[tt].hi, part == 1 ? m[ti].x.lo : m[ti].x.hi, part == 1 ? m[ti].y.lo : m[ti].y.hi);
+              for (int c = 0; c < kOwn; ++c) {
+                part[x][c] = j == 0 ? f2_mul(y[0], S[c][0]) : f2_fma(y[0], S[c][2 * j], part[x][c]);
+                part[x][c] = f2_fma(y[1], S[c][2 * j + 1], part[x][c]);
+              }
+            }
+          float sum[kTogether][kOwn];
+#pragma unroll
+          for (int x = 0; x < kTogether; ++x)
+#pragma unroll
+            for (int c = 0; c < kOwn; ++c) {
+              float y, z;
+              f2_unpack(part[x][c], y, z);
+              sum[x][c] = y + z;
+            }
+#pragma unroll
+          for (int m = kTogether / 2; m >= 1; m /= 2)
+#pragma unroll
+            for (int x = 0; x < m; ++x)
+#pragma unroll
+              for (int c = 0; c < kOwn; ++c) sum[x][c] += __shfl_xor_sync(kFullMask, sum[x + m][c], m * kOwn);
+#pragma unroll
+          for (int m = kOwn / 2; m >= 1; m /= 2)
+#pragma unroll
+            for (int c = 0; c < m; ++c) sum[0][c] += __shfl_xor_sync(kFullMask, sum[0][c + m], m);
+          sums[i2][k] = sum[0][0];
+        }
+      // ---- U, and the outputs with it: this lane's column and tokens, sums over the tokens up to them only ----
+      float x[kChunk];
+      auto column = [&](const float* of) {
+#pragma unroll
+        for (int j = 0; j < kChunk; j += 4) {
+          const float4 f = *reinterpret_cast<const float4*>(of + col * kPatch + j);
+          x[j] = f.x; x[j + 1] = f.y; x[j + 2] = f.z; x[j + 3] = f.w;
         }
       };
+      auto over_tokens = [&](const float* square, int i2, float sum) {            // of token i2 * kTogether + mine
+        const float* row = square + (i2 * kTogether + mine) * kChunk;
 #pragma unroll
-      for (int tt = 0; tt < 2; ++tt) {
-        float v[4];
+        for (int j = 0; j < (i2 + 1) * kTogether; j += 4) {
+          const float4 f = *reinterpret_cast<const float4*>(row + j);
+          const float y[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          v[e] = to_f32(*reinterpret_cast<const __nv_bfloat16*>(vs + (8 * tt + 2 * t4 + (e & 1)) * kVPitch + (e >> 1) * 16));
-          if (KIND == kDelta) v[e] -= ws[0][tt][e] + ws[1][tt][e] + ws[2][tt][e];
+          for (int e = 0; e < 4; ++e)
+            if (j + e - i2 * kTogether <= mine) sum = fmaf(y[e], x[j + e], sum);
         }
-        u[tt] = left<true>(v);
-      }
+        return sum;
+      };
       if (KIND == kDelta) {
-        float us[3][2][4] = {};
-        by_rows(st + Sh::kAtT, u, us, false, true);
 #pragma unroll
-        for (int tt = 0; tt < 2; ++tt) {
+        for (int i2 = 0; i2 < kChunk / kTogether; ++i2) put(seen, i2, v[i2] - sums[i2][0]);
+        __syncwarp();
+        column(seen);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) us[0][tt][e] += us[1][tt][e] + us[2][tt][e];
-          u[tt] = left<true>(us[0][tt]);
+        for (int i2 = 0; i2 < kChunk / kTogether; ++i2) put(u, i2, over_tokens(st + Sh::kAtT, i2, 0.f));
+        __syncwarp();
+      }
+      column(u);
+#pragma unroll
+      for (int i2 = 0; i2 < kChunk / kTogether; ++i2) {
+        const int t = i2 * kTogether + mine;
+        const float o = over_tokens(st + Sh::kAtM, i2, sums[i2][kSums - 1]);
+        if (t < n && real) out[(long long)(i * kChunk + t) * a.out_st] = __float2bfloat16_rn(o);
+      }
+      // ---- the state: decayed, and the chunk's keys times U ----
+#pragma unroll
+      for (int j = 0; j < kRuns; ++j) {
+        f2 g[2];
+        load4(st + Sh::kAtG + j * 64 + 4 * r, g);
+#pragma unroll
+        for (int c = 0; c < kOwn; ++c) {
+          S[c][2 * j] = f2_mul(S[c][2 * j], g[0]);
+          S[c][2 * j + 1] = f2_mul(S[c][2 * j + 1], g[1]);
         }
       }
-      by_rows(st + Sh::kAtM, u, os, KIND == kTimeMix, false);      // (time mixing's U are bf16)
-      const int n = min(kChunk, p.tokens - i * kChunk);
+      auto add = [&](int t, const float (&y)[kOwn]) {
+        f2 k[kRuns][2];
 #pragma unroll
-      for (int ti = 0; ti < 2; ++ti)
+        for (int j = 0; j < kRuns; ++j) load4(st + Sh::kAtK + t * D + j * 64 + 4 * r, k[j]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int tok = 8 * ti + 2 * t4 + (e & 1), col = g + (e >> 1) * 8;
-          if (tok < n && c0 + col < a.V) out[(long long)(i * kChunk + tok) * a.out_st + col] = __float2bfloat16_rn(os[0][ti][e] + os[1][ti][e] + os[2][ti][e]);
+        for (int c = 0; c < kOwn; ++c) {
+          const f2 y2 = f2_packf(y[c], y[c]);
+#pragma unroll
+          for (int j = 0; j < 2 * kRuns; ++j) S[c][j] = f2_fma(k[j / 2][j % 2], y2, S[c][j]);
         }
-      // the state: decayed, and the chunk's keys times U
-      constexpr int kTogether = 4;
+      };
+      const float* own_u = u + group * kOwn * kPatch;
+      if (n == kChunk) {
 #pragma unroll
-      for (int x0 = 0; x0 < NT; x0 += kTogether) {
-        Right k[kTogether][2];
-        float add[kTogether][4] = {}, small[kTogether][4] = {}, odd[kTogether][4] = {};
+        for (int t = 0; t < kChunk; t += 4) {
+          float y[4][kOwn];
 #pragma unroll
-        for (int x = 0; x < kTogether; ++x)
+          for (int c = 0; c < kOwn; ++c) {
+            const float4 f = *reinterpret_cast<const float4*>(own_u + (c ^ me) * kPatch + t);
+            y[0][c] = f.x; y[1][c] = f.y; y[2][c] = f.z; y[3][c] = f.w;
+          }
 #pragma unroll
-          for (int tt = 0; tt < 2; ++tt) k[x][tt] = right(st + Sh::kAtK + (4 * tt + t4) * Sh::kKPitch + 4 * (8 * (x0 + x) + g));
+          for (int e = 0; e < 4; ++e) add(t + e, y[e]);
+        }
+      } else {                                    // (what stands behind the last token may be no number)
+#pragma unroll 1
+        for (int t = 0; t < n; ++t) {
+          float y[kOwn];
 #pragma unroll
-        for (int tt = 0; tt < 2; ++tt)
-#pragma unroll
-          for (int x = 0; x < kTogether; ++x) mma_whole<KIND == kTimeMix>(tt > 0 ? odd[x] : add[x], small[x], u[tt], k[x][tt]);
-#pragma unroll
-        for (int x = 0; x < kTogether; ++x) {
-          const float2 f = *reinterpret_cast<const float2*>(st + Sh::kAtG + 8 * (x0 + x) + 2 * t4);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) S[x0 + x][e] = fmaf(S[x0 + x][e], e & 1 ? f.y : f.x, add[x][e] + (odd[x][e] + small[x][e]));
+          for (int c = 0; c < kOwn; ++c) y[c] = own_u[(c ^ me) * kPatch + t];
+          add(t, y);
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(empty0 + s * 8);
-      if (++s == p.ring) { s = 0; parity ^= 1; }
+      if (++s == kStages) { s = 0; parity ^= 1; }
     }
-    if (ok)
+    if (ok && real)
 #pragma unroll
-      for (int x = 0; x < NT; ++x)
+      for (int c = 0; c < kOwn; ++c)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int d = 8 * x + 2 * t4 + (e & 1), col = g + (e >> 1) * 8;
-          if (c0 + col < a.V) state[(long long)d * a.V + col] = S[x][e];
+        for (int j = 0; j < 2 * kRuns; ++j) {
+          float* at = state + (long long)row_of(j) * a.V + (c ^ me);
+          f2_unpack(S[c][j], at[0], at[a.V]);
         }
   }
   if (!ok && lane == 0 && a.status) atomicExch(a.status, (int)L3CI_ERR_DEVICE_WAIT);
   // a wait ran out: the copies still under way land before the shared memory is given back
   if (__syncthreads_or(!ok))
-    for (int f = asked > p.ring ? asked - p.ring : 0; f < asked; ++f) (void)mbar_wait_bounded_one(full0 + f % p.ring * 8, (uint32_t)(f / p.ring) & 1u);
+    for (int f = asked > kStages ? asked - kStages : 0; f < asked; ++f) (void)mbar_wait_bounded_one(full0 + f % kStages * 8, (uint32_t)(f / kStages) & 1u);
 }
 
-// Scratch of the chunks of `tokens` tokens of all heads.
+// Scratch of a chunk of all heads.
 size_t chunk_bytes(const l3ci_recurrent_scan_args* a) {
   const size_t floats = a->kind == kDelta ? (a->D == 64 ? ChunkShape<kDelta, 64>::kFloats : ChunkShape<kDelta, 128>::kFloats)
                                           : (a->D == 64 ? ChunkShape<kTimeMix, 64>::kFloats : ChunkShape<kTimeMix, 128>::kFloats);
   return (size_t)a->B * a->H * floats * 4;
 }
 constexpr size_t kMaxScratch = 256ull << 20;      // longer prompts go in segments
+
+// Warps of a CTA of the scan, eight columns each: the fewest columns for the busiest SM (96 heads' blocks of 64 columns leave a third of the SMs
+// idle; 48 heads of 128 x 128, 132 tokens of 32 heads: 6 and 4 warps 431 and 36.2 us, 8 warps 440 and 52.3).
+int scan_warps(const l3ci_recurrent_scan_args* a) {
+  const long long sms = sm_count() > 0 ? sm_count() : 148, heads = (long long)a->B * a->H;
+  long long least = -1;
+  int best = kMaxWarps;
+  for (int w = kMaxWarps; w >= kMaxWarps / 2; --w) {
+    const long long ctas = heads * ((a->V + w * kCols - 1) / (w * kCols)), load = (ctas + sms - 1) / sms * w;
+    if (least < 0 || load < least) { least = load; best = w; }
+  }
+  return best;
+}
 
 template <typename Q, int KIND, int D>
 int launch(const l3ci_recurrent_scan_args* a, void* scratch, size_t bytes) {
@@ -478,6 +478,7 @@ int launch(const l3ci_recurrent_scan_args* a, void* scratch, size_t bytes) {
   const int most = (int)(bytes / one < (size_t)all ? bytes / one : (size_t)all);
   if (!scratch || most < 1 || !aligned16(scratch)) return fail(L3CI_ERR_SCRATCH, "recurrent_scan: %zu bytes of scratch needed at least, %zu given", one, bytes);
   const int segments = (all + most - 1) / most, per = (all + segments - 1) / segments;
+  const int warps = scan_warps(a);
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(a->stream);
   auto inputs = chunk_inputs_kernel<Q, KIND, D>;
   auto scan = chunk_scan_kernel<KIND, D>;
@@ -485,23 +486,22 @@ int launch(const l3ci_recurrent_scan_args* a, void* scratch, size_t bytes) {
   int dev = 0;
   L3CI_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    L3CI_CUDA_TRY(cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 1024));
+    L3CI_CUDA_TRY(cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * Sh::kStage));
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   for (int c = 0; c < all; c += per) {
     ChunkParams p = {};
     p.a = *a;
-    p.col_blocks = (a->V + kBlockCols - 1) / kBlockCols;
+    p.warps = warps;
+    p.col_blocks = (a->V + warps * kCols - 1) / (warps * kCols);
     p.t0 = c * kChunk;
     p.chunks = per < all - c ? per : all - c;
     p.tokens = a->T - p.t0 < p.chunks * kChunk ? a->T - p.t0 : p.chunks * kChunk;
     p.last = c + per >= all;
     const long long heads = (long long)a->B * a->H, units = heads * p.chunks;
     p.blocks = static_cast<float*>(scratch);
-    const int stage = Sh::kStage, room = max_smem_optin() - 1024;
-    p.ring = room / stage < kMaxStages ? room / stage : kMaxStages;
     L3CI_LAUNCH("chunk_inputs_kernel", inputs, dim3((unsigned)((units + kInputWarps - 1) / kInputWarps)), dim3(32 * kInputWarps), 0, stream, p, units);
-    L3CI_LAUNCH("chunk_scan_kernel", scan, dim3((unsigned)(heads * p.col_blocks)), dim3(32 * (kScanWarps + 1)), (size_t)p.ring * stage, stream, p);
+    L3CI_LAUNCH("chunk_scan_kernel", scan, dim3((unsigned)(heads * p.col_blocks)), dim3(32 * (p.warps + 1)), (size_t)kStages * Sh::kStage, stream, p);
   }
   return L3CI_OK;
 }
@@ -516,11 +516,21 @@ bool applies(const l3ci_recurrent_scan_args* a) {
 }  // namespace
 
 size_t scan_chunks_scratch(const l3ci_recurrent_scan_args* a) {
-  // From where the chunks are the faster, in CTAs of the scan and tokens (us by tokens and by chunks): 32 CTAs of the delta rule 384 tokens 79.5 and
-  // 87.0, of time mixing 40.2 and 44.3, and a token more costs both the same; 64 CTAs 96 tokens 38.9 and 37.9, time mixing 128 25.5 and 25.6; 96
-  // CTAs 48 tokens 30.7 and 30.0, 64 24.1 and 22.2; 256 CTAs 48 tokens 54.8 and 43.6, 33.9 and 28.1.
-  const long long ctas = (long long)a->B * a->H * ((a->V + kBlockCols - 1) / kBlockCols);
-  if (!applies(a) || ctas < 64 || a->T < 40 || a->T * ctas * ctas < 540000) return 0;
+  // From where on the chunks are the faster, in CTAs of 64 columns and tokens; us by tokens and by chunks, heads of 128 x 128 and of 64 x 64.
+  //   delta rule   32 CTAs, 1000 tokens 187 and 171, 138 and 178;   64 CTAs, 132 tokens 46.3 and 37.4, 43.2 and 40.1;
+  //                96, 56 tokens 30.3 and 30.2;   128, 56 tokens 30.8 and 32.4, 64 tokens 33.9 and 32.4;   320, 56 tokens 72.5 and 79.5
+  //                64 x 64: 128 CTAs, 112 tokens 39.8 and 41.6, 128 tokens 44.7 and 43.9;   96, 128 tokens 44.7 and 40.0
+  //   time mixing  64 CTAs, 300 tokens 68.1 and 70.4, 400 tokens 87.5 and 81.6, 64 x 64 2000 tokens 269 and 352;
+  //                128 x 128: 96 CTAs, 64 tokens 27.0 and 25.5;   128, 64 tokens 27.5 and 27.5
+  //                64 x 64: 96 CTAs, 200 tokens 47.0 and 47.4, 240 tokens 55.0 and 50.6;   448, 240 tokens 108 and 88.8
+  const long long ctas = (long long)a->B * a->H * ((a->V + kMaxCols - 1) / kMaxCols);
+  if (!applies(a) || ctas < 64) return 0;
+  const bool some = ctas >= 96, wide = a->D == 128;
+  if (a->kind == kDelta && wide ? ctas < 128 ? a->T * ctas * ctas < 540000 : a->T < 80
+      : a->kind == kDelta       ? a->T < (some ? 128 : 132)
+      : wide                    ? a->T < (some ? 64 : 400)
+                                : !some || a->T < 240)
+    return 0;
   const size_t one = chunk_bytes(a), all = (size_t)((a->T + kChunk - 1) / kChunk);
   return one * all <= kMaxScratch ? one * all : one > kMaxScratch ? one : kMaxScratch / one * one;
 }

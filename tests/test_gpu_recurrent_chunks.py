@@ -24,9 +24,9 @@ def memory(chunks, bytes_of_one, device):
     return torch.full((chunks * bytes_of_one + 8,), 255, dtype=torch.uint8, device=device)[:chunks * bytes_of_one]     # (what it holds before is NaN)
 
 
-# bytes of a chunk of one head: 16 rows of 2 D + 16 floats (Q; the delta rule's W), 8 of 4 D + 8 (K), 16 of 20 (M; T), D decays
+# bytes of a chunk of one head: 16 rows of D floats each of Q and K (the delta rule's W), 16 of 16 of M (T), D decays
 def one(heads, D, delta):
-    return 4 * heads * ((2 if delta else 1) * 16 * (2 * D + 16) + 8 * (4 * D + 8) + (2 if delta else 1) * 320 + D)
+    return 4 * heads * ((3 if delta else 2) * 16 * D + (2 if delta else 1) * 256 + D)
 
 
 @pytest.mark.parametrize("chunks", [1, 2, 100])
@@ -99,7 +99,8 @@ def test_where_chunks_are_taken(pkg, device):
 
     assert need(2, 132, 16, 128, 128) == 9 * one(32, 128, True) and need(2, 131, 16, 128, 128) == 0 and need(1, 6000, 16, 128, 128) == 0
     assert need(3, 59, 16, 128, 128) == 4 * one(48, 128, True) and need(16, 39, 16, 128, 128) == 0
-    assert need(3, 59, 32, 64, 64, kind=1) == 4 * one(96, 64, False)
+    assert need(3, 240, 32, 64, 64, kind=1) == 15 * one(96, 64, False) and need(3, 239, 32, 64, 64, kind=1) == need(2, 6000, 32, 64, 64, kind=1) == 0
+    assert need(16, 79, 16, 128, 128) == 0 and need(16, 80, 16, 128, 128) == 5 * one(256, 128, True)
     assert 0 < need(8, 6000, 16, 128, 128) <= 256 << 20                             # longer prompts: segments
     assert need(3, 1000, 16, 128, 128, dtype=1) == need(3, 1000, 16, 32, 128) == need(3, 1000, 16, 128, 124) == need(3, 1000, 16, 128, 128, shift=2) == 0
     a = A()
