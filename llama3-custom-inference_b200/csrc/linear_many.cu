@@ -53,8 +53,8 @@ __device__ __forceinline__ float rcp(float x) { return __fdividef(1.f, x); }
 
 // x times the normal distribution's integral, two at a time: max(x, 0) - |x| erfc(|x| / sqrt 2) / 2 by the Chebyshev fit to erfc of Press et
 // al., "Numerical Recipes", section 6.2 (erfcc; fractional error below 1.2e-7 everywhere).  No branch, a third of the instructions of 0.5 x (1 +
-// erff(x / sqrt 2)), and no cancellation for negative x, where that form loses 4e-4 of the value at -4 and all of it below -5.6; over bf16
-// and normal x at most 4e-7 off, that form 4.5e-7.
+// erff(x / sqrt 2)), and no cancellation for negative x, where that form loses 4e-4 of the value at -4 and all of it below -5.6; of every
+// finite bf16 x with a normal result the rounded result is the nearest bf16.
 __device__ __forceinline__ void gelu(float& x, float& y) {
   constexpr float kLog2e = 1.4426950408889634f, kRoot = 0.70710678118654752f;
   const f2 m = f2_packf(fminf(fabsf(x), 30.f), fminf(fabsf(y), 30.f));        // (erfc is 0 from 15 on; an infinity keeps its sign)
@@ -72,7 +72,7 @@ __device__ __forceinline__ void gelu(float& x, float& y) {
   e = f2_fma(t, e, f2_same(-1.26551223f * kLog2e));
   f2_unpack(f2_fma(f2_mul(m, f2_same(-0.5f * kLog2e)), m, e), u, v);
   const f2 q = f2_mul(f2_mul(m, f2_same(-0.5f)), f2_mul(t, f2_packf(fast_exp2(u), fast_exp2(v))));
-  f2_unpack(f2_add(q, f2_packf(x < 0.f ? 0.f : x, y < 0.f ? 0.f : y)), x, y);
+  f2_unpack(f2_fma(f2_packf(x, y), f2_packf(x < 0.f ? 0.f : 1.f, y < 0.f ? 0.f : 1.f), q), x, y);   // (-infinity gives NaN, as 0.5 x (1 + erff) does)
 }
 // silu(z) u, both sides of the division a sixteenth: the divisor then stays below 2^126, where the short division is exact to 2 units of the last
 // place, for every z whose silu is not 0.  At most 2e-6 of the value off.

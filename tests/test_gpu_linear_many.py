@@ -64,3 +64,80 @@ def test_refused(capi, device):
     assert many(capi, x, w, 5, out) == capi.ERR_INVALID
     assert many(capi, x[:1].expand(300, 64), w, 0, out) == capi.ERR_INVALID
     assert many(capi, x, w[:60], 0, out[:, :60]) == capi.ERR_ALIGNMENT
+
+
+def every_number(device):
+    """The finite bf16 numbers, 255 x 256."""
+    bits = torch.arange(65536, dtype=torch.int32)
+    return bits[(bits & 0x7F80) != 0x7F80].to(torch.int16).view(BF16).view(255, 256).to(device)
+
+
+def sums(x, up=None):
+    """Operands whose product's sums are x, one term each (and, gated, `up`)."""
+    eye = torch.eye(256, dtype=BF16, device=x.device)
+    if up is None:
+        return x, eye
+    one = torch.zeros(x.shape[0], 8, dtype=BF16, device=x.device)
+    one[:, 0] = up
+    pick = torch.zeros(256, 264, dtype=BF16, device=x.device)
+    pick[:, 256] = 1.0
+    return torch.cat([x, one], 1), torch.cat([torch.cat([eye, torch.zeros(256, 8, dtype=BF16, device=x.device)], 1), pick])
+
+
+@pytest.mark.parametrize("act", [1, 2, 3])
+def test_activation_of_every_number(capi, device, act):
+    """One rounding to bf16 (2^-8 of a value) and at most 1e-5 of it, tails included; numbers below the least normal may be zeros, and silu is
+    zero where exp(-z) is no fp32 number."""
+    x = every_number(device)
+    a, w = sums(x, 1.0 if act == capi.ACT_SILU_GATE else None)
+    out, z = torch.empty(255, 256, dtype=BF16, device=device), x.double()
+    assert many(capi, a, w, act, out) == capi.OK
+    want = 0.5 * z * torch.special.erfc(-z * 0.5 ** 0.5) if act == capi.ACT_GELU else torch.tanh(z) if act == capi.ACT_TANH else z * torch.sigmoid(z)
+    bound = (2 ** -8 + 1e-5) * want.abs() + (3e-37 if act == capi.ACT_SILU_GATE else 2e-38)
+    assert bool(((out.double() - want).abs() <= bound).all())
+
+
+def test_silu_mul_of_every_number(ext, capi, device):
+    x = every_number(device) + 0.0                      # (a sum is never -0)
+    a, w = sums(x, 1.375)
+    out, up = torch.empty(255, 256, dtype=BF16, device=device), torch.full_like(x, 1.375)
+    args = capi.LinearArgs(x=a.data_ptr(), w=w.data_ptr(), out=out.data_ptr(), rows=255, x_st=264, out_st=256, K=264, N=256, groups=1, act=4,
+                           stream=torch.cuda.current_stream().cuda_stream)
+    assert capi.load().l3ci_linear_many(C.byref(args)) == capi.OK
+    assert torch.equal(out.view(torch.int16), ext.silu_mul(x, up).view(torch.int16))
+
+
+@pytest.mark.parametrize("act", [1, 2, 3, 4])
+def test_sums_that_are_not_finite(ext, pkg, capi, device, act):
+    """NaN where the activation of its own on a bf16 product has it."""
+    mx, odd = pkg.mixers, [float("nan"), float("inf"), -float("inf")]
+    w = torch.cat([torch.eye(256, dtype=BF16, device=device)] * (2 if act > 2 else 1))
+    x = torch.zeros(300, 256, dtype=BF16, device=device)
+    for r in range(300):
+        x[r, r % 256] = odd[r % 3]
+    out, plain = torch.empty(300, 256, dtype=BF16, device=device), torch.empty(300, w.shape[0], dtype=BF16, device=device)
+    args = capi.LinearArgs(x=x.data_ptr(), w=w.data_ptr(), out=out.data_ptr(), rows=300, x_st=256, out_st=256, K=256, N=256, groups=1, act=act,
+                           stream=torch.cuda.current_stream().cuda_stream)
+    assert capi.load().l3ci_linear_many(C.byref(args)) == capi.OK and many(capi, x, w, 0, plain) == capi.OK
+    want = (mx.gelu_(plain) if act == 1 else mx.tanh_(plain) if act == 2 else mx.gated_act(plain) if act == 3 else
+            ext.silu_mul(plain[:, :256], plain[:, 256:]))
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out[~out.isnan()], want[~want.isnan()])
+
+
+@pytest.mark.parametrize("B,T", [(1, 2048), (2, 1000)])
+def test_the_calls_that_choose_it(ext, capi, device, B, T):
+    """`many_rows` and a gated `linear` on a part of wider rows: the bits of the C call, near the fp32 product."""
+    K, N = 512, 2048
+    wide, w = rand(B, T, K + 64, seed=7), rand(2 * N, K, seed=8, scale=2 * K ** -0.5)
+    x = wide[..., 32:32 + K]
+    y = x.reshape(B * T, K)
+    for act, rows, got in ((capi.ACT_GELU, w, ext.many_rows(x, w, capi.ACT_GELU)), (capi.ACT_SILU_GATE, w, ext.many_rows(x, w, capi.ACT_SILU_GATE)),
+                           (4, w, ext.linear(x, w, gated=True))):
+        n = N if act > 2 else 2 * N
+        assert got is not None and got.shape == (B, T, n)
+        out = torch.empty(B * T, n, dtype=BF16, device=device)
+        args = capi.LinearArgs(x=y.data_ptr(), w=rows.data_ptr(), out=out.data_ptr(), rows=B * T, x_st=y.stride(0), out_st=n, K=K, N=n, groups=1, act=act,
+                               stream=torch.cuda.current_stream().cuda_stream)
+        assert capi.load().l3ci_linear_many(C.byref(args)) == capi.OK and torch.equal(got.view(B * T, n), out)
+        want = want_of(capi, y, rows, capi.ACT_SILU_GATE if act == 4 else act).double()
+        assert ((out.double() - want).norm() / want.norm()).item() < 6e-3
