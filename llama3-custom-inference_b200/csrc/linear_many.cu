@@ -19,6 +19,7 @@
 #include "bf16x8.cuh"
 #include "host_common.h"
 #include "linear_many.h"
+#include "mixer_types.cuh"
 #include "ptx_sm100.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.h"
@@ -74,10 +75,6 @@ __device__ __forceinline__ void gelu(float& x, float& y) {
   const f2 q = f2_mul(f2_mul(m, f2_same(-0.5f)), f2_mul(t, f2_packf(fast_exp2(u), fast_exp2(v))));
   f2_unpack(f2_fma(f2_packf(x, y), f2_packf(x < 0.f ? 0.f : 1.f, y < 0.f ? 0.f : 1.f), q), x, y);   // (-infinity gives NaN, as 0.5 x (1 + erff) does)
 }
-// silu(z) u, both sides of the division a sixteenth: the divisor then stays below 2^126, where the short division is exact to 2 units of the last
-// place, for every z whose silu is not 0.  At most 2e-6 of the value off.
-__device__ __forceinline__ float gated(float z, float u) { return __fdividef(z * 0.0625f, fmaf(__expf(-z), 0.0625f, 0.0625f)) * u; }
-
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -111,9 +108,14 @@ __device__ __forceinline__ void pair_commit(uint32_t bar, uint32_t elected) {
                ::"r"(bar), "r"(elected), "h"((uint16_t)3) : "memory");
 }
 
-// A pair of gate and up sums as a bf16 product has them, and silu's own rounding: l3ci_silu_mul's bits.
+// A pair of gate and up sums as a bf16 product has them, and silu's own rounding: l3ci_silu_mul's bits, by its short form of silu, whose error grows
+// with |z| but which rounds to the same bf16 for all the gates there are (rms_norm.cu).  The gate of unrounded sums is by expf and the full
+// division: of z between -85 and 0 the short form rounds some to another bf16 (2 x 8192 x 2048, 6001 rows: 276 us, by the short form 271).
 __device__ __forceinline__ float bf16_of(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-__device__ __forceinline__ float silu_mul(float z, float u) { return bf16_of(gated(bf16_of(z), 1.f)) * bf16_of(u); }
+__device__ __forceinline__ float silu_mul(float z, float u) {
+  z = bf16_of(z);
+  return bf16_of(__fdividef(z * 0.0625f, fmaf(__expf(-z), 0.0625f, 0.0625f))) * bf16_of(u);
+}
 
 template <int ACT>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -239,7 +241,7 @@ linear_many_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
             for (int i = 0; i < 8; ++i) {
               f[i] = __uint_as_float(y[v * 8 + i]);
               if (ACT == L3CI_ACT_SILU_MUL) f[i] = silu_mul(f[i], __uint_as_float(z[v * 8 + i]));
-              else if (GATED) f[i] = gated(f[i], __uint_as_float(z[v * 8 + i]));
+              else if (GATED) f[i] = gated_activation(f[i], __uint_as_float(z[v * 8 + i]), 0.f, 0.f);
               else if (ACT == L3CI_ACT_TANH) f[i] = tanhf(f[i]);
             }
             if (ACT == L3CI_ACT_GELU)

@@ -97,6 +97,25 @@ def test_activation_of_every_number(capi, device, act):
     assert bool(((out.double() - want).abs() <= bound).all())
 
 
+def test_gate_of_sums_as_in_few_rows(capi, device):
+    """silu(z) u with the bits of the product of few rows, which has expf and the full division: every bf16 number, and z of 24 bits where exp(-z) is
+    large, whose rounding a shorter exponential moves now and then."""
+    g = torch.Generator(device=device).manual_seed(5)
+    z = torch.cat([every_number(device).float(), -85 * torch.rand(4097, 256, generator=g, device=device)])
+    first = z.bfloat16()
+    a, w = sums(first, -1.375)
+    second = torch.where(z.abs() < 100, z - first.float(), 0.0).bfloat16()
+    a, w = torch.cat([a, second], 1), torch.cat([w, torch.cat([torch.eye(256), torch.zeros(256, 256)]).to(device, BF16)], 1)
+    out, few = torch.empty_like(first), torch.empty_like(first)
+    assert many(capi, a, w, capi.ACT_SILU_GATE, out) == capi.OK
+    for r in range(0, a.shape[0], 64):
+        part, to = a[r:r + 64], few[r:r + 64]
+        args = capi.LinearArgs(x=part.data_ptr(), w=w.data_ptr(), out=to.data_ptr(), rows=part.shape[0], x_st=520, out_st=256, K=520, N=256, groups=1,
+                               act=capi.ACT_SILU_GATE, stream=torch.cuda.current_stream().cuda_stream)
+        assert capi.load().l3ci_linear(C.byref(args)) == capi.OK
+    assert torch.equal(out.view(torch.int16), few.view(torch.int16))
+
+
 def test_silu_mul_of_every_number(ext, capi, device):
     x = every_number(device) + 0.0                      # (a sum is never -0)
     a, w = sums(x, 1.375)
