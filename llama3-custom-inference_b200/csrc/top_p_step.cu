@@ -697,7 +697,9 @@ top_p_count_kernel(const __nv_bfloat16* __restrict__ logits, long long vocab, lo
   auto order = [](uint32_t u) { const int t = (int)(short)u; return t ^ ((t >> 31) & 0x7fff); };
   const int star = all_kept ? -40000 : (int)key_star - 0x8000;
   const int star_low = star == 0 ? -1 : star;
-  const bool plain = !s_odd && !all_kept;                 // every entry has a number: bf16's own compare orders them (and ties -0 and +0)
+  // every entry here and the boundary (which may be another share's entry) has a number: bf16's own compare orders them (and ties -0 and +0)
+  const float boundary = key_logit(key_star);
+  const bool plain = !s_odd && !all_kept && boundary == boundary;
   auto at_least = [&](int it, const Group& g) {           // bit j: entry j of the group is in the nucleus or ties
     const int n = entries(it);
     uint32_t in = 0u;

@@ -46,3 +46,18 @@ def test_one_token_per_row_and_step(capi, device, kind, rows, vocab):
     y = torch.where(odd[:, None], torch.zeros_like(x), x)
     for a, b in zip(first, _run(capi, y)):
         assert torch.equal(a[~odd], b[~odd])
+
+
+@pytest.mark.parametrize("pattern", [-1, -64])           # 0xFFFF, 0xFFC0: NaN with the sign set, in order below every number
+@pytest.mark.parametrize("rows,vocab", [(1, 5001), (20, 70000), (40, 5001), (75, 70000)])
+def test_a_negative_nan_in_one_share_of_the_row(capi, device, rows, vocab, pattern):
+    """The boundary of the nucleus is then below all that the other shares hold: by counts as by masses (a tail of -inf, above the boundary
+    too, takes the row there)."""
+    long = 8 * 8191 * 8 + 8
+    x = (torch.randn(rows, vocab, generator=torch.Generator(device=device).manual_seed(vocab), device=device) * 3).bfloat16()
+    x.view(torch.int16)[torch.arange(rows, device=device), torch.arange(rows, device=device) * 997 % vocab] = pattern
+    wide = torch.full((rows, long), -INF, dtype=torch.bfloat16, device=device)
+    wide[:, :vocab] = x
+    got, want = _run(capi, x), _run(capi, wide)
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a + (long - vocab if i == 5 else 0), b)
