@@ -123,7 +123,7 @@ typedef struct l3ci_recurrent_scan_args {
   const void* conv_in;
   void* tail;
   const int32_t* positions;
-  int32_t* status;            /* optional device word: L3CI_ERR_DEVICE_WAIT when a bounded wait runs out          */
+  int32_t* status;            /* device word for L3CI_ERR_DEVICE_WAIT when a bounded wait runs out; null: the library's, for l3ci_recurrent_scan_poll */
   int64_t qk_st, qk_sh, v_st, v_sh, g_st, g_sh, gate_st, gate_sh, out_st, out_sh, norm_sh, state_sb, conv_st, tail_sb;
   int32_t kind, B, T, H, G, D, V, act, taps, dtype;
   float eps;
@@ -136,6 +136,9 @@ L3CI_API int l3ci_recurrent_scan(const l3ci_recurrent_scan_args* args);
  * l3ci_recurrent_scan is the faster. */
 L3CI_API int l3ci_recurrent_scan_chunks(const l3ci_recurrent_scan_args* args, void* scratch, size_t scratch_bytes);
 L3CI_API size_t l3ci_recurrent_scan_scratch_bytes(const l3ci_recurrent_scan_args* args);
+/* Waits for `stream`; L3CI_ERR_DEVICE_WAIT, once, if a scan without a status word of its own gave up on this device (should never happen): its outputs
+ * and states are not to be used. */
+L3CI_API int l3ci_recurrent_scan_poll(l3ci_stream_t stream);
 
 /* Mixture of experts.  Route: of the fp32 logits [rows, E] + bias [E] the `top` largest of a token (ties: the smaller index),
  * weights = softmax over these; experts, ranks int32 [rows, top] (rank: place of the pair among the pairs of its expert),

@@ -36,6 +36,9 @@
 namespace l3ci {
 namespace {
 
+// Where a wait that ran out is recorded by calls without a status word of their own, until l3ci_recurrent_scan_poll reads it.
+__device__ int g_wait_status = 0;
+
 constexpr int kDelta = 0, kTimeMix = 1;
 constexpr int kChunk = 16;         // tokens per stage
 constexpr int kMaxRing = 4;        // stages
@@ -220,7 +223,7 @@ recurrent_scan_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       __syncwarp();
     }
     if (a.tail && split == 0) move_tails<S>(a, b, h, lane, 32, fresh);
-    if (!ok && lane == 0 && a.status) atomicExch(a.status, (int)L3CI_ERR_DEVICE_WAIT);
+    if (!ok && lane == 0) atomicExch(a.status ? a.status : &g_wait_status, (int)L3CI_ERR_DEVICE_WAIT);
     return;
   }
 
@@ -286,7 +289,7 @@ recurrent_scan_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(ready0 + s * 8);
     }
-    if (!ok && lane == 0 && a.status) atomicExch(a.status, (int)L3CI_ERR_DEVICE_WAIT);
+    if (!ok && lane == 0) atomicExch(a.status ? a.status : &g_wait_status, (int)L3CI_ERR_DEVICE_WAIT);
     return;
   }
 
@@ -462,7 +465,7 @@ recurrent_scan_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     if (lane == 0) mbar_arrive(empty0 + s * 8);
   }
   if (!ok) {
-    if (lane == 0 && a.status) atomicExch(a.status, (int)L3CI_ERR_DEVICE_WAIT);
+    if (lane == 0) atomicExch(a.status ? a.status : &g_wait_status, (int)L3CI_ERR_DEVICE_WAIT);
     return;
   }
   if (KIND == kDelta) {
@@ -1059,6 +1062,24 @@ int l3ci_recurrent_scan(const l3ci_recurrent_scan_args* a) {
   if (a->kind == 0)
     return a->dtype == L3CI_BF16 ? scan_typed<__nv_bfloat16, float, kDelta>(a, s) : scan_typed<float, float, kDelta>(a, s);
   return a->dtype == L3CI_BF16 ? scan_typed<__nv_bfloat16, __nv_bfloat16, kTimeMix>(a, s) : scan_typed<float, float, kTimeMix>(a, s);
+}
+
+int l3ci_recurrent_scan_poll(l3ci_stream_t stream_) {
+  using namespace l3ci;
+  clear_error();
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  void* own = nullptr;
+  L3CI_CUDA_TRY(cudaGetSymbolAddress(&own, g_wait_status));
+  int* words[2] = {static_cast<int*>(own), scan_chunks_wait_status()};
+  int status[2] = {0, 0};
+  for (int i = 0; i < 2; ++i)
+    if (words[i]) L3CI_CUDA_TRY(cudaMemcpyAsync(&status[i], words[i], sizeof(int), cudaMemcpyDeviceToHost, stream));
+  L3CI_CUDA_TRY(cudaStreamSynchronize(stream));
+  if (status[0] == 0 && status[1] == 0) return L3CI_OK;
+  for (int i = 0; i < 2; ++i)
+    if (words[i]) L3CI_CUDA_TRY(cudaMemsetAsync(words[i], 0, sizeof(int), stream));
+  L3CI_CUDA_TRY(cudaStreamSynchronize(stream));
+  return fail(status[0] ? status[0] : status[1], "recurrent_scan: a bounded wait ran out in an earlier launch");
 }
 
 size_t l3ci_recurrent_scan_scratch_bytes(const l3ci_recurrent_scan_args* a) {

@@ -11,6 +11,8 @@ namespace l3ci {
 // it does not apply or the scan token by token is the faster; its launch, without the heads' norm and gate.
 size_t scan_chunks_scratch(const l3ci_recurrent_scan_args* a);
 int scan_chunks_launch(const l3ci_recurrent_scan_args* a, void* scratch, size_t bytes);
+// The device word where its waits that ran out are recorded (of the current device); null without a device.
+int* scan_chunks_wait_status();
 
 #if defined(__CUDACC__)
 // The convolution's carried inputs: row r of the tail becomes the input of token T - (taps - 1) + r.  Channel c of a sequence,

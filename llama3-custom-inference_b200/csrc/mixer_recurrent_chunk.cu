@@ -36,6 +36,8 @@
 namespace l3ci {
 namespace {
 
+__device__ int g_wait_status = 0;   // of calls without a status word of their own
+
 constexpr int kChunk = 16;
 constexpr int kDelta = 0, kTimeMix = 1;
 constexpr int kOwn = 4;                           // a lane's columns
@@ -443,7 +445,7 @@ chunk_scan_kernel(const __grid_constant__ ChunkParams p) {
           f2_unpack(S[c][j], at[0], at[a.V]);
         }
   }
-  if (!ok && lane == 0 && a.status) atomicExch(a.status, (int)L3CI_ERR_DEVICE_WAIT);
+  if (!ok && lane == 0) atomicExch(a.status ? a.status : &g_wait_status, (int)L3CI_ERR_DEVICE_WAIT);
   // a wait ran out: the copies still under way land before the shared memory is given back
   if (__syncthreads_or(!ok))
     for (int f = asked > kStages ? asked - kStages : 0; f < asked; ++f) (void)mbar_wait_bounded_one(full0 + f % kStages * 8, (uint32_t)(f / kStages) & 1u);
@@ -514,6 +516,11 @@ bool applies(const l3ci_recurrent_scan_args* a) {
 }
 
 }  // namespace
+
+int* scan_chunks_wait_status() {
+  void* at = nullptr;
+  return cudaGetSymbolAddress(&at, g_wait_status) == cudaSuccess ? static_cast<int*>(at) : nullptr;
+}
 
 size_t scan_chunks_scratch(const l3ci_recurrent_scan_args* a) {
   // From where on the chunks are the faster, in CTAs of 64 columns and tokens; us by tokens and by chunks, heads of 128 x 128 and of 64 x 64.

@@ -9,7 +9,7 @@ from pathlib import Path
 import torch
 import torch.nn.functional as F
 
-from .capi import ACT_GELU, ACT_NONE, ACT_SILU_GATE, ACT_TANH, LINEAR_MAX_ROWS, OK, L3ciError, _on, _stream
+from .capi import ACT_GELU, ACT_NONE, ACT_SILU_GATE, ACT_TANH, ERR_DEVICE_WAIT, LINEAR_MAX_ROWS, OK, L3ciError, _on, _stream
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libl3ci_mixers.so"
 
@@ -17,7 +17,7 @@ EXPORTS = ("l3ci_mixers_last_error", "l3ci_mixers_set_programmatic_launch", "l3c
            "l3ci_latent_cache", "l3ci_kv_cache_write", "l3ci_mixer_attention", "l3ci_mixer_attention_scratch_bytes",
            "l3ci_mixer_attention_variant", "l3ci_residual_norm", "l3ci_tanh", "l3ci_gated_act", "l3ci_qk_norm_cache",
            "l3ci_token_shift", "l3ci_delta_inputs", "l3ci_recurrent_scan", "l3ci_recurrent_scan_chunks",
-           "l3ci_recurrent_scan_scratch_bytes", "l3ci_moe_route", "l3ci_moe_gather",
+           "l3ci_recurrent_scan_scratch_bytes", "l3ci_recurrent_scan_poll", "l3ci_moe_route", "l3ci_moe_gather",
            "l3ci_moe_gather_places", "l3ci_moe_gemm", "l3ci_moe_gemm_variant")
 
 DTYPE_CODES = {torch.bfloat16: 0, torch.float32: 1}
@@ -107,6 +107,7 @@ def load() -> C.CDLL:
     lib.l3ci_delta_inputs.argtypes = [C.POINTER(DeltaInputsArgs)]
     lib.l3ci_recurrent_scan.argtypes = [C.POINTER(RecurrentScanArgs)]
     lib.l3ci_recurrent_scan_chunks.argtypes = [C.POINTER(RecurrentScanArgs), vp, C.c_size_t]
+    lib.l3ci_recurrent_scan_poll.argtypes = [vp]
     lib.l3ci_recurrent_scan_scratch_bytes.argtypes = [C.POINTER(RecurrentScanArgs)]
     lib.l3ci_recurrent_scan_scratch_bytes.restype = C.c_size_t
     lib.l3ci_moe_route.argtypes = [vp, vp, vp, vp, vp, vp, i64, i32, i32, vp]
@@ -412,6 +413,16 @@ def recurrent_scan(q, k, v, g, state, positions, norm, gate, *, act: int, eps: f
         else:
             _check(load().l3ci_recurrent_scan(C.byref(a)), "l3ci_recurrent_scan")
     return out.view(B, T, H * V)
+
+
+def scan_status(like) -> int:
+    """Of the recurrences' scans on the current stream of `like`'s device: 0, or 6 once after a device-side wait ran out."""
+    _cuda(like)
+    with _on(like):
+        status = load().l3ci_recurrent_scan_poll(_stream(like))
+    if status not in (OK, ERR_DEVICE_WAIT):
+        _check(status, "l3ci_recurrent_scan_poll")
+    return status
 
 
 def moe_route(logits, bias, top: int):

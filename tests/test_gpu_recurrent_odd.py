@@ -98,6 +98,7 @@ def test_the_call_that_chooses_chunks(pkg, device, monkeypatch, kind):
     (out, state), (same_out, same_state) = scan(pkg, monkeypatch, parts, "rule"), scan(pkg, monkeypatch, x, "rule")
     assert torch.equal(out, same_out) and torch.equal(state, same_state)
     want_out, want_state = scan(pkg, monkeypatch, x, "tokens")
+    assert pkg.mixers.scan_status(out) == 0                # neither form's waits ran out
     near = want_out.double().abs().amax(-1, keepdim=True)
     assert bool(((out.double() - want_out.double()).abs() <= 2 ** -7 * near).all())
     assert ((state - want_state).norm() / want_state.norm()).item() < 2e-6
