@@ -407,7 +407,10 @@ def recurrent_scan(q, k, v, g, state, positions, norm, gate, *, act: int, eps: f
     with _on(v):
         if scratch is None and T > 1:
             need = load().l3ci_recurrent_scan_scratch_bytes(C.byref(a))
-            scratch = torch.empty(need, dtype=torch.uint8, device=v.device) if need else None
+            try:
+                scratch = torch.empty(need, dtype=torch.uint8, device=v.device) if need else None
+            except torch.OutOfMemoryError:       # a device that is full: token by token, which takes none
+                pass
         if scratch is not None:
             _check(load().l3ci_recurrent_scan_chunks(C.byref(a), scratch.data_ptr(), scratch.numel()), "l3ci_recurrent_scan_chunks")
         else:

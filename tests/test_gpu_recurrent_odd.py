@@ -104,6 +104,25 @@ def test_the_call_that_chooses_chunks(pkg, device, monkeypatch, kind):
     assert ((state - want_state).norm() / want_state.norm()).item() < 2e-6
 
 
+def test_a_full_device(pkg, device, monkeypatch):
+    """No memory for the chunks: the scan token by token."""
+    x = inputs("delta", device, 2, 133, 16, 16, 128, 128, 0.3)
+    want = scan(pkg, monkeypatch, x, "tokens")
+    empty = torch.empty
+
+    def full(*size, **kw):
+        if kw.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("full")
+        return empty(*size, **kw)
+
+    with monkeypatch.context() as m:
+        m.setattr(torch, "empty", full)
+        state = x["state"].clone()
+        out = pkg.mixers.recurrent_scan(*[x[n] for n in "qkvg"], state, torch.full((2,), 3, dtype=torch.int32, device=device), x["norm"], x["gate"],
+                                        act=pkg.mixers.SIGMOID, eps=1e-5, beta=x["beta"])
+    assert torch.equal(out.view(want[0].shape), want[0]) and torch.equal(state, want[1])
+
+
 def exact(kind, x):
     """State after all tokens in float64."""
     S, out = x["state"].double(), {n: t.double() for n, t in x.items()}
