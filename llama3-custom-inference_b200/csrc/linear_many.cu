@@ -72,8 +72,8 @@ __device__ __forceinline__ void gelu(float& x, float& y) {
   e = f2_fma(t, e, f2_same(1.00002368f * kLog2e));
   e = f2_fma(t, e, f2_same(-1.26551223f * kLog2e));
   f2_unpack(f2_fma(f2_mul(m, f2_same(-0.5f * kLog2e)), m, e), u, v);
-  const f2 q = f2_mul(f2_mul(m, f2_same(-0.5f)), f2_mul(t, f2_packf(fast_exp2(u), fast_exp2(v))));
-  f2_unpack(f2_fma(f2_packf(x, y), f2_packf(x < 0.f ? 0.f : 1.f, y < 0.f ? 0.f : 1.f), q), x, y);   // (-infinity gives NaN, as 0.5 x (1 + erff) does)
+  const f2 over = f2_mul(f2_packf(x, y), f2_packf(x < 0.f ? 0.f : 1.f, y < 0.f ? 0.f : 1.f));   // max(x, 0); NaN for -infinity, as 0.5 x (1 + erff) gives
+  f2_unpack(f2_fma(f2_mul(m, f2_same(-0.5f)), f2_mul(t, f2_packf(fast_exp2(u), fast_exp2(v))), over), x, y);
 }
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
