@@ -140,7 +140,7 @@ L3CI_API size_t l3ci_recurrent_scan_scratch_bytes(const l3ci_recurrent_scan_args
  * and states are not to be used. */
 L3CI_API int l3ci_recurrent_scan_poll(l3ci_stream_t stream);
 
-/* Mixture of experts.  Route: of the fp32 logits [rows, E] + bias [E] the `top` largest of a token (ties: the smaller index),
+/* Mixture of experts.  Route: of the fp32 logits [rows, E] + bias [E] the `top` largest of a token (ties: the smaller index; NaN behind all numbers; each once),
  * weights = softmax over these; experts, ranks int32 [rows, top] (rank: place of the pair among the pairs of its expert),
  * weights fp32.  counts int32 [E] is set to the experts' pairs. */
 L3CI_API int l3ci_moe_route(const float* logits, const float* bias, int32_t* experts, int32_t* ranks, float* weights,

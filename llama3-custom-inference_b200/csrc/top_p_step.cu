@@ -942,10 +942,11 @@ TopPForm top_p_form(long long rows, long long vocab) {
   // the device (64 rows: 128 SMs; one row: 8).  A 148-SM part holds 15 clusters of 8, 33 of 4 or 74 of 2 of these
   // CTAs at a time (cudaOccupancyMaxActiveClusters); the bounds scale with the SM count.
   const int mass_ctas = sms <= 0 ? 1 : rows * 148 <= 15LL * sms ? 8 : rows * 148 <= 33LL * sms ? 4 : 2 * rows <= sms ? 2 : 1;
-  // By counts while a CTA's share of the row fits its registers and 16-bit counts: more CTAs per row where that takes more of
-  // them.  Longer rows yet, or a device without the shared memory: by masses.  So are short rows of one CTA each, where clearing
-  // and summing 65 536 counts takes longer than the passes over the row (75 rows: of 1000 logits 11.4 us by masses, 13.8 by counts; 4096:
-  // 13.5, 13.8; 8000: 16.8, 13.7).
+  // By counts while the counts of a CTA's share of the row fit 16 bits: more CTAs per row where that takes more of them.  Longer rows
+  // yet, or a device without the shared memory: by masses.  So are short rows of one CTA each: clearing and summing 65 536 counts took longer than
+  // the passes over the row before the nucleus was listed (75 rows, by masses and by counts: 1000 logits 11.4 and 13.8 us, 4096 13.5 and
+  // 13.8).  In chains, with the lists: 500 logits 10.6 and 9.8, 1000 9.9 and 9.8, 2000 10.5 and 9.8, 4096 12.0 and 10.0, 8000 15.2 and 9.9: the line
+  // is kept, and could be 0.
   const long long groups = (vocab + kVecElems - 1) / kVecElems;
   int ctas = mass_ctas;
   while (ctas < 8 && (groups + ctas - 1) / ctas > kMaxShare) ctas *= 2;
