@@ -359,7 +359,7 @@ class RupotarDecoder(DecodeLoop):
             return {"y": ops.linear(ops.linear(h, w.gate_up, mixers.ACT_SILU_GATE), w.down)}
         rows = h.view(-1, h.shape[-1])
         experts, ranks, weights, counts = mixers.moe_route(ops.product32(rows, w.router), w.router_b, ff.top)
-        if mixers.moe_places_pay(rows.shape[0], ff.experts, ff.top):
+        if rows.dtype == torch.bfloat16 and mixers.moe_places_pay(rows.shape[0], ff.experts, ff.top):
             x, part_rows = mixers.moe_places(rows, experts, ranks, ff.experts)
             a = ops.few_rows(x, w.gate_up.flatten(1, 2), mixers.ACT_SILU_GATE, limit=ff.limit, alpha=EXPERT_ALPHA)
             y = None if a is None else ops.few_rows(a, w.down, always=True)

@@ -68,6 +68,15 @@ def test_router_logits_without_numbers(pkg, device, rows, E, top, bad):
         assert torch.equal(stream[~odd], want[~odd]) and bool(stream[odd].isnan().all()) and bool(want.isfinite().all())
 
 
+def test_models_whose_products_are_others(pkg, device, monkeypatch):
+    """A model in fp32 gathers once, by sorted rows."""
+    from tests.rupotar_cases import case, weights
+    c = case("mixed", smooth=True)
+    model = pkg.rupotar.RupotarDecoder(None, pkg.rupotar.config_from_json(c), device, 1, 64, weights=weights(pkg, c, 3), dtype=torch.float32)
+    monkeypatch.setattr(pkg.mixers, "moe_places", lambda *a: pytest.fail("places"))
+    assert bool(model.extend("a", list(range(5)), range(5)).isfinite().all())
+
+
 def test_a_limit_belongs_to_a_gate(pkg, device):
     mx, x, w = pkg.mixers, rand(4, 64).to(device), rand(32, 64).to(device)
     for act, limit in ((mx.ACT_NONE, 1.0), (mx.ACT_GELU, 1.0), (mx.ACT_SILU_GATE, -1.0), (mx.ACT_SILU_GATE, float("nan"))):
