@@ -1025,7 +1025,7 @@ def bench_end_to_end(args, ext, pkg, dev, rank, world):
         "config": {"workload": f"C5 random-init Llama-3.2-1B architecture, batch {B}/GPU, prompt {P}, {G} greedy tokens",
                    "global_batch": B * world, "parallelism": "replicas x%d" % world,
                    "l2": "working set per decode step (2.5 GB weights + KV cache) >> 126 MB L2",
-                   "note": "products of the prompt, and beyond 32 sequences those of the attention layers, are cuBLAS via torch; the others, RMSNorm (+ residual add), SiLU*mul, RoPE + cache write, decode attention and the greedy step are this "
+                   "note": "products of the prompt but the gated one, and beyond 32 sequences those of the attention layers, are cuBLAS via torch; the others, RMSNorm (+ residual add), SiLU*mul, RoPE + cache write, decode attention and the greedy step are this "
                            "repository's kernels; the decode step is replayed from a CUDA graph",
                    "reference_published_rtx4060_tokens_per_s": 2041.67},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
@@ -1037,7 +1037,7 @@ def bench_end_to_end(args, ext, pkg, dev, rank, world):
                                      f"{products} products (16 with SiLU*mul), 1 greedy step; plus the embedding lookup and {65 - products} products of cuBLAS"},
         "e2e": e2e,
         # per decode step: 33 RMSNorm (32 with the residual add) + the RoPE/cache kernels + 16 flash-decode + the products
-        # (else 16 SiLU*mul) + 1 greedy-step launches of this library; the prefill pass: norms, RoPE, attention, SiLU*mul and the head's product
+        # (else 16 SiLU*mul) + 1 greedy-step launches of this library; the prefill pass: norms, RoPE, attention, the gated product (or SiLU*mul) and the head's product
         "gpu_launches": decode_steps * per_step + steps * (33 + 16 * 3 + 1), "clocks": sampler.summary(),
     }
     if cpu is not None:
